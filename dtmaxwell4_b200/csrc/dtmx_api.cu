@@ -1368,9 +1368,9 @@ static bool fused_usable(const dtmx_ctx* ctx, std::string* why) {
   return true;
 }
 
-template <int NR>
+template <int TY>
 static int build_fused_maps(dtmx_ctx* ctx, FusedMaps& fm, float* const* f) {
-  using L = FL<NR>;
+  using L = FL<TY>;
   int rc;
   for (int c = 0; c < 3; c++) {
     if ((rc = make_map(ctx, &fm.e[c], f[c], false, FE_W, L::FE_R))) return rc;
@@ -1386,8 +1386,8 @@ static int fused_prepare(dtmx_ctx* ctx) {
   if (ctx->fused_ready) return DTMX_OK;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(fused_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<2>::SMEM);
-    cudaFuncSetAttribute(fused_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<1>::SMEM);
+    cudaFuncSetAttribute(fused_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<16>::SMEM);
+    cudaFuncSetAttribute(fused_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<8>::SMEM);
     attr = true;
   }
   const dtmx_config& c = ctx->cfg;
@@ -1409,10 +1409,10 @@ static int fused_prepare(dtmx_ctx* ctx) {
     ctx->maps = save;
     for (int comp = 0; comp < 6; comp++) ctx->P.f[comp] = fsave[comp];
   }
-  if (!rc) rc = build_fused_maps<2>(ctx, ctx->fmaps[0], ctx->P.f);
-  if (!rc) rc = build_fused_maps<2>(ctx, ctx->fmaps[1], ctx->f_alt);
-  if (!rc) rc = build_fused_maps<1>(ctx, ctx->fmaps8[0], ctx->P.f);
-  if (!rc) rc = build_fused_maps<1>(ctx, ctx->fmaps8[1], ctx->f_alt);
+  if (!rc) rc = build_fused_maps<16>(ctx, ctx->fmaps[0], ctx->P.f);
+  if (!rc) rc = build_fused_maps<16>(ctx, ctx->fmaps[1], ctx->f_alt);
+  if (!rc) rc = build_fused_maps<8>(ctx, ctx->fmaps8[0], ctx->P.f);
+  if (!rc) rc = build_fused_maps<8>(ctx, ctx->fmaps8[1], ctx->f_alt);
   if (rc) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->fused_ready = true;
@@ -1484,10 +1484,10 @@ static int launch_fused_step(dtmx_ctx* ctx) {
     ctx->gcur = 1 - ctx->gcur;
     nl++;
   }
-  const dim3 blk(TZ, TW), grd((c.nz + TZ - 1) / TZ, (c.ny + ctx->frows - 1) / ctx->frows, (c.nx + PA.xchunk - 1) / PA.xchunk);
+  const dim3 grd((c.nz + TZ - 1) / TZ, (c.ny + ctx->frows - 1) / ctx->frows, (c.nx + PA.xchunk - 1) / PA.xchunk);
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], st);
-  if (ctx->frows == 8) fused_kernel<1><<<grd, blk, FL<1>::SMEM, st>>>(PA, fa, ctx->fmaps8[0]);
-  else fused_kernel<2><<<grd, blk, FL<2>::SMEM, st>>>(PA, fa, ctx->fmaps[0]);
+  if (ctx->frows == 8) fused_kernel<8><<<grd, FL<8>::NT, FL<8>::SMEM, st>>>(PA, fa, ctx->fmaps8[0]);
+  else fused_kernel<16><<<grd, FL<16>::NT, FL<16>::SMEM, st>>>(PA, fa, ctx->fmaps[0]);
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], st);
   nl++;
   if (PA.ade.Em[0] || ctx->has_gyro) {

@@ -11,31 +11,44 @@
 // (H, then E), each reading the field the other one writes; this engine makes
 // one.
 //
-// Tile: the per-step kernels' 32 (z, lanes) x 16 (y, 8 warps x 2 rows) node
-// tile, walked upwards along an x chunk.  Iteration t of the walk consumes the
-// stage of plane pc = x0 + t and
-//   * computes the new H of plane pc on the own nodes (and, split over warps
-//     0-3, the halo: Hz and Hx of row 16, Hy and Hx of column 32) from the old
+// Tile: 32 (z) x 16 or 8 (y) nodes, eight threads a row with four consecutive z
+// nodes each, walked upwards along an x chunk.  Iteration t of the walk
+// consumes the stage of plane pc = x0 + t and
+//   * computes the new H of plane pc on the own nodes (and the halo, one task a
+//     warp: Hz and Hx of the row above, Hy and Hx of column 32) from the old
 //     E of planes pc (staged) and pc - 1 (registers) and the old H of plane pc
 //     (staged); the own values go to B and, with the halo, to a shared-memory
 //     plane buffer;
 //   * computes the new E of plane pc - 1 on the own nodes from its old E
 //     (registers), the new H of plane pc - 1 (the other shared-memory plane
-//     buffer; own nodes from registers) and of plane pc (registers).
+//     buffer) and of plane pc (registers).
 // Each old value is therefore read from HBM once per step (the halo rows and
 // columns of the TMA boxes come from L2), and every plane costs one CTA
 // barrier.  One elected thread issues the TMA copies (cp.async.bulk.tensor,
-// no multicast) of a plane's E box (18 rows x 40 floats per component), old-H
-// boxes and, when the E update of the previous plane needs them, that plane's
-// material tiles, into a 3-stage ring (two planes in flight).  Everything
-// outside the grid reads as zero (TMA fill; new H forced to zero outside),
-// which is the box geometry; other geometries use the per-step engine.
+// no multicast) of a plane's E box (TY + 2 rows x 40 floats per component),
+// old-H boxes and, when the E update of the previous plane needs them, that
+// plane's material tiles, into a 3-stage ring (two planes in flight).
+// Everything outside the grid reads as zero (TMA fill; new H forced to zero
+// outside), which is the box geometry; other geometries use the per-step
+// engine.
+//
+// Why four nodes a thread: the sweep was bound by instructions, not by memory
+// or the loads' latency (a CTA alone on its SM took 4600 cycles for an
+// absorber plane, and loading the absorber's auxiliaries earlier made it
+// slower).  With 16-byte shared and global accesses a row of four nodes costs
+// 10 shared loads instead of 48 and a quarter of the address arithmetic and
+// stores, and the 4 warps of a 16-row tile have one halo task each, where 8
+// warps left the upper four waiting at the barrier.  Measured against two nodes
+// a thread (32 lanes along z, two rows): 384^3 with a 12-cell CPML 739 -> 592 us
+// a step (algorithmic bytes at 5.4 TB/s), without absorber 508 -> 454 us (6.0
+// TB/s), 128^3 with a 10-cell CPML 57 -> 40 us.
 //
 // The node updates are the expressions of plane_update (dtmx_device.cuh), in
-// the same order with the same explicitly rounded operations, so without a
-// TF/SF source this engine's fields are bit-identical to the per-step
-// engine's.  With one, the H correction is added to the old H before the sweep
-// (the update is linear in it), which rounds differently at the box faces.
+// the same order with the same explicitly rounded operations (sums with an
+// exact zero and products with an exact one left out), so without a TF/SF
+// source this engine's fields equal the per-step engine's.  With one, the H
+// correction is added to the old H before the sweep (the update is linear in
+// it), which rounds differently at the box faces.
 #pragma once
 #include "dtmx_stream.cuh"
 
@@ -44,15 +57,17 @@ namespace dtmx {
 constexpr int FE_W = 40;                     // E box: z in [k0-4, k0+36) (16-byte aligned start)
 constexpr int FHX_W = 36, FHY_W = 36, FHZ_W = 32;
 constexpr int F_NST = 3;
-constexpr int HN_P = TZ + 1;                 // new-H plane buffer: z in [k0, k0+33)
+constexpr int HN_P = 36;                     // new-H plane buffer: z in [k0, k0+33), rows 16-byte aligned
 constexpr int FX_MAX = 64;                   // longest x chunk
 constexpr int F_MROWS = 16;                  // material tiles: the per-step kernels' 32 x 16 boxes
 __host__ __device__ constexpr int f_up32(int v) { return (v + 31) / 32 * 32; }
 
-// Shared-memory layout of a tile of NR rows per warp (8 NR rows), in floats.
-template <int NR>
+// Shared-memory layout of a tile of TY rows, in floats.
+template <int TY>
 struct FL {
-  static constexpr int TY = TW * NR;                 // own rows of a tile (16 or 8)
+  static constexpr int NT = 8 * TY;                  // threads: eight a row
+  static constexpr int NW = NT / 32;
+  static constexpr int TASKS = NW >= 4 ? 1 : 4 / NW; // halo tasks of a warp (4 in all)
   static constexpr int FE_R = TY + 2;                // E box rows: y in [j0-1, j0+TY+1)
   static constexpr int FE_N = f_up32(FE_R * FE_W);
   static constexpr int FHX_R = TY + 1, FHY_R = TY, FHZ_R = TY + 1;   // old-H boxes
@@ -65,9 +80,14 @@ struct FL {
   static constexpr unsigned BYTES_MAT = 3 * F_MROWS * TZ;
   static constexpr int HN_N = (TY + 1) * HN_P;       // new-H plane, per component: y in [j0, j0+TY+1)
   static constexpr int HN = f_up32(3 * HN_N);
-  static constexpr size_t SMEM = (size_t)(F_NST * STAGE + 2 * HN) * 4 + sizeof(MatShared) + F_NST * 8 + 128;
+  // CPML coefficients (absorber runs): per x plane x0-1 .. x0+FX_MAX and per row
+  // j0 .. j0+TY six floats (b, a, 1/kappa - 1 at the half-coordinate 2v of the H
+  // components' derivatives, then at 2v + 1 of the E components'); per z
+  // column k0 .. k0+32 the same six as arrays of 36
+  static constexpr int FCO_X = 0, FCO_Y = (FX_MAX + 2) * 6, FCO_Z = (FCO_Y + (TY + 1) * 6 + 3) / 4 * 4, FCO_N = FCO_Z + 6 * 36;
+  static constexpr size_t SMEM = (size_t)(F_NST * STAGE + 2 * HN + f_up32(FCO_N)) * 4 + MAXMAT * 3 * 4 + F_NST * 8 + 128;
 };
-static_assert(FL<2>::STAGE == 4352 && FL<2>::OFF_HX == 2208, "16-row layout");
+static_assert(FL<16>::STAGE == 4352 && FL<16>::OFF_HX == 2208, "16-row layout");
 
 // TMA descriptors of one buffer set for one tile height
 struct FusedMaps {
@@ -83,64 +103,21 @@ struct FusedArgs {
   float* hdst[3][2];                         // ... and in B
 };
 
-// staged-tile accessors (tile-local y, z)
-template <int NR>
-__device__ __forceinline__ float fE(const float* st, int c, int y, int z) {
-  return st[c * FL<NR>::FE_N + (y + 1) * FE_W + z + 4];
+// four consecutive z nodes
+struct Q4 { float v[4]; };
+__device__ __forceinline__ Q4 ld4(const float* s) {
+  const float4 t = *reinterpret_cast<const float4*>(s);
+  return Q4{{t.x, t.y, t.z, t.w}};
 }
-template <int NR> __device__ __forceinline__ float fHx(const float* st, int y, int z) { return st[FL<NR>::OFF_HX + y * FHX_W + z]; }
-template <int NR> __device__ __forceinline__ float fHy(const float* st, int y, int z) { return st[FL<NR>::OFF_HY + y * FHY_W + z]; }
-template <int NR> __device__ __forceinline__ float fHz(const float* st, int y, int z) { return st[FL<NR>::OFF_HZ + y * FHZ_W + z]; }
-template <int NR>
-__device__ __forceinline__ int fM(const float* st, int c, int y, int z) {
-  return reinterpret_cast<const uint8_t*>(st + FL<NR>::OFF_M)[c * F_MROWS * TZ + y * TZ + z];
-}
-template <int NR>
-__device__ __forceinline__ float& fN(float* hn, int q, int y, int z) { return hn[q * FL<NR>::HN_N + y * HN_P + z]; }
-template <int NR>
-__device__ __forceinline__ float fN(const float* hn, int q, int y, int z) { return hn[q * FL<NR>::HN_N + y * HN_P + z]; }
+__device__ __forceinline__ void st4(float* d, const Q4& q) { *reinterpret_cast<float4*>(d) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]); }
 
-// CPML correction of component C at node (i, j, k) with slab indices si
-// (absorb_apply3 of the CPML form); H auxiliaries read from A and written to
-// B, E auxiliaries in place.  store false: a node whose new value this CTA
-// does not own (halo, the plane after the chunk) reads its auxiliaries only.
-template <int C>
-__device__ __forceinline__ float fused_cpml(const Params& p, const FusedArgs& fa, const int (&idx)[3], const int (&si)[3],
-                                            const float (&dif)[3], bool store) {
-  float corr = 0.f;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    const int sl = slot_of(C, a);
-    if (sl < 0 || si[a] < 0) continue;
-    const int h = 2 * idx[a] + comp_off(C, a);
-    const float k0 = __ldg(p.ab.c0[a] + h), k1 = __ldg(p.ab.c1[a] + h);
-    const float old = C >= 3 ? __ldg(fa.hsrc[a][sl - 2] + si[a]) : p.ab.aux[a][sl][si[a]];
-    const float nv = __fmaf_rn(k0, old, __fmul_rn(k1, dif[a]));
-    if (store) (C >= 3 ? fa.hdst[a][sl - 2] : p.ab.aux[a][sl])[si[a]] = nv;
-    corr = __fadd_rn(corr, __fmaf_rn(__fsub_rn(__ldg(p.ab.c2[a] + h), 1.f), dif[a], nv));
-  }
-  return corr;
-}
-
-// new H component C (3..5) = old + sum of the derivative terms d (+ CPML)
-template <int C, bool ABS>
-__device__ __forceinline__ float fused_hnode(const Params& p, const FusedArgs& fa, float old, float d0, float d1, float d2,
-                                             bool slab, const int (&idx)[3], const int (&si)[3], bool store) {
-  float inc = sum3(d0, d1, d2);
-  if (ABS && slab) {
-    const float dif[3] = {d0, d1, d2};
-    inc = __fadd_rn(inc, fused_cpml<C>(p, fa, idx, si, dif, store));
-  }
-  return __fadd_rn(old, inc);
-}
-
-// ---- absorber tiles
-// CPML coefficients are staged per CTA in shared memory, 6 floats per node
-// coordinate v of an axis: b, a, 1/kappa - 1 at half-coordinate 2v (the H
-// components' offset along a derivative axis) and at 2v + 1 (the E
-// components').  Rows: x planes x0-1 .. x0+FX_MAX, y rows j0 .. j0+16, z
-// columns k0 .. k0+32.
-constexpr int FCO_X = 0, FCO_Y = (FX_MAX + 2) * 6, FCO_Z = FCO_Y + (F_MROWS + 1) * 6, FCO_N = FCO_Z + (TZ + 1) * 6;
+// staged-tile addresses (tile-local y, z)
+template <int TY> __device__ __forceinline__ const float* fE(const float* st, int c, int y, int z) { return st + c * FL<TY>::FE_N + (y + 1) * FE_W + z + 4; }
+template <int TY> __device__ __forceinline__ const float* fHx(const float* st, int y, int z) { return st + FL<TY>::OFF_HX + y * FHX_W + z; }
+template <int TY> __device__ __forceinline__ const float* fHy(const float* st, int y, int z) { return st + FL<TY>::OFF_HY + y * FHY_W + z; }
+template <int TY> __device__ __forceinline__ const float* fHz(const float* st, int y, int z) { return st + FL<TY>::OFF_HZ + y * FHZ_W + z; }
+template <int TY> __device__ __forceinline__ float* fN(float* hn, int q, int y, int z) { return hn + q * FL<TY>::HN_N + y * HN_P + z; }
+template <int TY> __device__ __forceinline__ const float* fN(const float* hn, int q, int y, int z) { return hn + q * FL<TY>::HN_N + y * HN_P + z; }
 
 // index of coordinate v in the slab of its axis (-1 outside)
 __device__ __forceinline__ int slab_cs(const Params& p, int a, int v) {
@@ -148,278 +125,329 @@ __device__ __forceinline__ int slab_cs(const Params& p, int a, int v) {
   return v < lo ? v : (v >= n - hi ? lo + v - (n - hi) : -1);
 }
 
-// slab indices of node (i, j, k) along the axes of AXM (bit a: axis a may hold
-// a slab), from its slab coordinates xs, ys, zs (-1 outside); the slab_index32 layouts
-template <int AXM>
-__device__ __forceinline__ void fused_slabs(const Params& p, int i, int j, int k, int xs, int ys, int zs, int (&si)[3]) {
-  si[0] = ((AXM & 1) && xs >= 0) ? (xs * p.g.n[1] + j) * p.g.n[2] + k : -1;
-  si[1] = ((AXM & 2) && ys >= 0) ? (i * (p.ab.L[1][0] + p.ab.L[1][1]) + ys) * p.g.n[2] + k : -1;
-  si[2] = ((AXM & 4) && zs >= 0) ? (i * p.g.n[1] + j) * (p.ab.L[2][0] + p.ab.L[2][1]) + zs : -1;
+// slab index of node (i, j, k) along axis a from its slab coordinate s on that axis (>= 0)
+__device__ __forceinline__ int slab_at(const Params& p, int a, int i, int j, int k, int s) {
+  if (a == 0) return (s * p.g.n[1] + j) * p.g.n[2] + k;
+  if (a == 1) return (i * (p.ab.L[1][0] + p.ab.L[1][1]) + s) * p.g.n[2] + k;
+  return (i * p.g.n[1] + j) * (p.ab.L[2][0] + p.ab.L[2][1]) + s;
 }
 
-// the old auxiliaries of one node for one half of the update: per slab axis a
-// the two slots of that axis (H: slots 2, 3 from A; E: slots 0, 1 in place)
-template <int AXM, bool ISH>
-__device__ __forceinline__ void fused_aux_load(const Params& p, const FusedArgs& fa, const int (&si)[3], float (&old)[3][2]) {
+// What a thread keeps about its row and its four columns during the walk.
+struct FNode {
+  int y, z;                  // tile-local
+  int j, k;
+  int nv;                    // nodes of the four inside the grid (0: the row is outside)
+  int ys;                    // slab coordinate of the row (-1 outside)
+  int zs;                    // slab coordinate of node k (negative or past the slab where zm is 0)
+  unsigned zm;               // nodes of the four inside the z slab
+  bool vxy, vz;              // 16-byte accesses to the x and y slabs' / the z slab's auxiliaries
+};
+
+// Four old auxiliaries / four new ones.  The x and y slab arrays have rows of
+// nz floats, so with nz a multiple of 4 every row of four is aligned and whole;
+// the z slab's rows are as long as the slab is thick.
+template <bool RO>
+__device__ __forceinline__ Q4 aux4(const float* q, bool vec, unsigned m) {
+  Q4 r{{0.f, 0.f, 0.f, 0.f}};
+  if (vec) {
+    const float4 t = RO ? __ldg(reinterpret_cast<const float4*>(q)) : *reinterpret_cast<const float4*>(q);
+    r = Q4{{t.x, t.y, t.z, t.w}};
+  } else {
 #pragma unroll
-  for (int a = 0; a < 3; a++) {
-    old[a][0] = 0.f; old[a][1] = 0.f;
-    if (!((AXM >> a) & 1) || si[a] < 0) continue;
-    if (ISH) { old[a][0] = __ldg(fa.hsrc[a][0] + si[a]); old[a][1] = __ldg(fa.hsrc[a][1] + si[a]); }
-    else { old[a][0] = p.ab.aux[a][0][si[a]]; old[a][1] = p.ab.aux[a][1][si[a]]; }
+    for (int e = 0; e < 4; e++)
+      if ((m >> e) & 1) r.v[e] = RO ? __ldg(q + e) : q[e];
+  }
+  return r;
+}
+__device__ __forceinline__ void put4(float* q, bool vec, unsigned m, const Q4& v) {
+  if (vec) { st4(q, v); return; }
+#pragma unroll
+  for (int e = 0; e < 4; e++)
+    if ((m >> e) & 1) q[e] = v.v[e];
+}
+
+// The old auxiliaries of the thread's nodes in plane i, all axes: requested
+// before the stage wait, used after it.  H reads set A, E its own in place.
+template <bool ISH>
+__device__ __forceinline__ void fused_aux_load(const Params& p, const FusedArgs& fa, const FNode& f, int i, int xs, Q4 (&o)[3][2]) {
+  if (f.nv == 0) return;
+  const unsigned nm = (1u << f.nv) - 1u;
+  if (xs >= 0) {
+    const int s = slab_at(p, 0, i, f.j, f.k, xs);
+#pragma unroll
+    for (int q = 0; q < 2; q++) o[0][q] = aux4<ISH>((ISH ? fa.hsrc[0][q] : p.ab.aux[0][q]) + s, f.vxy, nm);
+  }
+  if (f.ys >= 0) {
+    const int s = slab_at(p, 1, i, f.j, f.k, f.ys);
+#pragma unroll
+    for (int q = 0; q < 2; q++) o[1][q] = aux4<ISH>((ISH ? fa.hsrc[1][q] : p.ab.aux[1][q]) + s, f.vxy, nm);
+  }
+  if (f.zm) {
+    const int s = slab_at(p, 2, i, f.j, f.k, f.zs);
+#pragma unroll
+    for (int q = 0; q < 2; q++) o[2][q] = aux4<ISH>((ISH ? fa.hsrc[2][q] : p.ab.aux[2][q]) + s, f.vz, f.zm);
   }
 }
 
-// CPML correction of component C from preloaded auxiliaries and staged
-// coefficients (the arithmetic of absorb_apply3, CPML form); store: the new
-// auxiliaries belong to this CTA.  Every axis of AXM takes part without a
-// branch: off its slab a node reads 0 and the coefficients there are b = 1,
-// a = 0, 1/kappa - 1 = 0, so its term is exactly zero and nothing is stored.
-template <int C, int AXM>
-__device__ __forceinline__ float fused_aux_apply(const Params& p, const FusedArgs& fa, const int (&si)[3],
-                                                 const float (&old)[3][2], const float (&dif)[3], const float* cx,
-                                                 const float* cy, const float* cz, bool store) {
-  float corr = 0.f;
+// one axis' term of four nodes of one component: psi <- b psi + a d, corr += (1/kappa - 1) d + psi
+__device__ __forceinline__ void cpml4(const Q4& d, const float (&b)[4], const float (&a)[4], const float (&c)[4], unsigned m, bool vec,
+                                      bool store, const Q4& old, float* mem, Q4& corr) {
+  Q4 nv;
 #pragma unroll
-  for (int a = 0; a < 3; a++) {
-    const int sl = slot_of(C, a);
-    if (sl < 0 || !((AXM >> a) & 1)) continue;
-    const int q = sl & 1;
-    const float* cf = (a == 0 ? cx : a == 1 ? cy : cz) + (C >= 3 ? 0 : 3);
-    const float nv = __fmaf_rn(cf[0], old[a][q], __fmul_rn(cf[1], dif[a]));
-    if (store && si[a] >= 0) (C >= 3 ? fa.hdst[a][q] : p.ab.aux[a][q])[si[a]] = nv;
-    corr = __fadd_rn(corr, __fmaf_rn(cf[2], dif[a], nv));
+  for (int e = 0; e < 4; e++) {
+    nv.v[e] = __fmaf_rn(b[e], old.v[e], __fmul_rn(a[e], d.v[e]));
+    const float t = __fmaf_rn(c[e], d.v[e], nv.v[e]);
+    corr.v[e] = __fadd_rn(corr.v[e], (m >> e) & 1 ? t : 0.f);
   }
-  return corr;
+  if (store) put4(mem, vec, m, nv);
 }
 
-// New H of plane i on the thread's own nodes: hc (registers), hn (shared
-// plane buffer), B (when the chunk owns plane i).  ec gets the old E of the
-// own nodes (the next plane's x taps and its E update); ep holds those of
-// plane i - 1.  AXM: the slab axes of the tile-plane (0: no absorber); the
-// slab coordinates xs (plane), ys (rows), zs (column) are per-thread constants.
-template <int NR, int AXM>
-__device__ __forceinline__ void fused_h_own(const Params& p, const FusedArgs& fa, const float* st, float* hn, int i,
-                                            int j0, int k0, bool store, const bool (&ok)[NR], const float (&ep)[NR][3],
-                                            float (&hc)[NR][3], float (&ec)[NR][3], const float* fco, int xs,
-                                            const int (&ys)[NR], int zs) {
-  const int lane = threadIdx.x, w = threadIdx.y;
+// CPML corrections of four nodes (the arithmetic of absorb_apply3) from their
+// scaled derivative terms dxy etc. (component, axis); inc += sum over the axes.
+template <int TY, bool ISH>
+__device__ __forceinline__ void fused_cpml(const Params& p, const FusedArgs& fa, const FNode& f, int i, int xs, const float* fco, int xrow,
+                                           const Q4 (&o)[3][2], bool store, const Q4& d01, const Q4& d02, const Q4& d10, const Q4& d12,
+                                           const Q4& d20, const Q4& d21, Q4 (&inc)[3]) {
+  if (f.nv == 0 || (xs < 0 && f.ys < 0 && f.zm == 0)) return;
+  constexpr int O = ISH ? 0 : 3;
+  const unsigned nm = (1u << f.nv) - 1u;
+  Q4 corr[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) corr[c] = Q4{{0.f, 0.f, 0.f, 0.f}};
+  auto same = [](float v, float (&r)[4]) { r[0] = r[1] = r[2] = r[3] = v; };
+  float b[4], a[4], c[4];
+  if (xs >= 0) {
+    const float* cf = fco + FL<TY>::FCO_X + xrow * 6 + O;
+    same(cf[0], b); same(cf[1], a); same(cf[2], c);
+    const int s = slab_at(p, 0, i, f.j, f.k, xs);
+    cpml4(d10, b, a, c, nm, f.vxy, store, o[0][0], (ISH ? fa.hdst[0][0] : p.ab.aux[0][0]) + s, corr[1]);
+    cpml4(d20, b, a, c, nm, f.vxy, store, o[0][1], (ISH ? fa.hdst[0][1] : p.ab.aux[0][1]) + s, corr[2]);
+  }
+  if (f.ys >= 0) {
+    const float* cf = fco + FL<TY>::FCO_Y + f.y * 6 + O;
+    same(cf[0], b); same(cf[1], a); same(cf[2], c);
+    const int s = slab_at(p, 1, i, f.j, f.k, f.ys);
+    cpml4(d01, b, a, c, nm, f.vxy, store, o[1][0], (ISH ? fa.hdst[1][0] : p.ab.aux[1][0]) + s, corr[0]);
+    cpml4(d21, b, a, c, nm, f.vxy, store, o[1][1], (ISH ? fa.hdst[1][1] : p.ab.aux[1][1]) + s, corr[2]);
+  }
+  if (f.zm) {
+    const float* cf = fco + FL<TY>::FCO_Z + O * 36 + f.z;
+    const Q4 tb = ld4(cf), ta = ld4(cf + 36), tc = ld4(cf + 72);
+    const int s = slab_at(p, 2, i, f.j, f.k, f.zs);
+    cpml4(d02, tb.v, ta.v, tc.v, f.zm, f.vz, store, o[2][0], (ISH ? fa.hdst[2][0] : p.ab.aux[2][0]) + s, corr[0]);
+    cpml4(d12, tb.v, ta.v, tc.v, f.zm, f.vz, store, o[2][1], (ISH ? fa.hdst[2][1] : p.ab.aux[2][1]) + s, corr[1]);
+  }
+#pragma unroll
+  for (int q = 0; q < 3; q++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) inc[q].v[e] = __fadd_rn(inc[q].v[e], corr[q].v[e]);
+}
+
+// scale * (u - l) of four nodes; l shifted by one node: the value below the first, then u's own
+__device__ __forceinline__ Q4 diff4(float s, const Q4& u, const Q4& l) {
+  Q4 r;
+#pragma unroll
+  for (int e = 0; e < 4; e++) r.v[e] = __fmul_rn(s, __fsub_rn(u.v[e], l.v[e]));
+  return r;
+}
+__device__ __forceinline__ Q4 below4(float first, const Q4& u) { return Q4{{first, u.v[0], u.v[1], u.v[2]}}; }
+__device__ __forceinline__ Q4 above4(const Q4& u, float last) { return Q4{{u.v[1], u.v[2], u.v[3], last}}; }
+__device__ __forceinline__ Q4 add4(const Q4& a, const Q4& b) {
+  Q4 r;
+#pragma unroll
+  for (int e = 0; e < 4; e++) r.v[e] = __fadd_rn(a.v[e], b.v[e]);
+  return r;
+}
+
+// New H of plane i on the thread's nodes: hc (registers), hn (shared plane
+// buffer), B (when the chunk owns plane i).  ec gets the old E of the own nodes
+// (the next plane's x taps and its E update); ep holds those of plane i - 1.
+template <int TY, bool ABS>
+__device__ __forceinline__ void fused_h_own(const Params& p, const FusedArgs& fa, const float* st, float* hn, const FNode& f, int i,
+                                            bool store, const Q4 (&ep)[3], Q4 (&hc)[3], Q4 (&ec)[3], const float* fco, int xrow, int xs,
+                                            const Q4 (&o)[3][2]) {
   const float cx = p.cdt[0], cy = p.cdt[1], cz = p.cdt[2];
-  const long long pb = (long long)i * p.g.sx;
-  int si[NR][3];
-  float old[NR][3][2];
-  if (AXM) {
-    // every auxiliary of the thread's nodes is requested before any is used
+  const Q4 ex = ld4(fE<TY>(st, 0, f.y, f.z)), ey = ld4(fE<TY>(st, 1, f.y, f.z)), ez = ld4(fE<TY>(st, 2, f.y, f.z));
+  const Q4 exm = ld4(fE<TY>(st, 0, f.y - 1, f.z)), ezm = ld4(fE<TY>(st, 2, f.y - 1, f.z));
+  const float exl = *fE<TY>(st, 0, f.y, f.z - 1), eyl = *fE<TY>(st, 1, f.y, f.z - 1);
+  // Hx -= dt(dy Ez - dz Ey); Hy -= dt(dz Ex - dx Ez); Hz -= dt(dx Ey - dy Ex)
+  const Q4 d01 = diff4(-cy, ez, ezm), d02 = diff4(cz, ey, below4(eyl, ey));
+  const Q4 d10 = diff4(cx, ez, ep[2]), d12 = diff4(-cz, ex, below4(exl, ex));
+  const Q4 d20 = diff4(-cx, ey, ep[1]), d21 = diff4(cy, ex, exm);
+  ec[0] = ex; ec[1] = ey; ec[2] = ez;
+  Q4 inc[3] = {add4(d01, d02), add4(d10, d12), add4(d20, d21)};
+  if (ABS) fused_cpml<TY, true>(p, fa, f, i, xs, fco, xrow, o, store, d01, d02, d10, d12, d20, d21, inc);
+  hc[0] = add4(ld4(fHx<TY>(st, f.y, f.z)), inc[0]);
+  hc[1] = add4(ld4(fHy<TY>(st, f.y, f.z)), inc[1]);
+  hc[2] = add4(ld4(fHz<TY>(st, f.y, f.z)), inc[2]);
+  if (f.nv < 4) {
 #pragma unroll
-    for (int r = 0; r < NR; r++) {
-      fused_slabs<AXM>(p, i, j0 + w + TW * r, k0 + lane, xs, ys[r], zs, si[r]);
-      if (!ok[r]) si[r][0] = si[r][1] = si[r][2] = -1;
-      fused_aux_load<AXM, true>(p, fa, si[r], old[r]);
-    }
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        if (e >= f.nv) hc[c].v[e] = 0.f;
   }
 #pragma unroll
-  for (int r = 0; r < NR; r++) {
-    const int y = w + TW * r, j = j0 + y, k = k0 + lane;
-    const float ez = fE<NR>(st, 2, y, lane), ey = fE<NR>(st, 1, y, lane), ex = fE<NR>(st, 0, y, lane);
-    ec[r][0] = ex; ec[r][1] = ey; ec[r][2] = ez;
-    // Hx -= dt(dy Ez - dz Ey); Hy -= dt(dz Ex - dx Ez); Hz -= dt(dx Ey - dy Ex)
-    const float dhx[3] = {0.f, __fmul_rn(-cy, __fsub_rn(ez, fE<NR>(st, 2, y - 1, lane))),
-                         __fmul_rn(cz, __fsub_rn(ey, fE<NR>(st, 1, y, lane - 1)))};
-    const float dhy[3] = {__fmul_rn(cx, __fsub_rn(ez, ep[r][2])), 0.f,
-                         __fmul_rn(-cz, __fsub_rn(ex, fE<NR>(st, 0, y, lane - 1)))};
-    const float dhz[3] = {__fmul_rn(-cx, __fsub_rn(ey, ep[r][1])), __fmul_rn(cy, __fsub_rn(ex, fE<NR>(st, 0, y - 1, lane))),
-                         0.f};
-    float ix = sum3(dhx[0], dhx[1], dhx[2]), iy = sum3(dhy[0], dhy[1], dhy[2]), iz = sum3(dhz[0], dhz[1], dhz[2]);
-    if (AXM && (si[r][0] & si[r][1] & si[r][2]) >= 0) {
-      const float* fx = fco + FCO_X + (i - p.x0 - blockIdx.z * p.xchunk + 1) * 6;
-      const float* fy = fco + FCO_Y + y * 6;
-      const float* fz = fco + FCO_Z + lane * 6;
-      ix = __fadd_rn(ix, fused_aux_apply<3, AXM>(p, fa, si[r], old[r], dhx, fx, fy, fz, store));
-      iy = __fadd_rn(iy, fused_aux_apply<4, AXM>(p, fa, si[r], old[r], dhy, fx, fy, fz, store));
-      iz = __fadd_rn(iz, fused_aux_apply<5, AXM>(p, fa, si[r], old[r], dhz, fx, fy, fz, store));
-    }
-    float vx = __fadd_rn(fHx<NR>(st, y, lane), ix), vy = __fadd_rn(fHy<NR>(st, y, lane), iy), vz = __fadd_rn(fHz<NR>(st, y, lane), iz);
-    if (!ok[r]) { vx = 0.f; vy = 0.f; vz = 0.f; }
-    hc[r][0] = vx; hc[r][1] = vy; hc[r][2] = vz;
-    fN<NR>(hn, 0, y, lane) = vx;
-    fN<NR>(hn, 1, y, lane) = vy;
-    fN<NR>(hn, 2, y, lane) = vz;
-    if (store && ok[r]) {
-      const long long off = pb + (long long)j * p.g.sy + k;
-      fa.dst[3][off] = vx;
-      fa.dst[4][off] = vy;
-      fa.dst[5][off] = vz;
-    }
+  for (int c = 0; c < 3; c++) st4(fN<TY>(hn, c, f.y, f.z), hc[c]);
+  if (store && f.nv > 0) {
+    const long long off = (long long)i * p.g.sx + (long long)f.j * p.g.sy + f.k;
+#pragma unroll
+    for (int c = 0; c < 3; c++) st4(fa.dst[3 + c] + off, hc[c]);
   }
 }
 
 // The halo of the new-H plane buffer (values the E update of the tile reads
-// beyond its own nodes), one component per warp:
-//   warp 0: Hz of row 16      warp 1: Hx of row 16
-//   warp 2: Hy of column 32   warp 3: Hx of column 32 (lanes 0-15)
-// xe: the warp's old E of the previous plane at its halo node (x tap), updated.
-// A CPML slab node takes the correction with the auxiliaries read, not written.
-template <int NR, bool ABS>
-__device__ __forceinline__ void fused_h_halo(const Params& p, const FusedArgs& fa, const float* st, float* hn, int i,
-                                             int j0, int k0, float& xe) {
-  const int lane = threadIdx.x, w = threadIdx.y;
-  if (w > 3 || (w > 1 && lane >= FL<NR>::TY)) return;
+// beyond its own nodes), one component per task, one node per lane:
+//   task 0: Hz of row TY      task 1: Hx of row TY
+//   task 2: Hy of column 32   task 3: Hx of column 32 (lanes below TY)
+// Each component has two derivative axes, a0 < a1.
+struct FHalo {
+  int y, z, j, k;
+  int ysh, zsh;              // slab coordinates of the node's row and column (-1 outside)
+  bool on, ok;               // the lane has a node / it lies in the grid
+};
+__device__ __forceinline__ int halo_a0(int task) { return task & 1; }
+__device__ __forceinline__ int halo_a1(int task) { return task == 0 ? 1 : 2; }
+// old auxiliaries of both axes (slots: Hz 1 and 1; Hx 0 and 0; Hy 0 on x, 1 on z), read only
+__device__ __forceinline__ void fused_halo_load(const Params& p, const FusedArgs& fa, int task, const FHalo& h, int i, int xs, float (&q)[2]) {
+  q[0] = q[1] = 0.f;
+  if (!h.ok) return;
+  const int s0 = task & 1 ? h.ysh : xs, s1 = task == 0 ? h.ysh : h.zsh;
+  if (s0 >= 0) q[0] = __ldg((task == 0 ? fa.hsrc[0][1] : task == 2 ? fa.hsrc[0][0] : fa.hsrc[1][0]) + slab_at(p, halo_a0(task), i, h.j, h.k, s0));
+  if (s1 >= 0) q[1] = __ldg((task == 0 ? fa.hsrc[1][1] : task == 2 ? fa.hsrc[2][1] : fa.hsrc[2][0]) + slab_at(p, halo_a1(task), i, h.j, h.k, s1));
+}
+// xe: the old E of the previous plane at the halo node (x tap), updated
+template <int TY, bool ABS>
+__device__ __forceinline__ void fused_h_halo(const Params& p, const float* st, float* hn, int task, const FHalo& h, float& xe,
+                                             const float* fco, int xrow, int xs, const float (&q)[2]) {
+  if (!h.on) return;
   const float cx = p.cdt[0], cy = p.cdt[1], cz = p.cdt[2];
-  const bool row = w < 2;
-  const int y = row ? FL<NR>::TY : lane, z = row ? lane : TZ;
-  const int j = j0 + y, k = k0 + z;
-  const bool ok = j < p.g.n[1] && k < p.g.n[2];
-  int si[3] = {-1, -1, -1};
-  const int idx[3] = {i, j, k};
-  const bool slab = ABS && ok && node_slabs(p, i, j, k, si);
-  float v;
-  if (w == 0) {
-    const float ey = fE<NR>(st, 1, y, z);
-    const float d0 = __fmul_rn(-cx, __fsub_rn(ey, xe));
-    const float d1 = __fmul_rn(cy, __fsub_rn(fE<NR>(st, 0, y, z), fE<NR>(st, 0, y - 1, z)));
-    v = fused_hnode<5, ABS>(p, fa, fHz<NR>(st, y, z), d0, d1, 0.f, slab, idx, si, false);
+  float d0, d1, old;
+  if (task == 0) {
+    const float ey = *fE<TY>(st, 1, h.y, h.z);
+    d0 = __fmul_rn(-cx, __fsub_rn(ey, xe));
+    d1 = __fmul_rn(cy, __fsub_rn(*fE<TY>(st, 0, h.y, h.z), *fE<TY>(st, 0, h.y - 1, h.z)));
+    old = *fHz<TY>(st, h.y, h.z);
     xe = ey;
-  } else if (w == 2) {
-    const float ez = fE<NR>(st, 2, y, z);
-    const float d0 = __fmul_rn(cx, __fsub_rn(ez, xe));
-    const float d2 = __fmul_rn(-cz, __fsub_rn(fE<NR>(st, 0, y, z), fE<NR>(st, 0, y, z - 1)));
-    v = fused_hnode<4, ABS>(p, fa, fHy<NR>(st, y, z), d0, 0.f, d2, slab, idx, si, false);
+  } else if (task == 2) {
+    const float ez = *fE<TY>(st, 2, h.y, h.z);
+    d0 = __fmul_rn(cx, __fsub_rn(ez, xe));
+    d1 = __fmul_rn(-cz, __fsub_rn(*fE<TY>(st, 0, h.y, h.z), *fE<TY>(st, 0, h.y, h.z - 1)));
+    old = *fHy<TY>(st, h.y, h.z);
     xe = ez;
   } else {
-    const float d1 = __fmul_rn(-cy, __fsub_rn(fE<NR>(st, 2, y, z), fE<NR>(st, 2, y - 1, z)));
-    const float d2 = __fmul_rn(cz, __fsub_rn(fE<NR>(st, 1, y, z), fE<NR>(st, 1, y, z - 1)));
-    v = fused_hnode<3, ABS>(p, fa, fHx<NR>(st, y, z), 0.f, d1, d2, slab, idx, si, false);
+    d0 = __fmul_rn(-cy, __fsub_rn(*fE<TY>(st, 2, h.y, h.z), *fE<TY>(st, 2, h.y - 1, h.z)));
+    d1 = __fmul_rn(cz, __fsub_rn(*fE<TY>(st, 1, h.y, h.z), *fE<TY>(st, 1, h.y, h.z - 1)));
+    old = *fHx<TY>(st, h.y, h.z);
   }
-  fN<NR>(hn, w == 0 ? 2 : w == 2 ? 1 : 0, y, z) = ok ? v : 0.f;
+  float inc = __fadd_rn(d0, d1);
+  if (ABS) {
+    float corr = 0.f;
+    if ((task & 1 ? h.ysh : xs) >= 0) {
+      const float* c = fco + (task & 1 ? FL<TY>::FCO_Y + h.y * 6 : FL<TY>::FCO_X + xrow * 6);
+      corr = __fmaf_rn(c[2], d0, __fmaf_rn(c[0], q[0], __fmul_rn(c[1], d0)));
+    }
+    if ((task == 0 ? h.ysh : h.zsh) >= 0) {
+      const float* c = fco + (task == 0 ? FL<TY>::FCO_Y + h.y * 6 : FL<TY>::FCO_Z + h.z);
+      const int s = task == 0 ? 1 : 36;
+      corr = __fadd_rn(corr, __fmaf_rn(c[2 * s], d1, __fmaf_rn(c[0], q[1], __fmul_rn(c[s], d1))));
+    }
+    inc = __fadd_rn(inc, corr);
+  }
+  *fN<TY>(hn, task == 0 ? 2 : task == 2 ? 1 : 0, h.y, h.z) = h.ok ? __fadd_rn(old, inc) : 0.f;
 }
 
 // New E of plane i on the own nodes.  ep: old E (registers), hn: new H of
 // plane i (shared), hc: new H of plane i + 1 (own nodes).
-//   MODE 1: uniform non-dispersive material um
-//   MODE 0: general (mixed materials, dispersive nodes left to the ADE pass,
-//           design region)
-// AXM: the slab axes of the tile-plane (0: no absorber).
-template <int NR, int MODE, int AXM>
-__device__ __forceinline__ void fused_e_own(const Params& p, const FusedArgs& fa, const float* st, const float* hn,
-                                            const MatShared& ms, int um, int i, int j0, int k0, const bool (&ok)[NR],
-                                            const float (&ep)[NR][3], const float (&hc)[NR][3], const float* fco, int xs,
-                                            const int (&ys)[NR], int zs) {
-  const int lane = threadIdx.x, w = threadIdx.y;
+//   MODE 2: vacuum; MODE 1: uniform non-dispersive material um;
+//   MODE 0: general (mixed materials, design region).  A dispersive node's table
+//           entry is 0, so it keeps its old E here and the ADE pass writes it
+//           (its absorber auxiliaries, if it has any, stay 0).
+template <int TY, int MODE, bool ABS>
+__device__ __forceinline__ void fused_e_own(const Params& p, const FusedArgs& fa, const float* st, const float* hn, const float* ies, int um,
+                                            const FNode& f, int i, const Q4 (&ep)[3], const Q4 (&hc)[3], const float* fco, int xrow, int xs,
+                                            const Q4 (&o)[3][2]) {
+  if (f.nv == 0) return;
   const float cx = p.cdt[0], cy = p.cdt[1], cz = p.cdt[2];
-  float iu[3] = {1.f, 1.f, 1.f};
-  if (MODE != 0) { iu[0] = ms.inv_eps[um][0]; iu[1] = ms.inv_eps[um][1]; iu[2] = ms.inv_eps[um][2]; }
-  const long long pb = (long long)i * p.g.sx;
-  int si[NR][3];
-  float old[NR][3][2];
-  if (AXM) {
+  const Q4 hx = ld4(fN<TY>(hn, 0, f.y, f.z)), hy = ld4(fN<TY>(hn, 1, f.y, f.z)), hz = ld4(fN<TY>(hn, 2, f.y, f.z));
+  const Q4 hxp = ld4(fN<TY>(hn, 0, f.y + 1, f.z)), hzp = ld4(fN<TY>(hn, 2, f.y + 1, f.z));
+  const float hxr = *fN<TY>(hn, 0, f.y, f.z + 4), hyr = *fN<TY>(hn, 1, f.y, f.z + 4);
+  // Ex += dt/eps(dy Hz - dz Hy); Ey += dt/eps(dz Hx - dx Hz); Ez += dt/eps(dx Hy - dy Hx)
+  Q4 d01 = diff4(cy, hzp, hz), d02 = diff4(-cz, above4(hy, hyr), hy);
+  Q4 d10 = diff4(-cx, hc[2], hz), d12 = diff4(cz, above4(hx, hxr), hx);
+  Q4 d20 = diff4(cx, hc[1], hy), d21 = diff4(-cy, hxp, hx);
+  if (MODE == 1) {
+    const float i0 = ies[um * 3], i1 = ies[um * 3 + 1], i2 = ies[um * 3 + 2];
 #pragma unroll
-    for (int r = 0; r < NR; r++) {
-      fused_slabs<AXM>(p, i, j0 + w + TW * r, k0 + lane, xs, ys[r], zs, si[r]);
-      if (!ok[r]) si[r][0] = si[r][1] = si[r][2] = -1;
-      fused_aux_load<AXM, false>(p, fa, si[r], old[r]);
+    for (int e = 0; e < 4; e++) {
+      d01.v[e] = __fmul_rn(d01.v[e], i0); d02.v[e] = __fmul_rn(d02.v[e], i0);
+      d10.v[e] = __fmul_rn(d10.v[e], i1); d12.v[e] = __fmul_rn(d12.v[e], i1);
+      d20.v[e] = __fmul_rn(d20.v[e], i2); d21.v[e] = __fmul_rn(d21.v[e], i2);
     }
   }
+  if (MODE == 0) {
+    const unsigned* mt = reinterpret_cast<const unsigned*>(st + FL<TY>::OFF_M);
+    unsigned m[3];
 #pragma unroll
-  for (int r = 0; r < NR; r++) {
-    if (!ok[r]) continue;
-    const int y = w + TW * r, j = j0 + y, k = k0 + lane;
-    const long long off = pb + (long long)j * p.g.sy + k;
-    const float hx = fN<NR>(hn, 0, y, lane), hy = fN<NR>(hn, 1, y, lane), hz = fN<NR>(hn, 2, y, lane);
-    // Ex += dt/eps(dy Hz - dz Hy); Ey += dt/eps(dz Hx - dx Hz); Ez += dt/eps(dx Hy - dy Hx)
-    float d[3][3];
-    d[0][0] = 0.f;
-    d[0][1] = __fmul_rn(cy, __fsub_rn(fN<NR>(hn, 2, y + 1, lane), hz));
-    d[0][2] = __fmul_rn(-cz, __fsub_rn(fN<NR>(hn, 1, y, lane + 1), hy));
-    d[1][0] = __fmul_rn(-cx, __fsub_rn(hc[r][2], hz));
-    d[1][1] = 0.f;
-    d[1][2] = __fmul_rn(cz, __fsub_rn(fN<NR>(hn, 0, y, lane + 1), hx));
-    d[2][0] = __fmul_rn(cx, __fsub_rn(hc[r][1], hy));
-    d[2][1] = __fmul_rn(-cy, __fsub_rn(fN<NR>(hn, 0, y + 1, lane), hx));
-    d[2][2] = 0.f;
-    const bool slab = AXM && (si[r][0] & si[r][1] & si[r][2]) >= 0;
-    const float* fx = fco + FCO_X + (i - p.x0 - blockIdx.z * p.xchunk + 1) * 6;
-    const float* fy = fco + FCO_Y + y * 6;
-    const float* fz = fco + FCO_Z + lane * 6;
+    for (int c = 0; c < 3; c++) m[c] = mt[(c * F_MROWS * TZ + f.y * TZ + f.z) / 4];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      float ie = iu[c];
-      if (MODE == 0) {
-        const int m = um >= 0 ? um : fM<NR>(st, c, y, lane);
-        if (ms.npoles[m] > 0) continue;              // dispersive node: the ADE pass writes it
-        ie = ms.inv_eps[m][c];
-        if (p.des_on) {
-          const long long di = design_index(p, i, j, k);
-          if (di >= 0) ie = p.des_ie[c][di];
+    for (int e = 0; e < 4; e++) {
+      float ie[3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) ie[c] = ies[((m[c] >> (8 * e)) & 255u) * 3 + c];
+      if (p.des_on) {
+        const long long di = design_index(p, i, f.j, f.k + e);
+        if (di >= 0) {
+#pragma unroll
+          for (int c = 0; c < 3; c++)
+            if (ie[c] != 0.f) ie[c] = p.des_ie[c][di];     // (a dispersive design node keeps its ADE update)
         }
       }
-      d[c][0] = __fmul_rn(d[c][0], ie); d[c][1] = __fmul_rn(d[c][1], ie); d[c][2] = __fmul_rn(d[c][2], ie);
-      float inc = sum3(d[c][0], d[c][1], d[c][2]);
-      if (slab) {
-        if (c == 0) inc = __fadd_rn(inc, fused_aux_apply<0, AXM>(p, fa, si[r], old[r], d[0], fx, fy, fz, true));
-        else if (c == 1) inc = __fadd_rn(inc, fused_aux_apply<1, AXM>(p, fa, si[r], old[r], d[1], fx, fy, fz, true));
-        else inc = __fadd_rn(inc, fused_aux_apply<2, AXM>(p, fa, si[r], old[r], d[2], fx, fy, fz, true));
-      }
-      fa.dst[c][off] = __fadd_rn(ep[r][c], inc);
+      d01.v[e] = __fmul_rn(d01.v[e], ie[0]); d02.v[e] = __fmul_rn(d02.v[e], ie[0]);
+      d10.v[e] = __fmul_rn(d10.v[e], ie[1]); d12.v[e] = __fmul_rn(d12.v[e], ie[1]);
+      d20.v[e] = __fmul_rn(d20.v[e], ie[2]); d21.v[e] = __fmul_rn(d21.v[e], ie[2]);
     }
   }
+  Q4 inc[3] = {add4(d01, d02), add4(d10, d12), add4(d20, d21)};
+  if (ABS) fused_cpml<TY, false>(p, fa, f, i, xs, fco, xrow, o, true, d01, d02, d10, d12, d20, d21, inc);
+  const long long off = (long long)i * p.g.sx + (long long)f.j * p.g.sy + f.k;
+#pragma unroll
+  for (int c = 0; c < 3; c++) st4(fa.dst[c] + off, add4(ep[c], inc[c]));
 }
 
 // Issue the copies of stage s (plane x0 - 1 + s; the material tiles of the
 // plane before it, whose E update runs while this stage is current).
-template <int NR>
+template <int TY>
 __device__ __forceinline__ void fused_issue(const FusedMaps& m, float* st, uint64_t* bar, int ip, int j0, int k0,
                                             bool want_mat) {
-  mbar_arrive_expect_tx(bar, FL<NR>::BYTES + (want_mat ? FL<NR>::BYTES_MAT : 0u));
+  mbar_arrive_expect_tx(bar, FL<TY>::BYTES + (want_mat ? FL<TY>::BYTES_MAT : 0u));
 #pragma unroll
-  for (int c = 0; c < 3; c++) tma_load_3d(st + c * FL<NR>::FE_N, &m.e[c], k0 - 4, j0 - 1, ip, bar);
-  tma_load_3d(st + FL<NR>::OFF_HX, &m.hx, k0, j0, ip, bar);
-  tma_load_3d(st + FL<NR>::OFF_HY, &m.hy, k0, j0, ip, bar);
-  tma_load_3d(st + FL<NR>::OFF_HZ, &m.hz, k0, j0, ip, bar);
+  for (int c = 0; c < 3; c++) tma_load_3d(st + c * FL<TY>::FE_N, &m.e[c], k0 - 4, j0 - 1, ip, bar);
+  tma_load_3d(st + FL<TY>::OFF_HX, &m.hx, k0, j0, ip, bar);
+  tma_load_3d(st + FL<TY>::OFF_HY, &m.hy, k0, j0, ip, bar);
+  tma_load_3d(st + FL<TY>::OFF_HZ, &m.hz, k0, j0, ip, bar);
   if (want_mat)
 #pragma unroll
     for (int c = 0; c < 3; c++)
-      tma_load_3d(reinterpret_cast<uint8_t*>(st + FL<NR>::OFF_M) + c * F_MROWS * TZ, &m.mat[c], k0, j0, ip - 1, bar);
+      tma_load_3d(reinterpret_cast<uint8_t*>(st + FL<TY>::OFF_M) + c * F_MROWS * TZ, &m.mat[c], k0, j0, ip - 1, bar);
 }
 
-// H of plane i over the own nodes for the tile-plane's slab axes m (bit 0: x
-// slab plane, bit 1: y slab rows, bit 2: z slab columns).  Tile-planes with
-// any slab take one general variant: variants per slab combination were
-// measured slower on every workload (a larger kernel).
-template <int NR>
-__device__ __forceinline__ void fused_h_dispatch(int m, const Params& p, const FusedArgs& fa, const float* st, float* hn,
-                                                 int i, int j0, int k0, bool store, const bool (&ok)[NR],
-                                                 const float (&ep)[NR][3], float (&hc)[NR][3], float (&ec)[NR][3],
-                                                 const float* fco, int xs, const int (&ys)[NR], int zs) {
-  switch (m) {
-    case 0: fused_h_own<NR, 0>(p, fa, st, hn, i, j0, k0, store, ok, ep, hc, ec, fco, xs, ys, zs); break;
-    default: fused_h_own<NR, 7>(p, fa, st, hn, i, j0, k0, store, ok, ep, hc, ec, fco, xs, ys, zs); break;
-  }
-}
-template <int NR, int MODE>
-__device__ __forceinline__ void fused_e_dispatch(int m, const Params& p, const FusedArgs& fa, const float* st,
-                                                 const float* hn, const MatShared& ms, int um, int i, int j0, int k0,
-                                                 const bool (&ok)[NR], const float (&ep)[NR][3], const float (&hc)[NR][3],
-                                                 const float* fco, int xs, const int (&ys)[NR], int zs) {
-  switch (m) {
-    case 0: fused_e_own<NR, MODE, 0>(p, fa, st, hn, ms, um, i, j0, k0, ok, ep, hc, fco, xs, ys, zs); break;
-    default: fused_e_own<NR, MODE, 7>(p, fa, st, hn, ms, um, i, j0, k0, ok, ep, hc, fco, xs, ys, zs); break;
-  }
-}
-
-// 3 CTAs per SM (shared memory: a 3-stage ring and two new-H planes)
-template <int NR>
-__global__ void __launch_bounds__(NTHR, NR == 2 ? 3 : 4)
+// 16 rows: 3 CTAs per SM, what shared memory allows (a 3-stage ring and two
+// new-H planes); 8 rows: 5
+template <int TY>
+__global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
     fused_kernel(const __grid_constant__ Params p, const __grid_constant__ FusedArgs fa,
                  const __grid_constant__ FusedMaps m) {
+  using L = FL<TY>;
   extern __shared__ __align__(128) float fsm[];
-  float* hnb = fsm + F_NST * FL<NR>::STAGE;                      // two new-H planes
-  MatShared& ms = *reinterpret_cast<MatShared*>(hnb + 2 * FL<NR>::HN);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<char*>(&ms) + sizeof(MatShared));
+  float* hnb = fsm + F_NST * L::STAGE;                           // two new-H planes
+  float* fco = hnb + 2 * L::HN;
+  float* ies = fco + f_up32(L::FCO_N);                           // 1/eps of the material table
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ies + MAXMAT * 3);
   __shared__ signed char umc[FX_MAX];
-  __shared__ float fco[FCO_N];
   __shared__ int gave_up;
-  const int lane = threadIdx.x, w = threadIdx.y, tid = w * TZ + lane;
-  const int k0 = blockIdx.x * TZ, j0 = blockIdx.y * FL<NR>::TY;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int k0 = blockIdx.x * TZ, j0 = blockIdx.y * TY;
   const int x0 = p.x0 + blockIdx.z * p.xchunk;
   const int x1 = min(x0 + p.xchunk, p.x1);
   const int len = x1 - x0;
@@ -430,61 +458,97 @@ __global__ void __launch_bounds__(NTHR, NR == 2 ? 3 : 4)
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     gave_up = 0;
   }
-  load_matshared(ms, p);
-  for (int q = tid; q < len; q += NTHR)
+  for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
+  for (int q = tid; q < len; q += L::NT)
     umc[q] = __ldg(p.umat + ((long long)(x0 + q) * p.nty + j0 / F_MROWS) * p.ntz + blockIdx.x);
-  if (cpml)
-    for (int q = tid; q < FCO_N / 6; q += NTHR) {
-      // row q: x plane x0 - 1 + q, y row j0 + q - (FX_MAX + 2), z column k0 + q - (FX_MAX + F_MROWS + 3)
-      const int a = q < FX_MAX + 2 ? 0 : q < FX_MAX + F_MROWS + 3 ? 1 : 2;
-      const int v = a == 0 ? x0 - 1 + q : a == 1 ? j0 + q - (FX_MAX + 2) : k0 + q - (FX_MAX + F_MROWS + 3);
+  if (cpml) {
+    // coefficient row q: x plane x0 - 1 + q, then y row j0 + ..., then z column k0 + ...
+    constexpr int RX = FX_MAX + 2, RY_ = TY + 1, RZ = TZ + 1;
+    for (int q = tid; q < RX + RY_ + RZ; q += L::NT) {
+      const int a = q < RX ? 0 : q < RX + RY_ ? 1 : 2;
+      const int v0 = a == 0 ? q : a == 1 ? q - RX : q - RX - RY_;
+      const int v = v0 + (a == 0 ? x0 - 1 : a == 1 ? j0 : k0);
+      if (a == 0 && v0 > len + 1) continue;
 #pragma unroll
       for (int o = 0; o < 2; o++) {
         const int h = 2 * v + o;
         const bool in = h >= 0 && h < 2 * p.g.n[a] + 2;
-        fco[q * 6 + 3 * o + 0] = in ? __ldg(p.ab.c0[a] + h) : 1.f;
-        fco[q * 6 + 3 * o + 1] = in ? __ldg(p.ab.c1[a] + h) : 0.f;
-        fco[q * 6 + 3 * o + 2] = in ? __fsub_rn(__ldg(p.ab.c2[a] + h), 1.f) : 0.f;
+        const float cb = in ? __ldg(p.ab.c0[a] + h) : 1.f, ca = in ? __ldg(p.ab.c1[a] + h) : 0.f;
+        const float cc = in ? __fsub_rn(__ldg(p.ab.c2[a] + h), 1.f) : 0.f;
+        float* d = a == 2 ? fco + L::FCO_Z + 3 * o * 36 + v0 : fco + (a == 0 ? L::FCO_X : L::FCO_Y) + v0 * 6 + 3 * o;
+        const int s = a == 2 ? 36 : 1;
+        d[0] = cb; d[s] = ca; d[2 * s] = cc;
       }
     }
+  }
   __syncthreads();
   auto issue = [&](int s) {
     const int ip = x0 - 1 + s;
-    fused_issue<NR>(m, fsm + (s % F_NST) * FL<NR>::STAGE, &bars[s % F_NST], ip, j0, k0, ip - 1 >= x0 && umc[ip - 1 - x0] < 0);
+    fused_issue<TY>(m, fsm + (s % F_NST) * L::STAGE, &bars[s % F_NST], ip, j0, k0, ip - 1 >= x0 && umc[ip - 1 - x0] < 0);
   };
   int issued = -1;
   if (tid == 0)
     for (int s = 0; s < F_NST && s <= slast; s++) { issue(s); issued = s; }
   // per-thread constants of the walk
-  bool ok[NR];
-  int ys[NR];
+  FNode f;
+  f.y = tid >> 3; f.z = 4 * (tid & 7);
+  f.j = j0 + f.y; f.k = k0 + f.z;
+  f.nv = f.j < p.g.n[1] ? min(4, max(0, p.g.n[2] - f.k)) : 0;
+  f.ys = cpml ? slab_cs(p, 1, f.j) : -1;
+  f.zs = 0; f.zm = 0;
+  if (cpml) {
+    // (the grid is at least four cells wider than both slabs, so four nodes meet one of them at most)
+    const int lo = p.ab.L[2][0], hi = p.g.n[2] - p.ab.L[2][1];
+    f.zs = f.k < lo ? f.k : f.k + lo - hi;
 #pragma unroll
-  for (int r = 0; r < NR; r++) {
-    ok[r] = j0 + w + TW * r < p.g.n[1] && k0 + lane < p.g.n[2];
-    ys[r] = cpml ? slab_cs(p, 1, j0 + w + TW * r) : -1;
+    for (int e = 0; e < 4; e++)
+      if (e < f.nv && (f.k + e < lo || f.k + e >= hi)) f.zm |= 1u << e;
   }
-  const int zs = cpml ? slab_cs(p, 2, k0 + lane) : -1;
-  // slab axes of the own nodes (y, z: fixed for the walk) and of the halo (row 16, column 32)
-  const int myz = cpml ? ((j0 < p.ab.L[1][0] || j0 + FL<NR>::TY > p.g.n[1] - p.ab.L[1][1]) ? 2 : 0) |
-                             ((k0 < p.ab.L[2][0] || k0 + TZ > p.g.n[2] - p.ab.L[2][1]) ? 4 : 0)
-                       : 0;
-  const bool halo_yz = cpml && (j0 < p.ab.L[1][0] || j0 + FL<NR>::TY + 1 > p.g.n[1] - p.ab.L[1][1] || k0 < p.ab.L[2][0] ||
-                                k0 + TZ + 1 > p.g.n[2] - p.ab.L[2][1]);
-  float ep[NR][3], hc[NR][3], ec[NR][3];
-  float xe = 0.f;
+  f.vxy = (p.g.n[2] & 3) == 0;
+  f.vz = f.zm == 15u && ((p.ab.L[2][0] + p.ab.L[2][1]) & 3) == 0 && (f.zs & 3) == 0;
+  FHalo hl[L::TASKS];
+  float xe[L::TASKS], hq[L::TASKS][2];
+#pragma unroll
+  for (int q = 0; q < L::TASKS; q++) {
+    const int task = w + q * L::NW;
+    const bool row = task < 2;
+    hl[q].y = row ? TY : lane; hl[q].z = row ? lane : TZ;
+    hl[q].j = j0 + hl[q].y; hl[q].k = k0 + hl[q].z;
+    hl[q].on = task < 4 && (row || lane < TY);
+    hl[q].ok = hl[q].on && hl[q].j < p.g.n[1] && hl[q].k < p.g.n[2];
+    hl[q].ysh = cpml ? slab_cs(p, 1, hl[q].j) : -1;
+    hl[q].zsh = cpml ? slab_cs(p, 2, hl[q].k) : -1;
+    xe[q] = 0.f; hq[q][0] = hq[q][1] = 0.f;
+  }
+  // does the tile (own nodes, then with the halo) meet a y or z slab?
+  const bool own_yz = cpml && (j0 < p.ab.L[1][0] || j0 + TY > p.g.n[1] - p.ab.L[1][1] || k0 < p.ab.L[2][0] ||
+                               k0 + TZ > p.g.n[2] - p.ab.L[2][1]);
+  const bool halo_yz = cpml && (own_yz || j0 + TY + 1 > p.g.n[1] - p.ab.L[1][1] || k0 + TZ + 1 > p.g.n[2] - p.ab.L[2][1]);
+  Q4 ep[3], hc[3], ec[3], oh[3][2], oe[3][2];
   // stage 0 (plane x0 - 1): the old E of the own nodes and of the halo nodes (x taps)
   if (tid == 0 && !mbar_wait(&bars[0], 0u, p.err, p.wait_limit)) gave_up = 1;
   __syncthreads();
   int t = 0, swait = 0;                                    // swait: the stage waited for last
   if (!gave_up) {
 #pragma unroll
-    for (int r = 0; r < NR; r++)
+    for (int c = 0; c < 3; c++) ep[c] = ld4(fE<TY>(fsm, c, f.y, f.z));
 #pragma unroll
-      for (int c = 0; c < 3; c++) ep[r][c] = fE<NR>(fsm, c, w + TW * r, lane);
-    if (w == 0) xe = fE<NR>(fsm, 1, FL<NR>::TY, lane);
-    else if (w == 2 && lane < FL<NR>::TY) xe = fE<NR>(fsm, 2, lane, TZ);
+    for (int q = 0; q < L::TASKS; q++) {
+      const int task = w + q * L::NW;
+      if (hl[q].on && !(task & 1)) xe[q] = *fE<TY>(fsm, task == 0 ? 1 : 2, hl[q].y, hl[q].z);
+    }
     for (; t <= len; t++) {
-      const int s = t + 1, pc = x0 + t;
+      const int s = t + 1, pc = x0 + t, pe = pc - 1;
+      const int xs = cpml ? slab_cs(p, 0, pc) : -1, xse = cpml ? slab_cs(p, 0, pe) : -1;
+      const bool abh = own_yz || xs >= 0, abe = own_yz || xse >= 0, abl = halo_yz || xs >= 0;
+      // absorber tile-planes: the old auxiliaries, requested before the stage wait
+      if (pc < p.g.n[0]) {
+        if (abh) fused_aux_load<true>(p, fa, f, pc, xs, oh);
+        if (abl)
+#pragma unroll
+          for (int q = 0; q < L::TASKS; q++) fused_halo_load(p, fa, w + q * L::NW, hl[q], pc, xs, hq[q]);
+      }
+      if (t >= 1 && abe) fused_aux_load<false>(p, fa, f, pe, xse, oe);
       swait = s;
       if (tid == 0 && !mbar_wait(&bars[s % F_NST], (unsigned)((s / F_NST) & 1), p.err, p.wait_limit)) gave_up = 1;
       // every thread is past iteration t - 1: the slot of stage t and the new-H
@@ -492,33 +556,37 @@ __global__ void __launch_bounds__(NTHR, NR == 2 ? 3 : 4)
       __syncthreads();
       if (gave_up) break;
       if (tid == 0 && t + F_NST <= slast) { issue(t + F_NST); issued = t + F_NST; }
-      const float* st = fsm + (s % F_NST) * FL<NR>::STAGE;
-      float* hn1 = hnb + (t & 1) * FL<NR>::HN;                   // new H of plane pc
-      const float* hn0 = hnb + ((t + 1) & 1) * FL<NR>::HN;       // new H of plane pc - 1
+      const float* st = fsm + (s % F_NST) * L::STAGE;
+      float* hn1 = hnb + (t & 1) * L::HN;                        // new H of plane pc
+      const float* hn0 = hnb + ((t + 1) & 1) * L::HN;            // new H of plane pc - 1
       if (pc < p.g.n[0]) {
-        const int xs = cpml ? slab_cs(p, 0, pc) : -1;
-        fused_h_dispatch<NR>(myz | (xs >= 0 ? 1 : 0), p, fa, st, hn1, pc, j0, k0, t < len, ok, ep, hc, ec, fco, xs, ys, zs);
-        if (halo_yz || xs >= 0) fused_h_halo<NR, true>(p, fa, st, hn1, pc, j0, k0, xe);
-        else fused_h_halo<NR, false>(p, fa, st, hn1, pc, j0, k0, xe);
+        if (abh) fused_h_own<TY, true>(p, fa, st, hn1, f, pc, t < len, ep, hc, ec, fco, t + 1, xs, oh);
+        else fused_h_own<TY, false>(p, fa, st, hn1, f, pc, t < len, ep, hc, ec, fco, t + 1, xs, oh);
+#pragma unroll
+        for (int q = 0; q < L::TASKS; q++) {
+          const int task = w + q * L::NW;
+          if (abl) fused_h_halo<TY, true>(p, st, hn1, task, hl[q], xe[q], fco, t + 1, xs, hq[q]);
+          else fused_h_halo<TY, false>(p, st, hn1, task, hl[q], xe[q], fco, t + 1, xs, hq[q]);
+        }
       } else {
         // beyond the last plane of the grid: H is zero there
 #pragma unroll
-        for (int r = 0; r < NR; r++)
-#pragma unroll
-          for (int c = 0; c < 3; c++) { hc[r][c] = 0.f; ec[r][c] = 0.f; }
+        for (int c = 0; c < 3; c++) { hc[c] = Q4{{0.f, 0.f, 0.f, 0.f}}; ec[c] = hc[c]; }
       }
       if (t >= 1) {
-        const int pe = pc - 1;
         const int um = umc[pe - x0];
-        const int xs = cpml ? slab_cs(p, 0, pe) : -1;
-        const int mm = myz | (xs >= 0 ? 1 : 0);
-        if (um >= 0) fused_e_dispatch<NR, 1>(mm, p, fa, st, hn0, ms, um, pe, j0, k0, ok, ep, hc, fco, xs, ys, zs);
-        else fused_e_dispatch<NR, 0>(mm, p, fa, st, hn0, ms, um, pe, j0, k0, ok, ep, hc, fco, xs, ys, zs);
+        const bool vac = um >= 0 && ies[um * 3] == 1.f && ies[um * 3 + 1] == 1.f && ies[um * 3 + 2] == 1.f;
+        switch ((vac ? 4 : um >= 0 ? 2 : 0) + (abe ? 1 : 0)) {
+          case 5: fused_e_own<TY, 2, true>(p, fa, st, hn0, ies, um, f, pe, ep, hc, fco, t, xse, oe); break;
+          case 4: fused_e_own<TY, 2, false>(p, fa, st, hn0, ies, um, f, pe, ep, hc, fco, t, xse, oe); break;
+          case 3: fused_e_own<TY, 1, true>(p, fa, st, hn0, ies, um, f, pe, ep, hc, fco, t, xse, oe); break;
+          case 2: fused_e_own<TY, 1, false>(p, fa, st, hn0, ies, um, f, pe, ep, hc, fco, t, xse, oe); break;
+          case 1: fused_e_own<TY, 0, true>(p, fa, st, hn0, ies, um, f, pe, ep, hc, fco, t, xse, oe); break;
+          default: fused_e_own<TY, 0, false>(p, fa, st, hn0, ies, um, f, pe, ep, hc, fco, t, xse, oe); break;
+        }
       }
 #pragma unroll
-      for (int r = 0; r < NR; r++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) ep[r][c] = ec[r][c];
+      for (int c = 0; c < 3; c++) ep[c] = ec[c];
     }
   }
   if (gave_up && tid == 0) {
