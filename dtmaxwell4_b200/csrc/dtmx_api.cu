@@ -128,6 +128,8 @@ struct dtmx_ctx {
   FusedMaps fmaps8[2]{};              // the same for 8-row tiles
   int frows = 16;                     // tile rows of the single sweep (16 or 8; dtmx_set_tile_rows, dtmx_autotune)
   bool fused_ready = false;
+  bool ptr_given = false;             // dtmx_field_device_ptr was called: see step_engine
+  bool auto_per_step = false;         // the automatic choice found no room for the second set
   int parity = 0;                     // 0: state in the buffers allocated first
   int* d_err = nullptr;
   bool has_gyro = false;
@@ -1419,6 +1421,35 @@ static int fused_prepare(dtmx_ctx* ctx) {
   return DTMX_OK;
 }
 
+static double free_device_bytes() {
+  size_t fr = 0, tot = 0;
+  return cudaMemGetInfo(&fr, &tot) == cudaSuccess ? (double)fr : 0.0;
+}
+
+// device bytes of the second set
+static double fused_set_bytes(const dtmx_ctx* ctx) {
+  double n = 6.0 * (ctx->nstore + 64);
+  for (int a = 0; a < 3; a++)
+    if (ctx->P.ab.aux[a][2]) n += 2.0 * (ctx->P.ab.L[a][0] + ctx->P.ab.L[a][1]) * (double)(ctx->ncell / (size_t)ctx->P.g.n[a]);
+  return 4.0 * n;
+}
+
+// Give a half-made second set back (plain allocations: the automatic choice leaves parkable contexts alone).
+static void fused_release(dtmx_ctx* ctx) {
+  if (ctx->fused_ready) return;
+  cudaStreamSynchronize(ctx->stream);
+  auto drop = [&](float*& q) {
+    if (!q) return;
+    auto it = std::find(ctx->allocs.begin(), ctx->allocs.end(), (void*)q);
+    if (it != ctx->allocs.end()) { cudaFree(q); ctx->allocs.erase(it); }
+    q = nullptr;
+  };
+  for (auto& q : ctx->f_alt) drop(q);
+  for (auto& a : ctx->hax_alt)
+    for (auto& q : a) drop(q);
+  cudaGetLastError();
+}
+
 // The state now lives in the other buffer set: swap the pointers (fields, H
 // auxiliaries, the maps reading them) so that P and every pass see it.
 static void fused_swap(dtmx_ctx* ctx) {
@@ -1432,16 +1463,26 @@ static void fused_swap(dtmx_ctx* ctx) {
   ctx->tmaps_ok = false;          // the wavefront engine's maps are rebuilt for the current buffer
 }
 
-// planes per CTA (at most FX_MAX): about eight waves of 3 CTAs per SM, and
-// at least 8 planes (each chunk stages one plane and updates one H plane more)
+// Planes per CTA (at most FX_MAX).  One wave of the 3 CTAs per SM that fit,
+// where that takes chunks of at most 12 planes: small grids are bound by the
+// latency of a CTA's walk, and a nearly empty last wave costs as much as a full
+// one (128^3 with a 10-cell CPML, 32 tile columns: 39.9 us with chunks of 10
+// = 416 CTAs, 45.8 with 8 = 512 CTAs; 48^3: 9.4 us with chunks of 1, 26.0 with
+// 8).  Larger grids: about eight waves, chunks of 6 to 32 planes (each chunk
+// stages one plane and updates one H plane more; 192x160x128: 68.0 us with 6,
+// 77.3 with 12; 384^3: 634 us with 32, 641 with 10, 669 with 64).
 static int fused_xchunk_for(const dtmx_ctx* ctx) {
   if (ctx->xchunk > 0) return std::min(ctx->xchunk, FX_MAX);
   const dtmx_config& c = ctx->cfg;
   const long long tiles = (long long)((c.nz + TZ - 1) / TZ) * ((c.ny + ctx->frows - 1) / ctx->frows);
-  const long long target = 148LL * 3 * 8;
-  const long long chunks = std::max<long long>(1, (target + tiles - 1) / tiles);
+  const long long fit = 148LL * (ctx->frows == 16 ? 3 : 5);
+  if (tiles <= fit) {
+    const long long xc = (c.nx + fit / tiles - 1) / (fit / tiles);
+    if (xc <= 12) return (int)xc;
+  }
+  const long long chunks = std::max<long long>(1, (fit * 8 + tiles - 1) / tiles);
   const long long xc = (c.nx + chunks - 1) / chunks;
-  return (int)std::min<long long>(32, std::max<long long>(8, xc));
+  return (int)std::min<long long>(32, std::max<long long>(6, xc));
 }
 
 // One time step of the single-sweep engine: the side passes that act on the
@@ -1539,8 +1580,32 @@ static int launch_fused_step(dtmx_ctx* ctx) {
   return DTMX_OK;
 }
 
+// The engine of a step: 3 where it was chosen, and for engine 0 (automatic)
+// wherever the single sweep applies: it was faster at every size measured
+// (48^3 9.4 against 34.9 us a step, 128^3 40 against 66, 640x512x384 1.30
+// against 1.79 ms).  The automatic choice stays with the per-step engine
+//   * once dtmx_field_device_ptr has handed out an address (the single sweep
+//     alternates between two sets of arrays, the per-step engine updates the
+//     one the caller holds),
+//   * while profiling (which times the H and the E kernel),
+//   * for parkable contexts and where the second set would take more than half
+//     of the free device memory (or cannot be had): it doubles the fields.
+// Needs fused_prepare's allocations, so call it outside a capture.
+static int step_engine(dtmx_ctx* ctx) {
+  if (ctx->engine != 0) return ctx->engine == 3 ? 3 : 1;
+  if (ctx->ptr_given || ctx->profiling || ctx->cfg.parkable || ctx->auto_per_step || !fused_usable(ctx, nullptr)) return 1;
+  if (!ctx->fused_ready) {
+    if (fused_set_bytes(ctx) > 0.5 * free_device_bytes() || fused_prepare(ctx) != DTMX_OK) {
+      fused_release(ctx);
+      ctx->auto_per_step = true;
+      return 1;
+    }
+  }
+  return 3;
+}
+
 // one time step of the selected per-step engine (per-step or single sweep)
-static int launch_one(dtmx_ctx* ctx) { return ctx->engine == 3 ? launch_fused_step(ctx) : launch_step(ctx); }
+static int launch_one(dtmx_ctx* ctx) { return step_engine(ctx) == 3 ? launch_fused_step(ctx) : launch_step(ctx); }
 
 // Capture (once per field buffer) and launch 16 per-step launch sequences as
 // one graph.  The host-side bookkeeping of the 16 steps (staging slots,
@@ -1552,7 +1617,7 @@ static int graph_steps16(dtmx_ctx* ctx) {
   const int par = ctx->parity;
   if (!ctx->graph16[par]) {
     set_kernel_attributes();
-    if (ctx->engine == 3) { int rc = fused_prepare(ctx); if (rc) return rc; }
+    if (step_engine(ctx) == 3) { int rc = fused_prepare(ctx); if (rc) return rc; }
     const long long launches0 = ctx->launches;
     const int gcur0 = ctx->gcur;
     std::vector<int> staged0;
@@ -1745,10 +1810,6 @@ struct FaRun {
 static double fa_history_bytes(const dtmx_ctx* ctx, int nsteps) {
   const Params& P = ctx->P;
   return (double)(nsteps + 1) * 3.0 * P.des_n[0] * P.des_n[1] * P.des_n[2] * 4.0;
-}
-static double free_device_bytes() {
-  size_t fr = 0, tot = 0;
-  return cudaMemGetInfo(&fr, &tot) == cudaSuccess ? (double)fr : 0.0;
 }
 static bool fa_history_fits(dtmx_ctx* ctx, int nsteps) {
   const double bytes = fa_history_bytes(ctx, nsteps);
@@ -2291,6 +2352,8 @@ extern "C" int dtmx_set_field(dtmx_ctx* ctx, int comp, const float* host_in) {
 extern "C" int dtmx_field_device_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]) {
   if (ctx && ctx->parked) return fail(ctx, DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
   if (!ctx || comp < 0 || comp > 5 || !dptr) return fail(ctx, DTMX_ERR_INVALID, "bad field request");
+  // the caller may keep the address: the automatic engine choice leaves the arrays where they are from here on
+  if (!ctx->ptr_given) { ctx->ptr_given = true; if (ctx->engine == 0) drop_graphs(ctx); }
   *dptr = ctx->P.f[comp];
   if (strides) { strides[0] = ctx->P.g.sx; strides[1] = ctx->P.g.sy; strides[2] = 1; }
   return DTMX_OK;

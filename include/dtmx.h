@@ -270,7 +270,9 @@ int  dtmx_get_step(const dtmx_ctx* ctx, int64_t* n);
 /* Field access (host buffers, nx*ny*nz floats, z fastest). */
 int  dtmx_get_field(dtmx_ctx* ctx, int comp, float* host_out);
 int  dtmx_set_field(dtmx_ctx* ctx, int comp, const float* host_in);
-/* Device pointer of a component and its element strides (x, y, z). */
+/* Device pointer of a component and its element strides (x, y, z).  The state
+ * stays at that address with engines 0, 1 and 2; engine 3 alternates between
+ * two sets of arrays, so ask again after each dtmx_step. */
 int  dtmx_field_device_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]);
 
 /* Host-side NaN/Inf check of the probe traces and a device reduction over E;
@@ -433,7 +435,11 @@ int  dtmx_load_state(dtmx_ctx* ctx, const char* path);
 #define DTMX_NOALLOC_MAX_ELEMS (DTMX_NOALLOC_BLOCK_ELEMS * DTMX_NOALLOC_MAX_BLOCKS)
 int  dtmx_count_nonfinite_noalloc(const float* const* d_fields, int nfields, int64_t nelem, int64_t* count_out);
 
-/* Engine choice for dtmx_step: 0 = auto, 1 = one launch per half step,
+/* Engine choice for dtmx_step: 0 = auto (the single sweep where it applies and
+ * its second set of arrays takes at most half of the free device memory; one
+ * launch per half step otherwise, for parkable contexts, while profiling, and
+ * once dtmx_field_device_ptr has handed out an address: its arrays then keep
+ * holding the state), 1 = one launch per half step,
  * 2 = L2-resident wavefront (several time steps per launch), 3 = single sweep
  * (one launch per time step updating H and then E over two field buffers; box
  * geometry, order 2, CPML or no absorber).  The reference compiles its kernel

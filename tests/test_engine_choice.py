@@ -1,0 +1,79 @@
+"""Engine 0 (automatic): the single sweep wherever it applies, with the state
+where the caller may look for it.  Every engine evaluates the same expressions
+without a TF/SF source, so the fields equal the per-step engine's exactly."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+N = (21, 34, 45)
+
+
+def _sim(engine, parkable=False, absorber=True):
+    from dtmaxwell4_b200 import Simulation, abi
+    s = Simulation(abi.make_config(*N, courant=0.5, absorber=abi.ABS_CPML if absorber else abi.ABS_NONE, pml=5 if absorber else 0,
+                                   parkable=parkable))
+    rng = np.random.default_rng(2)
+    for c in range(6):
+        s.set_field(c, rng.standard_normal(N).astype(np.float32))
+    s.set_engine(engine)
+    return s
+
+
+def _fields(s):
+    s.sync()
+    return [s.get_field(c) for c in range(6)]
+
+
+def _equal(a, b):
+    for c in range(6):
+        assert np.array_equal(a[c], b[c]), c
+
+
+@pytest.mark.parametrize("parkable", [False, True])
+@pytest.mark.parametrize("steps", [(3, 16, 18), (1,), (33, 2)])
+def test_automatic_equals_the_per_step_engine(steps, parkable):
+    a, b = _sim(1), _sim(0, parkable)
+    for n in steps:
+        a.step(n)
+        b.step(n)
+        _equal(_fields(b), _fields(a))
+    assert b.engine_config()[0] == 0
+    a.close()
+    b.close()
+
+
+def test_a_device_address_stays_the_state():
+    """After an odd number of single-sweep steps an address is handed out: from
+    then on every step leaves the state there (17 steps: a graph replay and one)."""
+    a, b = _sim(1), _sim(0)
+    b.step(19)
+    ptr = [b.device_ptr(c)[0] for c in range(6)]
+    a.step(19)
+    for n in (1, 17, 16):
+        a.step(n)
+        b.step(n)
+        assert [b.device_ptr(c)[0] for c in range(6)] == ptr
+        _equal(_fields(b), _fields(a))
+    b.set_engine(3)                   # the choice is the caller's again
+    a.step(4)
+    b.step(4)
+    _equal(_fields(b), _fields(a))
+    a.close()
+    b.close()
+
+
+def test_profiling_times_both_kernels():
+    s = _sim(0)
+    s.step(5)
+    s.set_profiling(True)
+    s.step(4)
+    h, e, n = s.read_profile()
+    assert n == 4 and h > 0 and e > 0
+    s.set_profiling(False)
+    a = _sim(1)
+    a.step(9 + 20)
+    s.step(20)
+    _equal(_fields(s), _fields(a))
+    a.close()
+    s.close()
