@@ -32,7 +32,17 @@ struct DftHost {
   double2* acc = nullptr;
   float* stage = nullptr;
   long long* sstep = nullptr;
-  int nstaged = 0;          // samples staged since the last flush
+};
+
+// The device tables of a set of DFT planes that are sampled and folded
+// together: their descriptors, the block map of the samples (tail_kernel) and
+// the work units of a fold (dft_flush_kernel).
+struct MonTable {
+  DftDev* tab = nullptr;
+  int2* map = nullptr;
+  FlushUnit* unit = nullptr;
+  int nmap = 0, nunit = 0;
+  int nstaged = 0;          // samples staged since the last fold, the same for every plane
 };
 
 // Six DFT patches of the tangential E and H components on the faces of a box
@@ -98,6 +108,9 @@ struct dtmx_ctx {
   int probe_cap = 0;
   std::vector<DftHost> dfts;
   std::vector<FluxHost> fluxes;
+  MonTable mon, objmon;         // tables of dfts and of the objective's plane
+  unsigned* d_ticket = nullptr; // blocks of a tail launch that are done
+  float* hist_out = nullptr;    // where the next step's design-region E goes (nullptr: not recorded)
   // state
   long long* d_step = nullptr;
   int* d_flag = nullptr;
@@ -561,6 +574,7 @@ extern "C" int dtmx_create(const dtmx_config* cfg, dtmx_ctx** out) {
   if (!rc) rc = dalloc(ctx, &ctx->d_mt, 1, true);
   if (!rc) rc = dalloc(ctx, &ctx->d_step, 1);
   if (!rc) rc = dalloc(ctx, &ctx->d_flag, 1);
+  if (!rc) rc = dalloc(ctx, &ctx->d_ticket, 1);
   if (!rc) rc = dalloc(ctx, &ctx->d_err, 1);
   for (int comp = 0; comp < 3 && !rc; comp++) rc = dalloc(ctx, &ctx->d_mat[comp], ctx->nstore + 64, true);
   if (!rc) rc = build_maps(ctx);
@@ -600,6 +614,7 @@ extern "C" void dtmx_destroy(dtmx_ctx* ctx) {
   }
   for (auto& d : ctx->dfts) { cudaFree(d.omega); cudaFree(d.acc); cudaFree(d.stage); cudaFree(d.sstep); }
   for (auto& fx : ctx->fluxes) cudaFree(fx.d_out);
+  for (MonTable* m : {&ctx->mon, &ctx->objmon}) { cudaFree(m->tab); cudaFree(m->map); cudaFree(m->unit); }
   cudaFree(ctx->obj.omega); cudaFree(ctx->obj.acc); cudaFree(ctx->obj.stage); cudaFree(ctx->obj.sstep);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -1001,13 +1016,48 @@ extern "C" int dtmx_flux_faces(dtmx_ctx* ctx, int id, int faces[6]) {
   return DTMX_OK;
 }
 
-// fold the staged samples of one DFT plane into its accumulators
-static void dft_flush(dtmx_ctx* ctx, DftHost& h) {
-  if (h.nstaged == 0) return;
-  const long long npts = (long long)h.d.n1 * h.d.n2;
-  dft_flush_kernel<<<(unsigned)((npts + 255) / 256), 256, 0, ctx->stream>>>(h.d, h.nstaged, ctx->cfg.dt);
+// Tables of a set of DFT planes (made once: the planes are fixed from the first step on).
+static int mon_build(dtmx_ctx* ctx, MonTable& m, const DftHost* h, int n) {
+  cudaFree(m.tab); cudaFree(m.map); cudaFree(m.unit);
+  m = MonTable{};
+  std::vector<DftDev> tab;
+  std::vector<int2> map;
+  std::vector<FlushUnit> unit;
+  for (int q = 0; q < n; q++) {
+    const DftDev& d = h[q].d;
+    tab.push_back(d);
+    const int nb = (int)(((long long)d.n1 * d.n2 + 255) / 256);
+    for (int b = 0; b < nb; b++) map.push_back(make_int2(q, b));
+    int slot = 0;
+    for (int c = 0; c < 6; c++) {
+      if (!(d.comp_mask & (1 << c))) continue;
+      for (int f = 0; f < d.nfreq; f += DFT_FCHUNK)
+        for (int b = 0; b < nb; b++) unit.push_back(FlushUnit{q, c, slot, f, b});
+      slot++;
+    }
+  }
+  if (tab.empty()) return DTMX_OK;
+  if (cudaMalloc(&m.tab, tab.size() * sizeof(DftDev)) != cudaSuccess || cudaMalloc(&m.map, map.size() * sizeof(int2)) != cudaSuccess ||
+      cudaMalloc(&m.unit, unit.size() * sizeof(FlushUnit)) != cudaSuccess) {
+    cudaFree(m.tab); cudaFree(m.map); cudaFree(m.unit);
+    m = MonTable{};
+    return fail(ctx, DTMX_ERR_OOM, "DFT tables");
+  }
+  CK(cudaMemcpyAsync(m.tab, tab.data(), tab.size() * sizeof(DftDev), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(m.map, map.data(), map.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(m.unit, unit.data(), unit.size() * sizeof(FlushUnit), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  m.nmap = (int)map.size();
+  m.nunit = (int)unit.size();
+  return DTMX_OK;
+}
+
+// fold the staged samples of a set of planes into their accumulators
+static void dft_flush(dtmx_ctx* ctx, MonTable& m) {
+  if (m.nstaged == 0) return;
+  dft_flush_kernel<<<m.nunit, 256, 0, ctx->stream>>>(m.tab, m.unit, m.nstaged, ctx->cfg.dt);
   ctx->launches++;
-  h.nstaged = 0;
+  m.nstaged = 0;
 }
 
 extern "C" int dtmx_read_dft(dtmx_ctx* ctx, int id, double* out, size_t out_len) {
@@ -1016,7 +1066,7 @@ extern "C" int dtmx_read_dft(dtmx_ctx* ctx, int id, double* out, size_t out_len)
   DftHost& h = ctx->dfts[id];
   const size_t n = (size_t)h.ncomp * h.d.nfreq * h.d.n1 * h.d.n2 * 2;
   if (out_len < n) return fail(ctx, DTMX_ERR_INVALID, "output buffer too small");
-  dft_flush(ctx, h);
+  dft_flush(ctx, ctx->mon);
   CK(cudaStreamSynchronize(ctx->stream));
   CK(cudaMemcpy(out, h.acc, n * sizeof(double), cudaMemcpyDeviceToHost));
   return DTMX_OK;
@@ -1028,9 +1078,9 @@ extern "C" int dtmx_read_flux(dtmx_ctx* ctx, int id, double* out, size_t out_len
   FluxHost& fx = ctx->fluxes[id];
   const int nf = fx.nfreq;
   if (out_len < (size_t)7 * nf) return fail(ctx, DTMX_ERR_INVALID, "output buffer too small");
+  dft_flush(ctx, ctx->mon);
   for (int q = 0; q < 6; q++) {
     DftHost& h = ctx->dfts[fx.face[q]];
-    dft_flush(ctx, h);
     flux_face_kernel<<<nf, FLUX_THREADS, 0, ctx->stream>>>(h.d, fx.sgn_area[q], fx.d_out + (size_t)q * nf);
     ctx->launches++;
   }
@@ -1055,13 +1105,10 @@ extern "C" int dtmx_ntff(dtmx_ctx* ctx, int id, int ndir, const double* theta, c
   if (out_len < (size_t)ndir * nf * 5) return fail(ctx, DTMX_ERR_INVALID, "output buffer too small");
   NtffFaces F{};
   const double ds[3] = {ctx->cfg.dx, ctx->cfg.dy, ctx->cfg.dz};
+  dft_flush(ctx, ctx->mon);
   for (int q = 0; q < 6; q++) {
-    DftHost& h = ctx->dfts[fx.ffe[q]];
-    dft_flush(ctx, h);
-    F.f[q] = h.d;
-    DftHost& h2 = ctx->dfts[fx.ffh[q]];
-    dft_flush(ctx, h2);
-    F.h[q] = h2.d;
+    F.f[q] = ctx->dfts[fx.ffe[q]].d;
+    F.h[q] = ctx->dfts[fx.ffh[q]].d;
   }
   for (int a = 0; a < 3; a++) {
     F.ds[a] = ds[a];
@@ -1111,6 +1158,49 @@ static int set_kernel_attributes() {
   cudaFuncSetAttribute(e_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Pipe<4, false>::SMEM_BYTES);
   done = true;
   return 0;
+}
+
+// The end of a step in one launch (two while the adjoint's objective is
+// recorded next to other DFT planes): soft sources, probes, DFT samples, the
+// design region's history, the step counter.  P.f is the state after the step.
+static long long launch_tail(dtmx_ctx* ctx, const Params& P, cudaStream_t st) {
+  const dtmx_config& c = ctx->cfg;
+  long long nl = 0;
+  TailArgs a{};
+  a.dt = c.dt;
+  a.ticket = ctx->d_ticket;
+  const int ns = (int)ctx->psrc.size();
+  if (ns > TAIL_SRC) {
+    point_source_kernel<<<(ns + 63) / 64, 64, 0, st>>>(P, ctx->d_psrc, ns, ctx->d_step, c.dt);
+    nl++;
+  } else {
+    a.src = ctx->d_psrc; a.ns = ns;
+  }
+  MonTable* sets[2] = {!ctx->monitors_off && ctx->mon.nmap ? &ctx->mon : nullptr, ctx->obj_on ? &ctx->objmon : nullptr};
+  if (!sets[0]) { sets[0] = sets[1]; sets[1] = nullptr; }
+  for (int q = 0; q < 2; q++) {
+    if (q == 1 && !sets[1]) break;
+    MonTable* m = sets[q];
+    const bool end = q == 1 || !sets[1];
+    TailArgs b = a;
+    if (q == 0 && !ctx->probes.empty() && !ctx->monitors_off) {
+      b.pr = ctx->d_probes; b.np = (int)ctx->probes.size();
+      b.traces = ctx->d_traces; b.cap = ctx->probe_cap;
+      b.every = c.probe_every > 0 ? c.probe_every : 1;
+    }
+    if (q == 1) b.ns = 0;                          // (the first launch has added the sources)
+    if (m) { b.dft = m->tab; b.map = m->map; b.nmap = m->nmap; b.slot = m->nstaged; }
+    if (end) {
+      b.hist = ctx->hist_out;
+      b.nd = P.des_on ? P.des_n[0] * P.des_n[1] * P.des_n[2] : 0;
+      b.advance = 1;
+    }
+    const int blocks = std::max(1, b.nmap + (b.hist ? (3 * b.nd + 255) / 256 : 0));
+    tail_kernel<<<blocks, 256, 0, st>>>(P, b, ctx->d_step);
+    nl++;
+    if (m && ++m->nstaged == DFT_STAGE) dft_flush(ctx, *m);
+  }
+  return nl;
 }
 
 static int launch_step(dtmx_ctx* ctx) {
@@ -1174,10 +1264,6 @@ static int launch_step(dtmx_ctx* ctx) {
     ctx->prof_ms_h += a; ctx->prof_ms_e += b; ctx->prof_count++;
   }
   nl++;
-  if (!ctx->psrc.empty()) {
-    point_source_kernel<<<((int)ctx->psrc.size() + 63) / 64, 64, 0, st>>>(P, ctx->d_psrc, (int)ctx->psrc.size(), ctx->d_step, c.dt);
-    nl++;
-  }
   if (ctx->has_tfsf) {
     if (o4) tfsf_kernel<4><<<tgrid[0], 256, 0, st>>>(P, ctx->T, ctx->d_step, 0);
     else tfsf_kernel<2><<<tgrid[0], 256, 0, st>>>(P, ctx->T, ctx->d_step, 0);
@@ -1189,28 +1275,7 @@ static int launch_step(dtmx_ctx* ctx) {
     else line_e_kernel<2><<<8, 256, 0, st>>>(ctx->line_e, ctx->line_h, ctx->T.line_n, r1, ctx->line_src, ctx->d_step, c.dt, s.amp, s.f0, s.tau, s.t0);
     nl++;
   }
-  if (!ctx->probes.empty() && !ctx->monitors_off) {
-    const int every = c.probe_every > 0 ? c.probe_every : 1;
-    probe_kernel<<<((int)ctx->probes.size() + 127) / 128, 128, 0, st>>>(P, ctx->d_probes, (int)ctx->probes.size(), ctx->d_traces,
-                                                                       ctx->probe_cap, ctx->d_step, every);
-    nl++;
-  }
-  for (auto& d : ctx->dfts) {
-    if (ctx->monitors_off) break;
-    const long long npts = (long long)d.d.n1 * d.d.n2;
-    dft_capture_kernel<<<(unsigned)((npts + 255) / 256), 256, 0, st>>>(P, d.d, ctx->d_step, d.nstaged);
-    nl++;
-    if (++d.nstaged == DFT_STAGE) dft_flush(ctx, d);
-  }
-  if (ctx->obj_on) {
-    DftHost& d = ctx->obj;
-    const long long npts = (long long)d.d.n1 * d.d.n2;
-    dft_capture_kernel<<<(unsigned)((npts + 255) / 256), 256, 0, st>>>(P, d.d, ctx->d_step, d.nstaged);
-    nl++;
-    if (++d.nstaged == DFT_STAGE) dft_flush(ctx, d);
-  }
-  advance_step_kernel<<<1, 1, 0, st>>>(ctx->d_step);
-  nl++;
+  nl += launch_tail(ctx, P, st);
   ctx->launches += nl;
   return DTMX_OK;
 }
@@ -1229,6 +1294,7 @@ static int prepare(dtmx_ctx* ctx) {
     CK(cudaMemcpyAsync(ctx->d_probes, ctx->probes.data(), ctx->probes.size() * sizeof(ProbeDev), cudaMemcpyHostToDevice, ctx->stream));
     if ((rc = dalloc(ctx, &ctx->d_traces, ctx->probes.size() * (size_t)ctx->probe_cap))) return rc;
   }
+  if ((rc = mon_build(ctx, ctx->mon, ctx->dfts.data(), (int)ctx->dfts.size()))) return rc;
   if (ctx->has_tfsf && ctx->h_mat[0].size()) {
     // every E node that gets a correction, and the E nodes next to them, must be non-dispersive
     const TfsfDev& T = ctx->T;
@@ -1543,38 +1609,13 @@ static int launch_fused_step(dtmx_ctx* ctx) {
     cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]);
     ctx->prof_ms_h += a; ctx->prof_count++;
   }
-  if (!ctx->psrc.empty()) {
-    point_source_kernel<<<((int)ctx->psrc.size() + 63) / 64, 64, 0, st>>>(PB, ctx->d_psrc, (int)ctx->psrc.size(), ctx->d_step, c.dt);
-    nl++;
-  }
   if (ctx->has_tfsf) { tfsf_kernel<2><<<tgrid[0], 256, 0, st>>>(PB, ctx->T, ctx->d_step, 0); nl++; }
   if (pw) {
     const dtmx_tfsf& s = ctx->tfsf;
     line_e_kernel<2><<<8, 256, 0, st>>>(ctx->line_e, ctx->line_h, ctx->T.line_n, r1, ctx->line_src, ctx->d_step, c.dt, s.amp, s.f0, s.tau, s.t0);
     nl++;
   }
-  if (!ctx->probes.empty() && !ctx->monitors_off) {
-    const int every = c.probe_every > 0 ? c.probe_every : 1;
-    probe_kernel<<<((int)ctx->probes.size() + 127) / 128, 128, 0, st>>>(PB, ctx->d_probes, (int)ctx->probes.size(), ctx->d_traces,
-                                                                       ctx->probe_cap, ctx->d_step, every);
-    nl++;
-  }
-  for (auto& d : ctx->dfts) {
-    if (ctx->monitors_off) break;
-    const long long npts = (long long)d.d.n1 * d.d.n2;
-    dft_capture_kernel<<<(unsigned)((npts + 255) / 256), 256, 0, st>>>(PB, d.d, ctx->d_step, d.nstaged);
-    nl++;
-    if (++d.nstaged == DFT_STAGE) dft_flush(ctx, d);
-  }
-  if (ctx->obj_on) {
-    DftHost& d = ctx->obj;
-    const long long npts = (long long)d.d.n1 * d.d.n2;
-    dft_capture_kernel<<<(unsigned)((npts + 255) / 256), 256, 0, st>>>(PB, d.d, ctx->d_step, d.nstaged);
-    nl++;
-    if (++d.nstaged == DFT_STAGE) dft_flush(ctx, d);
-  }
-  advance_step_kernel<<<1, 1, 0, st>>>(ctx->d_step);
-  nl++;
+  nl += launch_tail(ctx, PB, st);
   ctx->launches += nl;
   fused_swap(ctx);
   return DTMX_OK;
@@ -1620,8 +1661,7 @@ static int graph_steps16(dtmx_ctx* ctx) {
     if (step_engine(ctx) == 3) { int rc = fused_prepare(ctx); if (rc) return rc; }
     const long long launches0 = ctx->launches;
     const int gcur0 = ctx->gcur;
-    std::vector<int> staged0;
-    for (auto& d : ctx->dfts) staged0.push_back(d.nstaged);
+    const int staged0 = ctx->mon.nstaged;
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
       return fail(ctx, DTMX_ERR_CUDA, "graph capture could not start");
@@ -1634,8 +1674,7 @@ static int graph_steps16(dtmx_ctx* ctx) {
     if (e != cudaSuccess) { ctx->graph16[par] = nullptr; cudaGetLastError(); return fail(ctx, DTMX_ERR_CUDA, "graph instantiation failed"); }
     // the capture ran the bookkeeping of 16 steps; the graph below executes them
     if (ctx->gcur != gcur0 || ctx->parity != par) return fail(ctx, DTMX_ERR_STATE, "graph capture: unexpected buffer parity");
-    for (size_t q = 0; q < ctx->dfts.size(); q++)
-      if (ctx->dfts[q].nstaged != staged0[q]) return fail(ctx, DTMX_ERR_STATE, "graph capture: staging not aligned");
+    if (ctx->mon.nstaged != staged0) return fail(ctx, DTMX_ERR_STATE, "graph capture: staging not aligned");
     ctx->graph_launches[par] = ctx->launches - launches0;
   } else {
     ctx->launches += ctx->graph_launches[par];
@@ -1669,8 +1708,7 @@ extern "C" int dtmx_step(dtmx_ctx* ctx, int nsteps) {
     // (the captured sequence then repeats exactly: staging slots, the flush
     // every 16 steps and the gyrotropic buffer parity)
     bool aligned = left >= 16 && !ctx->profiling && !ctx->monitors_off && ctx->engine != 2;
-    for (auto& d : ctx->dfts) aligned = aligned && d.nstaged == 0;
-    if (ctx->obj_on) aligned = aligned && ctx->obj.nstaged == 0;
+    aligned = aligned && ctx->mon.nstaged == 0;
     if (aligned && !ctx->obj_on) {
       int rc = graph_steps16(ctx);
       if (rc) return rc;
@@ -1858,10 +1896,11 @@ static int fa_begin(dtmx_ctx* ctx, FaRun& R, int nsteps, int checkpoint_every, i
         cudaMalloc(&O.stage, (size_t)DFT_STAGE * 4 * R.npl * 4) != cudaSuccess || cudaMalloc(&O.sstep, DFT_STAGE * 8) != cudaSuccess)
       return fail(ctx, DTMX_ERR_OOM, "objective DFT allocation");
     O.d.omega = O.omega; O.d.acc = O.acc; O.d.stage = O.stage; O.d.sstep = O.sstep;
+    if ((rc = mon_build(ctx, ctx->objmon, &O, 1))) return rc;
   }
   CK(cudaMemcpyAsync(O.omega, &omega, 8, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(O.acc, 0, (size_t)4 * R.npl * sizeof(double2), ctx->stream));
-  O.nstaged = 0;
+  ctx->objmon.nstaged = 0;
   if (full) {
     // design-region history of every step: slot s holds E after s steps of the run
     void* h = R.take(ctx, (size_t)(R.N + 1) * 3 * R.nd * 4);
@@ -1892,13 +1931,11 @@ static int fa_forward(dtmx_ctx* ctx, FaRun& R, int st) {
   } else if (st % R.K == 0) {
     state_copy(ctx, R.ck[st / R.K], true);
   }
+  if (R.full) ctx->hist_out = R.hist + (size_t)(st + 1) * 3 * R.nd;
   int rc = launch_one(ctx);
+  ctx->hist_out = nullptr;
   if (rc) return rc;
   ctx->step++;
-  if (R.full) {
-    design_capture_kernel<<<design_blocks(R), 256, 0, ctx->stream>>>(ctx->P, R.hist, st + 1, R.nd);
-    ctx->launches++;
-  }
   return DTMX_OK;
 }
 
@@ -1908,7 +1945,7 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
   ctx->obj_on = false;
   if (!R.full) state_copy(ctx, R.ck[R.nseg], true);
   DftHost& O = ctx->obj;
-  dft_flush(ctx, O);
+  dft_flush(ctx, ctx->objmon);
   std::vector<double> F((size_t)8 * R.npl);
   CK(cudaMemcpyAsync(F.data(), O.acc, F.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1975,10 +2012,11 @@ static int fa_segment_begin(dtmx_ctx* ctx, FaRun& R, int seg) {
 // recompute step q (1..len) of the current segment
 static int fa_recompute(dtmx_ctx* ctx, FaRun& R, int q) {
   if (R.full) return DTMX_OK;
+  ctx->hist_out = R.hist + (size_t)q * 3 * R.nd;
   int rc = launch_one(ctx);
+  ctx->hist_out = nullptr;
   if (rc) return rc;
   ctx->step++;
-  design_capture_kernel<<<design_blocks(R), 256, 0, ctx->stream>>>(ctx->P, R.hist, q, R.nd);
   return DTMX_OK;
 }
 

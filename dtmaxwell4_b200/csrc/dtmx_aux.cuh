@@ -217,49 +217,25 @@ __global__ void line_e_kernel(double* e, const double* h, int n, double r, int s
 struct PointSrcDev {
   int comp; long long id; double amp, f0, tau, t0;
 };
+__device__ __forceinline__ float source_value(const PointSrcDev& s, long long n, double dt) {
+  const double u = ((double)n + 0.5) * dt - s.t0;
+  return (float)(s.amp * sin(2.0 * M_PI * s.f0 * u) * exp(-(u / s.tau) * (u / s.tau)));
+}
 
+// More soft sources than the tail kernel's list holds.  Sources on one node are
+// added in their order by the first of them.
 __global__ void point_source_kernel(Params p, const PointSrcDev* s, int ns, const long long* d_step, double dt) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= ns) return;
-  const double u = ((double)(*d_step) + 0.5) * dt - s[q].t0;
-  const double v = s[q].amp * sin(2.0 * M_PI * s[q].f0 * u) * exp(-(u / s[q].tau) * (u / s[q].tau));
-  p.f[s[q].comp][s[q].id] += (float)v;
+  for (int e = 0; e < q; e++)
+    if (s[e].comp == s[q].comp && s[e].id == s[q].id) return;
+  float v = p.f[s[q].comp][s[q].id];
+  for (int e = q; e < ns; e++)
+    if (s[e].comp == s[q].comp && s[e].id == s[q].id) v += source_value(s[e], *d_step, dt);
+  p.f[s[q].comp][s[q].id] = v;
 }
 
 struct ProbeDev { int comp, i, j, k, mode; };
-
-__device__ __forceinline__ float probe_get(const Params& p, int c, int i, int j, int k) {
-  if (i < 0 || i >= p.g.n[0] || j < 0 || j >= p.g.n[1] || k < 0 || k >= p.g.n[2]) return 0.f;
-  return p.f[c][(long long)i * p.g.sx + (long long)j * p.g.sy + k];
-}
-
-// Reference Sensor::write averaging (sensor.h:51-83); for Hz the reference's
-// second point is never assigned and reads a zero node outside the domain.
-__global__ void probe_kernel(Params p, const ProbeDev* pr, int np, float* traces, int cap, const long long* d_step,
-                             int every) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const long long s = *d_step + 1;
-  if (q >= np || (s % every) != 0) return;
-  const long long sample = s / every - 1;
-  if (sample >= cap) return;
-  const ProbeDev d = pr[q];
-  const int c = d.comp, x = d.i, y = d.j, z = d.k;
-  float v;
-  if (d.mode == 0) {
-    v = probe_get(p, c, x, y, z);
-  } else {
-    const int zM = z == 0 ? z + 1 : z - 1;
-    switch (c) {
-      case 0: v = 0.25f * (probe_get(p, c, x, y - 1, zM) + probe_get(p, c, x, y - 1, z) + probe_get(p, c, x, y, zM) + probe_get(p, c, x, y, z)); break;
-      case 1: v = 0.25f * (probe_get(p, c, x - 1, y, zM) + probe_get(p, c, x - 1, y, z) + probe_get(p, c, x, y, zM) + probe_get(p, c, x, y, z)); break;
-      case 2: v = 0.25f * (probe_get(p, c, x - 1, y - 1, z) + probe_get(p, c, x - 1, y, z) + probe_get(p, c, x, y - 1, z) + probe_get(p, c, x, y, z)); break;
-      case 3: v = 0.5f * (probe_get(p, c, x - 1, y, z) + probe_get(p, c, x, y, z)); break;
-      case 4: v = 0.5f * (probe_get(p, c, x, y - 1, z) + probe_get(p, c, x, y, z)); break;
-      default: v = 0.5f * probe_get(p, c, x, y, zM); break;
-    }
-  }
-  traces[(long long)q * cap + sample] = v;
-}
 
 struct DftDev {
   int axis, index, comp_mask, nfreq, n1, n2;
@@ -271,70 +247,173 @@ struct DftDev {
 };
 constexpr int DFT_STAGE = 16;
 
-// Running DFT with FP64 accumulators: acc += f(t) exp(-i w t) dt, t = s*dt for E,
-// (s-1/2)*dt for H, s = steps completed.  Every step stages the plane's values
-// (dft_capture_kernel); every DFT_STAGE steps dft_flush_kernel folds the staged
-// samples into the accumulators in step order, so the accumulator update
-// sequence (and its rounding) is that of a per-step update while the
-// accumulators are read and written once per DFT_STAGE steps.
-__global__ void dft_capture_kernel(Params p, DftDev d, const long long* d_step, int slot) {
-  const long long npts = (long long)d.n1 * d.n2;
-  const long long pt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (pt == 0) d.sstep[slot] = *d_step + 1;
-  if (pt >= npts) return;
-  const int u = d.lo1 + (int)(pt / d.n2), v = d.lo2 + (int)(pt % d.n2);
-  int i, j, k;
-  if (d.axis == 0) { i = d.index; j = u; k = v; }
-  else if (d.axis == 1) { i = u; j = d.index; k = v; }
-  else { i = u; j = v; k = d.index; }
+// ---- the end of a time step in one launch: soft sources, probes, DFT samples,
+// the design region's history and the step counter.  Each of them is small
+// (1 to 4 us as a launch of its own, 4.6 us a step together for a dipole run
+// with probes, 52 us for a flux box' 18 windows), so they share one: a block
+// map assigns the blocks to the DFT planes.
+// A source changes a node that a sample may read in the same launch.  So the
+// blocks read the fields as they are and add the sources of the node they
+// read; the block that finishes last (a ticket) adds them to the fields, after
+// every read, and advances the step counter.
+constexpr int TAIL_SRC = 32;
+struct TailArgs {
+  const PointSrcDev* src; int ns; double dt;
+  const ProbeDev* pr; int np; float* traces; int cap; int every;
+  const DftDev* dft; const int2* map; int nmap; int slot;      // map[block] = {plane, its block of 256 points}
+  float* hist; int nd;                                         // design-region E of this step (nullptr: none)
+  unsigned* ticket;
+  int advance;
+};
+struct TailSources { float v[TAIL_SRC]; long long id[TAIL_SRC]; int comp[TAIL_SRC]; };
+
+__device__ __forceinline__ float tail_get(const Params& p, const TailSources& s, int ns, int c, int i, int j, int k) {
+  if (i < 0 || i >= p.g.n[0] || j < 0 || j >= p.g.n[1] || k < 0 || k >= p.g.n[2]) return 0.f;
   const long long id = (long long)i * p.g.sx + (long long)j * p.g.sy + k;
-  int ci = 0;
-  const int ncomp = __popc(d.comp_mask);
-  for (int c = 0; c < 6; c++) {
-    if (!(d.comp_mask & (1 << c))) continue;
-    d.stage[((long long)slot * ncomp + ci) * npts + pt] = p.f[c][id];
-    ci++;
+  float v = p.f[c][id];
+  for (int q = 0; q < ns; q++)
+    if (s.comp[q] == c && s.id[q] == id) v += s.v[q];
+  return v;
+}
+
+// Reference Sensor::write averaging (sensor.h:51-83); for Hz the reference's
+// second point is never assigned and reads a zero node outside the domain.
+__device__ __forceinline__ float tail_probe(const Params& p, const TailSources& s, int ns, const ProbeDev& d) {
+  const int c = d.comp, x = d.i, y = d.j, z = d.k;
+  if (d.mode == 0) return tail_get(p, s, ns, c, x, y, z);
+  const int zM = z == 0 ? z + 1 : z - 1;
+  auto get = [&](int i, int j, int k) { return tail_get(p, s, ns, c, i, j, k); };
+  switch (c) {
+    case 0: return 0.25f * (get(x, y - 1, zM) + get(x, y - 1, z) + get(x, y, zM) + get(x, y, z));
+    case 1: return 0.25f * (get(x - 1, y, zM) + get(x - 1, y, z) + get(x, y, zM) + get(x, y, z));
+    case 2: return 0.25f * (get(x - 1, y - 1, z) + get(x - 1, y, z) + get(x, y - 1, z) + get(x, y, z));
+    case 3: return 0.5f * (get(x - 1, y, z) + get(x, y, z));
+    case 4: return 0.5f * (get(x, y - 1, z) + get(x, y, z));
+    default: return 0.5f * get(x, y, zM);
   }
 }
 
-__global__ void __launch_bounds__(256) dft_flush_kernel(DftDev d, int nslots, double dt) {
-  __shared__ double2 phE[DFT_STAGE][64], phH[DFT_STAGE][64];
-  for (int q = threadIdx.x; q < nslots * d.nfreq; q += blockDim.x) {
-    const int sl = q / d.nfreq, f = q - sl * d.nfreq;
-    const long long s = d.sstep[sl];
-    double sn, cs;
-    sincos(d.omega[f] * (double)s * dt, &sn, &cs);
-    phE[sl][f] = make_double2(cs * dt, -sn * dt);
-    sincos(d.omega[f] * ((double)s - 0.5) * dt, &sn, &cs);
-    phH[sl][f] = make_double2(cs * dt, -sn * dt);
+__global__ void __launch_bounds__(256) tail_kernel(const __grid_constant__ Params p, const __grid_constant__ TailArgs a, long long* d_step) {
+  __shared__ TailSources s;
+  __shared__ bool last;
+  const int tid = threadIdx.x, b = blockIdx.x;
+  const long long n = *d_step;
+  if (tid < a.ns) {
+    const PointSrcDev& q = a.src[tid];
+    s.v[tid] = source_value(q, n, a.dt);
+    s.id[tid] = q.id;
+    s.comp[tid] = q.comp;
   }
   __syncthreads();
-  const long long npts = (long long)d.n1 * d.n2;
-  const long long pt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (pt >= npts) return;
-  const int ncomp = __popc(d.comp_mask);
-  int ci = 0;
-  for (int c = 0; c < 6; c++) {
-    if (!(d.comp_mask & (1 << c))) continue;
-    double val[DFT_STAGE];
-#pragma unroll
-    for (int sl = 0; sl < DFT_STAGE; sl++)
-      val[sl] = sl < nslots ? (double)d.stage[((long long)sl * ncomp + ci) * npts + pt] : 0.0;
-    const double2(*ph)[64] = c < 3 ? phE : phH;
-    double2* acc = d.acc + (long long)ci * d.nfreq * npts + pt;
-    for (int f = 0; f < d.nfreq; f++) {
-      double2 a = acc[(long long)f * npts];
-#pragma unroll
-      for (int sl = 0; sl < DFT_STAGE; sl++) {
-        if (sl < nslots) {
-          a.x += val[sl] * ph[sl][f].x;
-          a.y += val[sl] * ph[sl][f].y;
-        }
-      }
-      acc[(long long)f * npts] = a;
-    }
-    ci++;
+  if (b == 0 && a.np > 0 && (n + 1) % a.every == 0) {
+    const long long sample = (n + 1) / a.every - 1;
+    if (sample < a.cap)
+      for (int q = tid; q < a.np; q += blockDim.x) a.traces[(long long)q * a.cap + sample] = tail_probe(p, s, a.ns, a.pr[q]);
   }
+  if (b < a.nmap) {
+    const int2 e = a.map[b];
+    const DftDev& d = a.dft[e.x];
+    const int npts = d.n1 * d.n2, n2 = d.n2, mask = d.comp_mask, ncomp = __popc(mask);
+    const int pt = e.y * 256 + tid;
+    if (pt == 0) d.sstep[a.slot] = n + 1;
+    if (pt < npts) {
+      const int u = d.lo1 + pt / n2, v = d.lo2 + pt % n2, axis = d.axis;
+      const int i = axis == 0 ? d.index : u, j = axis == 0 ? u : axis == 1 ? d.index : v, k = axis == 2 ? d.index : v;
+      float* out = d.stage + (long long)a.slot * ncomp * npts + pt;
+      int ci = 0;
+#pragma unroll
+      for (int c = 0; c < 6; c++)
+        if (mask & (1 << c)) out[(long long)(ci++) * npts] = tail_get(p, s, a.ns, c, i, j, k);
+    }
+  } else if (a.hist && b - a.nmap < (3 * a.nd + 255) / 256) {
+    const int q = (b - a.nmap) * 256 + tid;
+    if (q < 3 * a.nd) {
+      const int c = q / a.nd, di = q - c * a.nd;
+      const int i = p.des_lo[0] + di / (p.des_n[1] * p.des_n[2]);
+      const int j = p.des_lo[1] + (di / p.des_n[2]) % p.des_n[1];
+      const int k = p.des_lo[2] + di % p.des_n[2];
+      a.hist[q] = p.f[c][(long long)i * p.g.sx + (long long)j * p.g.sy + k];   // (no source lies in the design region)
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    last = true;
+    if (gridDim.x > 1) {
+      __threadfence();
+      last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  if (tid < a.ns) {
+    // sources on one node are added in their order by the first of them
+    bool first = true;
+    for (int q = 0; q < tid; q++) first = first && !(s.comp[q] == s.comp[tid] && s.id[q] == s.id[tid]);
+    if (first) {
+      float v = p.f[s.comp[tid]][s.id[tid]];
+      for (int q = tid; q < a.ns; q++)
+        if (s.comp[q] == s.comp[tid] && s.id[q] == s.id[tid]) v += s.v[q];
+      p.f[s.comp[tid]][s.id[tid]] = v;
+    }
+  }
+  if (tid == 0) {
+    if (gridDim.x > 1) *a.ticket = 0u;
+    if (a.advance) *d_step = n + 1;
+  }
+}
+
+// Running DFT with FP64 accumulators: acc += f(t) exp(-i w t) dt, t = s*dt for E,
+// (s-1/2)*dt for H, s = steps completed.  Every step stages the planes' values
+// (tail_kernel); every DFT_STAGE steps dft_flush_kernel folds the staged
+// samples into the accumulators in step order, so the accumulator update
+// sequence (and its rounding) is that of a per-step update while the
+// accumulators are read and written once per DFT_STAGE steps.
+// One launch for all planes: a block takes 256 points of one component and up
+// to DFT_FCHUNK frequencies, from a map made once.  (A launch per plane with
+// all components and frequencies in one thread took 74 us for each of a flux
+// box' 18 windows of 41^2 points and 32 frequencies, seven blocks wide, and 119
+// us for a 384^2 plane of 4 components and 16 frequencies, whose accumulators'
+// bytes take 47.)
+constexpr int DFT_FCHUNK = 8;
+struct FlushUnit { int plane, comp, slot, f0, ptb; };
+__global__ void __launch_bounds__(256) dft_flush_kernel(const DftDev* tab, const FlushUnit* unit, int nslots, double dt) {
+  __shared__ double2 ph[DFT_STAGE][DFT_FCHUNK];
+  const FlushUnit u = unit[blockIdx.x];
+  const DftDev& d = tab[u.plane];
+  const int nf = min(DFT_FCHUNK, d.nfreq - u.f0);
+  if (threadIdx.x < DFT_STAGE * DFT_FCHUNK) {
+    const int sl = threadIdx.x / DFT_FCHUNK, f = threadIdx.x % DFT_FCHUNK;
+    if (sl < nslots && f < nf) {
+      const double t = (double)d.sstep[sl] - (u.comp < 3 ? 0.0 : 0.5);
+      double sn, cs;
+      sincos(d.omega[u.f0 + f] * t * dt, &sn, &cs);
+      ph[sl][f] = make_double2(cs * dt, -sn * dt);
+    }
+  }
+  __syncthreads();
+  const int npts = d.n1 * d.n2, ncomp = __popc(d.comp_mask);
+  const int pt = u.ptb * 256 + threadIdx.x;
+  if (pt >= npts) return;
+  float val[DFT_STAGE];
+  const float* st = d.stage + (long long)u.slot * npts + pt;
+#pragma unroll
+  for (int sl = 0; sl < DFT_STAGE; sl++) val[sl] = sl < nslots ? st[(long long)sl * ncomp * npts] : 0.f;
+  double2* acc = d.acc + ((long long)u.slot * d.nfreq + u.f0) * npts + pt;
+  double2 v[DFT_FCHUNK];
+#pragma unroll
+  for (int f = 0; f < DFT_FCHUNK; f++)
+    if (f < nf) v[f] = acc[(long long)f * npts];
+#pragma unroll
+  for (int sl = 0; sl < DFT_STAGE; sl++)
+    if (sl < nslots) {
+      const double x = (double)val[sl];
+#pragma unroll
+      for (int f = 0; f < DFT_FCHUNK; f++)
+        if (f < nf) { v[f].x += x * ph[sl][f].x; v[f].y += x * ph[sl][f].y; }
+    }
+#pragma unroll
+  for (int f = 0; f < DFT_FCHUNK; f++)
+    if (f < nf) acc[(long long)f * npts] = v[f];
 }
 
 // Outward Poynting flux of one face of a flux box at every frequency of its
@@ -606,8 +685,6 @@ __global__ void mask_nonlive_kernel(Params p, int comp, long long ncell) {
     if (!is_live(p.g, comp, i, j, k)) p.f[comp][(long long)i * p.g.sx + (long long)j * p.g.sy + k] = 0.f;
   }
 }
-
-__global__ void advance_step_kernel(long long* d_step) { *d_step += 1; }
 
 __global__ void nonfinite_kernel(Params p, int comp, long long ncell, int* flag) {
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < ncell; q += (long long)gridDim.x * blockDim.x) {

@@ -1,0 +1,81 @@
+"""The end of a step in one launch (sources, probes, DFT samples, step counter)
+and the one-launch DFT fold, against the FP64 oracle: sources on sampled and
+probed nodes, several on one node, more sources than the launch's list holds
+(32), windows of one point and around a block of 256, frequencies around a
+chunk of 8, and reads in the middle of a 16-step cycle.
+
+Tolerance: 1e-5 of the strongest trace / of the spectrum, the bound of the
+other GPU-against-oracle tests for runs of this length.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+N = (24, 20, 37)
+
+
+def _setup(sim, nsrc, nfreq):
+    from dtmaxwell4_b200 import abi
+    rng = np.random.default_rng(9)
+    at = [(abi.EZ, 12, 10, 18), (abi.EZ, 12, 10, 18), (abi.EY, 12, 11, 19)]
+    while len(at) < nsrc:
+        at.append((int(rng.integers(3)),) + tuple(int(rng.integers(6, m - 6)) for m in N))
+    for q, (c, i, j, k) in enumerate(at[:nsrc]):
+        sim.add_point_source(abi.PointSource(comp=c, i=i, j=j, k=k, waveform=abi.WAVE_GAUSS_SINE, amp=1.0 + 0.1 * q, f0=0.05,
+                                             tau=15.0, t0=10.0 + q))
+    for p in ((abi.EZ, 12, 10, 18, 0), (abi.EY, 12, 11, 19, 0), (abi.HX, 9, 9, 9, 0), (abi.EZ, 13, 11, 18, 1)):
+        sim.add_probe(*p)
+    om = list(2 * np.pi * np.linspace(0.02, 0.08, nfreq))
+    ids = [sim.add_dft_plane(0, 12, (1 << abi.EY) | (1 << abi.EZ) | (1 << abi.HZ), om)]         # 740 points
+    return ids, om
+
+
+@pytest.mark.parametrize("nsrc,nfreq", [(1, 1), (3, 8), (32, 9), (40, 64)])
+def test_sources_probes_and_spectra(nsrc, nfreq):
+    import pyoracle
+    from dtmaxwell4_b200 import Simulation, abi
+    cfg = abi.make_config(*N, courant=0.5, pml=5, probe_capacity=128)
+    g, o = Simulation(cfg), pyoracle.OracleSim(cfg)
+    gid, om = _setup(g, nsrc, nfreq)
+    oid, _ = _setup(o, nsrc, nfreq)
+    steps = 45                                    # two whole cycles and 13 steps of a third
+    g.step(steps)
+    o.step(steps)
+    tg, to = g.read_probes(), o.read_probes(128)
+    assert tg.shape == to.shape
+    assert np.abs(tg - to).max() <= 1e-5 * np.abs(to).max()
+    dg, do = g.read_dft(gid[0]), o.read_dft(oid[0])
+    assert np.linalg.norm(dg - do) <= 1e-5 * np.linalg.norm(do)
+    g.close()
+
+
+@pytest.mark.parametrize("window", [(3, 1, 4, 1), (2, 5, 1, 51), (2, 16, 3, 16), (0, 20, 7, 13)])
+def test_windows_and_reads_mid_cycle(window):
+    """Windows of 1, 255, 256 and 260 points next to a plane of other size; a
+    read after 5 steps folds early and changes nothing."""
+    from dtmaxwell4_b200 import Simulation, abi
+    lo1, n1, lo2, n2 = window
+    n = (20, 22, 60)
+    cfg = abi.make_config(*n, courant=0.5, pml=4)
+    rng = np.random.default_rng(1)
+    fields = [rng.standard_normal(n).astype(np.float32) for _ in range(6)]
+    om = list(np.linspace(0.1, 0.4, 9))
+    mask = (1 << abi.EX) | (1 << abi.HY)
+    got = []
+    for split in ((37,), (5, 32), (16, 21)):
+        s = Simulation(cfg)
+        w = s.add_dft_patch(0, 9, lo1, n1, lo2, n2, mask, om)
+        a = s.add_dft_plane(0, 9, mask, om)
+        b = s.add_dft_plane(2, 30, 1 << abi.EZ, om[:3])
+        for c in range(6):
+            s.set_field(c, fields[c])
+        for q in split:
+            s.step(q)
+            out = (s.read_dft(w), s.read_dft(a), s.read_dft(b))
+        got.append(out)
+        assert np.array_equal(out[0], out[1][:, :, lo1:lo1 + n1, lo2:lo2 + n2])
+        s.close()
+    for out in got[1:]:
+        for x, y in zip(out, got[0]):
+            assert np.array_equal(x, y)
