@@ -384,9 +384,9 @@ class Simulation:
 
     def read_dft(self, did):
         ncomp, nf, n1, n2 = self._dft[did]
-        out = np.zeros((ncomp, nf, n1, n2, 2), dtype=np.float64)
-        self._ck(self._L.dtmx_read_dft(self._h, did, out.ctypes.data, out.size))
-        return out[..., 0] + 1j * out[..., 1]
+        out = np.empty((ncomp, nf, n1, n2), dtype=np.complex128)
+        self._ck(self._L.dtmx_read_dft(self._h, did, out.ctypes.data, 2 * out.size))
+        return out
 
     def stream_handle(self):
         """cudaStream_t of the context (for torch.cuda.ExternalStream)."""

@@ -1,0 +1,70 @@
+"""Fields and spectra between the device and host memory of every kind: rows
+that are padded on the device, more than one piece of the threaded read (1 MB
+pieces from 4 MB on), pinned memory, and reads of two contexts at once."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [(9, 8, 11), (64, 161, 103), (40, 64, 512), (1100, 33, 31)])
+def test_field_roundtrip(n):
+    import torch
+    from dtmaxwell4_b200 import Simulation, abi
+    s = Simulation(abi.make_config(*n, absorber=abi.ABS_NONE, pml=0))
+    rng = np.random.default_rng(4)
+    a = [rng.standard_normal(n).astype(np.float32) for _ in range(2)]
+    for c in (0, 4):
+        s.set_field(c, a[c // 4])
+    pinned = torch.empty(n, dtype=torch.float32).pin_memory().numpy()
+    for c in (0, 4):
+        assert np.array_equal(s.get_field(c), a[c // 4])
+        assert np.array_equal(s.get_field(c, out=pinned), a[c // 4])
+    assert not s.get_field(1).any()
+    s.close()
+
+
+def test_two_contexts_read_at_once():
+    from dtmaxwell4_b200 import Simulation, abi
+    n = (48, 150, 170)
+    rng = np.random.default_rng(6)
+    sims, want, got = [], [], [None, None]
+    for q in range(2):
+        s = Simulation(abi.make_config(*n, absorber=abi.ABS_NONE, pml=0))
+        want.append(rng.standard_normal(n).astype(np.float32))
+        s.set_field(2, want[q])
+        sims.append(s)
+
+    def read(q):
+        for _ in range(8):
+            got[q] = sims[q].get_field(2)
+            if not np.array_equal(got[q], want[q]):
+                return
+    th = [threading.Thread(target=read, args=(q,)) for q in range(2)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    for q in range(2):
+        assert np.array_equal(got[q], want[q])
+        sims[q].close()
+
+
+def test_spectra_are_complex_arrays():
+    from dtmaxwell4_b200 import Simulation, abi
+    n = (12, 150, 160)
+    s = Simulation(abi.make_config(*n, absorber=abi.ABS_NONE, pml=0))
+    om = [0.2, 0.3, 0.5, 0.7, 0.9, 1.1, 1.3, 1.5]
+    d = s.add_dft_plane(0, 6, (1 << abi.EY) | (1 << abi.HZ), om)          # 6.1 MB
+    f = np.random.default_rng(3).standard_normal(n).astype(np.float32)
+    s.set_field(abi.EY, f)
+    s.step(1)
+    e = s.get_field(abi.EY)[6]
+    out = s.read_dft(d)
+    assert out.dtype == np.complex128 and out.shape == (2, len(om)) + n[1:]
+    dt = s.cfg.dt
+    for k, w in enumerate(om):
+        assert np.allclose(out[0, k], e * np.exp(-1j * w * dt) * dt, rtol=0, atol=1e-12 * np.abs(e).max())
+    s.close()
