@@ -31,6 +31,7 @@ struct AdjDev {
   float* lEm[3];            // adjoint of the ADE state (Em, Jp, Jm) over the ADE box
   float* lJp[3][MAXPOLE];
   float* lJm[3][MAXPOLE];
+  float* lE[3];             // lam_E of the dispersive nodes next to the sweep's part (single-sweep adjoint only)
   float* lJg[3];            // adjoint of the gyrotropic current, ADE box
   float* lT[3];             // muJ of the gyrotropic nodes during one adjoint step, ADE box
 };

@@ -9,7 +9,7 @@
 // new G of the tile's halo recomputed, one CTA barrier a plane.  The kernels
 // it replaces (adj_w_kernel, adj_curl_kernel: w of both curl terms to memory
 // and back, twice a step) move 168 bytes a cell, this one 48 and the absorber's
-// auxiliaries; on a 192x160x128 grid they took 187 us a step, this one %ADJ%.
+// auxiliaries; on a 192x160x128 grid they took 187 us a step, this one 112.
 //
 // The absorber does differ: the transposed CPML stretches a value before the
 // difference is taken.  For a derivative along axis a a tap reads

@@ -24,6 +24,7 @@
 #include "dtmx_torre.cuh"
 #include "dtmx_adjoint.cuh"
 #include "dtmx_fused.cuh"
+#include "dtmx_adjsweep.cuh"
 
 using namespace dtmx;
 
@@ -1647,11 +1648,9 @@ static void fused_swap(dtmx_ctx* ctx) {
 // 8).  Larger grids: about eight waves, chunks of 6 to 32 planes (each chunk
 // stages one plane and updates one H plane more; 192x160x128: 68.0 us with 6,
 // 77.3 with 12; 384^3: 634 us with 32, 641 with 10, 669 with 64).
-static int fused_xchunk_for(const dtmx_ctx* ctx) {
-  if (ctx->xchunk > 0) return std::min(ctx->xchunk, FX_MAX);
-  const dtmx_config& c = ctx->cfg;
-  const long long tiles = (long long)((c.nz + TZ - 1) / TZ) * ((c.ny + ctx->frows - 1) / ctx->frows);
-  const long long fit = 148LL * (ctx->frows == 16 ? 3 : 5);
+static int sweep_xchunk(const dtmx_config& c, int rows, int per_sm) {
+  const long long tiles = (long long)((c.nz + TZ - 1) / TZ) * ((c.ny + rows - 1) / rows);
+  const long long fit = 148LL * per_sm;
   if (tiles <= fit) {
     const long long xc = (c.nx + fit / tiles - 1) / (fit / tiles);
     if (xc <= 12) return (int)xc;
@@ -1659,6 +1658,10 @@ static int fused_xchunk_for(const dtmx_ctx* ctx) {
   const long long chunks = std::max<long long>(1, (fit * 8 + tiles - 1) / tiles);
   const long long xc = (c.nx + chunks - 1) / chunks;
   return (int)std::min<long long>(32, std::max<long long>(6, xc));
+}
+static int fused_xchunk_for(const dtmx_ctx* ctx) {
+  if (ctx->xchunk > 0) return std::min(ctx->xchunk, FX_MAX);
+  return sweep_xchunk(ctx->cfg, ctx->frows, ctx->frows == 16 ? 3 : 5);
 }
 
 // One time step of the single-sweep engine: the side passes that act on the
@@ -1927,6 +1930,12 @@ struct FaRun {
   bool full = false;          // the forward pass records the whole design history: no checkpoints, no recompute
   cudaStream_t st = nullptr;
   std::vector<void*> bufs;
+  // single-sweep adjoint: A.lam / A.lpsi are the current set, these the other
+  // one (swapped after every step), the maps read set 0 and set 1
+  bool sweep = false;
+  float* lam_alt[6] = {};
+  float* lpsi_alt[3][4] = {};
+  FusedMaps fm[2]{};
   // Device buffers of the run come from the device's stream-ordered pool:
   // released blocks stay in the pool (release threshold raised once per
   // process), so later runs -- on this context or a fresh one -- reuse them
@@ -1963,6 +1972,18 @@ static bool fa_history_fits(dtmx_ctx* ctx, int nsteps) {
   const double bytes = fa_history_bytes(ctx, nsteps);
   if (ctx->adj_budget >= 0) return bytes <= (double)ctx->adj_budget;
   return bytes <= 0.25 * free_device_bytes();
+}
+
+// The adjoint as one sweep a step (dtmx_adjsweep.cuh): the Yee stencil without
+// gyrotropic material, and no dispersive node in a slab (its taps there would
+// be stretched).  Never slower than the two-pass kernels where both apply.
+static bool adj_sweep_usable(const dtmx_ctx* ctx) {
+  const Params& P = ctx->P;
+  if (ctx->cfg.order != 2 || ctx->has_gyro) return false;
+  if (P.ade.Em[0])
+    for (int a = 0; a < 3; a++)
+      if (P.ade.lo[a] < P.ab.L[a][0] || P.ade.lo[a] + P.ade.n[a] > P.g.n[a] - P.ab.L[a][1]) return false;
+  return true;
 }
 
 static int fa_begin(dtmx_ctx* ctx, FaRun& R, int nsteps, int checkpoint_every, int plane_x, double omega, bool full) {
@@ -2074,13 +2095,16 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
     return cudaMemsetAsync(*q, 0, bytes, ctx->stream) == cudaSuccess;
   };
   bool ok = true;
+  R.sweep = adj_sweep_usable(ctx);
   for (int comp = 0; comp < 6; comp++) ok = ok && talloc((void**)&A.lam[comp], (ctx->nstore + 64) * 4);
   for (int a = 0; a < 3; a++) {
     const size_t cnt = (size_t)(P.ab.L[a][0] + P.ab.L[a][1]) * (ctx->ncell / (size_t)P.g.n[a]);
     if (!P.ab.aux[a][0]) continue;
     for (int q = 0; q < 4; q++) ok = ok && talloc((void**)&A.lpsi[a][q], cnt * 4);
+    for (int q = 0; q < 4 && R.sweep; q++) ok = ok && talloc((void**)&R.lpsi_alt[a][q], cnt * 4);
   }
-  for (int c3 = 0; c3 < 3; c3++)
+  for (int comp = 0; comp < 6 && R.sweep; comp++) ok = ok && talloc((void**)&R.lam_alt[comp], (ctx->nstore + 64) * 4);
+  for (int c3 = 0; c3 < 3 && !R.sweep; c3++)
     for (int t = 0; t < 2; t++) ok = ok && talloc((void**)&A.w[c3][t], (ctx->nstore + 64) * 4);
   if (ctx->has_gyro) {
     const size_t na = (size_t)P.ade.n[0] * P.ade.n[1] * P.ade.n[2];
@@ -2091,6 +2115,7 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
     const size_t na = (size_t)P.ade.n[0] * P.ade.n[1] * P.ade.n[2];
     for (int c3 = 0; c3 < 3; c3++) {
       ok = ok && talloc((void**)&A.lEm[c3], na * 4);
+      if (R.sweep) ok = ok && talloc((void**)&A.lE[c3], na * 4);
       for (int r = 0; r < MAXPOLE; r++)
         if (P.ade.Jp[c3][r]) ok = ok && talloc((void**)&A.lJp[c3][r], na * 4) && talloc((void**)&A.lJm[c3][r], na * 4);
     }
@@ -2099,6 +2124,12 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
   if (!R.full) ok = ok && talloc((void**)&R.hist, (size_t)(R.K + 1) * 3 * R.nd * 4);
   if (!ok) { R.release(); return fail(ctx, DTMX_ERR_OOM, "adjoint allocation"); }
   A.hist = R.hist;
+  if (R.sweep) {
+    int rc;
+    if ((rc = build_fused_maps<16>(ctx, R.fm[0], A.lam)) || (rc = build_fused_maps<16>(ctx, R.fm[1], R.lam_alt))) return rc;
+    if (cudaFuncSetAttribute(adj_sweep_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AL<16>::SMEM) != cudaSuccess)
+      return fail(ctx, DTMX_ERR_CUDA, "adjoint sweep: shared memory attribute");
+  }
   CK(cudaMemcpyAsync(R.dF, F.data(), F.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->monitors_off = true;
@@ -2136,6 +2167,38 @@ static int fa_adjoint(dtmx_ctx* ctx, FaRun& R, int q) {
   const dtmx_config& c = ctx->cfg;
   AdjDev& A = R.A;
   cudaStream_t st = ctx->stream;
+  if (R.sweep) {
+    const long long s = R.s0 + (long long)R.seg * R.K + q;
+    const int ns = (R.npl + 255) / 256, ng = (int)design_blocks(R);
+    // the sources and the gradient share a launch unless the plane cuts the design region
+    if (R.plane_x >= P.des_lo[0] && R.plane_x < P.des_lo[0] + P.des_n[0]) {
+      adj_pre_kernel<<<ns, 256, 0, st>>>(P, A, R.dF, s, R.plane_x, R.omega, c.dt, ns, q);
+      adj_pre_kernel<<<ng, 256, 0, st>>>(P, A, R.dF, s, R.plane_x, R.omega, c.dt, 0, q);
+      ctx->launches++;
+    } else {
+      adj_pre_kernel<<<ns + ng, 256, 0, st>>>(P, A, R.dF, s, R.plane_x, R.omega, c.dt, ns, q);
+    }
+    if (P.ade.Em[0]) {
+      const dim3 blk(32, 8), grd((P.ade.n[2] + 31) / 32, (P.ade.n[1] + 7) / 8, std::max(1, P.ade.n[0]));
+      adj_ade_sweep_kernel<<<grd, blk, 0, st>>>(P, A);
+      ctx->launches++;
+    }
+    Params PS = P;
+    PS.x0 = 0; PS.x1 = c.nx;
+    PS.xchunk = sweep_xchunk(c, 16, 3);
+    AdjSweepArgs sa{};
+    for (int comp = 0; comp < 6; comp++) sa.dst[comp] = R.lam_alt[comp];
+    for (int a = 0; a < 3; a++)
+      for (int k = 0; k < 4; k++) { sa.psrc[a][k] = A.lpsi[a][k]; sa.pdst[a][k] = R.lpsi_alt[a][k]; }
+    const dim3 grd((c.nz + TZ - 1) / TZ, (c.ny + 15) / 16, (c.nx + PS.xchunk - 1) / PS.xchunk);
+    adj_sweep_kernel<16><<<grd, FL<16>::NT, AL<16>::SMEM, st>>>(PS, sa, R.fm[0]);
+    ctx->launches += 2;
+    for (int comp = 0; comp < 6; comp++) std::swap(A.lam[comp], R.lam_alt[comp]);
+    for (int a = 0; a < 3; a++)
+      for (int k = 0; k < 4; k++) std::swap(A.lpsi[a][k], R.lpsi_alt[a][k]);
+    std::swap(R.fm[0], R.fm[1]);
+    return DTMX_OK;
+  }
   adj_source_kernel<<<(R.npl + 255) / 256, 256, 0, st>>>(P, A, R.dF, R.s0 + (long long)R.seg * R.K + q, R.plane_x, R.omega, c.dt);
   adj_grad_kernel<<<design_blocks(R), 256, 0, st>>>(P, A, q);
   const dim3 blk(32, 8), grd((c.nz + 31) / 32, (c.ny + 7) / 8, c.nx);
