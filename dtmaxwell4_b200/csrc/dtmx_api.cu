@@ -519,7 +519,7 @@ static int build_maps(dtmx_ctx* ctx) {
   const int rows[6] = {rows_h, TYT, rows_h, rows_e, TYT, rows_e};
   int rc;
   for (int comp = 0; comp < 6; comp++) {
-    if ((rc = make_map(ctx, &ctx->maps.src[comp], ctx->P.f[comp], false, TW_ROW, rows[comp]))) return rc;
+    if ((rc = make_map(ctx, &ctx->maps.src[comp], ctx->P.f[comp], false, TZ + 8, rows[comp]))) return rc;
     if ((rc = make_map(ctx, &ctx->maps.own[comp], ctx->P.f[comp], false, TZ, TYT))) return rc;
   }
   for (int comp = 0; comp < 3; comp++)
@@ -1320,7 +1320,7 @@ static int launch_step(dtmx_ctx* ctx) {
   Params P = ctx->P;
   P.x0 = 0; P.x1 = c.nx;
   P.xchunk = xchunk_for(ctx);
-  const dim3 blk(TZ, TW);
+  const int blk = STREAM_NT;
   const dim3 grd((c.nz + TZ - 1) / TZ, (c.ny + TYT - 1) / TYT, (c.nx + P.xchunk - 1) / P.xchunk);
   const bool o4 = c.order == 4;
   cudaStream_t st = ctx->stream;

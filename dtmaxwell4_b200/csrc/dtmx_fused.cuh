@@ -103,14 +103,6 @@ struct FusedArgs {
   float* hdst[3][2];                         // ... and in B
 };
 
-// four consecutive z nodes
-struct Q4 { float v[4]; };
-__device__ __forceinline__ Q4 ld4(const float* s) {
-  const float4 t = *reinterpret_cast<const float4*>(s);
-  return Q4{{t.x, t.y, t.z, t.w}};
-}
-__device__ __forceinline__ void st4(float* d, const Q4& q) { *reinterpret_cast<float4*>(d) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]); }
-
 // staged-tile addresses (tile-local y, z)
 template <int TY> __device__ __forceinline__ const float* fE(const float* st, int c, int y, int z) { return st + c * FL<TY>::FE_N + (y + 1) * FE_W + z + 4; }
 template <int TY> __device__ __forceinline__ const float* fHx(const float* st, int y, int z) { return st + FL<TY>::OFF_HX + y * FHX_W + z; }
@@ -118,53 +110,6 @@ template <int TY> __device__ __forceinline__ const float* fHy(const float* st, i
 template <int TY> __device__ __forceinline__ const float* fHz(const float* st, int y, int z) { return st + FL<TY>::OFF_HZ + y * FHZ_W + z; }
 template <int TY> __device__ __forceinline__ float* fN(float* hn, int q, int y, int z) { return hn + q * FL<TY>::HN_N + y * HN_P + z; }
 template <int TY> __device__ __forceinline__ const float* fN(const float* hn, int q, int y, int z) { return hn + q * FL<TY>::HN_N + y * HN_P + z; }
-
-// index of coordinate v in the slab of its axis (-1 outside)
-__device__ __forceinline__ int slab_cs(const Params& p, int a, int v) {
-  const int n = p.g.n[a], lo = p.ab.L[a][0], hi = p.ab.L[a][1];
-  return v < lo ? v : (v >= n - hi ? lo + v - (n - hi) : -1);
-}
-
-// slab index of node (i, j, k) along axis a from its slab coordinate s on that axis (>= 0)
-__device__ __forceinline__ int slab_at(const Params& p, int a, int i, int j, int k, int s) {
-  if (a == 0) return (s * p.g.n[1] + j) * p.g.n[2] + k;
-  if (a == 1) return (i * (p.ab.L[1][0] + p.ab.L[1][1]) + s) * p.g.n[2] + k;
-  return (i * p.g.n[1] + j) * (p.ab.L[2][0] + p.ab.L[2][1]) + s;
-}
-
-// What a thread keeps about its row and its four columns during the walk.
-struct FNode {
-  int y, z;                  // tile-local
-  int j, k;
-  int nv;                    // nodes of the four inside the grid (0: the row is outside)
-  int ys;                    // slab coordinate of the row (-1 outside)
-  int zs;                    // slab coordinate of node k (negative or past the slab where zm is 0)
-  unsigned zm;               // nodes of the four inside the z slab
-  bool vxy, vz;              // 16-byte accesses to the x and y slabs' / the z slab's auxiliaries
-};
-
-// Four old auxiliaries / four new ones.  The x and y slab arrays have rows of
-// nz floats, so with nz a multiple of 4 every row of four is aligned and whole;
-// the z slab's rows are as long as the slab is thick.
-template <bool RO>
-__device__ __forceinline__ Q4 aux4(const float* q, bool vec, unsigned m) {
-  Q4 r{{0.f, 0.f, 0.f, 0.f}};
-  if (vec) {
-    const float4 t = RO ? __ldg(reinterpret_cast<const float4*>(q)) : *reinterpret_cast<const float4*>(q);
-    r = Q4{{t.x, t.y, t.z, t.w}};
-  } else {
-#pragma unroll
-    for (int e = 0; e < 4; e++)
-      if ((m >> e) & 1) r.v[e] = RO ? __ldg(q + e) : q[e];
-  }
-  return r;
-}
-__device__ __forceinline__ void put4(float* q, bool vec, unsigned m, const Q4& v) {
-  if (vec) { st4(q, v); return; }
-#pragma unroll
-  for (int e = 0; e < 4; e++)
-    if ((m >> e) & 1) q[e] = v.v[e];
-}
 
 // The old auxiliaries of the thread's nodes in plane i, all axes: requested
 // before the stage wait, used after it.  H reads set A, E its own in place.
@@ -241,22 +186,6 @@ __device__ __forceinline__ void fused_cpml(const Params& p, const FusedArgs& fa,
   for (int q = 0; q < 3; q++)
 #pragma unroll
     for (int e = 0; e < 4; e++) inc[q].v[e] = __fadd_rn(inc[q].v[e], corr[q].v[e]);
-}
-
-// scale * (u - l) of four nodes; l shifted by one node: the value below the first, then u's own
-__device__ __forceinline__ Q4 diff4(float s, const Q4& u, const Q4& l) {
-  Q4 r;
-#pragma unroll
-  for (int e = 0; e < 4; e++) r.v[e] = __fmul_rn(s, __fsub_rn(u.v[e], l.v[e]));
-  return r;
-}
-__device__ __forceinline__ Q4 below4(float first, const Q4& u) { return Q4{{first, u.v[0], u.v[1], u.v[2]}}; }
-__device__ __forceinline__ Q4 above4(const Q4& u, float last) { return Q4{{u.v[1], u.v[2], u.v[3], last}}; }
-__device__ __forceinline__ Q4 add4(const Q4& a, const Q4& b) {
-  Q4 r;
-#pragma unroll
-  for (int e = 0; e < 4; e++) r.v[e] = __fadd_rn(a.v[e], b.v[e]);
-  return r;
 }
 
 // New H of plane i on the thread's nodes: hc (registers), hn (shared plane
