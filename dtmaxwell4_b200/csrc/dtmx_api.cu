@@ -958,6 +958,7 @@ extern "C" int dtmx_set_tfsf(dtmx_ctx* ctx, const dtmx_tfsf* s) {
         for (int side = 0; side < 2; side++) {
           TfsfJob jb{};
           jb.c = comp;
+          jb.a = a; jb.g = g; jb.sg = term == 0 ? 1 : -1;
           bool empty = false;
           for (int b = 0; b < 3; b++) {
             int X0, X1, o;
@@ -1314,6 +1315,39 @@ static long long launch_tail(dtmx_ctx* ctx, const Params& P, cudaStream_t st) {
   return nl;
 }
 
+// TF/SF corrections of one half step, and the plane wave's line
+static long long launch_tfsf(dtmx_ctx* ctx, const Params& P, cudaStream_t st, bool isH) {
+  if (!ctx->has_tfsf) return 0;
+  const TfsfDev& T = ctx->T;
+  const int hs = isH ? 1 : 0;
+  const bool o4 = ctx->cfg.order == 4;
+  if (ctx->tfsf.kind == DTMX_TFSF_PLANE_X) {
+    const dtmx_tfsf& s = ctx->tfsf;
+    const LineDev l{ctx->line_e, ctx->line_h, T.line_n, ctx->line_src, ctx->cfg.dt / ctx->cfg.dx, ctx->cfg.dt, s.amp, s.f0, s.tau, s.t0};
+    long long units = 64;                          // warps of a job (128 nodes each); at least 8 blocks for the line
+    for (int r = 0; r < T.njob[hs]; r++) {
+      const TfsfJob& jb = T.job[hs][r];
+      const int la = jb.a == 2 ? 1 : 2;
+      const long long nl = jb.hi[la] - jb.lo[la] + 1;
+      units = std::max(units, jb.cells / nl * ((nl + 127) / 128));
+    }
+    const dim3 grd((unsigned)((units + 7) / 8), T.njob[hs] + 1);
+    if (o4) tfsf_plane_kernel<4><<<grd, 256, 0, st>>>(P, T, l, ctx->d_step, isH);
+    else tfsf_plane_kernel<2><<<grd, 256, 0, st>>>(P, T, l, ctx->d_step, isH);
+    return 1;
+  }
+  long long mx = 1;
+  for (int r = 0; r < T.njob[hs]; r++) mx = std::max(mx, T.job[hs][r].cells);
+  const dim3 grd((unsigned)((mx + 255) / 256), std::max(1, T.njob[hs]));
+  if (o4) tfsf_kernel<4><<<grd, 256, 0, st>>>(P, T, ctx->d_step, isH);
+  else tfsf_kernel<2><<<grd, 256, 0, st>>>(P, T, ctx->d_step, isH);
+  return 1;
+}
+// grid of the passes over the ADE box (ade_cell)
+static dim3 ade_grid(const Params& P) {
+  return dim3((unsigned)(((long long)P.ade.n[1] * P.ade.n[2] + 255) / 256), std::max(1, P.ade.n[0]));
+}
+
 static int launch_step(dtmx_ctx* ctx) {
   set_kernel_attributes();
   const dtmx_config& c = ctx->cfg;
@@ -1324,35 +1358,17 @@ static int launch_step(dtmx_ctx* ctx) {
   const dim3 grd((c.nz + TZ - 1) / TZ, (c.ny + TYT - 1) / TYT, (c.nx + P.xchunk - 1) / P.xchunk);
   const bool o4 = c.order == 4;
   cudaStream_t st = ctx->stream;
-  const bool pw = ctx->has_tfsf && ctx->tfsf.kind == DTMX_TFSF_PLANE_X;
   long long nl = 0;
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], st);
   if (o4) h_kernel<4><<<grd, blk, Pipe<4, true>::SMEM_BYTES, st>>>(P, ctx->maps);
   else h_kernel<2><<<grd, blk, Pipe<2, true>::SMEM_BYTES, st>>>(P, ctx->maps);
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], st);
   nl++;
-  dim3 tgrid[2];
-  for (int hs = 0; hs < 2 && ctx->has_tfsf; hs++) {
-    long long mx = 1;
-    for (int r = 0; r < ctx->T.njob[hs]; r++) mx = std::max(mx, ctx->T.job[hs][r].cells);
-    tgrid[hs] = dim3((unsigned)((mx + 255) / 256), std::max(1, ctx->T.njob[hs]));
-  }
-  if (ctx->has_tfsf) {
-    if (o4) tfsf_kernel<4><<<tgrid[1], 256, 0, st>>>(P, ctx->T, ctx->d_step, 1);
-    else tfsf_kernel<2><<<tgrid[1], 256, 0, st>>>(P, ctx->T, ctx->d_step, 1);
-    nl++;
-  }
-  const double r1 = c.dt / c.dx;
-  if (pw) {
-    if (o4) line_h_kernel<4><<<8, 256, 0, st>>>(ctx->line_e, ctx->line_h, ctx->T.line_n, r1);
-    else line_h_kernel<2><<<8, 256, 0, st>>>(ctx->line_e, ctx->line_h, ctx->T.line_n, r1);
-    nl++;
-  }
-  const dim3 ablk(32, 8), agrd((P.ade.n[2] + 31) / 32, (P.ade.n[1] + 7) / 8, std::max(1, P.ade.n[0]));
+  nl += launch_tfsf(ctx, P, st, true);
+  const int cur = ctx->gcur;
   if (ctx->has_gyro) {
-    gyro_current_kernel<<<agrd, ablk, 0, st>>>(P, ctx->gcur);
-    P.ade.gnew = 1 - ctx->gcur;
-    ctx->gcur = 1 - ctx->gcur;
+    gyro_current_kernel<<<ade_grid(P), 256, 0, st>>>(P, cur);
+    ctx->gcur = 1 - cur;
     nl++;
   }
   if (ctx->profiling) cudaEventRecord(ctx->ev[2], st);
@@ -1361,8 +1377,8 @@ static int launch_step(dtmx_ctx* ctx) {
   if (P.ade.Em[0] || ctx->has_gyro) {
     // dispersive and gyrotropic nodes of the E half step (e_kernel skipped them)
     const bool box = c.geometry == DTMX_GEOM_BOX;
-    if (o4) { if (box) ade_node_kernel<4, true><<<agrd, ablk, 0, st>>>(P); else ade_node_kernel<4, false><<<agrd, ablk, 0, st>>>(P); }
-    else { if (box) ade_node_kernel<2, true><<<agrd, ablk, 0, st>>>(P); else ade_node_kernel<2, false><<<agrd, ablk, 0, st>>>(P); }
+    if (o4) { if (box) ade_node_kernel<4, true, false><<<ade_grid(P), 256, 0, st>>>(P, cur); else ade_node_kernel<4, false, false><<<ade_grid(P), 256, 0, st>>>(P, cur); }
+    else { if (box) ade_node_kernel<2, true, false><<<ade_grid(P), 256, 0, st>>>(P, cur); else ade_node_kernel<2, false, false><<<ade_grid(P), 256, 0, st>>>(P, cur); }
     nl++;
   }
   if (ctx->profiling) {
@@ -1375,17 +1391,7 @@ static int launch_step(dtmx_ctx* ctx) {
     ctx->prof_ms_h += a; ctx->prof_ms_e += b; ctx->prof_count++;
   }
   nl++;
-  if (ctx->has_tfsf) {
-    if (o4) tfsf_kernel<4><<<tgrid[0], 256, 0, st>>>(P, ctx->T, ctx->d_step, 0);
-    else tfsf_kernel<2><<<tgrid[0], 256, 0, st>>>(P, ctx->T, ctx->d_step, 0);
-    nl++;
-  }
-  if (pw) {
-    const dtmx_tfsf& s = ctx->tfsf;
-    if (o4) line_e_kernel<4><<<8, 256, 0, st>>>(ctx->line_e, ctx->line_h, ctx->T.line_n, r1, ctx->line_src, ctx->d_step, c.dt, s.amp, s.f0, s.tau, s.t0);
-    else line_e_kernel<2><<<8, 256, 0, st>>>(ctx->line_e, ctx->line_h, ctx->T.line_n, r1, ctx->line_src, ctx->d_step, c.dt, s.amp, s.f0, s.tau, s.t0);
-    nl++;
-  }
+  nl += launch_tfsf(ctx, P, st, false);
   nl += launch_tail(ctx, P, st);
   ctx->launches += nl;
   return DTMX_OK;
@@ -1685,25 +1691,8 @@ static int launch_fused_step(dtmx_ctx* ctx) {
       PB.ab.aux[a][2 + q] = ctx->hax_alt[a][q];
     }
   cudaStream_t st = ctx->stream;
-  const bool pw = ctx->has_tfsf && ctx->tfsf.kind == DTMX_TFSF_PLANE_X;
-  long long nl = 0;
-  dim3 tgrid[2];
-  for (int hs = 0; hs < 2 && ctx->has_tfsf; hs++) {
-    long long mx = 1;
-    for (int r = 0; r < ctx->T.njob[hs]; r++) mx = std::max(mx, ctx->T.job[hs][r].cells);
-    tgrid[hs] = dim3((unsigned)((mx + 255) / 256), std::max(1, ctx->T.njob[hs]));
-  }
   // TF/SF correction of H, added to the old H (the H update is linear in it)
-  if (ctx->has_tfsf) { tfsf_kernel<2><<<tgrid[1], 256, 0, st>>>(PA, ctx->T, ctx->d_step, 1); nl++; }
-  const double r1 = c.dt / c.dx;
-  if (pw) { line_h_kernel<2><<<8, 256, 0, st>>>(ctx->line_e, ctx->line_h, ctx->T.line_n, r1); nl++; }
-  const dim3 ablk(32, 8), agrd((PA.ade.n[2] + 31) / 32, (PA.ade.n[1] + 7) / 8, std::max(1, PA.ade.n[0]));
-  if (ctx->has_gyro) {
-    gyro_current_kernel<<<agrd, ablk, 0, st>>>(PA, ctx->gcur);
-    PA.ade.gnew = PB.ade.gnew = 1 - ctx->gcur;
-    ctx->gcur = 1 - ctx->gcur;
-    nl++;
-  }
+  long long nl = launch_tfsf(ctx, PA, st, true);
   const dim3 grd((c.nz + TZ - 1) / TZ, (c.ny + ctx->frows - 1) / ctx->frows, (c.nx + PA.xchunk - 1) / PA.xchunk);
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], st);
   if (ctx->frows == 8) fused_kernel<8><<<grd, FL<8>::NT, FL<8>::SMEM, st>>>(PA, fa, ctx->fmaps8[0]);
@@ -1711,9 +1700,15 @@ static int launch_fused_step(dtmx_ctx* ctx) {
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], st);
   nl++;
   if (PA.ade.Em[0] || ctx->has_gyro) {
-    // dispersive nodes (left by the sweep) from the old E in A; E -= dt/eps_inf J on gyrotropic nodes
+    // dispersive nodes (left by the sweep) from the old E in A; on gyrotropic nodes the current from the
+    // old E, then E -= dt/eps_inf J
     for (int comp = 0; comp < 3; comp++) PB.fe_old[comp] = PA.f[comp];
-    ade_node_kernel<2, true><<<agrd, ablk, 0, st>>>(PB);
+    if (ctx->has_gyro) {
+      ade_node_kernel<2, true, true><<<ade_grid(PB), 256, 0, st>>>(PB, ctx->gcur);
+      ctx->gcur = 1 - ctx->gcur;
+    } else {
+      ade_node_kernel<2, true, false><<<ade_grid(PB), 256, 0, st>>>(PB, 0);
+    }
     nl++;
   }
   if (ctx->profiling) {
@@ -1722,12 +1717,7 @@ static int launch_fused_step(dtmx_ctx* ctx) {
     cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]);
     ctx->prof_ms_h += a; ctx->prof_count++;
   }
-  if (ctx->has_tfsf) { tfsf_kernel<2><<<tgrid[0], 256, 0, st>>>(PB, ctx->T, ctx->d_step, 0); nl++; }
-  if (pw) {
-    const dtmx_tfsf& s = ctx->tfsf;
-    line_e_kernel<2><<<8, 256, 0, st>>>(ctx->line_e, ctx->line_h, ctx->T.line_n, r1, ctx->line_src, ctx->d_step, c.dt, s.amp, s.f0, s.tau, s.t0);
-    nl++;
-  }
+  nl += launch_tfsf(ctx, PB, st, false);
   nl += launch_tail(ctx, PB, st);
   ctx->launches += nl;
   fused_swap(ctx);
@@ -2179,8 +2169,7 @@ static int fa_adjoint(dtmx_ctx* ctx, FaRun& R, int q) {
       adj_pre_kernel<<<ns + ng, 256, 0, st>>>(P, A, R.dF, s, R.plane_x, R.omega, c.dt, ns, q);
     }
     if (P.ade.Em[0]) {
-      const dim3 blk(32, 8), grd((P.ade.n[2] + 31) / 32, (P.ade.n[1] + 7) / 8, std::max(1, P.ade.n[0]));
-      adj_ade_sweep_kernel<<<grd, blk, 0, st>>>(P, A);
+      adj_ade_sweep_kernel<<<ade_grid(P), 256, 0, st>>>(P, A);
       ctx->launches++;
     }
     Params PS = P;
@@ -2207,7 +2196,8 @@ static int fa_adjoint(dtmx_ctx* ctx, FaRun& R, int q) {
   // the gyrotropic current's transposition reads lam_E' (after adj_w) and gathers over the box
   const bool ade = P.ade.Em[0] != nullptr;
   const bool gyro = ctx->has_gyro;
-  const dim3 ablk(32, 8), agrd((P.ade.n[2] + 31) / 32, (P.ade.n[1] + 7) / 8, std::max(1, P.ade.n[0]));
+  const int ablk = 256;
+  const dim3 agrd = ade_grid(P);
   if (c.order == 4) {
     adj_w_kernel<4, 0><<<wgrd, blk, 0, st>>>(P, A);
     if (ade) adj_ade_kernel<<<agrd, ablk, 0, st>>>(P, A);

@@ -10,6 +10,7 @@ namespace dtmx {
 // node of c whose taps along one curl axis cross one face of the box.
 struct TfsfJob {
   int c;
+  int a, g, sg;              // the job's curl term: axis, source component, sign in the curl
   int lo[3], hi[3];
   long long cells;
 };
@@ -180,37 +181,112 @@ __global__ void tfsf_kernel(Params p, TfsfDev t, const long long* d_step, int is
   p.f[c][id] += (float)total;
 }
 
-// 1-D incident line (Ez at odd X, Hy at even X), same stencil and time step.
+// ---- plane wave: corrections of one half step and the 1-D incident line (Ez
+// at odd X, Hy at even X, same stencil and time step) in one launch.  The
+// corrections read the line's other field, so neither waits for the other: the
+// H half step reads e and advances h, the E half step reads h and advances e.
+struct LineDev {
+  double* e; double* h;
+  int n, src;
+  double r, dt, amp, f0, tau, t0;
+};
+
 template <int ORDER>
-__global__ void line_h_kernel(double* e, double* h, int n, double r) {
-  for (int m = threadIdx.x + blockIdx.x * blockDim.x; m < n; m += blockDim.x * gridDim.x) {
-    const double e0 = e[m], em1 = m >= 1 ? e[m - 1] : 0.0;
-    double d;
-    if (ORDER == 4) {
-      const double ep1 = m + 1 < n ? e[m + 1] : 0.0, em2 = m >= 2 ? e[m - 2] : 0.0;
-      d = (27.0 * (e0 - em1) - (ep1 - em2)) / 24.0;
+__device__ __forceinline__ void line_update(const LineDev& l, bool isH, long long n, int m0, int stride) {
+  const double ts = ((double)n + 0.5) * l.dt - l.t0;
+  for (int m = m0; m < l.n; m += stride) {
+    if (isH) {
+      const double e0 = l.e[m], em1 = m >= 1 ? l.e[m - 1] : 0.0;
+      double d = e0 - em1;
+      if (ORDER == 4) {
+        const double ep1 = m + 1 < l.n ? l.e[m + 1] : 0.0, em2 = m >= 2 ? l.e[m - 2] : 0.0;
+        d = (27.0 * (e0 - em1) - (ep1 - em2)) / 24.0;
+      }
+      l.h[m] += l.r * d;
     } else {
-      d = e0 - em1;
+      const double h0 = l.h[m], hp1 = m + 1 < l.n ? l.h[m + 1] : 0.0;
+      double d = hp1 - h0;
+      if (ORDER == 4) {
+        const double hp2 = m + 2 < l.n ? l.h[m + 2] : 0.0, hm1 = m >= 1 ? l.h[m - 1] : 0.0;
+        d = (27.0 * (hp1 - h0) - (hp2 - hm1)) / 24.0;
+      }
+      double v = l.e[m] + l.r * d;
+      if (m == l.src) v += l.amp * sin(2.0 * M_PI * l.f0 * ts) * exp(-(ts / l.tau) * (ts / l.tau));
+      l.e[m] = v;
     }
-    h[m] += r * d;
   }
 }
+
+// A plane wave has only Ez and Hy, so a component has one curl term with an
+// incident tap, and on one node it depends on the node's index along the
+// term's axis and on x alone.  A warp takes 128 nodes of a row of a job: along
+// z, or along y where the job is the face normal to z and a row along z would
+// hold one node.  Measured on a 384^3 grid: 18 us a half step with one thread a
+// node and the general tap search, 12.5 with this, the line's update included (5
+// and 2 us as launches of their own); what is left is a chain of dependent loads.
 template <int ORDER>
-__global__ void line_e_kernel(double* e, const double* h, int n, double r, int src, const long long* d_step,
-                              double dt, double amp, double f0, double tau, double t0) {
-  const double ts = ((double)(*d_step) + 0.5) * dt - t0;
-  for (int m = threadIdx.x + blockIdx.x * blockDim.x; m < n; m += blockDim.x * gridDim.x) {
-    const double h0 = h[m], hp1 = m + 1 < n ? h[m + 1] : 0.0;
-    double d;
-    if (ORDER == 4) {
-      const double hp2 = m + 2 < n ? h[m + 2] : 0.0, hm1 = m >= 1 ? h[m - 1] : 0.0;
-      d = (27.0 * (hp1 - h0) - (hp2 - hm1)) / 24.0;
-    } else {
-      d = hp1 - h0;
+__global__ void __launch_bounds__(256) tfsf_plane_kernel(const __grid_constant__ Params p, const __grid_constant__ TfsfDev t, const LineDev l,
+                                                         const long long* d_step, int isH) {
+  const long long n = *d_step;
+  const int hs = isH ? 1 : 0, r = blockIdx.y;
+  if (r == t.njob[hs]) {                           // the line's own update
+    line_update<ORDER>(l, isH, n, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256);
+    return;
+  }
+  if (!tfsf_on(t, n)) return;
+  const TfsfJob& jb = t.job[hs][r];
+  const int c = jb.c, a = jb.a, g = jb.g, lane = threadIdx.x & 31;
+  const int la = a == 2 ? 1 : 2, ra = a == 2 ? 2 : 1;              // axis of a row, and the other one beside x
+  const int nl = jb.hi[la] - jb.lo[la] + 1, nr = jb.hi[ra] - jb.lo[ra] + 1, ni = jb.hi[0] - jb.lo[0] + 1;
+  const int parts = (nl + 127) / 128;
+  const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (unit >= ni * nr * parts) return;
+  const int part = unit % parts, row = unit / parts;
+  int idx[3];
+  idx[0] = jb.lo[0] + row / nr;
+  idx[ra] = jb.lo[ra] + row % nr;
+  const int first = jb.lo[la] + part * 128 + lane;
+  // the correction of the row's nodes, but for 1/eps (a is not the row's axis)
+  const int t0 = isH ? -2 : -1, o = comp_off(c, a), og = comp_off(g, a);
+  const int S = 2 * idx[a] + o;
+  const bool sin_ = S >= t.lo[a] && S <= t.hi[a];
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if (ORDER == 2 && (q == 0 || q == 3)) continue;
+    const int G = 2 * (idx[a] + t0 + q) + og;
+    if ((G >= t.lo[a] && G <= t.hi[a]) == sin_) continue;
+    const int X = a == 0 ? G : 2 * idx[0] + comp_off(g, 0);
+    const int m = (g == 2 ? (X - 1) >> 1 : X >> 1) + t.line_M;
+    const double inc = m >= 0 && m < t.line_n ? (g == 2 ? t.line_e[m] : t.line_h[m]) : 0.0;
+    v[q] = sin_ ? -inc : inc;
+  }
+  const double dv = ORDER == 2 ? v[2] - v[1] : (27.0 * (v[2] - v[1]) - (v[3] - v[0])) / 24.0;
+  const double total = (isH ? -jb.sg : jb.sg) * (double)p.cdt[a] * dv;
+  long long id[4];
+  float f[4];
+  bool on[4];
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    idx[la] = first + 32 * e;
+    on[e] = idx[la] <= jb.hi[la] && is_live(p.g, c, idx[0], idx[1], idx[2]);
+    // a node of an earlier job of the component is that job's
+    for (int q = 0; q < r && on[e]; q++)
+      if (t.job[hs][q].c == c && in_job(t.job[hs][q], idx[0], idx[1], idx[2])) on[e] = false;
+    id[e] = (long long)idx[0] * p.g.sx + (long long)idx[1] * p.g.sy + idx[2];
+    f[e] = on[e] ? p.f[c][id[e]] : 0.f;
+  }
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    if (!on[e]) continue;
+    double w = total;
+    if (!isH) {
+      idx[la] = first + 32 * e;
+      const int mi = p.mat[c] ? (int)__ldg(p.mat[c] + id[e]) : 0;
+      const long long di = design_index(p, idx[0], idx[1], idx[2]);
+      w *= (double)(di >= 0 ? p.des_ie[c][di] : __ldg(&p.mt->inv_eps[mi][c]));
     }
-    double v = e[m] + r * d;
-    if (m == src) v += amp * sin(2.0 * M_PI * f0 * ts) * exp(-(ts / tau) * (ts / tau));
-    e[m] = v;
+    p.f[c][id[e]] = f[e] + (float)w;
   }
 }
 
@@ -581,99 +657,167 @@ __device__ __forceinline__ float gyro_old(const Params& p, int cur, int c, int i
   return __ldg(p.ade.Jg[cur][c] + ((long long)bi * p.ade.n[1] + bj) * p.ade.n[2] + bk);
 }
 
-// Thread layout of the passes over the ADE box: (threadIdx.x, blockIdx.x) = z,
-// (threadIdx.y, blockIdx.y) = y, blockIdx.z = x (no index division).
+// Thread layout of the passes over the ADE box: 256 threads along the box'
+// (y, z) plane, blockIdx.y = x.
 __device__ __forceinline__ bool ade_cell(const Params& p, int& bi, int& bj, int& bk, long long& q) {
-  bk = blockIdx.x * blockDim.x + threadIdx.x;
-  bj = blockIdx.y * blockDim.y + threadIdx.y;
-  bi = blockIdx.z;
-  if (bj >= p.ade.n[1] || bk >= p.ade.n[2]) return false;
-  q = ((long long)bi * p.ade.n[1] + bj) * p.ade.n[2] + bk;
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r >= p.ade.n[1] * p.ade.n[2]) return false;
+  bj = r / p.ade.n[2];
+  bk = r - bj * p.ade.n[2];
+  bi = blockIdx.y;
+  q = (long long)bi * p.ade.n[1] * p.ade.n[2] + r;
   return true;
 }
 
-__global__ void gyro_current_kernel(Params p, int cur) {
+// The three new current components of node (i, j, k), box index q, from the
+// old ones (buffer cur) and E^n; m: material indices, E: E^n, on: gyrotropic
+__device__ __forceinline__ void gyro_new(const Params& p, int cur, int i, int j, int k, long long q, const int (&m)[3], const float (&E)[3],
+                                         const bool (&on)[3], float (&J)[3]) {
   const MatTable& mt = *p.mt;
-  int bi, bj, bk;
-  long long q;
-  if (ade_cell(p, bi, bj, bk, q)) {
-    const int i = p.ade.lo[0] + bi, j = p.ade.lo[1] + bj, k = p.ade.lo[2] + bk;
-    const long long id = (long long)i * p.g.sx + (long long)j * p.g.sy + k;
+  // every load before its use
+  float own[3], near[2][4];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      // (E, the old current, materials and table are read-only in this pass)
-      const int m = p.mat[c] ? (int)__ldg(p.mat[c] + id) : 0;
-      if (__ldg(&mt.gjc[m]) == 0.f) continue;
-      const float E = __ldg(p.f[c] + id), Jo = __ldg(p.ade.Jg[cur][c] + q);
-      float t;
-      if (c == 0) {
-        const float avg = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(gyro_old(p, cur, 1, i - 1, j, k), gyro_old(p, cur, 1, i, j, k)),
-                                                               gyro_old(p, cur, 1, i - 1, j + 1, k)),
-                                                     gyro_old(p, cur, 1, i, j + 1, k)));
-        t = __fmaf_rn(__ldg(&mt.gC[m]), Jo, __fmul_rn(__ldg(&mt.gS[m]), avg));
-      } else if (c == 1) {
-        const float avg = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(gyro_old(p, cur, 0, i, j - 1, k), gyro_old(p, cur, 0, i + 1, j - 1, k)),
-                                                               gyro_old(p, cur, 0, i, j, k)),
-                                                     gyro_old(p, cur, 0, i + 1, j, k)));
-        t = __fmaf_rn(__ldg(&mt.gC[m]), Jo, -__fmul_rn(__ldg(&mt.gS[m]), avg));
-      } else {
-        t = Jo;
-      }
-      p.ade.Jg[1 - cur][c][q] = __fmaf_rn(__ldg(&mt.gA[m]), t, __fmul_rn(__ldg(&mt.gB[m]), E));
+  for (int c = 0; c < 3; c++) own[c] = on[c] ? __ldg(p.ade.Jg[cur][c] + q) : 0.f;
+  if (on[0]) {
+    near[0][0] = gyro_old(p, cur, 1, i - 1, j, k); near[0][1] = gyro_old(p, cur, 1, i, j, k);
+    near[0][2] = gyro_old(p, cur, 1, i - 1, j + 1, k); near[0][3] = gyro_old(p, cur, 1, i, j + 1, k);
+  }
+  if (on[1]) {
+    near[1][0] = gyro_old(p, cur, 0, i, j - 1, k); near[1][1] = gyro_old(p, cur, 0, i + 1, j - 1, k);
+    near[1][2] = gyro_old(p, cur, 0, i, j, k); near[1][3] = gyro_old(p, cur, 0, i + 1, j, k);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    J[c] = 0.f;
+    if (!on[c]) continue;
+    float t = own[c];
+    if (c < 2) {
+      const float avg = __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(near[c][0], near[c][1]), near[c][2]), near[c][3]));
+      const float s = __fmul_rn(__ldg(&mt.gS[m[c]]), avg);
+      t = __fmaf_rn(__ldg(&mt.gC[m[c]]), own[c], c == 0 ? s : -s);
     }
+    J[c] = __fmaf_rn(__ldg(&mt.gA[m[c]]), t, __fmul_rn(__ldg(&mt.gB[m[c]]), E[c]));
   }
 }
 
-// Dispersive and gyrotropic E nodes, after e_kernel (which leaves dispersive
-// nodes untouched): the ADE recursion (countDisp, dispersion.cpp:85-99) with
-// rot = dt curl H recomputed from H exactly as the field kernels compute it,
-// and E -= dt/eps_inf J^{n+1/2} on gyrotropic nodes.  One thread per cell of
-// the ADE box; BOX: zero-outside geometry (bounds-checked taps).
-template <int ORDER, bool BOX>
-__global__ void ade_node_kernel(Params p) {
+// J^{n+1/2} into buffer 1-cur (per-step engine: before the E half step changes E)
+__global__ void __launch_bounds__(256) gyro_current_kernel(const __grid_constant__ Params p, int cur) {
+  int bi, bj, bk;
+  long long q;
+  if (!ade_cell(p, bi, bj, bk, q)) return;
+  const int i = p.ade.lo[0] + bi, j = p.ade.lo[1] + bj, k = p.ade.lo[2] + bk;
+  const long long id = (long long)i * p.g.sx + (long long)j * p.g.sy + k;
+  // (E, the old current, materials and table are read-only in this pass)
+  int m[3];
+  float E[3], J[3];
+  bool on[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) { m[c] = p.mat[c] ? (int)__ldg(p.mat[c] + id) : 0; E[c] = __ldg(p.f[c] + id); }
+#pragma unroll
+  for (int c = 0; c < 3; c++) on[c] = __ldg(&p.mt->gjc[m[c]]) != 0.f;
+  gyro_new(p, cur, i, j, k, q, m, E, on, J);
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    if (on[c]) p.ade.Jg[1 - cur][c][q] = J[c];
+}
+
+// Dispersive and gyrotropic E nodes, after the field pass (which leaves
+// dispersive nodes at their old value): the ADE recursion (countDisp,
+// dispersion.cpp:85-99) with rot = dt curl H recomputed from H exactly as the
+// field kernels compute it, and E -= dt/eps_inf J^{n+1/2} on gyrotropic nodes.
+// One thread per cell of the ADE box; BOX: zero-outside geometry (bounds-checked
+// taps).  CUR: the gyrotropic current is advanced here too, from E^n in the
+// single sweep's other set (p.fe_old): one pass over it instead of two.
+// The three components' loads are issued together (materials, then flags, then
+// state and taps: three round trips a cell, where a component at a time made
+// nine).  A 236x236x76 gyrotropic layer took 84 + 102 us in two passes and takes
+// 83; the Drude film of the reference geometry (8 cells along z, so lanes run along
+// y and z together) 76 -> 32 us.
+template <int ORDER, bool BOX, bool CUR>
+__global__ void __launch_bounds__(256) ade_node_kernel(const __grid_constant__ Params p, int cur) {
   const MatTable& mt = *p.mt;
   int bi, bj, bk;
   long long q;
-  if (ade_cell(p, bi, bj, bk, q)) {
-    const int i = p.ade.lo[0] + bi, j = p.ade.lo[1] + bj, k = p.ade.lo[2] + bk;
-    const long long id = (long long)i * p.g.sx + (long long)j * p.g.sy + k;
-    const int idx[3] = {i, j, k};
+  if (!ade_cell(p, bi, bj, bk, q)) return;
+  const int i = p.ade.lo[0] + bi, j = p.ade.lo[1] + bj, k = p.ade.lo[2] + bk;
+  const long long id = (long long)i * p.g.sx + (long long)j * p.g.sy + k;
+  // (materials, table, H and the old E are read-only in this pass)
+  int m[3], np[3];
+  float gj[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) m[c] = p.mat[c] ? (int)__ldg(p.mat[c] + id) : 0;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const bool live = BOX || is_live(p.g, c, i, j, k);
+    np[c] = live ? __ldg(&mt.npoles[m[c]]) : 0;
+    gj[c] = live ? __ldg(&mt.gjc[m[c]]) : 0.f;
+  }
+  if (np[0] > 0 || np[1] > 0 || np[2] > 0) {
+    // taps of H: the node's own and, per curl term, those along its axis (E taps at -1..+2)
+    float v[3][2][4], E0[3];
+    bool inside = true;
+    if (!BOX) {
+      const int ix[3] = {i, j, k};
+#pragma unroll
+      for (int a = 0; a < 3; a++) inside = inside && ix[a] - 1 >= p.g.all_lo[a] && ix[a] + 2 <= p.g.all_hi[a];
+    }
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      if (!is_live(p.g, c, i, j, k)) continue;
-      // (materials, table, H and the new current are read-only in this pass)
-      const int m = p.mat[c] ? (int)__ldg(p.mat[c] + id) : 0;
-      const int np = __ldg(&mt.npoles[m]);
-      if (np > 0) {
-        float d[3] = {0.f, 0.f, 0.f};
+      if (np[c] <= 0) continue;
+      E0[c] = p.fe_old[c] ? __ldg(p.fe_old[c] + id) : p.f[c][id];
 #pragma unroll
-        for (int t = 0; t < 2; t++) {
-          const int a = (c + 1 + t) % 3;             // curl axis of term t
-          const int g = 3 + (c + 2 - t) % 3;         // source H component of term t
-          float v[4];
+      for (int t = 0; t < 2; t++) {
+        const int a = (c + 1 + t) % 3;             // curl axis of term t
+        const int g = 3 + (c + 2 - t) % 3;         // source H component of term t
+        const long long sa = a == 0 ? p.g.sx : a == 1 ? p.g.sy : 1;
+        const int ia = a == 0 ? i : a == 1 ? j : k;
 #pragma unroll
-          for (int o = 0; o < 4; o++) {
-            v[o] = 0.f;
-            if (ORDER == 2 && (o == 0 || o == 3)) continue;
-            int m3[3] = {i, j, k};
-            m3[a] += o - 1;                          // E taps at -1..+2
-            if (BOX) {
-              const long long sa = a == 0 ? p.g.sx : a == 1 ? p.g.sy : 1;
-              v[o] = (m3[a] >= 0 && m3[a] < p.g.n[a]) ? __ldg(p.f[g] + id + (long long)(o - 1) * sa) : 0.f;
-            } else {
-              v[o] = fetch<1>(p, g, m3[0], m3[1], m3[2]);
-            }
+        for (int o = 0; o < 4; o++) {
+          v[c][t][o] = 0.f;
+          if (ORDER == 2 && (o == 0 || o == 3)) continue;
+          if (BOX || inside) {
+            if (!BOX || (ia + o - 1 >= 0 && ia + o - 1 < p.g.n[a])) v[c][t][o] = __ldg(p.f[g] + id + (long long)(o - 1) * sa);
+          } else {
+            v[c][t][o] = fetch<1>(p, g, a == 0 ? i + o - 1 : i, a == 1 ? j + o - 1 : j, a == 2 ? k + o - 1 : k);
           }
-          d[a] = __fmul_rn(t == 0 ? p.cdt[a] : -p.cdt[a], dstencil<ORDER>(v[0], v[1], v[2], v[3]));
         }
-        (void)idx;
-        const float E0 = p.fe_old[c] ? __ldg(p.fe_old[c] + id) : p.f[c][id];
-        p.f[c][id] = ade_update(p, c, m, np, q, sum3(d[0], d[1], d[2]), E0);
-      } else if (__ldg(&mt.gjc[m]) != 0.f) {
-        p.f[c][id] = __fsub_rn(p.f[c][id], __fmul_rn(__ldg(&mt.gjc[m]), __ldg(p.ade.Jg[p.ade.gnew][c] + q)));
       }
     }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (np[c] <= 0) continue;
+      float d[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+      for (int t = 0; t < 2; t++) {
+        const int a = (c + 1 + t) % 3;
+        d[a] = __fmul_rn(t == 0 ? p.cdt[a] : -p.cdt[a], dstencil<ORDER>(v[c][t][0], v[c][t][1], v[c][t][2], v[c][t][3]));
+      }
+      p.f[c][id] = ade_update(p, c, m[c], np[c], q, sum3(d[0], d[1], d[2]), E0[c]);
+    }
   }
+  bool on[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) on[c] = np[c] <= 0 && gj[c] != 0.f;
+  if (!(on[0] || on[1] || on[2])) return;
+  float J[3], F[3];
+  if (CUR) {
+    float E[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) { F[c] = on[c] ? p.f[c][id] : 0.f; E[c] = on[c] ? __ldg(p.fe_old[c] + id) : 0.f; }
+    gyro_new(p, cur, i, j, k, q, m, E, on, J);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      if (on[c]) p.ade.Jg[1 - cur][c][q] = J[c];
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      F[c] = on[c] ? p.f[c][id] : 0.f;
+      J[c] = on[c] ? __ldg(p.ade.Jg[1 - cur][c] + q) : 0.f;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    if (on[c]) p.f[c][id] = __fsub_rn(F[c], __fmul_rn(gj[c], J[c]));
 }
 
 __global__ void mask_nonlive_kernel(Params p, int comp, long long ncell) {

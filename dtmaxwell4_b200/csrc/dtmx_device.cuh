@@ -254,15 +254,19 @@ __device__ __forceinline__ float ade_update(const Params& p, int c, int m, int n
   const float Em = p.ade.Em[c][ai];
   const float Etmp = F;
   float sum = 0.f;
-  float jp[MAXPOLE], jm[MAXPOLE];
-  for (int q = 0; q < np; q++) {
-    jp[q] = p.ade.Jp[c][q][ai]; jm[q] = p.ade.Jm[c][q][ai];
-    sum = __fadd_rn(sum, __fmaf_rn(__ldg(&mt.kEJ[m][c][q][0]), jp[q], __fmul_rn(__ldg(&mt.kEJ[m][c][q][1]), jm[q])));
-  }
+  float jp[MAXPOLE] = {}, jm[MAXPOLE] = {};
+#pragma unroll
+  for (int q = 0; q < MAXPOLE; q++)
+    if (q < np) { jp[q] = p.ade.Jp[c][q][ai]; jm[q] = p.ade.Jm[c][q][ai]; }
+#pragma unroll
+  for (int q = 0; q < MAXPOLE; q++)
+    if (q < np) sum = __fadd_rn(sum, __fmaf_rn(__ldg(&mt.kEJ[m][c][q][0]), jp[q], __fmul_rn(__ldg(&mt.kEJ[m][c][q][1]), jm[q])));
   const float Ep = __fsub_rn(__fmaf_rn(__ldg(&mt.kE[m][c][0]), Em,
                                        __fmaf_rn(__ldg(&mt.kE[m][c][1]), F, __fmul_rn(__ldg(&mt.kE[m][c][2]), rot))),
                              sum);
-  for (int q = 0; q < np; q++) {
+#pragma unroll
+  for (int q = 0; q < MAXPOLE; q++) {
+    if (q >= np) continue;
     float a = __fmul_rn(__ldg(&mt.kJ[m][c][q][4]), Etmp);
     a = __fmaf_rn(__ldg(&mt.kJ[m][c][q][3]), Em, a);
     a = __fmaf_rn(__ldg(&mt.kJ[m][c][q][2]), Ep, a);
