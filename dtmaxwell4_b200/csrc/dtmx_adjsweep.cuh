@@ -361,10 +361,17 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
   const int len = x1 - x0;
   const int slast = len + 1;                               // stages 0 .. len + 1: planes x0 - 1 .. x1
   const bool cpml = p.ab.kind == 1;
+  auto issue = [&](int s, bool want_mat) {
+    fused_issue<TY>(m, fsm + (s % F_NST) * L::STAGE, &bars[s % F_NST], x0 - 1 + s, j0, k0, want_mat);
+  };
+  int issued = -1;
   if (tid == 0) {
     for (int q = 0; q < F_NST; q++) mbar_init(&bars[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     gave_up = 0;
+    // the first two stages hold no material tile: they need not wait for the tables below
+    pdl_wait();
+    for (int s = 0; s < 2; s++) { issue(s, false); issued = s; }
   }
   for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
   for (int q = tid; q < len; q += L::NT)
@@ -389,14 +396,11 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
       }
     }
   }
+  pdl_wait();
+  pdl_trigger();
   __syncthreads();
-  auto issue = [&](int s) {
-    const int ip = x0 - 1 + s;
-    fused_issue<TY>(m, fsm + (s % F_NST) * L::STAGE, &bars[s % F_NST], ip, j0, k0, ip - 1 >= x0 && umc[ip - 1 - x0] < 0);
-  };
-  int issued = -1;
-  if (tid == 0)
-    for (int s = 0; s < F_NST && s <= slast; s++) { issue(s); issued = s; }
+  // stage s: plane x0 - 1 + s, with the materials of the plane before it (s >= 2)
+  if (tid == 0 && slast >= 2) { issue(2, umc[0] < 0); issued = 2; }
   FNode f;
   f.y = tid >> 3; f.z = 4 * (tid & 7);
   f.j = j0 + f.y; f.k = k0 + f.z;
@@ -467,7 +471,7 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
       // plane written two iterations ago are free
       __syncthreads();
       if (gave_up) break;
-      if (tid == 0 && t + F_NST <= slast) { issue(t + F_NST); issued = t + F_NST; }
+      if (tid == 0 && t + F_NST <= slast) { issue(t + F_NST, umc[t + F_NST - 2] < 0); issued = t + F_NST; }
       const float* st = fsm + (s % F_NST) * L::STAGE;
       float* hn1 = hnb + (t & 1) * L::HN;                        // new G of plane pc
       const float* hn0 = hnb + ((t + 1) & 1) * L::HN;            // new G of plane pc - 1
@@ -518,6 +522,8 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
 // design region share no node in one launch: the gradient reads U after the sources.
 __global__ void __launch_bounds__(256) adj_pre_kernel(const __grid_constant__ Params p, const __grid_constant__ AdjDev A, const double* F,
                                                       long long s, int X, double omega, double dt, int ns, int st) {
+  pdl_wait();
+  pdl_trigger();
   if ((int)blockIdx.x < ns) {
     __shared__ double ph[4];
     if (threadIdx.x < 2) {
@@ -564,7 +570,9 @@ __global__ void __launch_bounds__(256) adj_pre_kernel(const __grid_constant__ Pa
 // Transposed ADE recursion before the sweep (the recursion of adj_ade_kernel):
 // the sweep left curl G' in the U array of a dispersive node, lE holds the rest of
 // its lam_E; writes kE2 mu for the node's taps.
-__global__ void adj_ade_sweep_kernel(Params p, AdjDev A) {
+__global__ void __launch_bounds__(256) adj_ade_sweep_kernel(const __grid_constant__ Params p, const __grid_constant__ AdjDev A) {
+  pdl_wait();
+  pdl_trigger();
   const MatTable& mt = *p.mt;
   int bi, bj, bk;
   long long q;

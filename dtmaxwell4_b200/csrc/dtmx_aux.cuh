@@ -150,7 +150,9 @@ __device__ __forceinline__ bool in_job(const TfsfJob& jb, int i, int j, int k) {
 // earlier job of the same component is left to that job, so every node is
 // corrected exactly once with the sum of all its crossing taps.
 template <int ORDER>
-__global__ void tfsf_kernel(Params p, TfsfDev t, const long long* d_step, int isH) {
+__global__ void tfsf_kernel(const __grid_constant__ Params p, const __grid_constant__ TfsfDev t, const long long* d_step, int isH) {
+  pdl_wait();
+  pdl_trigger();
   const long long n = *d_step;
   if (!tfsf_on(t, n)) return;
   const int hs = isH ? 1 : 0;
@@ -227,6 +229,8 @@ __device__ __forceinline__ void line_update(const LineDev& l, bool isH, long lon
 template <int ORDER>
 __global__ void __launch_bounds__(256) tfsf_plane_kernel(const __grid_constant__ Params p, const __grid_constant__ TfsfDev t, const LineDev l,
                                                          const long long* d_step, int isH) {
+  pdl_wait();
+  pdl_trigger();
   const long long n = *d_step;
   const int hs = isH ? 1 : 0, r = blockIdx.y;
   if (r == t.njob[hs]) {                           // the line's own update
@@ -300,7 +304,9 @@ __device__ __forceinline__ float source_value(const PointSrcDev& s, long long n,
 
 // More soft sources than the tail kernel's list holds.  Sources on one node are
 // added in their order by the first of them.
-__global__ void point_source_kernel(Params p, const PointSrcDev* s, int ns, const long long* d_step, double dt) {
+__global__ void point_source_kernel(const __grid_constant__ Params p, const PointSrcDev* s, int ns, const long long* d_step, double dt) {
+  pdl_wait();
+  pdl_trigger();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= ns) return;
   for (int e = 0; e < q; e++)
@@ -373,6 +379,8 @@ __global__ void __launch_bounds__(256) tail_kernel(const __grid_constant__ Param
   __shared__ TailSources s;
   __shared__ bool last;
   const int tid = threadIdx.x, b = blockIdx.x;
+  pdl_wait();
+  pdl_trigger();
   const long long n = *d_step;
   if (tid < a.ns) {
     const PointSrcDev& q = a.src[tid];
@@ -702,6 +710,8 @@ __device__ __forceinline__ void gyro_new(const Params& p, int cur, int i, int j,
 
 // J^{n+1/2} into buffer 1-cur (per-step engine: before the E half step changes E)
 __global__ void __launch_bounds__(256) gyro_current_kernel(const __grid_constant__ Params p, int cur) {
+  pdl_wait();
+  pdl_trigger();
   int bi, bj, bk;
   long long q;
   if (!ade_cell(p, bi, bj, bk, q)) return;
@@ -735,6 +745,8 @@ __global__ void __launch_bounds__(256) gyro_current_kernel(const __grid_constant
 // y and z together) 76 -> 32 us.
 template <int ORDER, bool BOX, bool CUR>
 __global__ void __launch_bounds__(256) ade_node_kernel(const __grid_constant__ Params p, int cur) {
+  pdl_wait();
+  pdl_trigger();
   const MatTable& mt = *p.mt;
   int bi, bj, bk;
   long long q;

@@ -26,6 +26,15 @@ constexpr int TYT = 16;          // tile extent along y
 constexpr int MAXMAT = 64;
 constexpr int MAXPOLE = 2;
 
+// Programmatic dependent launch.  A step is a chain of launches on one stream, on
+// small grids of a few microseconds each.  Every kernel of the chain lets the
+// next one start its set-up (pdl_trigger) and itself waits for the one before
+// (pdl_wait) ahead of anything that one may have written; what comes before
+// the wait reads only tables that no step changes.  Each kernel waits in all
+// its threads, so a finished kernel means that all before it have finished.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // half-cell offset of component c along axis a (lattice in dtmx.h)
 __host__ __device__ __forceinline__ int comp_off(int c, int a) { return c < 3 ? (a != c) : (a == c - 3); }
 

@@ -382,10 +382,17 @@ __global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
   const int len = x1 - x0;
   const int slast = len + 1;                               // stages 0 .. len + 1: planes x0 - 1 .. x1
   const bool cpml = p.ab.kind == 1;
+  auto issue = [&](int s, bool want_mat) {
+    fused_issue<TY>(m, fsm + (s % F_NST) * L::STAGE, &bars[s % F_NST], x0 - 1 + s, j0, k0, want_mat);
+  };
+  int issued = -1;
   if (tid == 0) {
     for (int q = 0; q < F_NST; q++) mbar_init(&bars[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     gave_up = 0;
+    // the first two stages hold no material tile: they need not wait for the tables below
+    pdl_wait();
+    for (int s = 0; s < 2; s++) { issue(s, false); issued = s; }
   }
   for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
   for (int q = tid; q < len; q += L::NT)
@@ -410,14 +417,11 @@ __global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
       }
     }
   }
+  pdl_wait();
+  pdl_trigger();
   __syncthreads();
-  auto issue = [&](int s) {
-    const int ip = x0 - 1 + s;
-    fused_issue<TY>(m, fsm + (s % F_NST) * L::STAGE, &bars[s % F_NST], ip, j0, k0, ip - 1 >= x0 && umc[ip - 1 - x0] < 0);
-  };
-  int issued = -1;
-  if (tid == 0)
-    for (int s = 0; s < F_NST && s <= slast; s++) { issue(s); issued = s; }
+  // stage s: plane x0 - 1 + s, with the materials of the plane before it (s >= 2)
+  if (tid == 0 && slast >= 2) { issue(2, umc[0] < 0); issued = 2; }
   // per-thread constants of the walk
   FNode f;
   f.y = tid >> 3; f.z = 4 * (tid & 7);
@@ -484,7 +488,7 @@ __global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
       // plane written two iterations ago are free
       __syncthreads();
       if (gave_up) break;
-      if (tid == 0 && t + F_NST <= slast) { issue(t + F_NST); issued = t + F_NST; }
+      if (tid == 0 && t + F_NST <= slast) { issue(t + F_NST, umc[t + F_NST - 2] < 0); issued = t + F_NST; }
       const float* st = fsm + (s % F_NST) * L::STAGE;
       float* hn1 = hnb + (t & 1) * L::HN;                        // new H of plane pc
       const float* hn0 = hnb + ((t + 1) & 1) * L::HN;            // new H of plane pc - 1

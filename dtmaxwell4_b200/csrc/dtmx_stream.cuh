@@ -266,6 +266,7 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
     coeff(2, k0 + tid, c);
     zc[0][tid] = c[0]; zc[1][tid] = c[1]; zc[2][tid] = c[2];
   }
+  pdl_wait();
   __syncthreads();
   // uniform material of stage number sq (0 for planes outside the array)
   auto um_of = [&](int sq) -> int {
