@@ -1361,7 +1361,7 @@ static long long launch_tfsf(dtmx_ctx* ctx, const Params& P, cudaStream_t st, bo
   }
   long long mx = 1;
   for (int r = 0; r < T.njob[hs]; r++) mx = std::max(mx, T.job[hs][r].cells);
-  const dim3 grd((unsigned)((mx + 255) / 256), std::max(1, T.njob[hs]));
+  const dim3 grd((unsigned)((mx * 8 + 255) / 256), std::max(1, T.njob[hs]));
   if (o4) launch_after(ctx->early, tfsf_kernel<4>, grd, 256, 0, st, P, T, ctx->d_step, isH);
   else launch_after(ctx->early, tfsf_kernel<2>, grd, 256, 0, st, P, T, ctx->d_step, isH);
   return 1;

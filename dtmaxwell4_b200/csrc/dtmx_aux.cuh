@@ -70,13 +70,6 @@ __device__ double dipole_field(const TfsfDev& t, int comp, int X, int Y, int Z, 
   return b1 / (c * c * R) + b2 / (c * R * R);
 }
 
-__device__ __forceinline__ double incident(const TfsfDev& t, int g, int X, int Y, int Z, double tt) {
-  if (t.kind == 0) return dipole_field(t, g, X, Y, Z, tt);
-  if (g == 2) { const int m = ((X - 1) >> 1) + t.line_M; return (m >= 0 && m < t.line_n) ? t.line_e[m] : 0.0; }
-  if (g == 4) { const int m = (X >> 1) + t.line_M; return (m >= 0 && m < t.line_n) ? t.line_h[m] : 0.0; }
-  return 0.0;
-}
-
 // curl terms of component c: {axis, source component} for (+) and (-) terms
 __host__ __device__ __forceinline__ void curl_terms(int c, int& a0, int& g0, int& a1, int& g1) {
   switch (c) {
@@ -94,63 +87,41 @@ __host__ __device__ __forceinline__ void curl_terms(int c, int& a0, int& g0, int
 // inside, -inc in the opposite case.  The update is linear in the taps, so
 // the correction is added after the bulk update as dt/d * D(corrections),
 // summed over both curl terms of the node in double precision.
+// This is the part of one tap: q of curl term `term` (0 where the tap does not
+// cross or the term cannot).
 template <int ORDER>
-__device__ __forceinline__ bool tfsf_node(const Params& p, const TfsfDev& t, int c, int i, int j, int k, bool isH,
-                                          double tt, double& total) {
-  const int t0 = isH ? -2 : -1;
-  const int idx[3] = {i, j, k};
-  const int Xs[3] = {2 * i + comp_off(c, 0), 2 * j + comp_off(c, 1), 2 * k + comp_off(c, 2)};
+__device__ __forceinline__ double tfsf_tap(const Params& p, const TfsfDev& t, int c, int i, int j, int k, bool isH, double tt, int term, int q) {
+  if (ORDER == 2 && (q == 0 || q == 3)) return 0.0;
   int ax[2], gs[2];
   curl_terms(c, ax[0], gs[0], ax[1], gs[1]);
-  total = 0.0;
-  bool any = false;
-  bool self_known = false, self_in = false;
-  for (int term = 0; term < 2; term++) {
-    const int a = ax[term], g = gs[term];
-    // the plane wave has only Ez and Hy incident components
-    if (t.kind == 1 && g != 2 && g != 4) continue;
-    // a tap along a crosses the surface only if the node lies inside the box
-    // range on the other two axes and within 3 half cells of a face along a
-    const int b1 = (a + 1) % 3, b2 = (a + 2) % 3;
-    const int gb1 = 2 * idx[b1] + comp_off(g, b1), gb2 = 2 * idx[b2] + comp_off(g, b2);
-    if (gb1 < t.lo[b1] || gb1 > t.hi[b1] || gb2 < t.lo[b2] || gb2 > t.hi[b2]) continue;
-    const int Xa = Xs[a];
-    if (!((Xa >= t.lo[a] - 4 && Xa <= t.lo[a] + 3) || (Xa >= t.hi[a] - 3 && Xa <= t.hi[a] + 4))) continue;
-    if (!self_known) { self_in = in_box(t, Xs[0], Xs[1], Xs[2]); self_known = true; }
-    double v[4];
-    bool hit = false;
-    for (int q = 0; q < 4; q++) {
-      v[q] = 0.0;
-      if (ORDER == 2 && (q == 0 || q == 3)) continue;
-      int m[3] = {idx[0], idx[1], idx[2]};
-      m[a] += t0 + q;
-      const int TX = 2 * m[0] + comp_off(g, 0), TY_ = 2 * m[1] + comp_off(g, 1), TZ_ = 2 * m[2] + comp_off(g, 2);
-      const bool tin = in_box(t, TX, TY_, TZ_);
-      if (tin != self_in) {
-        const double inc = incident(t, g, TX, TY_, TZ_, tt);
-        v[q] = self_in ? -inc : inc;
-        hit = true;
-      }
-    }
-    if (!hit) continue;
-    any = true;
-    double sg = term == 0 ? 1.0 : -1.0;
-    if (isH) sg = -sg;
-    const double dv = ORDER == 2 ? v[2] - v[1] : (27.0 * (v[2] - v[1]) - (v[3] - v[0])) / 24.0;
-    total += sg * (double)p.cdt[a] * dv;
-  }
-  return any;
+  const int a = term ? ax[1] : ax[0], g = term ? gs[1] : gs[0];
+  const int t0 = (isH ? -2 : -1) + q;
+  const int S[3] = {2 * i + comp_off(c, 0), 2 * j + comp_off(c, 1), 2 * k + comp_off(c, 2)};
+  const int G[3] = {2 * (i + (a == 0 ? t0 : 0)) + comp_off(g, 0), 2 * (j + (a == 1 ? t0 : 0)) + comp_off(g, 1),
+                    2 * (k + (a == 2 ? t0 : 0)) + comp_off(g, 2)};
+  const bool sin_ = in_box(t, S[0], S[1], S[2]);
+  if (in_box(t, G[0], G[1], G[2]) == sin_) return 0.0;
+  // (a tap differs from its node along a alone, so it is the face along a that it crosses)
+  const double w = ORDER == 2 ? (q == 2 ? 1.0 : -1.0) : q == 0 ? 1.0 / 24.0 : q == 1 ? -27.0 / 24.0 : q == 2 ? 27.0 / 24.0 : -1.0 / 24.0;
+  double sg = term == 0 ? 1.0 : -1.0;
+  if (isH) sg = -sg;
+  const double inc = dipole_field(t, g, G[0], G[1], G[2], tt);
+  return sg * (double)p.cdt[a] * w * (sin_ ? -inc : inc);
 }
 
 __device__ __forceinline__ bool in_job(const TfsfJob& jb, int i, int j, int k) {
   return i >= jb.lo[0] && i <= jb.hi[0] && j >= jb.lo[1] && j <= jb.hi[1] && k >= jb.lo[2] && k <= jb.hi[2];
 }
 
-// One thread per node of a job (blockIdx.y); a node that also lies in an
-// earlier job of the same component is left to that job, so every node is
-// corrected exactly once with the sum of all its crossing taps.
+// Eight threads per node of a job (blockIdx.y), one for each tap of both curl
+// terms: the incident field of a tap is a chain of FP64 sines, and one thread
+// that walked a node's taps took 10 us a half step for any box (the jobs are far
+// too small to fill the chip).  A node that also lies in an earlier job of the
+// same component is left to that job, so every node is corrected exactly once
+// with the sum of all its crossing taps.
 template <int ORDER>
-__global__ void tfsf_kernel(const __grid_constant__ Params p, const __grid_constant__ TfsfDev t, const long long* d_step, int isH) {
+__global__ void __launch_bounds__(256) tfsf_kernel(const __grid_constant__ Params p, const __grid_constant__ TfsfDev t, const long long* d_step,
+                                                   int isH) {
   pdl_wait();
   pdl_trigger();
   const long long n = *d_step;
@@ -160,20 +131,20 @@ __global__ void tfsf_kernel(const __grid_constant__ Params p, const __grid_const
   if (r >= t.njob[hs]) return;
   const TfsfJob& jb = t.job[hs][r];
   // a job is a thin shell (cells < 2^31, checked when the jobs are built): 32-bit indexing
-  const int cell = blockIdx.x * blockDim.x + threadIdx.x;
-  if (cell >= (int)jb.cells) return;
+  const long long cell8 = (long long)blockIdx.x * 256 + threadIdx.x;
+  const int cell = (int)min(cell8 >> 3, jb.cells - 1);          // (threads past the end help the last node and store nothing)
   const int ey = jb.hi[1] - jb.lo[1] + 1, ez = jb.hi[2] - jb.lo[2] + 1;
   const int i = jb.lo[0] + cell / (ey * ez);
   const int rest = cell - (i - jb.lo[0]) * (ey * ez);
   const int j = jb.lo[1] + rest / ez;
   const int k = jb.lo[2] + (rest - (j - jb.lo[1]) * ez);
   const int c = jb.c;
-  if (!is_live(p.g, c, i, j, k)) return;
+  double total = tfsf_tap<ORDER>(p, t, c, i, j, k, isH, isH ? (double)n : (double)n + 0.5, (threadIdx.x >> 2) & 1, threadIdx.x & 3);
+#pragma unroll
+  for (int s = 1; s < 8; s <<= 1) total += __shfl_xor_sync(0xffffffffu, total, s);
+  if ((threadIdx.x & 7) != 0 || (cell8 >> 3) >= jb.cells || total == 0.0 || !is_live(p.g, c, i, j, k)) return;
   for (int q = 0; q < r; q++)
     if (t.job[hs][q].c == c && in_job(t.job[hs][q], i, j, k)) return;
-  const double tt = isH ? (double)n : (double)n + 0.5;
-  double total;
-  if (!tfsf_node<ORDER>(p, t, c, i, j, k, isH, tt, total)) return;
   const long long id = (long long)i * p.g.sx + (long long)j * p.g.sy + k;
   if (!isH) {
     const int mi = p.mat[c] ? (int)p.mat[c][id] : 0;
