@@ -104,13 +104,48 @@ __device__ __forceinline__ Q4 psi_old(const Params& p, const float* q, int a, in
   return aux4<true>(q + slab_at(p, a, i, j, k, s), vec, m);
 }
 
+// The old psi of the thread's nodes: what the G update of plane i reads (U's
+// slots on all axes, own nodes; the row below) and what the U update of plane i
+// reads (G's slots along y and z), requested before the stage wait.
+struct AdjPsi {
+  Q4 g[3][2], gm[2], u[2][2];
+};
+__device__ __forceinline__ void adj_psi_g(const Params& p, const AdjSweepArgs& fa, const FNode& f, const AdjNode& an, int i, int xs, AdjPsi& o) {
+  const unsigned nm = (1u << f.nv) - 1u;
+  if (f.nv > 0) {
+    if (xs >= 0)
+#pragma unroll
+      for (int q = 0; q < 2; q++) o.g[0][q] = psi_old(p, fa.psrc[0][q], 0, i, f.j, f.k, xs, f.vxy, nm);
+    if (f.ys >= 0)
+#pragma unroll
+      for (int q = 0; q < 2; q++) o.g[1][q] = psi_old(p, fa.psrc[1][q], 1, i, f.j, f.k, f.ys, f.vxy, nm);
+    if (f.zm)
+#pragma unroll
+      for (int q = 0; q < 2; q++) o.g[2][q] = psi_old(p, fa.psrc[2][q], 2, i, f.j, f.k, f.zs, f.vz, f.zm);
+  }
+  const unsigned cm = (1u << min(4, max(0, p.g.n[2] - f.k))) - 1u;   // columns inside the grid, whatever the row
+  if (an.ysm >= 0 && cm)
+#pragma unroll
+    for (int q = 0; q < 2; q++) o.gm[q] = psi_old(p, fa.psrc[1][q], 1, i, f.j - 1, f.k, an.ysm, f.vxy, cm);
+}
+__device__ __forceinline__ void adj_psi_u(const Params& p, const AdjSweepArgs& fa, const FNode& f, int i, AdjPsi& o) {
+  if (f.nv == 0) return;
+  const unsigned nm = (1u << f.nv) - 1u;
+  if (f.ys >= 0)
+#pragma unroll
+    for (int q = 0; q < 2; q++) o.u[0][q] = psi_old(p, fa.psrc[1][2 + q], 1, i, f.j, f.k, f.ys, f.vxy, nm);
+  if (f.zm)
+#pragma unroll
+    for (int q = 0; q < 2; q++) o.u[1][q] = psi_old(p, fa.psrc[2][2 + q], 2, i, f.j, f.k, f.zs, f.vz, f.zm);
+}
+
 // New G of plane i on the thread's nodes; ec gets the old U, ux the stretched
 // old Uy, Uz of this plane (x taps of the next one; in: those of plane i - 1), hcx
 // the stretched new Gy, Gz (x taps of the U update).
 template <int TY, bool ABS>
 __device__ __forceinline__ void adj_g_own(const Params& p, const AdjSweepArgs& fa, const float* st, float* hn, const FNode& f,
                                           const AdjNode& an, int i, bool store, Q4 (&ux)[2], Q4 (&hc)[3], Q4 (&hcx)[2], Q4 (&ec)[3],
-                                          const float* fco, int xrow, int xs) {
+                                          const float* fco, int xrow, int xs, const AdjPsi& ps) {
   const float cx = p.cdt[0], cy = p.cdt[1], cz = p.cdt[2];
   const Q4 ex = ld4(fE<TY>(st, 0, f.y, f.z)), ey = ld4(fE<TY>(st, 1, f.y, f.z)), ez = ld4(fE<TY>(st, 2, f.y, f.z));
   ec[0] = ex; ec[1] = ey; ec[2] = ez;
@@ -124,12 +159,11 @@ __device__ __forceinline__ void adj_g_own(const Params& p, const AdjSweepArgs& f
     d20 = diff4(-cx, ey, ux[0]); d21 = diff4(cy, ex, exm);
     ux[0] = ey; ux[1] = ez;
   } else {
-    const Q4 zero{{0.f, 0.f, 0.f, 0.f}};
     // x: Uy (slot 0), Uz (slot 1)
     Q4 xy = ey, xz = ez;
     if (xs >= 0 && f.nv > 0) {
       const Str4 c = str_same(cfx<TY>(fco, xrow, 3));
-      const Q4 p0 = psi_old(p, fa.psrc[0][0], 0, i, f.j, f.k, xs, f.vxy, nm), p1 = psi_old(p, fa.psrc[0][1], 0, i, f.j, f.k, xs, f.vxy, nm);
+      const Q4 p0 = ps.g[0][0], p1 = ps.g[0][1];
       xy = stretch4(ey, p0, c); xz = stretch4(ez, p1, c);
       if (store) {
         const int s = slab_at(p, 0, i, f.j, f.k, xs);
@@ -144,7 +178,7 @@ __device__ __forceinline__ void adj_g_own(const Params& p, const AdjSweepArgs& f
     const unsigned cm = (1u << min(4, max(0, p.g.n[2] - f.k))) - 1u;   // columns inside the grid, whatever the row
     if (f.ys >= 0 && f.nv > 0) {
       const Str4 c = str_same(cfy<TY>(fco, f.y, 3));
-      const Q4 p0 = psi_old(p, fa.psrc[1][0], 1, i, f.j, f.k, f.ys, f.vxy, nm), p1 = psi_old(p, fa.psrc[1][1], 1, i, f.j, f.k, f.ys, f.vxy, nm);
+      const Q4 p0 = ps.g[1][0], p1 = ps.g[1][1];
       yx = stretch4(ex, p0, c); yz = stretch4(ez, p1, c);
       if (store) {
         const int s = slab_at(p, 1, i, f.j, f.k, f.ys);
@@ -154,15 +188,15 @@ __device__ __forceinline__ void adj_g_own(const Params& p, const AdjSweepArgs& f
     }
     if (an.ysm >= 0 && cm) {
       const Str4 c = str_same(cfy<TY>(fco, f.y - 1, 3));
-      yxm = stretch4(exm, psi_old(p, fa.psrc[1][0], 1, i, f.j - 1, f.k, an.ysm, f.vxy, cm), c);
-      yzm = stretch4(ezm, psi_old(p, fa.psrc[1][1], 1, i, f.j - 1, f.k, an.ysm, f.vxy, cm), c);
+      yxm = stretch4(exm, ps.gm[0], c);
+      yzm = stretch4(ezm, ps.gm[1], c);
     }
     d01 = diff4(-cy, yz, yzm); d21 = diff4(cy, yx, yxm);
     // z: Ux (slot 0), Uy (slot 1), own columns and the one below
     Q4 zx = ex, zy = ey;
     if (f.zm) {
       const Str4 c = str_cols(cfz<TY>(fco, f.z, 3), AL<TY>::ZS);
-      const Q4 p0 = psi_old(p, fa.psrc[2][0], 2, i, f.j, f.k, f.zs, f.vz, f.zm), p1 = psi_old(p, fa.psrc[2][1], 2, i, f.j, f.k, f.zs, f.vz, f.zm);
+      const Q4 p0 = ps.g[2][0], p1 = ps.g[2][1];
       zx = stretch4(ex, p0, c); zy = stretch4(ey, p1, c);
       if (store) {
         const int s = slab_at(p, 2, i, f.j, f.k, f.zs);
@@ -181,7 +215,6 @@ __device__ __forceinline__ void adj_g_own(const Params& p, const AdjSweepArgs& f
       }
     }
     d02 = diff4(cz, zy, below4(ly, zy)); d12 = diff4(-cz, zx, below4(lx, zx));
-    (void)zero;
   }
   hc[0] = add4(ld4(fHx<TY>(st, f.y, f.z)), add4(d01, d02));
   hc[1] = add4(ld4(fHy<TY>(st, f.y, f.z)), add4(d10, d12));
@@ -261,7 +294,7 @@ __device__ __forceinline__ void adj_g_halo(const Params& p, const AdjSweepArgs& 
 template <int TY, int MODE, bool ABS>
 __device__ __forceinline__ void adj_u_own(const Params& p, const AdjSweepArgs& fa, const float* st, const float* hn, const float* ies, int um,
                                           const FNode& f, const AdjNode& an, int i, const Q4 (&ep)[3], const Q4 (&hpx)[2],
-                                          const Q4 (&hcx)[2], const float* fco) {
+                                          const Q4 (&hcx)[2], const float* fco, const AdjPsi& ps) {
   const float cx = p.cdt[0], cy = p.cdt[1], cz = p.cdt[2];
   const Q4 hx = ld4(fN<TY>(hn, 0, f.y, f.z)), hy = ld4(fN<TY>(hn, 1, f.y, f.z)), hz = ld4(fN<TY>(hn, 2, f.y, f.z));
   const Q4 hxp = ld4(fN<TY>(hn, 0, f.y + 1, f.z)), hzp = ld4(fN<TY>(hn, 2, f.y + 1, f.z));
@@ -277,7 +310,7 @@ __device__ __forceinline__ void adj_u_own(const Params& p, const AdjSweepArgs& f
     Q4 yx = hx, yz = hz, yxp = hxp, yzp = hzp;
     if (f.ys >= 0 && f.nv > 0) {
       const Str4 c = str_same(cfy<TY>(fco, f.y, 0));
-      const Q4 p0 = psi_old(p, fa.psrc[1][2], 1, i, f.j, f.k, f.ys, f.vxy, nm), p1 = psi_old(p, fa.psrc[1][3], 1, i, f.j, f.k, f.ys, f.vxy, nm);
+      const Q4 p0 = ps.u[0][0], p1 = ps.u[0][1];
       yx = stretch4(hx, p0, c); yz = stretch4(hz, p1, c);
       const int s = slab_at(p, 1, i, f.j, f.k, f.ys);
       put4(fa.pdst[1][2] + s, f.vxy, nm, psi4(hx, p0, c));
@@ -293,7 +326,7 @@ __device__ __forceinline__ void adj_u_own(const Params& p, const AdjSweepArgs& f
     Q4 zx = hx, zy = hy;
     if (f.zm) {
       const Str4 c = str_cols(cfz<TY>(fco, f.z, 0), AL<TY>::ZS);
-      const Q4 p0 = psi_old(p, fa.psrc[2][2], 2, i, f.j, f.k, f.zs, f.vz, f.zm), p1 = psi_old(p, fa.psrc[2][3], 2, i, f.j, f.k, f.zs, f.vz, f.zm);
+      const Q4 p0 = ps.u[1][0], p1 = ps.u[1][1];
       zx = stretch4(hx, p0, c); zy = stretch4(hy, p1, c);
       const int s = slab_at(p, 2, i, f.j, f.k, f.zs);
       put4(fa.pdst[2][2] + s, f.vz, f.zm, psi4(hx, p0, c));
@@ -439,6 +472,7 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
   const bool ab_yz = cpml && (j0 - 1 < p.ab.L[1][0] || j0 + TY + 1 > p.g.n[1] - p.ab.L[1][1] || k0 - 1 < p.ab.L[2][0] ||
                               k0 + TZ + 1 > p.g.n[2] - p.ab.L[2][1]);
   Q4 ep[3], hc[3], ec[3], ux[2], hpx[2], hcx[2];
+  AdjPsi ps;
   // stage 0 (plane x0 - 1): the stretched old Uy, Uz of the own nodes and of the halo nodes (x taps)
   if (tid == 0 && !mbar_wait(&bars[0], 0u, p.err, p.wait_limit)) gave_up = 1;
   __syncthreads();
@@ -465,6 +499,10 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
     }
     for (; t <= len; t++) {
       const int s = t + 1, pc = x0 + t, pe = pc - 1;
+      const int xs = cpml && pc < p.g.n[0] ? slab_cs(p, 0, pc) : -1;
+      const bool ab = ab_yz || xs >= 0;
+      if (ab && pc < p.g.n[0]) adj_psi_g(p, fa, f, an, pc, xs, ps);
+      if (ab_yz && t >= 1) adj_psi_u(p, fa, f, pe, ps);
       swait = s;
       if (tid == 0 && !mbar_wait(&bars[s % F_NST], (unsigned)((s / F_NST) & 1), p.err, p.wait_limit)) gave_up = 1;
       // every thread is past iteration t - 1: the slot of stage t and the new-G
@@ -475,11 +513,9 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
       const float* st = fsm + (s % F_NST) * L::STAGE;
       float* hn1 = hnb + (t & 1) * L::HN;                        // new G of plane pc
       const float* hn0 = hnb + ((t + 1) & 1) * L::HN;            // new G of plane pc - 1
-      const int xs = cpml && pc < p.g.n[0] ? slab_cs(p, 0, pc) : -1;
-      const bool ab = ab_yz || xs >= 0;
       if (pc < p.g.n[0]) {
-        if (ab) adj_g_own<TY, true>(p, fa, st, hn1, f, an, pc, t < len, ux, hc, hcx, ec, fco, t + 1, xs);
-        else adj_g_own<TY, false>(p, fa, st, hn1, f, an, pc, t < len, ux, hc, hcx, ec, fco, t + 1, xs);
+        if (ab) adj_g_own<TY, true>(p, fa, st, hn1, f, an, pc, t < len, ux, hc, hcx, ec, fco, t + 1, xs, ps);
+        else adj_g_own<TY, false>(p, fa, st, hn1, f, an, pc, t < len, ux, hc, hcx, ec, fco, t + 1, xs, ps);
 #pragma unroll
         for (int q = 0; q < L::TASKS; q++) {
           const int task = w + q * L::NW;
@@ -496,12 +532,12 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
         const int um = umc[pe - x0];
         const bool vac = um >= 0 && ies[um * 3] == 1.f && ies[um * 3 + 1] == 1.f && ies[um * 3 + 2] == 1.f;
         switch ((vac ? 4 : um >= 0 ? 2 : 0) + (ab_yz ? 1 : 0)) {
-          case 5: adj_u_own<TY, 2, true>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco); break;
-          case 4: adj_u_own<TY, 2, false>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco); break;
-          case 3: adj_u_own<TY, 1, true>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco); break;
-          case 2: adj_u_own<TY, 1, false>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco); break;
-          case 1: adj_u_own<TY, 0, true>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco); break;
-          default: adj_u_own<TY, 0, false>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco); break;
+          case 5: adj_u_own<TY, 2, true>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco, ps); break;
+          case 4: adj_u_own<TY, 2, false>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco, ps); break;
+          case 3: adj_u_own<TY, 1, true>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco, ps); break;
+          case 2: adj_u_own<TY, 1, false>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco, ps); break;
+          case 1: adj_u_own<TY, 0, true>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco, ps); break;
+          default: adj_u_own<TY, 0, false>(p, fa, st, hn0, ies, um, f, an, pe, ep, hpx, hcx, fco, ps); break;
         }
       }
 #pragma unroll
