@@ -17,7 +17,7 @@
 // and psi <- b (x + psi).  A tap may lie in a neighbouring tile, which needs
 // that node's old psi, so psi of both fields is kept twice as well.
 //
-// A dispersive node (table entry 1/eps = 0; none lies in a slab) holds in the
+// A dispersive node (none lies in a slab) holds in the
 // U array the value its taps read (kE2 mu, written before the sweep by
 // adj_ade_sweep_kernel) and gets curl G' alone from the sweep; its lam_E is kept
 // with its ADE state.
@@ -358,9 +358,9 @@ __device__ __forceinline__ void adj_u_own(const Params& p, const AdjSweepArgs& f
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         float ie = ies[((m[c] >> (8 * e)) & 255u) * 3 + c];
-        if (di >= 0 && ie != 0.f) ie = __ldg(p.des_ie[c] + di);
+        if (di >= 0 && !is_dispersive(ie)) ie = __ldg(p.des_ie[c] + di);
         // (a dispersive node: curl G' alone)
-        out[c].v[e] = ie != 0.f ? __fmaf_rn(ie, inc[c].v[e], ep[c].v[e]) : inc[c].v[e];
+        out[c].v[e] = is_dispersive(ie) ? inc[c].v[e] : __fmaf_rn(ie, inc[c].v[e], ep[c].v[e]);
       }
     }
   } else {
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
     pdl_wait();
     for (int s = 0; s < 2; s++) { issue(s, false); issued = s; }
   }
-  for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
+  for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = staged_ie(p.mt, q);
   for (int q = tid; q < len; q += L::NT)
     umc[q] = __ldg(p.umat + ((long long)(x0 + q) * p.nty + j0 / F_MROWS) * p.ntz + blockIdx.x);
   if (cpml) {
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(256) adj_pre_kernel(const __grid_constant__ Pa
     for (int c = 1; c < 3; c++) {
       const int mat = p.mat[c] ? (int)__ldg(p.mat[c] + id) : 0;
       ie[c] = __ldg(&p.mt->inv_eps[mat][c]);
-      if (ie[c] == 0.f) ie[c] = 1.f;                   // dispersive node: lam_E itself
+      if (__ldg(&p.mt->npoles[mat]) > 0) ie[c] = 1.f;  // dispersive node: lam_E itself
       else if (di >= 0) ie[c] = __ldg(p.des_ie[c] + di);
     }
     A.lam[1][id] += (float)((ph[0] * hz.x + ph[1] * hz.y) * (double)ie[1]);

@@ -205,6 +205,18 @@ static void read_slots_drop() {
   S.buf = nullptr;
 }
 
+// the calling thread's device while it uses another one
+struct DeviceGuard {
+  int was = -1;
+  explicit DeviceGuard(int dev) {
+    int cur = -1;
+    if (cudaGetDevice(&cur) == cudaSuccess && cur != dev && cudaSetDevice(dev) == cudaSuccess) was = cur;
+  }
+  ~DeviceGuard() {
+    if (was >= 0) cudaSetDevice(was);
+  }
+};
+
 // bytes of device memory to host memory, after the work queued on the stream; waits for it
 static cudaError_t copy_to_host(int dev, cudaStream_t st, void* host, const void* devp, size_t bytes) {
   ReadSlots& S = read_slots();
@@ -224,7 +236,7 @@ static cudaError_t copy_to_host(int dev, cudaStream_t st, void* host, const void
     std::atomic<size_t> next{0};
     std::atomic<int> bad{(int)cudaSuccess};
     auto work = [&](int w) {
-      cudaSetDevice(dev);
+      const DeviceGuard guard(dev);
       char* slot[2] = {S.buf + (size_t)w * 2 * kReadPiece, S.buf + (size_t)(w * 2 + 1) * kReadPiece};
       cudaEvent_t ev[2] = {};
       size_t at[2] = {pieces, pieces};
@@ -1656,6 +1668,17 @@ static void fused_release(dtmx_ctx* ctx) {
   cudaGetLastError();
 }
 
+// The automatic choice's second set given back for another use of the memory:
+// the context goes on with the per-step engine (the state is always in P.f).
+static bool fused_give_back(dtmx_ctx* ctx) {
+  if (ctx->engine != 0 || !ctx->fused_ready || ctx->cfg.parkable) return false;
+  drop_graphs(ctx);
+  ctx->fused_ready = false;
+  ctx->auto_per_step = true;
+  fused_release(ctx);
+  return true;
+}
+
 // The state now lives in the other buffer set: swap the pointers (fields, H
 // auxiliaries, the maps reading them) so that P and every pass see it.
 static void fused_swap(dtmx_ctx* ctx) {
@@ -1964,7 +1987,11 @@ struct FaRun {
     (void)pool_kept;
     st = ctx->stream;
     void* q = nullptr;
-    if (cudaMallocAsync(&q, bytes, ctx->stream) != cudaSuccess) return nullptr;
+    if (cudaMallocAsync(&q, bytes, ctx->stream) != cudaSuccess) {
+      // an automatic second set of fields makes room for the adjoint
+      cudaGetLastError();
+      if (!fused_give_back(ctx) || cudaMallocAsync(&q, bytes, ctx->stream) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    }
     bufs.push_back(q);
     return q;
   }
@@ -2114,11 +2141,10 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
     const size_t cnt = (size_t)(P.ab.L[a][0] + P.ab.L[a][1]) * (ctx->ncell / (size_t)P.g.n[a]);
     if (!P.ab.aux[a][0]) continue;
     for (int q = 0; q < 4; q++) ok = ok && talloc((void**)&A.lpsi[a][q], cnt * 4);
-    for (int q = 0; q < 4 && R.sweep; q++) ok = ok && talloc((void**)&R.lpsi_alt[a][q], cnt * 4);
   }
-  for (int comp = 0; comp < 6 && R.sweep; comp++) ok = ok && talloc((void**)&R.lam_alt[comp], (ctx->nstore + 64) * 4);
-  for (int c3 = 0; c3 < 3 && !R.sweep; c3++)
-    for (int t = 0; t < 2; t++) ok = ok && talloc((void**)&A.w[c3][t], (ctx->nstore + 64) * 4);
+  // six more field arrays: the sweep's second set, or the two-pass kernels' w
+  float* six[6] = {};
+  for (int comp = 0; comp < 6; comp++) ok = ok && talloc((void**)&six[comp], (ctx->nstore + 64) * 4);
   if (ctx->has_gyro) {
     const size_t na = (size_t)P.ade.n[0] * P.ade.n[1] * P.ade.n[2];
     for (int c3 = 0; c3 < 3; c3++) ok = ok && talloc((void**)&A.lJg[c3], na * 4) && talloc((void**)&A.lT[c3], na * 4);
@@ -2128,7 +2154,6 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
     const size_t na = (size_t)P.ade.n[0] * P.ade.n[1] * P.ade.n[2];
     for (int c3 = 0; c3 < 3; c3++) {
       ok = ok && talloc((void**)&A.lEm[c3], na * 4);
-      if (R.sweep) ok = ok && talloc((void**)&A.lE[c3], na * 4);
       for (int r = 0; r < MAXPOLE; r++)
         if (P.ade.Jp[c3][r]) ok = ok && talloc((void**)&A.lJp[c3][r], na * 4) && talloc((void**)&A.lJm[c3][r], na * 4);
     }
@@ -2136,6 +2161,13 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
   ok = ok && talloc((void**)&A.grad, (size_t)3 * R.nd * 8) && talloc((void**)&R.dF, F.size() * 8);
   if (!R.full) ok = ok && talloc((void**)&R.hist, (size_t)(R.K + 1) * 3 * R.nd * 4);
   if (!ok) { R.release(); return fail(ctx, DTMX_ERR_OOM, "adjoint allocation"); }
+  // what the sweep needs beyond the two-pass kernels' arrays comes last: without room for it they serve
+  for (int a = 0; a < 3 && R.sweep; a++)
+    for (int q = 0; q < 4 && R.sweep && P.ab.aux[a][0]; q++)
+      R.sweep = talloc((void**)&R.lpsi_alt[a][q], (size_t)(P.ab.L[a][0] + P.ab.L[a][1]) * (ctx->ncell / (size_t)P.g.n[a]) * 4);
+  for (int c3 = 0; c3 < 3 && R.sweep && P.ade.Em[0]; c3++)
+    R.sweep = talloc((void**)&A.lE[c3], (size_t)P.ade.n[0] * P.ade.n[1] * P.ade.n[2] * 4);
+  for (int comp = 0; comp < 6; comp++) (R.sweep ? R.lam_alt[comp] : A.w[comp / 2][comp % 2]) = six[comp];
   A.hist = R.hist;
   if (R.sweep) {
     int rc;
@@ -2568,6 +2600,7 @@ extern "C" int dtmx_get_field(dtmx_ctx* ctx, int comp, float* host_out) {
   if (!ctx || comp < 0 || comp > 5 || !host_out) return fail(ctx, DTMX_ERR_INVALID, "bad field request");
   const dtmx_config& c = ctx->cfg;
   const size_t rows = (size_t)c.nx * c.ny;
+  const DeviceGuard guard(ctx->dev);
   if (c.nz == ctx->nzp) return copy_out(ctx, host_out, ctx->P.f[comp], rows * c.nz * 4);
   float* dense = nullptr;
   const size_t per = dense_rows(c.nz, rows);

@@ -290,7 +290,7 @@ __device__ __forceinline__ void fused_h_halo(const Params& p, const float* st, f
 // plane i (shared), hc: new H of plane i + 1 (own nodes).
 //   MODE 2: vacuum; MODE 1: uniform non-dispersive material um;
 //   MODE 0: general (mixed materials, design region).  A dispersive node's table
-//           entry is 0, so it keeps its old E here and the ADE pass writes it
+//           entry is -0, so it keeps its old E here and the ADE pass writes it
 //           (its absorber auxiliaries, if it has any, stay 0).
 template <int TY, int MODE, bool ABS>
 __device__ __forceinline__ void fused_e_own(const Params& p, const FusedArgs& fa, const float* st, const float* hn, const float* ies, int um,
@@ -329,7 +329,7 @@ __device__ __forceinline__ void fused_e_own(const Params& p, const FusedArgs& fa
         if (di >= 0) {
 #pragma unroll
           for (int c = 0; c < 3; c++)
-            if (ie[c] != 0.f) ie[c] = p.des_ie[c][di];     // (a dispersive design node keeps its ADE update)
+            if (!is_dispersive(ie[c])) ie[c] = p.des_ie[c][di];     // (a dispersive design node keeps its ADE update)
         }
       }
       d01.v[e] = __fmul_rn(d01.v[e], ie[0]); d02.v[e] = __fmul_rn(d02.v[e], ie[0]);
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
     pdl_wait();
     for (int s = 0; s < 2; s++) { issue(s, false); issued = s; }
   }
-  for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
+  for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = staged_ie(p.mt, q);
   for (int q = tid; q < len; q += L::NT)
     umc[q] = __ldg(p.umat + ((long long)(x0 + q) * p.nty + j0 / F_MROWS) * p.ntz + blockIdx.x);
   if (cpml) {

@@ -246,7 +246,7 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
     gave_up = 0;
   }
   if (!ISH) {
-    for (int q = tid; q < MAXMAT * 3; q += STREAM_NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
+    for (int q = tid; q < MAXMAT * 3; q += STREAM_NT) ies[q] = staged_ie(p.mt, q);
     for (int sq = tid; sq <= slast && sq < UMC; sq += STREAM_NT) {
       const int ip = i0 + DIR * sq;
       umc[sq] = (ip >= 0 && ip < p.g.n[0]) ? __ldg(p.umat + ((long long)ip * p.nty + blockIdx.y) * p.ntz + blockIdx.x)
@@ -408,7 +408,7 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
           d20 = scale4(e2, d20); d21 = scale4(e2, d21);
         }
       } else {
-        // mixed materials or the design region; a dispersive node's table entry is 0, so it
+        // mixed materials or the design region; a dispersive node's table entry is -0, so it
         // keeps its old E here and the ADE pass writes it
         const unsigned* mt = reinterpret_cast<const unsigned*>(cur + P::OFF_MAT);
         unsigned mm[3];
@@ -424,7 +424,7 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
             if (di >= 0) {
 #pragma unroll
               for (int c = 0; c < 3; c++)
-                if (ie[c] != 0.f) ie[c] = p.des_ie[c][di];
+                if (!is_dispersive(ie[c])) ie[c] = p.des_ie[c][di];
             }
           }
           d01.v[e] = __fmul_rn(d01.v[e], ie[0]); d02.v[e] = __fmul_rn(d02.v[e], ie[0]);

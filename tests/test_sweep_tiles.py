@@ -48,3 +48,60 @@ def test_tile_edges_equal_the_per_step_engine(n, pml, rows):
     got = _run(n, pml, 3, rows)
     for c in range(6):
         assert np.array_equal(got[c], want[c]), (c, np.abs(got[c] - want[c]).max())
+
+
+@pytest.mark.parametrize("n,pml", [
+    ((70, 40, 40), ((6, 6), (6, 6), (6, 6))),        # one wave, pieces of equal cost
+    ((44, 300, 290), ((6, 5), (0, 7), (8, 8))),      # several waves
+    ((150, 17, 20), None),                           # pieces as long as a CTA's tables allow (64 planes)
+])
+def test_pieces_of_equal_cost(n, pml):
+    """The tile columns cut into pieces of equal cost (automatic) against equal
+    pieces of 7 planes, on both streaming engines."""
+    from dtmaxwell4_b200 import Simulation, abi
+    cfg = abi.make_config(*n, courant=0.5, absorber=abi.ABS_CPML if pml else abi.ABS_NONE, pml=pml or 0)
+    rng = np.random.default_rng(3)
+    fields = [rng.standard_normal(n).astype(np.float32) for _ in range(6)]
+    got = []
+    for engine, planes in ((1, 7), (1, 0), (3, 7), (3, 0)):
+        s = Simulation(cfg)
+        for c in range(6):
+            s.set_field(c, fields[c])
+        s.set_engine(engine)
+        s.set_xchunk(planes)
+        s.step(5)
+        got.append([s.get_field(c) for c in range(6)])
+        s.close()
+    for out in got[1:]:
+        for c in range(6):
+            assert np.array_equal(out[c], got[0][c]), c
+
+
+def test_design_nodes_in_a_material_of_huge_permittivity():
+    """1/eps of the material rounds to 0 in FP32; the design permittivity replaces
+    it all the same (a dispersive material's nodes keep theirs)."""
+    from dtmaxwell4_b200 import Simulation, abi
+    n = (20, 18, 36)
+    cfg = abi.make_config(*n, courant=0.5, pml=4)
+    rng = np.random.default_rng(7)
+    fields = [rng.standard_normal(n).astype(np.float32) for _ in range(6)]
+    idx = np.zeros(n, np.uint8)
+    idx[6:14, 5:13, 8:30] = 1
+    mats = [abi.make_material(1.0), abi.make_material(1e60)]
+    eps = rng.uniform(1.0, 4.0, size=(3, 4, 4, 9)).astype(np.float32)
+    got = []
+    for engine in (1, 3):
+        s = Simulation(cfg)
+        s.set_materials(mats, idx)
+        s.set_design((8, 7, 12), eps)
+        for c in range(6):
+            s.set_field(c, fields[c])
+        s.set_engine(engine)
+        s.step(6)
+        got.append([s.get_field(c) for c in range(6)])
+        s.close()
+    for c in range(6):
+        assert np.array_equal(got[0][c], got[1][c]), c
+    e = got[0][2]
+    assert (e[8:12, 7:11, 12:21] != fields[2][8:12, 7:11, 12:21]).all()
+    assert np.array_equal(e[6:8, 5:13, 8:30], fields[2][6:8, 5:13, 8:30])
