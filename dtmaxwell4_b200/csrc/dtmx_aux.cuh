@@ -630,11 +630,6 @@ __global__ void __launch_bounds__(FLUX_THREADS) ntff_kernel(NtffFaces F, const d
 
 // Magnetised-Drude current over the ADE box (dtmx.h, dtmx_material):
 // J^{n+1/2} into buffer 1-cur from J^{n-1/2} (buffer cur) and E^n.
-__device__ __forceinline__ float gyro_old(const Params& p, int cur, int c, int i, int j, int k) {
-  const int bi = i - p.ade.lo[0], bj = j - p.ade.lo[1], bk = k - p.ade.lo[2];
-  if (bi < 0 || bi >= p.ade.n[0] || bj < 0 || bj >= p.ade.n[1] || bk < 0 || bk >= p.ade.n[2]) return 0.f;
-  return __ldg(p.ade.Jg[cur][c] + ((long long)bi * p.ade.n[1] + bj) * p.ade.n[2] + bk);
-}
 
 // Thread layout of the passes over the ADE box: 256 threads along the box'
 // (y, z) plane, blockIdx.y = x.
@@ -648,22 +643,27 @@ __device__ __forceinline__ bool ade_cell(const Params& p, int& bi, int& bj, int&
   return true;
 }
 
-// The three new current components of node (i, j, k), box index q, from the
-// old ones (buffer cur) and E^n; m: material indices, E: E^n, on: gyrotropic
-__device__ __forceinline__ void gyro_new(const Params& p, int cur, int i, int j, int k, long long q, const int (&m)[3], const float (&E)[3],
+// The three new current components of the node at box position (bi, bj), box
+// index q, from the old ones (buffer cur; 0 outside the box and off the
+// gyrotropic nodes) and E^n; m: material indices, E: E^n, on: gyrotropic
+__device__ __forceinline__ void gyro_new(const Params& p, int cur, int bi, int bj, long long q, const int (&m)[3], const float (&E)[3],
                                          const bool (&on)[3], float (&J)[3]) {
   const MatTable& mt = *p.mt;
+  const int dj = p.ade.n[2];
+  const long long di = (long long)p.ade.n[1] * dj;
+  const float *Jx = p.ade.Jg[cur][0] + q, *Jy = p.ade.Jg[cur][1] + q;
+  const bool im = bi > 0, ip = bi + 1 < p.ade.n[0], jm = bj > 0, jp = bj + 1 < p.ade.n[1];
   // every load before its use
   float own[3], near[2][4];
 #pragma unroll
   for (int c = 0; c < 3; c++) own[c] = on[c] ? __ldg(p.ade.Jg[cur][c] + q) : 0.f;
   if (on[0]) {
-    near[0][0] = gyro_old(p, cur, 1, i - 1, j, k); near[0][1] = gyro_old(p, cur, 1, i, j, k);
-    near[0][2] = gyro_old(p, cur, 1, i - 1, j + 1, k); near[0][3] = gyro_old(p, cur, 1, i, j + 1, k);
+    near[0][0] = im ? __ldg(Jy - di) : 0.f; near[0][1] = on[1] ? own[1] : __ldg(Jy);
+    near[0][2] = im && jp ? __ldg(Jy - di + dj) : 0.f; near[0][3] = jp ? __ldg(Jy + dj) : 0.f;
   }
   if (on[1]) {
-    near[1][0] = gyro_old(p, cur, 0, i, j - 1, k); near[1][1] = gyro_old(p, cur, 0, i + 1, j - 1, k);
-    near[1][2] = gyro_old(p, cur, 0, i, j, k); near[1][3] = gyro_old(p, cur, 0, i + 1, j, k);
+    near[1][0] = jm ? __ldg(Jx - dj) : 0.f; near[1][1] = ip && jm ? __ldg(Jx + di - dj) : 0.f;
+    near[1][2] = on[0] ? own[0] : __ldg(Jx); near[1][3] = ip ? __ldg(Jx + di) : 0.f;
   }
 #pragma unroll
   for (int c = 0; c < 3; c++) {
@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(256) gyro_current_kernel(const __grid_constant
   for (int c = 0; c < 3; c++) { m[c] = p.mat[c] ? (int)__ldg(p.mat[c] + id) : 0; E[c] = __ldg(p.f[c] + id); }
 #pragma unroll
   for (int c = 0; c < 3; c++) on[c] = __ldg(&p.mt->gjc[m[c]]) != 0.f;
-  gyro_new(p, cur, i, j, k, q, m, E, on, J);
+  gyro_new(p, cur, bi, bj, q, m, E, on, J);
 #pragma unroll
   for (int c = 0; c < 3; c++)
     if (on[c]) p.ade.Jg[1 - cur][c][q] = J[c];
@@ -712,10 +712,10 @@ __global__ void __launch_bounds__(256) gyro_current_kernel(const __grid_constant
 // The three components' loads are issued together (materials, then flags, then
 // state and taps: three round trips a cell, where a component at a time made
 // nine).  A 236x236x76 gyrotropic layer took 84 + 102 us in two passes and takes
-// 83; the Drude film of the reference geometry (8 cells along z, so lanes run along
+// 78 (98 with 68 registers a thread: five blocks per SM hide its loads better than three); the Drude film of the reference geometry (8 cells along z, so lanes run along
 // y and z together) 76 -> 32 us.
 template <int ORDER, bool BOX, bool CUR>
-__global__ void __launch_bounds__(256) ade_node_kernel(const __grid_constant__ Params p, int cur) {
+__global__ void __launch_bounds__(256, CUR ? 5 : 4) ade_node_kernel(const __grid_constant__ Params p, int cur) {
   pdl_wait();
   pdl_trigger();
   const MatTable& mt = *p.mt;
@@ -787,7 +787,7 @@ __global__ void __launch_bounds__(256) ade_node_kernel(const __grid_constant__ P
     float E[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) { F[c] = on[c] ? p.f[c][id] : 0.f; E[c] = on[c] ? __ldg(p.fe_old[c] + id) : 0.f; }
-    gyro_new(p, cur, i, j, k, q, m, E, on, J);
+    gyro_new(p, cur, bi, bj, q, m, E, on, J);
 #pragma unroll
     for (int c = 0; c < 3; c++)
       if (on[c]) p.ade.Jg[1 - cur][c][q] = J[c];
