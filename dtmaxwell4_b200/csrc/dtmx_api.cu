@@ -851,7 +851,7 @@ extern "C" int dtmx_set_materials(dtmx_ctx* ctx, const dtmx_material* table, int
   for (int m = 0; m < nmat; m++) {
     ctx->mats[m] = table[m];
     t.npoles[m] = table[m].npoles;
-    for (int c = 0; c < 3; c++) t.inv_eps[m][c] = table[m].npoles > 0 ? 0.f : (float)(1.0 / table[m].eps[c]);
+    for (int c = 0; c < 3; c++) t.inv_eps[m][c] = table[m].npoles > 0 ? -0.f : (float)(1.0 / table[m].eps[c]);
     if (table[m].npoles > 0) disp_coeffs(table[m], ctx->cfg.dt, t, m);
     if (table[m].gyro_wp > 0) {
       const double dt = ctx->cfg.dt;

@@ -294,13 +294,8 @@ struct MatShared {
   float gjc[MAXMAT];
 };
 
-// 1/eps entries of the material table in shared memory; a dispersive material's
-// is -0: it adds nothing to E, and is told from a permittivity too large for
-// 1/eps by its sign.
-__device__ __forceinline__ float staged_ie(const MatTable* mt, int q) {
-  const float v = __ldg(&mt->inv_eps[0][0] + q);
-  return __ldg(&mt->npoles[q / 3]) > 0 ? -0.f : v;
-}
+// The 1/eps entry of a dispersive material is -0 (dtmx_set_materials): it adds
+// nothing to E, and is told from a permittivity too large for 1/eps by its sign.
 __device__ __forceinline__ bool is_dispersive(float ie) { return __float_as_uint(ie) == 0x80000000u; }
 
 // ---- four consecutive z nodes a thread (the single sweep, its adjoint and the

@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
     pdl_wait();
     for (int s = 0; s < 2; s++) { issue(s, false); issued = s; }
   }
-  for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = staged_ie(p.mt, q);
+  for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
   for (int q = tid; q < len; q += L::NT)
     umc[q] = __ldg(p.umat + ((long long)(x0 + q) * p.nty + j0 / F_MROWS) * p.ntz + blockIdx.x);
   if (cpml) {

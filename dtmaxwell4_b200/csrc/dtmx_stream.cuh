@@ -246,7 +246,7 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
     gave_up = 0;
   }
   if (!ISH) {
-    for (int q = tid; q < MAXMAT * 3; q += STREAM_NT) ies[q] = staged_ie(p.mt, q);
+    for (int q = tid; q < MAXMAT * 3; q += STREAM_NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
     for (int sq = tid; sq <= slast && sq < UMC; sq += STREAM_NT) {
       const int ip = i0 + DIR * sq;
       umc[sq] = (ip >= 0 && ip < p.g.n[0]) ? __ldg(p.umat + ((long long)ip * p.nty + blockIdx.y) * p.ntz + blockIdx.x)
