@@ -9,7 +9,8 @@
 // new G of the tile's halo recomputed, one CTA barrier a plane.  The kernels
 // it replaces (adj_w_kernel, adj_curl_kernel: w of both curl terms to memory
 // and back, twice a step) move 168 bytes a cell, this one 48 and the absorber's
-// auxiliaries; on a 192x160x128 grid they took 187 us a step, this one 112.
+// auxiliaries; on a 192x160x128 grid they took 187 us a step, this one takes 86
+// (94 in pieces of equal length, plan_work).
 //
 // The absorber does differ: the transposed CPML stretches a value before the
 // difference is taken.  For a derivative along axis a a tap reads
@@ -376,9 +377,10 @@ __device__ __forceinline__ void adj_u_own(const Params& p, const AdjSweepArgs& f
   for (int c = 0; c < 3; c++) st4(fa.dst[c] + off, out[c]);
 }
 
-template <int TY>
+template <int TY, bool TAB>
 __global__ void __launch_bounds__(FL<TY>::NT, 3)
-    adj_sweep_kernel(const __grid_constant__ Params p, const __grid_constant__ AdjSweepArgs fa, const __grid_constant__ FusedMaps m) {
+    adj_sweep_kernel(const __grid_constant__ Params p, const __grid_constant__ AdjSweepArgs fa, const __grid_constant__ FusedMaps m,
+                     const __grid_constant__ Work<TAB> work) {
   using L = FL<TY>;
   extern __shared__ __align__(128) float fsm[];
   float* hnb = fsm + F_NST * L::STAGE;                           // two new-G planes
@@ -388,10 +390,9 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
   __shared__ signed char umc[FX_MAX];
   __shared__ int gave_up;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int k0 = blockIdx.x * TZ, j0 = blockIdx.y * TY;
-  const int x0 = p.x0 + blockIdx.z * p.xchunk;
-  const int x1 = min(x0 + p.xchunk, p.x1);
-  const int len = x1 - x0;
+  const int4 job = cta_job<TAB>(p, work);
+  const int k0 = job.x * TZ, j0 = job.y * TY;
+  const int x0 = job.z, len = job.w - job.z;
   const int slast = len + 1;                               // stages 0 .. len + 1: planes x0 - 1 .. x1
   const bool cpml = p.ab.kind == 1;
   auto issue = [&](int s, bool want_mat) {
@@ -408,7 +409,7 @@ __global__ void __launch_bounds__(FL<TY>::NT, 3)
   }
   for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
   for (int q = tid; q < len; q += L::NT)
-    umc[q] = __ldg(p.umat + ((long long)(x0 + q) * p.nty + j0 / F_MROWS) * p.ntz + blockIdx.x);
+    umc[q] = __ldg(p.umat + ((long long)(x0 + q) * p.nty + j0 / F_MROWS) * p.ntz + job.x);
   if (cpml) {
     // coefficient row q: x plane x0 - 1 + q, then y row j0 - 1 + ..., then z column k0 - 1 + ...
     constexpr int RX = FX_MAX + 2, RY_ = TY + 2, RZ = TZ + 2;

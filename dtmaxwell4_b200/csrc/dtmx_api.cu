@@ -13,6 +13,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <array>
 #include <atomic>
 #include <thread>
 
@@ -74,6 +75,14 @@ struct VmmBlock {
   bool saved_prepared = false;  // the host copy was taken after the context first stepped
 };
 
+// the pieces of a streaming launch (plan_work)
+struct WorkPlan {
+  bool table = false, alone = false;   // alone: to be launched when the kernel ahead has finished
+  int xchunk = 0;
+  dim3 grid;
+  Work<true> work{};
+};
+
 struct dtmx_ctx {
   dtmx_config cfg{};
   int dev = 0;
@@ -85,6 +94,7 @@ struct dtmx_ctx {
   std::vector<void*> allocs;
   std::vector<VmmBlock> vmm;    // the arrays of a parkable context (instead of allocs)
   bool parked = false;
+  std::map<std::array<int, 4>, WorkPlan> work;   // by (kind, tile rows, planes per CTA asked for, early launches)
   bool early = false;           // launches may overlap their set-up with the kernel ahead (launch_after)
   // coefficient tables
   float* ctab[3][3] = {};
@@ -1284,25 +1294,132 @@ extern "C" int dtmx_ntff(dtmx_ctx* ctx, int id, int ndir, const double* theta, c
 }
 
 // ---------------------------------------------------------------- stepping
-static int xchunk_for(const dtmx_ctx* ctx) {
-  if (ctx->xchunk > 0) return ctx->xchunk;
+// How a streaming launch cuts the tile columns along x, one CTA a piece.
+//   * One wave of the CTAs that fit, where that takes about a dozen planes a CTA:
+//     small grids are bound by the latency of a CTA's walk, and a nearly empty last
+//     wave costs as much as a full one (single sweep, 48^3: 9.4 us with pieces of one
+//     plane, 26 with eight; per-step kernels, 64^3: 17.8 with four, 10.6 with one).
+//   * With an absorber, in pieces of equal cost, not equal length: a plane next to a
+//     slab costs about one interior plane more per slab axis, and on 128^3 in equal
+//     pieces the busiest SM issued 1.43 times the average (single sweep 41.1 -> 36.3
+//     us; per-step kernels 42.2 -> 37.4, 149x93x211 59.8 -> 50.0; adjoint sweep on
+//     192x160x128 94 -> 86).  Such pieces serve one wave up to about 40 units (single
+//     sweep, 192x160x128: 68.1 us in eight waves of equal pieces, 60.2 in one wave;
+//     149x93x211 59.3 -> 52.5); above that several waves even out as well (384^3).
+//     One wave has no slack for what the cost leaves out, nor for slots that other
+//     kernels hold: the long pieces are not for the single sweep with a design region
+//     (its tile-planes cost several others: the forward runs of a gradient on
+//     192x160x128 18.8 -> 20.8 ms) or in a batch, and their launch waits for the
+//     kernel ahead.  The single sweep's pieces below six planes stay equal: the lookup
+//     ahead of the first copy costs them more than it evens out (96^3: 18.7 -> 20.7 us).
+//     The order-4 per-step kernels stay at equal pieces (64.5 + 54.0 -> 75.1 + 55.3 us in
+//     the reference geometry).
+//   * Otherwise several waves of equal pieces: of 6 to 32 planes for the single sweep
+//     (192x160x128: 68 us with 6, 77 with 12; 384^3: 634 us with 32, 641 with 10, 669
+//     with 64), 4 to 10 for the per-step kernels (384^3 712 us with 10, 830 with about 40).
+// planes > 0: equal pieces of that many planes (dtmx_set_xchunk, dtmx_autotune).
+static int tile_axes(const dtmx_ctx* ctx, int j0, int rows, int k0) {
+  const Absorb& ab = ctx->P.ab;
+  if (ab.kind == 0) return 0;
   const dtmx_config& c = ctx->cfg;
-  const long long tiles = (long long)((c.nz + TZ - 1) / TZ) * ((c.ny + TYT - 1) / TYT);
-  const long long target = 148LL * 8 * 3;   // about three waves of 8 CTAs per SM
-  long long chunks = std::max<long long>(1, (target + tiles - 1) / tiles);
-  long long xc = (c.nx + chunks - 1) / chunks;
-  // at most 10 planes per CTA: the autotuner picks 8-10 on 384^3 and
-  // 1024x1024x1536 grids (longer chunks leave the tail of each CTA alone on its SM)
-  return (int)std::min<long long>(10, std::max<long long>(4, xc));
+  return (j0 < ab.L[1][0] || j0 + rows > c.ny - ab.L[1][1] ? 1 : 0) + (k0 < ab.L[2][0] || k0 + TZ > c.nz - ab.L[2][1] ? 1 : 0);
+}
+// pieces of at most `budget` units: an interior plane is one, a piece's start two
+static void work_cut(const dtmx_ctx* ctx, int rows, int budget, std::vector<int4>* out, long long* count) {
+  const dtmx_config& c = ctx->cfg;
+  const Absorb& ab = ctx->P.ab;
+  constexpr int kStart = 2;
+  std::vector<int> cuts[3];            // the cuts depend on the number of the column's slab axes alone
+  for (int a = 0; a < 3; a++) {
+    int cost = kStart, first = 0;
+    cuts[a].push_back(0);
+    for (int i = 0; i < c.nx; i++) {
+      const int w = 1 + a + (ab.kind != 0 && (i < ab.L[0][0] || i >= c.nx - ab.L[0][1]) ? 1 : 0);
+      if (i > first && (cost + w > budget || i - first >= FX_MAX)) { cuts[a].push_back(i); cost = kStart; first = i; }
+      cost += w;
+    }
+    cuts[a].push_back(c.nx);
+  }
+  const int ntz = (c.nz + TZ - 1) / TZ, nty = (c.ny + rows - 1) / rows;
+  size_t longest = 0;
+  for (int a = 0; a < 3; a++) longest = std::max(longest, cuts[a].size() - 1);
+  long long n = 0;
+  // in order of their place along x, so that CTAs that start together share halos
+  for (size_t q = 0; q < longest; q++)
+    for (int ty = 0; ty < nty; ty++)
+      for (int tz = 0; tz < ntz; tz++) {
+        const std::vector<int>& cut = cuts[tile_axes(ctx, ty * rows, rows, tz * TZ)];
+        if (q + 1 >= cut.size()) continue;
+        n++;
+        if (out) out->push_back(make_int4(tz, ty, cut[q], cut[q + 1]));
+      }
+  if (count) *count = n;
+}
+enum { WK_STREAM, WK_SWEEP, WK_ADJ };
+constexpr int kOneWave = 40;            // most units of a piece in a single wave
+// The plan of a launch; its table is made on first use, never while a stream is captured.
+static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, const WorkPlan** plan) {
+  const dtmx_config& c = ctx->cfg;
+  const int ntz = (c.nz + TZ - 1) / TZ, nty = (c.ny + rows - 1) / rows;
+  const long long tiles = (long long)ntz * nty, fit = 148LL * per_sm;
+  const bool many = ctx->early && !ctx->P.des_on;     // may take long pieces in one wave
+  const std::array<int, 4> key{kind, rows, planes, many ? 1 : 0};
+  auto it = ctx->work.find(key);
+  if (it == ctx->work.end()) {
+    WorkPlan w;
+    w.xchunk = planes;
+    if (planes == 0) {
+      const long long one = tiles <= fit ? (c.nx + fit / tiles - 1) / (fit / tiles) : c.nx;      // one wave of equal pieces
+      int budget = kOneWave + 1;
+      if (c.absorber != DTMX_ABS_NONE && rows == 16 && tiles <= fit && one >= (kind == WK_STREAM ? 5 : 6) && !(kind == WK_STREAM && c.order == 4) &&
+          (kind != WK_SWEEP || one <= 12 || many)) {
+        for (budget = 3; budget <= kOneWave; budget++) {
+          long long n = 0;
+          work_cut(ctx, rows, budget, nullptr, &n);
+          if (n <= fit) break;
+        }
+      }
+      if (budget <= kOneWave) {
+        std::vector<int4> v;
+        work_cut(ctx, rows, budget, &v, nullptr);
+        int4* d = nullptr;
+        int rc = dalloc(ctx, &d, v.size(), true);
+        if (rc) return rc;
+        CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        w.table = true;
+        w.alone = kind == WK_SWEEP && one > 12;
+        w.work.e = d;
+        w.grid = dim3((unsigned)v.size());
+      } else if (kind == WK_STREAM) {
+        const long long chunks = std::max<long long>(1, (148LL * 8 * 3 + tiles - 1) / tiles), xc = (c.nx + chunks - 1) / chunks;
+        w.xchunk = (int)(one <= 2 && c.order == 2 ? one : std::min<long long>(10, std::max<long long>(4, xc)));
+      } else {
+        const long long chunks = std::max<long long>(1, (8 * fit + tiles - 1) / tiles), xc = (c.nx + chunks - 1) / chunks;
+        w.xchunk = (int)(one <= 12 ? one : std::min<long long>(32, std::max<long long>(6, xc)));
+      }
+    }
+    if (!w.table) w.grid = dim3(ntz, nty, (c.nx + w.xchunk - 1) / w.xchunk);
+    it = ctx->work.emplace(key, w).first;
+  }
+  if (plan) *plan = &it->second;
+  return DTMX_OK;
+}
+static int plan_stream(dtmx_ctx* ctx, const WorkPlan** w) { return plan_work(ctx, WK_STREAM, TYT, ctx->cfg.order == 4 ? 3 : 4, ctx->xchunk, w); }
+static int plan_sweep(dtmx_ctx* ctx, const WorkPlan** w) {
+  return plan_work(ctx, WK_SWEEP, ctx->frows, ctx->frows == 16 ? 3 : 5, std::min(ctx->xchunk, FX_MAX), w);
 }
 
 static int set_kernel_attributes() {
   static bool done = false;
   if (done) return 0;
-  cudaFuncSetAttribute(h_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Pipe<2, true>::SMEM_BYTES);
-  cudaFuncSetAttribute(h_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Pipe<4, true>::SMEM_BYTES);
-  cudaFuncSetAttribute(e_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Pipe<2, false>::SMEM_BYTES);
-  cudaFuncSetAttribute(e_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Pipe<4, false>::SMEM_BYTES);
+  auto allow = [](const void* k, size_t smem) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); };
+  allow((const void*)h_kernel<2, false>, Pipe<2, true>::SMEM_BYTES);
+  allow((const void*)h_kernel<2, true>, Pipe<2, true>::SMEM_BYTES);
+  allow((const void*)h_kernel<4, false>, Pipe<4, true>::SMEM_BYTES);
+  allow((const void*)e_kernel<2, false>, Pipe<2, false>::SMEM_BYTES);
+  allow((const void*)e_kernel<2, true>, Pipe<2, false>::SMEM_BYTES);
+  allow((const void*)e_kernel<4, false>, Pipe<4, false>::SMEM_BYTES);
   done = true;
   return 0;
 }
@@ -1387,16 +1504,19 @@ static int launch_step(dtmx_ctx* ctx) {
   set_kernel_attributes();
   const dtmx_config& c = ctx->cfg;
   Params P = ctx->P;
-  P.x0 = 0; P.x1 = c.nx;
-  P.xchunk = xchunk_for(ctx);
+  const WorkPlan* wp;
+  if (int rc = plan_stream(ctx, &wp)) return rc;
+  const WorkPlan& plan = *wp;
+  P.xchunk = plan.xchunk;
   const int blk = STREAM_NT;
-  const dim3 grd((c.nz + TZ - 1) / TZ, (c.ny + TYT - 1) / TYT, (c.nx + P.xchunk - 1) / P.xchunk);
+  const dim3 grd = plan.grid;
   const bool o4 = c.order == 4;
   cudaStream_t st = ctx->stream;
   long long nl = 0;
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], st);
-  if (o4) launch_after(ctx->early, h_kernel<4>, grd, blk, Pipe<4, true>::SMEM_BYTES, st, P, ctx->maps);
-  else launch_after(ctx->early, h_kernel<2>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps);
+  if (o4) launch_after(ctx->early, h_kernel<4, false>, grd, blk, Pipe<4, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  else if (plan.table) launch_after(ctx->early, h_kernel<2, true>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, plan.work);
+  else launch_after(ctx->early, h_kernel<2, false>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], st);
   nl++;
   nl += launch_tfsf(ctx, P, st, true);
@@ -1407,8 +1527,9 @@ static int launch_step(dtmx_ctx* ctx) {
     nl++;
   }
   if (ctx->profiling) cudaEventRecord(ctx->ev[2], st);
-  if (o4) launch_after(ctx->early, e_kernel<4>, grd, blk, Pipe<4, false>::SMEM_BYTES, st, P, ctx->maps);
-  else launch_after(ctx->early, e_kernel<2>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps);
+  if (o4) launch_after(ctx->early, e_kernel<4, false>, grd, blk, Pipe<4, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  else if (plan.table) launch_after(ctx->early, e_kernel<2, true>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, plan.work);
+  else launch_after(ctx->early, e_kernel<2, false>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
   if (P.ade.Em[0] || ctx->has_gyro) {
     // dispersive and gyrotropic nodes of the E half step (e_kernel skipped them)
     const bool box = c.geometry == DTMX_GEOM_BOX;
@@ -1606,8 +1727,9 @@ static int fused_prepare(dtmx_ctx* ctx) {
   if (ctx->fused_ready) return DTMX_OK;
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(fused_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<16>::SMEM);
-    cudaFuncSetAttribute(fused_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<8>::SMEM);
+    cudaFuncSetAttribute(fused_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<16>::SMEM);
+    cudaFuncSetAttribute(fused_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<16>::SMEM);
+    cudaFuncSetAttribute(fused_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<8>::SMEM);
     attr = true;
   }
   const dtmx_config& c = ctx->cfg;
@@ -1692,30 +1814,6 @@ static void fused_swap(dtmx_ctx* ctx) {
   ctx->tmaps_ok = false;          // the wavefront engine's maps are rebuilt for the current buffer
 }
 
-// Planes per CTA (at most FX_MAX).  One wave of the 3 CTAs per SM that fit,
-// where that takes chunks of at most 12 planes: small grids are bound by the
-// latency of a CTA's walk, and a nearly empty last wave costs as much as a full
-// one (128^3 with a 10-cell CPML, 32 tile columns: 39.9 us with chunks of 10
-// = 416 CTAs, 45.8 with 8 = 512 CTAs; 48^3: 9.4 us with chunks of 1, 26.0 with
-// 8).  Larger grids: about eight waves, chunks of 6 to 32 planes (each chunk
-// stages one plane and updates one H plane more; 192x160x128: 68.0 us with 6,
-// 77.3 with 12; 384^3: 634 us with 32, 641 with 10, 669 with 64).
-static int sweep_xchunk(const dtmx_config& c, int rows, int per_sm) {
-  const long long tiles = (long long)((c.nz + TZ - 1) / TZ) * ((c.ny + rows - 1) / rows);
-  const long long fit = 148LL * per_sm;
-  if (tiles <= fit) {
-    const long long xc = (c.nx + fit / tiles - 1) / (fit / tiles);
-    if (xc <= 12) return (int)xc;
-  }
-  const long long chunks = std::max<long long>(1, (fit * 8 + tiles - 1) / tiles);
-  const long long xc = (c.nx + chunks - 1) / chunks;
-  return (int)std::min<long long>(32, std::max<long long>(6, xc));
-}
-static int fused_xchunk_for(const dtmx_ctx* ctx) {
-  if (ctx->xchunk > 0) return std::min(ctx->xchunk, FX_MAX);
-  return sweep_xchunk(ctx->cfg, ctx->frows, ctx->frows == 16 ? 3 : 5);
-}
-
 // One time step of the single-sweep engine: the side passes that act on the
 // old state (TF/SF H correction, gyrotropic current), the sweep A -> B, the
 // passes on the new state (dispersive nodes, sources, TF/SF E correction,
@@ -1723,10 +1821,11 @@ static int fused_xchunk_for(const dtmx_ctx* ctx) {
 static int launch_fused_step(dtmx_ctx* ctx) {
   int rc = fused_prepare(ctx);
   if (rc) return rc;
-  const dtmx_config& c = ctx->cfg;
   Params PA = ctx->P;
-  PA.x0 = 0; PA.x1 = c.nx;
-  PA.xchunk = fused_xchunk_for(ctx);
+  const WorkPlan* wp;
+  if ((rc = plan_sweep(ctx, &wp))) return rc;
+  const WorkPlan& plan = *wp;
+  PA.xchunk = plan.xchunk;
   Params PB = PA;
   FusedArgs fa{};
   for (int comp = 0; comp < 6; comp++) { PB.f[comp] = ctx->f_alt[comp]; fa.dst[comp] = ctx->f_alt[comp]; }
@@ -1739,10 +1838,11 @@ static int launch_fused_step(dtmx_ctx* ctx) {
   cudaStream_t st = ctx->stream;
   // TF/SF correction of H, added to the old H (the H update is linear in it)
   long long nl = launch_tfsf(ctx, PA, st, true);
-  const dim3 grd((c.nz + TZ - 1) / TZ, (c.ny + ctx->frows - 1) / ctx->frows, (c.nx + PA.xchunk - 1) / PA.xchunk);
+  const dim3 grd = plan.grid;
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], st);
-  if (ctx->frows == 8) launch_after(ctx->early, fused_kernel<8>, grd, FL<8>::NT, FL<8>::SMEM, st, PA, fa, ctx->fmaps8[0]);
-  else launch_after(ctx->early, fused_kernel<16>, grd, FL<16>::NT, FL<16>::SMEM, st, PA, fa, ctx->fmaps[0]);
+  if (ctx->frows == 8) launch_after(ctx->early, fused_kernel<8, false>, grd, FL<8>::NT, FL<8>::SMEM, st, PA, fa, ctx->fmaps8[0], Work<false>{});
+  else if (plan.table) launch_after(ctx->early && !plan.alone, fused_kernel<16, true>, grd, FL<16>::NT, FL<16>::SMEM, st, PA, fa, ctx->fmaps[0], plan.work);
+  else launch_after(ctx->early, fused_kernel<16, false>, grd, FL<16>::NT, FL<16>::SMEM, st, PA, fa, ctx->fmaps[0], Work<false>{});
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], st);
   nl++;
   if (PA.ade.Em[0] || ctx->has_gyro) {
@@ -1807,7 +1907,13 @@ static int graph_steps16(dtmx_ctx* ctx) {
   const int par = ctx->parity;
   if (!ctx->graph16[par]) {
     set_kernel_attributes();
-    if (step_engine(ctx) == 3) { int rc = fused_prepare(ctx); if (rc) return rc; }
+    if (step_engine(ctx) == 3) {
+      int rc = fused_prepare(ctx);
+      if (!rc) rc = plan_sweep(ctx, nullptr);
+      if (rc) return rc;
+    } else if (int rc = plan_stream(ctx, nullptr)) {
+      return rc;
+    }
     const long long launches0 = ctx->launches;
     const int gcur0 = ctx->gcur;
     const int staged0 = ctx->mon.nstaged;
@@ -2172,7 +2278,8 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
   if (R.sweep) {
     int rc;
     if ((rc = build_fused_maps<16>(ctx, R.fm[0], A.lam)) || (rc = build_fused_maps<16>(ctx, R.fm[1], R.lam_alt))) return rc;
-    if (cudaFuncSetAttribute(adj_sweep_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AL<16>::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(adj_sweep_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AL<16>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(adj_sweep_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AL<16>::SMEM) != cudaSuccess)
       return fail(ctx, DTMX_ERR_CUDA, "adjoint sweep: shared memory attribute");
   }
   CK(cudaMemcpyAsync(R.dF, F.data(), F.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
@@ -2228,14 +2335,17 @@ static int fa_adjoint(dtmx_ctx* ctx, FaRun& R, int q) {
       ctx->launches++;
     }
     Params PS = P;
-    PS.x0 = 0; PS.x1 = c.nx;
-    PS.xchunk = sweep_xchunk(c, 16, 3);
+    const WorkPlan* wp;
+    if (int rc = plan_work(ctx, WK_ADJ, 16, 3, 0, &wp)) return rc;
+    const WorkPlan& plan = *wp;
+    PS.xchunk = plan.xchunk;
     AdjSweepArgs sa{};
     for (int comp = 0; comp < 6; comp++) sa.dst[comp] = R.lam_alt[comp];
     for (int a = 0; a < 3; a++)
       for (int k = 0; k < 4; k++) { sa.psrc[a][k] = A.lpsi[a][k]; sa.pdst[a][k] = R.lpsi_alt[a][k]; }
-    const dim3 grd((c.nz + TZ - 1) / TZ, (c.ny + 15) / 16, (c.nx + PS.xchunk - 1) / PS.xchunk);
-    launch_after(ctx->early, adj_sweep_kernel<16>, grd, FL<16>::NT, AL<16>::SMEM, st, PS, sa, R.fm[0]);
+    const dim3 grd = plan.grid;
+    if (plan.table) launch_after(ctx->early, adj_sweep_kernel<16, true>, grd, FL<16>::NT, AL<16>::SMEM, st, PS, sa, R.fm[0], plan.work);
+    else launch_after(ctx->early, adj_sweep_kernel<16, false>, grd, FL<16>::NT, AL<16>::SMEM, st, PS, sa, R.fm[0], Work<false>{});
     ctx->launches += 2;
     for (int comp = 0; comp < 6; comp++) std::swap(A.lam[comp], R.lam_alt[comp]);
     for (int a = 0; a < 3; a++)
@@ -2446,6 +2556,9 @@ extern "C" int dtmx_autotune(dtmx_ctx* ctx, int trial_steps, int* engine_out, in
       ctx->frows = cd.rows;
       int r = DTMX_OK;
       const int n = cd.engine == 2 ? (trial_steps / cd.tblock) * cd.tblock : trial_steps;
+      // (the work table is made outside the timed steps)
+      if (cd.engine == 1) r = plan_stream(ctx, nullptr);
+      else if (cd.engine == 3) r = plan_sweep(ctx, nullptr);
       cudaEventRecord(e0, ctx->stream);
       if (cd.engine == 2) {
         for (int q = 0; q < n && !r; q += cd.tblock) r = launch_torre(ctx, cd.tblock);

@@ -712,8 +712,8 @@ __global__ void __launch_bounds__(256) gyro_current_kernel(const __grid_constant
 // The three components' loads are issued together (materials, then flags, then
 // state and taps: three round trips a cell, where a component at a time made
 // nine).  A 236x236x76 gyrotropic layer took 84 + 102 us in two passes and takes
-// 78 (98 with 68 registers a thread: five blocks per SM hide its loads better than three); the Drude film of the reference geometry (8 cells along z, so lanes run along
-// y and z together) 76 -> 32 us.
+// 78 (98 at three blocks per SM instead of five); the Drude film of the reference
+// geometry (8 cells along z, so lanes run along y and z together) 76 -> 32 us.
 template <int ORDER, bool BOX, bool CUR>
 __global__ void __launch_bounds__(256, CUR ? 5 : 4) ade_node_kernel(const __grid_constant__ Params p, int cur) {
   pdl_wait();

@@ -85,8 +85,8 @@ struct Params {
   const uint8_t* mat[3];     // per E component material index (nullptr -> material 0)
   const MatTable* mt;
   Ade ade;
-  int x0, x1;                // planes [x0, x1) processed by a streaming launch
-  int xchunk;                // planes per CTA along x
+  int x0, x1;                // planes [x0, x1) of a wavefront launch
+  int xchunk;                // planes per CTA of a streaming launch without a work table
   int* err;                  // device error word (bounded waits that gave up)
   long long wait_limit;      // polls of one bounded wait (2^26; lowered only to test the timeout paths)
   // per (plane, y tile, z tile): the single non-dispersive material of all E
@@ -101,6 +101,22 @@ struct Params {
   int des_lo[3], des_n[3];
   int des_on;
 };
+
+// The piece of work of a CTA of a streaming launch: z tile, y tile, first plane
+// and plane past the last, from the block index (equal pieces) or from a table
+// (plan_work).  The table is in global memory: as a kernel argument of 4.7 KB it
+// was no faster (128^3: 37.5 against 36.7 us).
+template <bool TAB> struct Work { const int4* e; };
+template <> struct Work<false> {};
+template <bool TAB>
+__device__ __forceinline__ int4 cta_job(const Params& p, const Work<TAB>& w) {
+  if constexpr (TAB) {
+    return __ldg(w.e + blockIdx.x);
+  } else {
+    const int x0 = blockIdx.z * p.xchunk;
+    return make_int4(blockIdx.x, blockIdx.y, x0, min(x0 + p.xchunk, p.g.n[0]));
+  }
+}
 
 __host__ __device__ __forceinline__ long long design_index(const Params& p, int i, int j, int k) {
   if (!p.des_on) return -1;

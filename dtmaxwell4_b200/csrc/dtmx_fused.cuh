@@ -363,10 +363,10 @@ __device__ __forceinline__ void fused_issue(const FusedMaps& m, float* st, uint6
 
 // 16 rows: 3 CTAs per SM, what shared memory allows (a 3-stage ring and two
 // new-H planes); 8 rows: 5
-template <int TY>
+template <int TY, bool TAB>
 __global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
     fused_kernel(const __grid_constant__ Params p, const __grid_constant__ FusedArgs fa,
-                 const __grid_constant__ FusedMaps m) {
+                 const __grid_constant__ FusedMaps m, const __grid_constant__ Work<TAB> work) {
   using L = FL<TY>;
   extern __shared__ __align__(128) float fsm[];
   float* hnb = fsm + F_NST * L::STAGE;                           // two new-H planes
@@ -376,10 +376,9 @@ __global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
   __shared__ signed char umc[FX_MAX];
   __shared__ int gave_up;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int k0 = blockIdx.x * TZ, j0 = blockIdx.y * TY;
-  const int x0 = p.x0 + blockIdx.z * p.xchunk;
-  const int x1 = min(x0 + p.xchunk, p.x1);
-  const int len = x1 - x0;
+  const int4 job = cta_job<TAB>(p, work);
+  const int k0 = job.x * TZ, j0 = job.y * TY;
+  const int x0 = job.z, len = job.w - job.z;
   const int slast = len + 1;                               // stages 0 .. len + 1: planes x0 - 1 .. x1
   const bool cpml = p.ab.kind == 1;
   auto issue = [&](int s, bool want_mat) {
@@ -396,7 +395,7 @@ __global__ void __launch_bounds__(FL<TY>::NT, TY == 16 ? 3 : 5)
   }
   for (int q = tid; q < MAXMAT * 3; q += L::NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
   for (int q = tid; q < len; q += L::NT)
-    umc[q] = __ldg(p.umat + ((long long)(x0 + q) * p.nty + j0 / F_MROWS) * p.ntz + blockIdx.x);
+    umc[q] = __ldg(p.umat + ((long long)(x0 + q) * p.nty + j0 / F_MROWS) * p.ntz + job.x);
   if (cpml) {
     // coefficient row q: x plane x0 - 1 + q, then y row j0 + ..., then z column k0 + ...
     constexpr int RX = FX_MAX + 2, RY_ = TY + 1, RZ = TZ + 1;

@@ -215,8 +215,8 @@ __device__ __forceinline__ void absorb4(int kind, const Q4& d, const float (&c0)
   put4(mem, vec && lm == 15u, m & lm, nv);
 }
 
-template <int ORDER, bool ISH>
-__device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, float* dsm) {
+template <int ORDER, bool ISH, bool TAB>
+__device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, const Work<TAB>& work, float* dsm) {
   using P = Pipe<ORDER, ISH>;
   constexpr int NST = P::NST, AHEAD = P::AHEAD, BEHIND = P::BEHIND, BASE = P::BASE, DIR = P::DIR;
   constexpr int c0 = ISH ? 0 : 3, cf = ISH ? 3 : 0;          // source and updated components
@@ -225,9 +225,9 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
   float* ies = dsm + NST * P::STAGE;                         // 1/eps of the material table (E step)
   uint64_t* bars = reinterpret_cast<uint64_t*>(ies + MAXMAT * 3);
   const int tid = threadIdx.x;
-  const int k0 = blockIdx.x * TZ, j0 = blockIdx.y * TYT;
-  const int xa = p.x0 + blockIdx.z * p.xchunk;
-  const int xb = min(xa + p.xchunk, p.x1);
+  const int4 job = cta_job<TAB>(p, work);
+  const int k0 = job.x * TZ, j0 = job.y * TYT;
+  const int xa = job.z, xb = job.w;
   const int len = xb - xa;
   const int i0 = DIR > 0 ? xa : xb - 1;      // first plane of the walk; step t works on plane i0 + DIR t
   // the uniform-material entries of the planes this CTA stages (stage number s),
@@ -249,7 +249,7 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
     for (int q = tid; q < MAXMAT * 3; q += STREAM_NT) ies[q] = __ldg(&p.mt->inv_eps[0][0] + q);
     for (int sq = tid; sq <= slast && sq < UMC; sq += STREAM_NT) {
       const int ip = i0 + DIR * sq;
-      umc[sq] = (ip >= 0 && ip < p.g.n[0]) ? __ldg(p.umat + ((long long)ip * p.nty + blockIdx.y) * p.ntz + blockIdx.x)
+      umc[sq] = (ip >= 0 && ip < p.g.n[0]) ? __ldg(p.umat + ((long long)ip * p.nty + job.y) * p.ntz + job.x)
                                           : (signed char)0;
     }
   }
@@ -273,7 +273,7 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
     if (ISH) return 0;
     if (sq < UMC) return umc[sq];
     const int ip = i0 + DIR * sq;
-    return (ip >= 0 && ip < p.g.n[0]) ? (int)__ldg(p.umat + ((long long)ip * p.nty + blockIdx.y) * p.ntz + blockIdx.x) : 0;
+    return (ip >= 0 && ip < p.g.n[0]) ? (int)__ldg(p.umat + ((long long)ip * p.nty + job.y) * p.ntz + job.x) : 0;
   };
   auto issue = [&](int sq) {
     const int ip = i0 + DIR * sq;
@@ -496,18 +496,18 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, f
 }
 
 // 4 CTAs per SM: what shared memory allows for the 3-stage rings
-template <int ORDER>
+template <int ORDER, bool TAB>
 __global__ void __launch_bounds__(STREAM_NT, ORDER == 2 ? 4 : 3)
-    h_kernel(const __grid_constant__ Params p, const __grid_constant__ TmaMaps m) {
+    h_kernel(const __grid_constant__ Params p, const __grid_constant__ TmaMaps m, const __grid_constant__ Work<TAB> work) {
   extern __shared__ __align__(128) float dsm[];
-  stream_body<ORDER, true>(p, m, dsm);
+  stream_body<ORDER, true, TAB>(p, m, work, dsm);
 }
 
-template <int ORDER>
+template <int ORDER, bool TAB>
 __global__ void __launch_bounds__(STREAM_NT, ORDER == 2 ? 4 : 3)
-    e_kernel(const __grid_constant__ Params p, const __grid_constant__ TmaMaps m) {
+    e_kernel(const __grid_constant__ Params p, const __grid_constant__ TmaMaps m, const __grid_constant__ Work<TAB> work) {
   extern __shared__ __align__(128) float dsm[];
-  stream_body<ORDER, false>(p, m, dsm);
+  stream_body<ORDER, false, TAB>(p, m, work, dsm);
 }
 
 }  // namespace dtmx

@@ -18,6 +18,8 @@ pytestmark = pytest.mark.gpu
     ((26, 34, 66), ((4, 4), (0, 5), (12, 16)), (8, 10, 14), (8, 10, 12), 12, False),  # the plane cuts the region
     ((24, 17, 40), None, (6, 3, 4), (8, 9, 20), 18, False),
     ((40, 36, 44), ((5, 5), (5, 5), (6, 5)), (12, 12, 12), (8, 9, 11), 33, True),
+    ((48, 150, 140), ((5, 5), (5, 5), (5, 5)), (20, 60, 60), (6, 9, 7), 40, False),   # pieces of equal cost, both sweeps
+    ((30, 300, 290), ((5, 5), (5, 5), (5, 5)), (9, 90, 90), (6, 9, 7), 22, False),    # the adjoint's alone
 ])
 def test_gradient_against_the_oracle(n, pml, lo, d, plane, drude):
     import pyoracle

@@ -51,8 +51,10 @@ def test_tile_edges_equal_the_per_step_engine(n, pml, rows):
 
 
 @pytest.mark.parametrize("n,pml", [
-    ((70, 40, 40), ((6, 6), (6, 6), (6, 6))),        # one wave, pieces of equal cost
-    ((44, 300, 290), ((6, 5), (0, 7), (8, 8))),      # several waves
+    ((70, 40, 40), ((6, 6), (6, 6), (6, 6))),        # one wave, pieces of one plane
+    ((61, 170, 150), ((6, 6), (6, 6), (6, 6))),      # one wave, pieces of equal cost
+    ((44, 300, 290), ((6, 5), (0, 7), (8, 8))),      # one wave of long pieces
+    ((20, 520, 530), ((6, 5), (0, 7), (8, 8))),      # several waves
     ((150, 17, 20), None),                           # pieces as long as a CTA's tables allow (64 planes)
 ])
 def test_pieces_of_equal_cost(n, pml):
