@@ -95,6 +95,8 @@ struct dtmx_ctx {
   std::vector<VmmBlock> vmm;    // the arrays of a parkable context (instead of allocs)
   bool parked = false;
   std::map<std::array<int, 4>, WorkPlan> work;   // by (kind, tile rows, planes per CTA asked for, early launches)
+  WorkPlan work_once;                            // while the caller captures the stream
+  bool own_capture = false;                      // the capture under way is graph_steps16's
   bool early = false;           // launches may overlap their set-up with the kernel ahead (launch_after)
   // coefficient tables
   float* ctab[3][3] = {};
@@ -1355,6 +1357,11 @@ static void work_cut(const dtmx_ctx* ctx, int rows, int budget, std::vector<int4
       }
   if (count) *count = n;
 }
+// the caller captures the context's stream: no allocation, no wait
+static bool capturing(const dtmx_ctx* ctx) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
 enum { WK_STREAM, WK_SWEEP, WK_ADJ };
 constexpr int kOneWave = 40;            // most units of a piece in a single wave
 // The plan of a launch; its table is made on first use, never while a stream is captured.
@@ -1367,6 +1374,7 @@ static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, 
   auto it = ctx->work.find(key);
   if (it == ctx->work.end()) {
     WorkPlan w;
+    bool keep = true;
     w.xchunk = planes;
     if (planes == 0) {
       const long long one = tiles <= fit ? (c.nx + fit / tiles - 1) / (fit / tiles) : c.nx;      // one wave of equal pieces
@@ -1379,12 +1387,15 @@ static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, 
           if (n <= fit) break;
         }
       }
+      std::vector<int4> v;
+      int4* d = nullptr;
       if (budget <= kOneWave) {
-        std::vector<int4> v;
+        // no table while the caller captures the stream, nor without memory for one: equal pieces serve
+        keep = !capturing(ctx);
         work_cut(ctx, rows, budget, &v, nullptr);
-        int4* d = nullptr;
-        int rc = dalloc(ctx, &d, v.size(), true);
-        if (rc) return rc;
+        if (keep && dalloc(ctx, &d, v.size(), true) != DTMX_OK) { cudaGetLastError(); d = nullptr; }
+      }
+      if (d) {
         CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         w.table = true;
@@ -1400,6 +1411,11 @@ static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, 
       }
     }
     if (!w.table) w.grid = dim3(ntz, nty, (c.nx + w.xchunk - 1) / w.xchunk);
+    if (!keep) {
+      ctx->work_once = w;
+      if (plan) *plan = &ctx->work_once;
+      return DTMX_OK;
+    }
     it = ctx->work.emplace(key, w).first;
   }
   if (plan) *plan = &it->second;
@@ -1883,6 +1899,7 @@ static int launch_fused_step(dtmx_ctx* ctx) {
 // Needs fused_prepare's allocations, so call it outside a capture.
 static int step_engine(dtmx_ctx* ctx) {
   if (ctx->engine != 0) return ctx->engine == 3 ? 3 : 1;
+  if (!ctx->own_capture && capturing(ctx)) return 1;     // a graph of the caller's may be replayed any number of times: in place
   if (ctx->ptr_given || ctx->profiling || ctx->cfg.parkable || ctx->auto_per_step || !fused_usable(ctx, nullptr)) return 1;
   if (!ctx->fused_ready) {
     if (fused_set_bytes(ctx) > 0.5 * free_device_bytes() || fused_prepare(ctx) != DTMX_OK) {
@@ -1921,7 +1938,9 @@ static int graph_steps16(dtmx_ctx* ctx) {
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
       return fail(ctx, DTMX_ERR_CUDA, "graph capture could not start");
     int rc = DTMX_OK;
+    ctx->own_capture = true;
     for (int q = 0; q < 16 && !rc; q++) rc = launch_one(ctx);
+    ctx->own_capture = false;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
     if (rc || e != cudaSuccess) { if (g) cudaGraphDestroy(g); cudaGetLastError(); return rc ? rc : fail(ctx, DTMX_ERR_CUDA, "graph capture failed"); }
     e = cudaGraphInstantiate(&ctx->graph16[par], g, 0);

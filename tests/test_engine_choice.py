@@ -77,3 +77,38 @@ def test_profiling_times_both_kernels():
     _equal(_fields(s), _fields(a))
     a.close()
     s.close()
+
+
+def test_steps_captured_by_the_caller():
+    """Steps in a graph of the caller's, replayed an odd and an even number of
+    times, against plain steps."""
+    import torch
+    from dtmaxwell4_b200 import Simulation, abi
+    n = (61, 170, 150)
+    cfg = abi.make_config(*n, courant=0.5, absorber=abi.ABS_CPML, pml=6)
+    rng = np.random.default_rng(3)
+    fields = [rng.standard_normal(n).astype(np.float32) for _ in range(6)]
+    got = []
+    for replays in (0, 3):
+        s = Simulation(cfg)
+        for c in range(6):
+            s.set_field(c, fields[c])
+        s.step(2)
+        if replays:
+            s.sync()
+            st = torch.cuda.ExternalStream(s.stream_handle())
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=st):
+                s.step(1)
+            with torch.cuda.stream(st):
+                for _ in range(replays):
+                    g.replay()
+            torch.cuda.synchronize()
+        else:
+            s.step(3)
+        got.append([s.get_field(c) for c in range(6)])
+        if replays:
+            del g
+        s.close()
+    for c in range(6):
+        assert np.array_equal(got[0][c], got[1][c]), c
