@@ -96,7 +96,6 @@ struct dtmx_ctx {
   bool parked = false;
   std::map<std::array<int, 4>, WorkPlan> work;   // by (kind, tile rows, planes per CTA asked for, early launches)
   WorkPlan work_once;                            // while the caller captures the stream
-  bool own_capture = false;                      // the capture under way is graph_steps16's
   bool early = false;           // launches may overlap their set-up with the kernel ahead (launch_after)
   // coefficient tables
   float* ctab[3][3] = {};
@@ -157,7 +156,8 @@ struct dtmx_ctx {
   FusedMaps fmaps8[2]{};              // the same for 8-row tiles
   int frows = 16;                     // tile rows of the single sweep (16 or 8; dtmx_set_tile_rows, dtmx_autotune)
   bool fused_ready = false;
-  bool ptr_given = false;             // dtmx_field_device_ptr was called: see step_engine
+  bool pinned = false;                // the caller holds the fields' addresses: see step_engine
+  bool graphs_stale = false;          // the step graphs were made before that
   bool auto_per_step = false;         // the automatic choice found no room for the second set
   int parity = 0;                     // 0: state in the buffers allocated first
   int* d_err = nullptr;
@@ -302,6 +302,7 @@ static size_t dense_rows(int nz, size_t rows) { return std::min(rows, std::max<s
 static void drop_graphs(dtmx_ctx* ctx) {
   for (auto& g : ctx->graph16)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+  ctx->graphs_stale = false;
 }
 
 static const char* kErrStr[] = {"ok", "invalid argument", "CUDA error", "out of device memory", "non-finite value",
@@ -1890,17 +1891,18 @@ static int launch_fused_step(dtmx_ctx* ctx) {
 // wherever the single sweep applies: it was faster at every size measured
 // (48^3 9.4 against 34.9 us a step, 128^3 40 against 66, 640x512x384 1.30
 // against 1.79 ms).  The automatic choice stays with the per-step engine
-//   * once dtmx_field_device_ptr has handed out an address (the single sweep
-//     alternates between two sets of arrays, the per-step engine updates the
-//     one the caller holds),
+//   * once the caller holds the fields' addresses, from dtmx_field_device_ptr
+//     or in a graph that steps were captured into, which may be replayed any
+//     number of times and between other steps (the single sweep alternates
+//     between two sets of arrays, the per-step engine updates the one the caller
+//     holds),
 //   * while profiling (which times the H and the E kernel),
 //   * for parkable contexts and where the second set would take more than half
 //     of the free device memory (or cannot be had): it doubles the fields.
 // Needs fused_prepare's allocations, so call it outside a capture.
 static int step_engine(dtmx_ctx* ctx) {
   if (ctx->engine != 0) return ctx->engine == 3 ? 3 : 1;
-  if (!ctx->own_capture && capturing(ctx)) return 1;     // a graph of the caller's may be replayed any number of times: in place
-  if (ctx->ptr_given || ctx->profiling || ctx->cfg.parkable || ctx->auto_per_step || !fused_usable(ctx, nullptr)) return 1;
+  if (ctx->pinned || ctx->profiling || ctx->cfg.parkable || ctx->auto_per_step || !fused_usable(ctx, nullptr)) return 1;
   if (!ctx->fused_ready) {
     if (fused_set_bytes(ctx) > 0.5 * free_device_bytes() || fused_prepare(ctx) != DTMX_OK) {
       fused_release(ctx);
@@ -1909,6 +1911,14 @@ static int step_engine(dtmx_ctx* ctx) {
     }
   }
   return 3;
+}
+
+// From here on the caller holds the addresses of the fields.  (The step graphs go
+// later: this may be called while a stream is captured.)
+static void pin_fields(dtmx_ctx* ctx) {
+  if (ctx->pinned) return;
+  ctx->pinned = true;
+  ctx->graphs_stale = ctx->engine == 0;
 }
 
 // one time step of the selected per-step engine (per-step or single sweep)
@@ -1922,6 +1932,7 @@ static int launch_one(dtmx_ctx* ctx) { return step_engine(ctx) == 3 ? launch_fus
 // (16 single-sweep steps come back to it).
 static int graph_steps16(dtmx_ctx* ctx) {
   const int par = ctx->parity;
+  if (ctx->graphs_stale) drop_graphs(ctx);
   if (!ctx->graph16[par]) {
     set_kernel_attributes();
     if (step_engine(ctx) == 3) {
@@ -1938,9 +1949,7 @@ static int graph_steps16(dtmx_ctx* ctx) {
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
       return fail(ctx, DTMX_ERR_CUDA, "graph capture could not start");
     int rc = DTMX_OK;
-    ctx->own_capture = true;
     for (int q = 0; q < 16 && !rc; q++) rc = launch_one(ctx);
-    ctx->own_capture = false;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
     if (rc || e != cudaSuccess) { if (g) cudaGraphDestroy(g); cudaGetLastError(); return rc ? rc : fail(ctx, DTMX_ERR_CUDA, "graph capture failed"); }
     e = cudaGraphInstantiate(&ctx->graph16[par], g, 0);
@@ -1964,6 +1973,9 @@ extern "C" int dtmx_step(dtmx_ctx* ctx, int nsteps) {
   int rc0 = prepare(ctx);
   if (rc0) return rc0;
   int left = nsteps;
+  // steps that the caller captures: with engine 0 in place, one by one
+  const bool captured = ctx->engine == 0 && nsteps > 0 && capturing(ctx);
+  if (captured) pin_fields(ctx);
   if (ctx->engine == 2) {
     std::string why;
     if (!torre_features_ok(ctx, &why)) return fail(ctx, DTMX_ERR_UNSUPPORTED, "wavefront engine: " + why);
@@ -1981,7 +1993,7 @@ extern "C" int dtmx_step(dtmx_ctx* ctx, int nsteps) {
     // 16 steps as one CUDA graph when every DFT staging cycle is at its start
     // (the captured sequence then repeats exactly: staging slots, the flush
     // every 16 steps and the gyrotropic buffer parity)
-    bool aligned = left >= 16 && !ctx->profiling && !ctx->monitors_off && ctx->engine != 2;
+    bool aligned = left >= 16 && !ctx->profiling && !ctx->monitors_off && ctx->engine != 2 && !captured;
     aligned = aligned && ctx->mon.nstaged == 0;
     if (aligned && !ctx->obj_on) {
       int rc = graph_steps16(ctx);
@@ -2786,7 +2798,7 @@ extern "C" int dtmx_field_device_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64
   if (ctx && ctx->parked) return fail(ctx, DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
   if (!ctx || comp < 0 || comp > 5 || !dptr) return fail(ctx, DTMX_ERR_INVALID, "bad field request");
   // the caller may keep the address: the automatic engine choice leaves the arrays where they are from here on
-  if (!ctx->ptr_given) { ctx->ptr_given = true; if (ctx->engine == 0) drop_graphs(ctx); }
+  pin_fields(ctx);
   *dptr = ctx->P.f[comp];
   if (strides) { strides[0] = ctx->P.g.sx; strides[1] = ctx->P.g.sy; strides[2] = 1; }
   return DTMX_OK;

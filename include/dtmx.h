@@ -438,8 +438,9 @@ int  dtmx_count_nonfinite_noalloc(const float* const* d_fields, int nfields, int
 /* Engine choice for dtmx_step: 0 = auto (the single sweep where it applies and
  * its second set of arrays takes at most half of the free device memory; one
  * launch per half step otherwise, for parkable contexts, while profiling, and
- * once dtmx_field_device_ptr has handed out an address: its arrays then keep
- * holding the state), 1 = one launch per half step,
+ * once the caller holds the fields' addresses, from dtmx_field_device_ptr or in
+ * a graph that steps were captured into: those arrays then keep holding the
+ * state), 1 = one launch per half step,
  * 2 = L2-resident wavefront (several time steps per launch), 3 = single sweep
  * (one launch per time step updating H and then E over two field buffers; box
  * geometry, order 2, CPML or no absorber).  The reference compiles its kernel

@@ -112,3 +112,53 @@ def test_steps_captured_by_the_caller():
         s.close()
     for c in range(6):
         assert np.array_equal(got[0][c], got[1][c]), c
+
+
+@pytest.mark.parametrize("before", [2, 17])
+@pytest.mark.parametrize("inside", [1, 18])
+def test_captured_steps_between_plain_ones(before, inside):
+    """Replays of the caller's graph and plain steps in turn: the captured steps
+    find the state where the plain ones left it, after a gradient run too."""
+    import torch
+    from dtmaxwell4_b200 import Simulation, abi
+    cfg = abi.make_config(*N, courant=0.5, absorber=abi.ABS_CPML, pml=5)
+    rng = np.random.default_rng(4)
+    fields = [rng.standard_normal(N).astype(np.float32) for _ in range(6)]
+    eps = np.full((3, 3, 4, 5), 2.0, np.float32)
+    got = []
+    for graph in (False, True):
+        s = Simulation(cfg)
+        s.set_design((8, 14, 20), eps)
+        for c in range(6):
+            s.set_field(c, fields[c])
+        if not graph:
+            s.set_engine(1)
+        s.step(before)
+        s.sync()
+        out = []
+        if graph:
+            st = torch.cuda.ExternalStream(s.stream_handle())
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=st):
+                s.step(inside)
+        for plain in (0, 1, 19):
+            if graph:
+                with torch.cuda.stream(st):
+                    g.replay()
+            else:
+                s.step(inside)
+            s.step(plain)
+            out.append(_fields(s))
+        s.forward_adjoint(5, 15, 0.4)
+        if graph:
+            with torch.cuda.stream(st):
+                g.replay()
+        else:
+            s.step(inside)
+        out.append(_fields(s))
+        got.append(out)
+        if graph:
+            del g
+        s.close()
+    for a, b in zip(*got):
+        _equal(b, a)
