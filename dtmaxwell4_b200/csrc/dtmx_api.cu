@@ -175,6 +175,7 @@ struct dtmx_ctx {
   bool tmaps_ok = false;
   int* d_ctr = nullptr;
   signed char* d_umat = nullptr;
+  int fail_in[1] = {-1};        // dtmx_fail_next: requests left before one is refused (-1: none)
   std::string err;
 };
 
@@ -430,9 +431,22 @@ static CUresult vmm_back(int dev, VmmBlock& b) {
   return r;
 }
 
+// is this request the one that dtmx_fail_next asked to refuse?
+static bool refuse(dtmx_ctx* ctx, int what) { return ctx->fail_in[what] >= 0 && ctx->fail_in[what]-- == 0; }
+
+// device memory beside the context's own arrays (which dalloc makes); *p is nullptr without it
+template <class T>
+static cudaError_t dev_malloc(dtmx_ctx* ctx, T** p, size_t bytes) {
+  *p = nullptr;
+  const cudaError_t e = refuse(ctx, DTMX_FAIL_ALLOC) ? cudaErrorMemoryAllocation : cudaMalloc((void**)p, bytes);
+  if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); *p = nullptr; }
+  return e;
+}
+
 template <class T>
 static int dalloc(dtmx_ctx* ctx, T** p, size_t count, bool fixed = false) {
   if (ctx->cfg.parkable) {
+    if (refuse(ctx, DTMX_FAIL_ALLOC)) return fail(ctx, DTMX_ERR_OOM, "device memory");
     const VmmApi& A = vmm_api();
     if (!A.ok) return fail(ctx, DTMX_ERR_CUDA, "CUDA virtual memory management is unavailable");
     const CUmemAllocationProp prop = vmm_prop(ctx->dev);
@@ -451,7 +465,7 @@ static int dalloc(dtmx_ctx* ctx, T** p, size_t count, bool fixed = false) {
     return DTMX_OK;
   }
   void* q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
+  cudaError_t e = dev_malloc(ctx, &q, std::max<size_t>(count, 1) * sizeof(T));
   if (e != cudaSuccess) {
     ctx->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? DTMX_ERR_OOM : DTMX_ERR_CUDA;
@@ -760,6 +774,12 @@ extern "C" int dtmx_create(const dtmx_config* cfg, dtmx_ctx** out) {
   return DTMX_OK;
 }
 
+static void dft_free(DftHost& h);
+static void mon_free(MonTable& m) {
+  cudaFree(m.tab); cudaFree(m.map); cudaFree(m.unit);
+  m = MonTable{};
+}
+
 extern "C" void dtmx_destroy(dtmx_ctx* ctx) {
   if (!ctx) return;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
@@ -772,10 +792,10 @@ extern "C" void dtmx_destroy(dtmx_ctx* ctx) {
     A.vfree(b.va, b.size);
     if (b.host) cudaFreeHost(b.host);
   }
-  for (auto& d : ctx->dfts) { cudaFree(d.omega); cudaFree(d.acc); cudaFree(d.stage); cudaFree(d.sstep); }
+  for (auto& d : ctx->dfts) dft_free(d);
   for (auto& fx : ctx->fluxes) cudaFree(fx.d_out);
-  for (MonTable* m : {&ctx->mon, &ctx->objmon}) { cudaFree(m->tab); cudaFree(m->map); cudaFree(m->unit); }
-  cudaFree(ctx->obj.omega); cudaFree(ctx->obj.acc); cudaFree(ctx->obj.stage); cudaFree(ctx->obj.sstep);
+  for (MonTable* m : {&ctx->mon, &ctx->objmon}) mon_free(*m);
+  dft_free(ctx->obj);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   read_slots_drop();
   delete ctx;
@@ -1089,6 +1109,19 @@ extern "C" int dtmx_read_probes(dtmx_ctx* ctx, float* out, int max_samples, int*
   return DTMX_OK;
 }
 
+static void dft_free(DftHost& h) {
+  cudaFree(h.omega); cudaFree(h.acc); cudaFree(h.stage); cudaFree(h.sstep);
+  h.omega = nullptr; h.acc = nullptr; h.stage = nullptr; h.sstep = nullptr;
+}
+// all four arrays of a DFT plane, or none of them
+static bool dft_malloc(dtmx_ctx* ctx, DftHost& h, size_t nfreq, size_t nacc, size_t nstage) {
+  if (dev_malloc(ctx, &h.omega, nfreq * sizeof(double)) == cudaSuccess && dev_malloc(ctx, &h.acc, nacc * sizeof(double2)) == cudaSuccess &&
+      dev_malloc(ctx, &h.stage, nstage * sizeof(float)) == cudaSuccess && dev_malloc(ctx, &h.sstep, DFT_STAGE * sizeof(long long)) == cudaSuccess)
+    return true;
+  dft_free(h);
+  return false;
+}
+
 extern "C" int dtmx_add_dft_patch(dtmx_ctx* ctx, int axis, int index, int lo1, int n1, int lo2, int n2, int comp_mask,
                                   int nfreq, const double* omegas, int* id_out) {
   if (ctx && ctx->parked) return fail(ctx, DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
@@ -1106,13 +1139,8 @@ extern "C" int dtmx_add_dft_patch(dtmx_ctx* ctx, int axis, int index, int lo1, i
   h.d.lo2 = lo2; h.d.n2 = n2;
   h.ncomp = __builtin_popcount(comp_mask);
   const size_t nacc = (size_t)h.ncomp * nfreq * h.d.n1 * h.d.n2;
-  if (cudaMalloc(&h.omega, nfreq * sizeof(double)) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "DFT allocation");
   const size_t nstage = (size_t)DFT_STAGE * h.ncomp * h.d.n1 * h.d.n2;
-  if (cudaMalloc(&h.acc, nacc * sizeof(double2)) != cudaSuccess || cudaMalloc(&h.stage, nstage * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&h.sstep, DFT_STAGE * sizeof(long long)) != cudaSuccess) {
-    cudaFree(h.omega); cudaFree(h.acc); cudaFree(h.stage); cudaFree(h.sstep);
-    return fail(ctx, DTMX_ERR_OOM, "DFT allocation");
-  }
+  if (!dft_malloc(ctx, h, nfreq, nacc, nstage)) return fail(ctx, DTMX_ERR_OOM, "DFT allocation");
   CK(cudaMemsetAsync(h.acc, 0, nacc * sizeof(double2), ctx->stream));
   CK(cudaMemcpyAsync(h.omega, omegas, nfreq * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   h.d.omega = h.omega; h.d.acc = h.acc; h.d.stage = h.stage; h.d.sstep = h.sstep;
@@ -1164,7 +1192,7 @@ extern "C" int dtmx_add_flux_box(dtmx_ctx* ctx, const int lo[3], const int hi[3]
       fx.ffh[2 * a + side] = hid;
     }
   }
-  if (cudaMalloc(&fx.d_out, (size_t)6 * nfreq * sizeof(double)) != cudaSuccess)
+  if (dev_malloc(ctx, &fx.d_out, (size_t)6 * nfreq * sizeof(double)) != cudaSuccess)
     return fail(ctx, DTMX_ERR_OOM, "flux box allocation");
   ctx->fluxes.push_back(fx);
   if (id_out) *id_out = (int)ctx->fluxes.size() - 1;
@@ -1180,8 +1208,7 @@ extern "C" int dtmx_flux_faces(dtmx_ctx* ctx, int id, int faces[6]) {
 
 // Tables of a set of DFT planes (made once: the planes are fixed from the first step on).
 static int mon_build(dtmx_ctx* ctx, MonTable& m, const DftHost* h, int n) {
-  cudaFree(m.tab); cudaFree(m.map); cudaFree(m.unit);
-  m = MonTable{};
+  mon_free(m);
   std::vector<DftDev> tab;
   std::vector<int2> map;
   std::vector<FlushUnit> unit;
@@ -1199,10 +1226,9 @@ static int mon_build(dtmx_ctx* ctx, MonTable& m, const DftHost* h, int n) {
     }
   }
   if (tab.empty()) return DTMX_OK;
-  if (cudaMalloc(&m.tab, tab.size() * sizeof(DftDev)) != cudaSuccess || cudaMalloc(&m.map, map.size() * sizeof(int2)) != cudaSuccess ||
-      cudaMalloc(&m.unit, unit.size() * sizeof(FlushUnit)) != cudaSuccess) {
-    cudaFree(m.tab); cudaFree(m.map); cudaFree(m.unit);
-    m = MonTable{};
+  if (dev_malloc(ctx, &m.tab, tab.size() * sizeof(DftDev)) != cudaSuccess || dev_malloc(ctx, &m.map, map.size() * sizeof(int2)) != cudaSuccess ||
+      dev_malloc(ctx, &m.unit, unit.size() * sizeof(FlushUnit)) != cudaSuccess) {
+    mon_free(m);
     return fail(ctx, DTMX_ERR_OOM, "DFT tables");
   }
   CK(cudaMemcpyAsync(m.tab, tab.data(), tab.size() * sizeof(DftDev), cudaMemcpyHostToDevice, ctx->stream));
@@ -1279,8 +1305,8 @@ extern "C" int dtmx_ntff(dtmx_ctx* ctx, int id, int ndir, const double* theta, c
   }
   double *dth = nullptr, *dph = nullptr, *dout = nullptr;
   const size_t nout = (size_t)ndir * nf * 5;
-  if (cudaMalloc(&dth, ndir * 8) != cudaSuccess || cudaMalloc(&dph, ndir * 8) != cudaSuccess ||
-      cudaMalloc(&dout, nout * 8) != cudaSuccess) {
+  if (dev_malloc(ctx, &dth, ndir * 8) != cudaSuccess || dev_malloc(ctx, &dph, ndir * 8) != cudaSuccess ||
+      dev_malloc(ctx, &dout, nout * 8) != cudaSuccess) {
     cudaFree(dth); cudaFree(dph); cudaFree(dout);
     return fail(ctx, DTMX_ERR_OOM, "far-field allocation");
   }
@@ -2124,7 +2150,7 @@ struct FaRun {
     (void)pool_kept;
     st = ctx->stream;
     void* q = nullptr;
-    if (cudaMallocAsync(&q, bytes, ctx->stream) != cudaSuccess) {
+    if (refuse(ctx, DTMX_FAIL_ALLOC) || cudaMallocAsync(&q, bytes, ctx->stream) != cudaSuccess) {
       // an automatic second set of fields makes room for the adjoint
       cudaGetLastError();
       if (!fused_give_back(ctx) || cudaMallocAsync(&q, bytes, ctx->stream) != cudaSuccess) { cudaGetLastError(); return nullptr; }
@@ -2195,14 +2221,13 @@ static int fa_begin(dtmx_ctx* ctx, FaRun& R, int nsteps, int checkpoint_every, i
   R.plane_x = plane_x; R.omega = omega;
   // objective flux DFT on the plane x = plane_x: Ey, Ez, Hy, Hz at omega
   DftHost& O = ctx->obj;
-  if (!O.acc || O.d.index != plane_x) {
-    cudaFree(O.omega); cudaFree(O.acc); cudaFree(O.stage); cudaFree(O.sstep);
+  if (!ctx->objmon.tab || O.d.index != plane_x) {
+    mon_free(ctx->objmon);
+    dft_free(O);
     O = DftHost{};
     O.d.axis = 0; O.d.index = plane_x; O.d.comp_mask = (1 << 1) | (1 << 2) | (1 << 4) | (1 << 5); O.d.nfreq = 1;
     O.d.n1 = c.ny; O.d.n2 = c.nz; O.ncomp = 4;
-    if (cudaMalloc(&O.omega, 8) != cudaSuccess || cudaMalloc(&O.acc, (size_t)4 * R.npl * sizeof(double2)) != cudaSuccess ||
-        cudaMalloc(&O.stage, (size_t)DFT_STAGE * 4 * R.npl * 4) != cudaSuccess || cudaMalloc(&O.sstep, DFT_STAGE * 8) != cudaSuccess)
-      return fail(ctx, DTMX_ERR_OOM, "objective DFT allocation");
+    if (!dft_malloc(ctx, O, 1, (size_t)4 * R.npl, (size_t)DFT_STAGE * 4 * R.npl)) return fail(ctx, DTMX_ERR_OOM, "objective DFT allocation");
     O.d.omega = O.omega; O.d.acc = O.acc; O.d.stage = O.stage; O.d.sstep = O.sstep;
     if ((rc = mon_build(ctx, ctx->objmon, &O, 1))) return rc;
   }
@@ -2562,7 +2587,7 @@ extern "C" int dtmx_autotune(dtmx_ctx* ctx, int trial_steps, int* engine_out, in
     best = it->second;
   } else {
     char* ck = nullptr;
-    if (cudaMalloc(&ck, state_bytes(ctx)) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "autotune state copy");
+    if (dev_malloc(ctx, &ck, state_bytes(ctx)) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "autotune state copy");
     state_copy(ctx, ck, true);
     const long long step0 = ctx->step;
     const int gcur0 = ctx->gcur, eng0 = ctx->engine, tb0 = ctx->tblock, xc0 = ctx->xchunk, fr0 = ctx->frows;
@@ -2666,7 +2691,7 @@ extern "C" int dtmx_save_state(dtmx_ctx* ctx, const char* path) {
   if (rc) return rc;
   const size_t sb = state_bytes(ctx);
   char* dev = nullptr;
-  if (cudaMalloc(&dev, sb) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "state buffer");
+  if (dev_malloc(ctx, &dev, sb) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "state buffer");
   state_copy(ctx, dev, true);
   std::vector<char> host(sb);
   cudaError_t e = cudaMemcpyAsync(host.data(), dev, sb, cudaMemcpyDeviceToHost, ctx->stream);
@@ -2709,7 +2734,7 @@ extern "C" int dtmx_load_state(dtmx_ctx* ctx, const char* path) {
   fclose(f);
   if (!ok) return fail(ctx, DTMX_ERR_INVALID, "truncated state file");
   char* dev = nullptr;
-  if (cudaMalloc(&dev, sb) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "state buffer");
+  if (dev_malloc(ctx, &dev, sb) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "state buffer");
   cudaError_t e = cudaMemcpyAsync(dev, host.data(), sb, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) { state_copy(ctx, dev, false); e = cudaStreamSynchronize(ctx->stream); }
   cudaFree(dev);
@@ -3127,6 +3152,12 @@ extern "C" int dtmx_set_xchunk(dtmx_ctx* ctx, int planes) {
 extern "C" int dtmx_set_wait_limit(dtmx_ctx* ctx, int64_t polls) {
   if (!ctx) return DTMX_ERR_INVALID;
   ctx->P.wait_limit = polls > 0 ? (long long)polls : kWaitPolls;
+  return DTMX_OK;
+}
+
+extern "C" int dtmx_fail_next(dtmx_ctx* ctx, int what, int skip) {
+  if (!ctx || what != DTMX_FAIL_ALLOC) return fail(ctx, DTMX_ERR_INVALID, "bad failure request");
+  ctx->fail_in[what] = skip < 0 ? -1 : skip;
   return DTMX_OK;
 }
 

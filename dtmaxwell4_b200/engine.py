@@ -26,7 +26,7 @@ EXPORTS = (
     "dtmx_set_design", "dtmx_forward_adjoint", "dtmx_batch_forward_adjoint", "dtmx_autotune",
     "dtmx_write_arr", "dtmx_save_state", "dtmx_load_state",
     "dtmx_add_dft_patch", "dtmx_add_flux_box", "dtmx_read_flux", "dtmx_flux_faces",
-    "dtmx_set_adjoint_memory", "dtmx_ntff", "dtmx_set_wait_limit",
+    "dtmx_set_adjoint_memory", "dtmx_ntff", "dtmx_set_wait_limit", "dtmx_fail_next",
 )
 
 
@@ -99,6 +99,7 @@ def load():
                                              C.POINTER(C.c_double), C.POINTER(vp)]
     L.dtmx_count_nonfinite_noalloc.argtypes = [C.POINTER(C.c_void_p), C.c_int, C.c_int64, C.POINTER(C.c_int64)]
     L.dtmx_set_wait_limit.argtypes = [vp, C.c_int64]
+    L.dtmx_fail_next.argtypes = [vp, ip, ip]
     _lib = L
     return L
 
@@ -342,6 +343,11 @@ class Simulation:
     def set_wait_limit(self, polls):
         """Bound of the device-side waits (polls); <= 0 restores the default."""
         self._ck(self._L.dtmx_set_wait_limit(self._h, int(polls)))
+
+    def fail_next(self, what, skip=0):
+        """Testing aid: the (skip + 1)-th request of a kind (abi.FAIL_ALLOC: a device
+        allocation) from now on is refused on the host; skip < 0: none."""
+        self._ck(self._L.dtmx_fail_next(self._h, int(what), int(skip)))
 
     @property
     def nstep(self):
