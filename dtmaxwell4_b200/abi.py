@@ -22,7 +22,7 @@ MAX_MATERIALS = 64
 WAVE_GAUSS_SINE = 0
 TFSF_DIPOLE, TFSF_PLANE_X = 0, 1
 PROBE_NODE, PROBE_REFERENCE = 0, 1
-FAIL_ALLOC = 0
+FAIL_ALLOC, FAIL_LAUNCH = 0, 1
 
 
 class Config(C.Structure):

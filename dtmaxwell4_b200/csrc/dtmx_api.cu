@@ -96,7 +96,7 @@ struct dtmx_ctx {
   bool parked = false;
   std::map<std::array<int, 4>, WorkPlan> work;   // by (kind, tile rows, planes per CTA asked for, early launches)
   WorkPlan work_once;                            // while the caller captures the stream
-  bool early = false;           // launches may overlap their set-up with the kernel ahead (launch_after)
+  bool early = false;           // launches may overlap their set-up with the kernel ahead (launch)
   // coefficient tables
   float* ctab[3][3] = {};
   // materials
@@ -175,7 +175,8 @@ struct dtmx_ctx {
   bool tmaps_ok = false;
   int* d_ctr = nullptr;
   signed char* d_umat = nullptr;
-  int fail_in[1] = {-1};        // dtmx_fail_next: requests left before one is refused (-1: none)
+  cudaError_t launch_err = cudaSuccess;   // the first launch that failed and has not been reported
+  int fail_in[2] = {-1, -1};    // dtmx_fail_next: requests left before one is refused (-1: none)
   std::string err;
 };
 
@@ -235,14 +236,17 @@ static cudaError_t copy_to_host(int dev, cudaStream_t st, void* host, const void
   ReadSlots& S = read_slots();
   cudaPointerAttributes at{};
   bool direct = bytes < kReadMin;
-  if (!direct && cudaPointerGetAttributes(&at, host) == cudaSuccess) direct = at.type != cudaMemoryTypeUnregistered;
+  if (!direct) {
+    if (cudaPointerGetAttributes(&at, host) == cudaSuccess) direct = at.type != cudaMemoryTypeUnregistered;
+    else cudaGetLastError();
+  }
   std::unique_lock<std::mutex> lk(S.use, std::defer_lock);
   if (!direct && !lk.try_lock()) direct = true;
   if (!direct && !S.buf && cudaHostAlloc((void**)&S.buf, kReadPiece * 2 * kReadThreads, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
     S.buf = nullptr;
     direct = true;
   }
-  cudaGetLastError();
   cudaError_t e = cudaSuccess;
   if (!direct) {
     const size_t pieces = (bytes + kReadPiece - 1) / kReadPiece;
@@ -319,6 +323,9 @@ static const char* kErrStr[] = {"ok", "invalid argument", "CUDA error", "out of 
     }                                                                                      \
   } while (0)
 
+// is this request the one that dtmx_fail_next asked to refuse?
+static bool refuse(dtmx_ctx* ctx, int what) { return ctx->fail_in[what] >= 0 && ctx->fail_in[what]-- == 0; }
+
 // A launch; early: it may start its set-up before the kernel ahead of it on the
 // stream has finished (pdl_wait in the kernel).  Captured into graphs like any
 // other.  A context takes early launches up to 2^23 cells (kEarlyCells) and
@@ -327,20 +334,33 @@ static const char* kErrStr[] = {"ok", "invalid argument", "CUDA error", "out of 
 // a gyrotropic layer 402 -> 409 us and on 57 M with TF/SF and dispersive passes
 // 672 -> 700, and the waiting CTAs take room from the other contexts of a batch
 // (23.2 -> 23.7 ms).
+// A launch that failed is kept in the context until launched() reports it.
 template <class... P, class... A>
-static cudaError_t launch_after(bool early, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+static cudaError_t launch(dtmx_ctx* ctx, bool early, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c{};
   c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st;
-  c.attrs = at; c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, k, P(args)...);
+  c.attrs = at; c.numAttrs = early ? 1 : 0;
+  const cudaError_t e = refuse(ctx, DTMX_FAIL_LAUNCH) ? cudaErrorLaunchOutOfResources : cudaLaunchKernelEx(&c, k, P(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (ctx->launch_err == cudaSuccess) ctx->launch_err = e;
+  }
+  return e;
 }
 
 static int fail(dtmx_ctx* ctx, int code, const std::string& msg) {
   if (ctx) ctx->err = msg;
   return code;
+}
+
+// have all kernels been launched since the last call?
+static int launched(dtmx_ctx* ctx) {
+  const cudaError_t e = ctx->launch_err;
+  ctx->launch_err = cudaSuccess;
+  return e == cudaSuccess ? DTMX_OK : fail(ctx, DTMX_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
 }
 
 static int copy_out(dtmx_ctx* ctx, void* host, const void* devp, size_t bytes) {
@@ -430,9 +450,6 @@ static CUresult vmm_back(int dev, VmmBlock& b) {
   if ((r = A.access(b.va, b.size, &acc, 1)) != CUDA_SUCCESS) { A.unmap(b.va, b.size); A.release(b.h); }
   return r;
 }
-
-// is this request the one that dtmx_fail_next asked to refuse?
-static bool refuse(dtmx_ctx* ctx, int what) { return ctx->fail_in[what] >= 0 && ctx->fail_in[what]-- == 0; }
 
 // device memory beside the context's own arrays (which dalloc makes); *p is nullptr without it
 template <class T>
@@ -1243,9 +1260,9 @@ static int mon_build(dtmx_ctx* ctx, MonTable& m, const DftHost* h, int n) {
 // fold the staged samples of a set of planes into their accumulators
 static void dft_flush(dtmx_ctx* ctx, MonTable& m) {
   if (m.nstaged == 0) return;
-  dft_flush_kernel<<<m.nunit, 256, 0, ctx->stream>>>(m.tab, m.unit, m.nstaged, ctx->cfg.dt);
+  const cudaError_t e = launch(ctx, false, dft_flush_kernel, m.nunit, 256, 0, ctx->stream, m.tab, m.unit, m.nstaged, ctx->cfg.dt);
   ctx->launches++;
-  m.nstaged = 0;
+  if (e == cudaSuccess || m.nstaged == DFT_STAGE) m.nstaged = 0;     // (a fold that did not start is made by the next one, while there is room)
 }
 
 extern "C" int dtmx_read_dft(dtmx_ctx* ctx, int id, double* out, size_t out_len) {
@@ -1255,6 +1272,7 @@ extern "C" int dtmx_read_dft(dtmx_ctx* ctx, int id, double* out, size_t out_len)
   const size_t n = (size_t)h.ncomp * h.d.nfreq * h.d.n1 * h.d.n2 * 2;
   if (out_len < n) return fail(ctx, DTMX_ERR_INVALID, "output buffer too small");
   dft_flush(ctx, ctx->mon);
+  if (int rc = launched(ctx)) return rc;
   return copy_out(ctx, out, h.acc, n * sizeof(double));
 }
 
@@ -1267,10 +1285,10 @@ extern "C" int dtmx_read_flux(dtmx_ctx* ctx, int id, double* out, size_t out_len
   dft_flush(ctx, ctx->mon);
   for (int q = 0; q < 6; q++) {
     DftHost& h = ctx->dfts[fx.face[q]];
-    flux_face_kernel<<<nf, FLUX_THREADS, 0, ctx->stream>>>(h.d, fx.sgn_area[q], fx.d_out + (size_t)q * nf);
+    launch(ctx, false, flux_face_kernel, nf, FLUX_THREADS, 0, ctx->stream, h.d, fx.sgn_area[q], fx.d_out + (size_t)q * nf);
     ctx->launches++;
   }
-  CK(cudaGetLastError());
+  if (int rc = launched(ctx)) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
   CK(cudaMemcpy(out, fx.d_out, (size_t)6 * nf * sizeof(double), cudaMemcpyDeviceToHost));
   for (int f = 0; f < nf; f++) {
@@ -1312,9 +1330,10 @@ extern "C" int dtmx_ntff(dtmx_ctx* ctx, int id, int ndir, const double* theta, c
   }
   CK(cudaMemcpyAsync(dth, theta, ndir * 8, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(dph, phi, ndir * 8, cudaMemcpyHostToDevice, ctx->stream));
-  ntff_kernel<<<dim3(ndir, nf), FLUX_THREADS, 0, ctx->stream>>>(F, dth, dph, nf, dout);
+  launch(ctx, false, ntff_kernel, dim3(ndir, nf), FLUX_THREADS, 0, ctx->stream, F, dth, dph, nf, dout);
   ctx->launches++;
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = ctx->launch_err;
+  ctx->launch_err = cudaSuccess;
   if (e == cudaSuccess) e = cudaMemcpyAsync(out, dout, nout * 8, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   cudaFree(dth); cudaFree(dph); cudaFree(dout);
@@ -1420,7 +1439,7 @@ static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, 
         // no table while the caller captures the stream, nor without memory for one: equal pieces serve
         keep = !capturing(ctx);
         work_cut(ctx, rows, budget, &v, nullptr);
-        if (keep && dalloc(ctx, &d, v.size(), true) != DTMX_OK) { cudaGetLastError(); d = nullptr; }
+        if (keep && dalloc(ctx, &d, v.size(), true) != DTMX_OK) d = nullptr;
       }
       if (d) {
         CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
@@ -1478,7 +1497,7 @@ static long long launch_tail(dtmx_ctx* ctx, const Params& P, cudaStream_t st) {
   a.ticket = ctx->d_ticket;
   const int ns = (int)ctx->psrc.size();
   if (ns > TAIL_SRC) {
-    launch_after(ctx->early, point_source_kernel, (ns + 63) / 64, 64, 0, st, P, ctx->d_psrc, ns, ctx->d_step, c.dt);
+    launch(ctx, ctx->early, point_source_kernel, (ns + 63) / 64, 64, 0, st, P, ctx->d_psrc, ns, ctx->d_step, c.dt);
     nl++;
   } else {
     a.src = ctx->d_psrc; a.ns = ns;
@@ -1503,7 +1522,7 @@ static long long launch_tail(dtmx_ctx* ctx, const Params& P, cudaStream_t st) {
       b.advance = 1;
     }
     const int blocks = std::max(1, b.nmap + (b.hist ? (3 * b.nd + 255) / 256 : 0));
-    launch_after(ctx->early, tail_kernel, blocks, 256, 0, st, P, b, ctx->d_step);
+    launch(ctx, ctx->early, tail_kernel, blocks, 256, 0, st, P, b, ctx->d_step);
     nl++;
     if (m && ++m->nstaged == DFT_STAGE) dft_flush(ctx, *m);
   }
@@ -1527,15 +1546,15 @@ static long long launch_tfsf(dtmx_ctx* ctx, const Params& P, cudaStream_t st, bo
       units = std::max(units, jb.cells / nl * ((nl + 127) / 128));
     }
     const dim3 grd((unsigned)((units + 7) / 8), T.njob[hs] + 1);
-    if (o4) launch_after(ctx->early, tfsf_plane_kernel<4>, grd, 256, 0, st, P, T, l, ctx->d_step, isH);
-    else launch_after(ctx->early, tfsf_plane_kernel<2>, grd, 256, 0, st, P, T, l, ctx->d_step, isH);
+    if (o4) launch(ctx, ctx->early, tfsf_plane_kernel<4>, grd, 256, 0, st, P, T, l, ctx->d_step, isH);
+    else launch(ctx, ctx->early, tfsf_plane_kernel<2>, grd, 256, 0, st, P, T, l, ctx->d_step, isH);
     return 1;
   }
   long long mx = 1;
   for (int r = 0; r < T.njob[hs]; r++) mx = std::max(mx, T.job[hs][r].cells);
   const dim3 grd((unsigned)((mx * 8 + 255) / 256), std::max(1, T.njob[hs]));
-  if (o4) launch_after(ctx->early, tfsf_kernel<4>, grd, 256, 0, st, P, T, ctx->d_step, isH);
-  else launch_after(ctx->early, tfsf_kernel<2>, grd, 256, 0, st, P, T, ctx->d_step, isH);
+  if (o4) launch(ctx, ctx->early, tfsf_kernel<4>, grd, 256, 0, st, P, T, ctx->d_step, isH);
+  else launch(ctx, ctx->early, tfsf_kernel<2>, grd, 256, 0, st, P, T, ctx->d_step, isH);
   return 1;
 }
 // grid of the passes over the ADE box (ade_cell)
@@ -1557,27 +1576,27 @@ static int launch_step(dtmx_ctx* ctx) {
   cudaStream_t st = ctx->stream;
   long long nl = 0;
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], st);
-  if (o4) launch_after(ctx->early, h_kernel<4, false>, grd, blk, Pipe<4, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
-  else if (plan.table) launch_after(ctx->early, h_kernel<2, true>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, plan.work);
-  else launch_after(ctx->early, h_kernel<2, false>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  if (o4) launch(ctx, ctx->early, h_kernel<4, false>, grd, blk, Pipe<4, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  else if (plan.table) launch(ctx, ctx->early, h_kernel<2, true>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, plan.work);
+  else launch(ctx, ctx->early, h_kernel<2, false>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], st);
   nl++;
   nl += launch_tfsf(ctx, P, st, true);
   const int cur = ctx->gcur;
   if (ctx->has_gyro) {
-    launch_after(ctx->early, gyro_current_kernel, ade_grid(P), 256, 0, st, P, cur);
+    launch(ctx, ctx->early, gyro_current_kernel, ade_grid(P), 256, 0, st, P, cur);
     ctx->gcur = 1 - cur;
     nl++;
   }
   if (ctx->profiling) cudaEventRecord(ctx->ev[2], st);
-  if (o4) launch_after(ctx->early, e_kernel<4, false>, grd, blk, Pipe<4, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
-  else if (plan.table) launch_after(ctx->early, e_kernel<2, true>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, plan.work);
-  else launch_after(ctx->early, e_kernel<2, false>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  if (o4) launch(ctx, ctx->early, e_kernel<4, false>, grd, blk, Pipe<4, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  else if (plan.table) launch(ctx, ctx->early, e_kernel<2, true>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, plan.work);
+  else launch(ctx, ctx->early, e_kernel<2, false>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
   if (P.ade.Em[0] || ctx->has_gyro) {
     // dispersive and gyrotropic nodes of the E half step (e_kernel skipped them)
     const bool box = c.geometry == DTMX_GEOM_BOX;
-    if (o4) { if (box) launch_after(ctx->early, ade_node_kernel<4, true, false>, ade_grid(P), 256, 0, st, P, cur); else launch_after(ctx->early, ade_node_kernel<4, false, false>, ade_grid(P), 256, 0, st, P, cur); }
-    else { if (box) launch_after(ctx->early, ade_node_kernel<2, true, false>, ade_grid(P), 256, 0, st, P, cur); else launch_after(ctx->early, ade_node_kernel<2, false, false>, ade_grid(P), 256, 0, st, P, cur); }
+    if (o4) { if (box) launch(ctx, ctx->early, ade_node_kernel<4, true, false>, ade_grid(P), 256, 0, st, P, cur); else launch(ctx, ctx->early, ade_node_kernel<4, false, false>, ade_grid(P), 256, 0, st, P, cur); }
+    else { if (box) launch(ctx, ctx->early, ade_node_kernel<2, true, false>, ade_grid(P), 256, 0, st, P, cur); else launch(ctx, ctx->early, ade_node_kernel<2, false, false>, ade_grid(P), 256, 0, st, P, cur); }
     nl++;
   }
   if (ctx->profiling) {
@@ -1593,7 +1612,7 @@ static int launch_step(dtmx_ctx* ctx) {
   nl += launch_tfsf(ctx, P, st, false);
   nl += launch_tail(ctx, P, st);
   ctx->launches += nl;
-  return DTMX_OK;
+  return launched(ctx);
 }
 
 // First-step preparation: upload the source and probe lists, allocate the
@@ -1735,8 +1754,9 @@ static int launch_torre(dtmx_ctx* ctx, int T) {
     cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]);
     ctx->prof_ms_h += a; ctx->prof_count += T;
   }
-  advance_step_by_kernel<<<1, 1, 0, ctx->stream>>>(ctx->d_step, T);
+  launch(ctx, false, advance_step_by_kernel, 1, 1, 0, ctx->stream, ctx->d_step, T);
   ctx->launches += 2;
+  if (int bad = launched(ctx)) return bad;
   ctx->step += T;
   return DTMX_OK;
 }
@@ -1830,7 +1850,6 @@ static void fused_release(dtmx_ctx* ctx) {
   for (auto& q : ctx->f_alt) drop(q);
   for (auto& a : ctx->hax_alt)
     for (auto& q : a) drop(q);
-  cudaGetLastError();
 }
 
 // The automatic choice's second set given back for another use of the memory:
@@ -1883,9 +1902,9 @@ static int launch_fused_step(dtmx_ctx* ctx) {
   long long nl = launch_tfsf(ctx, PA, st, true);
   const dim3 grd = plan.grid;
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], st);
-  if (ctx->frows == 8) launch_after(ctx->early, fused_kernel<8, false>, grd, FL<8>::NT, FL<8>::SMEM, st, PA, fa, ctx->fmaps8[0], Work<false>{});
-  else if (plan.table) launch_after(ctx->early && !plan.alone, fused_kernel<16, true>, grd, FL<16>::NT, FL<16>::SMEM, st, PA, fa, ctx->fmaps[0], plan.work);
-  else launch_after(ctx->early, fused_kernel<16, false>, grd, FL<16>::NT, FL<16>::SMEM, st, PA, fa, ctx->fmaps[0], Work<false>{});
+  if (ctx->frows == 8) launch(ctx, ctx->early, fused_kernel<8, false>, grd, FL<8>::NT, FL<8>::SMEM, st, PA, fa, ctx->fmaps8[0], Work<false>{});
+  else if (plan.table) launch(ctx, ctx->early && !plan.alone, fused_kernel<16, true>, grd, FL<16>::NT, FL<16>::SMEM, st, PA, fa, ctx->fmaps[0], plan.work);
+  else launch(ctx, ctx->early, fused_kernel<16, false>, grd, FL<16>::NT, FL<16>::SMEM, st, PA, fa, ctx->fmaps[0], Work<false>{});
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], st);
   nl++;
   if (PA.ade.Em[0] || ctx->has_gyro) {
@@ -1893,10 +1912,10 @@ static int launch_fused_step(dtmx_ctx* ctx) {
     // old E, then E -= dt/eps_inf J
     for (int comp = 0; comp < 3; comp++) PB.fe_old[comp] = PA.f[comp];
     if (ctx->has_gyro) {
-      launch_after(ctx->early, ade_node_kernel<2, true, true>, ade_grid(PB), 256, 0, st, PB, ctx->gcur);
+      launch(ctx, ctx->early, ade_node_kernel<2, true, true>, ade_grid(PB), 256, 0, st, PB, ctx->gcur);
       ctx->gcur = 1 - ctx->gcur;
     } else {
-      launch_after(ctx->early, ade_node_kernel<2, true, false>, ade_grid(PB), 256, 0, st, PB, 0);
+      launch(ctx, ctx->early, ade_node_kernel<2, true, false>, ade_grid(PB), 256, 0, st, PB, 0);
     }
     nl++;
   }
@@ -1909,6 +1928,7 @@ static int launch_fused_step(dtmx_ctx* ctx) {
   nl += launch_tfsf(ctx, PB, st, false);
   nl += launch_tail(ctx, PB, st);
   ctx->launches += nl;
+  if ((rc = launched(ctx))) return rc;
   fused_swap(ctx);
   return DTMX_OK;
 }
@@ -1977,7 +1997,15 @@ static int graph_steps16(dtmx_ctx* ctx) {
     int rc = DTMX_OK;
     for (int q = 0; q < 16 && !rc; q++) rc = launch_one(ctx);
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-    if (rc || e != cudaSuccess) { if (g) cudaGraphDestroy(g); cudaGetLastError(); return rc ? rc : fail(ctx, DTMX_ERR_CUDA, "graph capture failed"); }
+    if (rc || e != cudaSuccess) {
+      // nothing of it ran: the bookkeeping goes back too
+      if (ctx->parity != par) fused_swap(ctx);
+      ctx->gcur = gcur0;
+      ctx->mon.nstaged = staged0;
+      if (g) cudaGraphDestroy(g);
+      if (e != cudaSuccess) cudaGetLastError();
+      return rc ? rc : fail(ctx, DTMX_ERR_CUDA, "graph capture failed");
+    }
     e = cudaGraphInstantiate(&ctx->graph16[par], g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) { ctx->graph16[par] = nullptr; cudaGetLastError(); return fail(ctx, DTMX_ERR_CUDA, "graph instantiation failed"); }
@@ -2258,14 +2286,14 @@ static unsigned design_blocks(const FaRun& R) { return (unsigned)((3 * R.nd + 25
 static int fa_forward(dtmx_ctx* ctx, FaRun& R, int st) {
   if (R.full) {
     if (st == 0) {
-      design_capture_kernel<<<design_blocks(R), 256, 0, ctx->stream>>>(ctx->P, R.hist, 0, R.nd);
+      launch(ctx, false, design_capture_kernel, design_blocks(R), 256, 0, ctx->stream, ctx->P, R.hist, 0, R.nd);
       ctx->launches++;
     }
   } else if (st % R.K == 0) {
     state_copy(ctx, R.ck[st / R.K], true);
   }
   if (R.full) ctx->hist_out = R.hist + (size_t)(st + 1) * 3 * R.nd;
-  int rc = launch_one(ctx);
+  int rc = launch_one(ctx);                      // (reports the launch above too)
   ctx->hist_out = nullptr;
   if (rc) return rc;
   ctx->step++;
@@ -2279,6 +2307,7 @@ static int fa_forward_done(dtmx_ctx* ctx, FaRun& R) {
   if (!R.full) state_copy(ctx, R.ck[R.nseg], true);
   DftHost& O = ctx->obj;
   dft_flush(ctx, ctx->objmon);
+  if (int rc = launched(ctx)) return rc;
   std::vector<double> F((size_t)8 * R.npl);
   CK(cudaMemcpyAsync(F.data(), O.acc, F.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -2354,8 +2383,8 @@ static int fa_segment_begin(dtmx_ctx* ctx, FaRun& R, int seg) {
   state_copy(ctx, R.ck[seg], false);
   ctx->step = R.s0 + start;
   ctx->gcur = R.gcur0 ^ (start & 1);
-  design_capture_kernel<<<design_blocks(R), 256, 0, ctx->stream>>>(ctx->P, R.hist, 0, R.nd);
-  return DTMX_OK;
+  launch(ctx, false, design_capture_kernel, design_blocks(R), 256, 0, ctx->stream, ctx->P, R.hist, 0, R.nd);
+  return launched(ctx);
 }
 
 // recompute step q (1..len) of the current segment
@@ -2380,14 +2409,14 @@ static int fa_adjoint(dtmx_ctx* ctx, FaRun& R, int q) {
     const int ns = (R.npl + 255) / 256, ng = (int)design_blocks(R);
     // the sources and the gradient share a launch unless the plane cuts the design region
     if (R.plane_x >= P.des_lo[0] && R.plane_x < P.des_lo[0] + P.des_n[0]) {
-      launch_after(ctx->early, adj_pre_kernel, ns, 256, 0, st, P, A, R.dF, s, R.plane_x, R.omega, c.dt, ns, q);
-      launch_after(ctx->early, adj_pre_kernel, ng, 256, 0, st, P, A, R.dF, s, R.plane_x, R.omega, c.dt, 0, q);
+      launch(ctx, ctx->early, adj_pre_kernel, ns, 256, 0, st, P, A, R.dF, s, R.plane_x, R.omega, c.dt, ns, q);
+      launch(ctx, ctx->early, adj_pre_kernel, ng, 256, 0, st, P, A, R.dF, s, R.plane_x, R.omega, c.dt, 0, q);
       ctx->launches++;
     } else {
-      launch_after(ctx->early, adj_pre_kernel, ns + ng, 256, 0, st, P, A, R.dF, s, R.plane_x, R.omega, c.dt, ns, q);
+      launch(ctx, ctx->early, adj_pre_kernel, ns + ng, 256, 0, st, P, A, R.dF, s, R.plane_x, R.omega, c.dt, ns, q);
     }
     if (P.ade.Em[0]) {
-      launch_after(ctx->early, adj_ade_sweep_kernel, ade_grid(P), 256, 0, st, P, A);
+      launch(ctx, ctx->early, adj_ade_sweep_kernel, ade_grid(P), 256, 0, st, P, A);
       ctx->launches++;
     }
     Params PS = P;
@@ -2400,17 +2429,17 @@ static int fa_adjoint(dtmx_ctx* ctx, FaRun& R, int q) {
     for (int a = 0; a < 3; a++)
       for (int k = 0; k < 4; k++) { sa.psrc[a][k] = A.lpsi[a][k]; sa.pdst[a][k] = R.lpsi_alt[a][k]; }
     const dim3 grd = plan.grid;
-    if (plan.table) launch_after(ctx->early, adj_sweep_kernel<16, true>, grd, FL<16>::NT, AL<16>::SMEM, st, PS, sa, R.fm[0], plan.work);
-    else launch_after(ctx->early, adj_sweep_kernel<16, false>, grd, FL<16>::NT, AL<16>::SMEM, st, PS, sa, R.fm[0], Work<false>{});
+    if (plan.table) launch(ctx, ctx->early, adj_sweep_kernel<16, true>, grd, FL<16>::NT, AL<16>::SMEM, st, PS, sa, R.fm[0], plan.work);
+    else launch(ctx, ctx->early, adj_sweep_kernel<16, false>, grd, FL<16>::NT, AL<16>::SMEM, st, PS, sa, R.fm[0], Work<false>{});
     ctx->launches += 2;
     for (int comp = 0; comp < 6; comp++) std::swap(A.lam[comp], R.lam_alt[comp]);
     for (int a = 0; a < 3; a++)
       for (int k = 0; k < 4; k++) std::swap(A.lpsi[a][k], R.lpsi_alt[a][k]);
     std::swap(R.fm[0], R.fm[1]);
-    return DTMX_OK;
+    return launched(ctx);
   }
-  adj_source_kernel<<<(R.npl + 255) / 256, 256, 0, st>>>(P, A, R.dF, R.s0 + (long long)R.seg * R.K + q, R.plane_x, R.omega, c.dt);
-  adj_grad_kernel<<<design_blocks(R), 256, 0, st>>>(P, A, q);
+  launch(ctx, false, adj_source_kernel, (R.npl + 255) / 256, 256, 0, st, P, A, R.dF, R.s0 + (long long)R.seg * R.K + q, R.plane_x, R.omega, c.dt);
+  launch(ctx, false, adj_grad_kernel, design_blocks(R), 256, 0, st, P, A, q);
   const dim3 blk(32, 8), grd((c.nz + 31) / 32, (c.ny + 7) / 8, c.nx);
   const dim3 wgrd((c.nz + 31) / 32, (c.ny + 7) / 8, (c.nx + ADJ_XP - 1) / ADJ_XP);   // adj_w: ADJ_XP planes per thread
   // the dispersive nodes' transposed ADE recursion replaces their w (after adj_w, before adj_curl);
@@ -2420,23 +2449,23 @@ static int fa_adjoint(dtmx_ctx* ctx, FaRun& R, int q) {
   const int ablk = 256;
   const dim3 agrd = ade_grid(P);
   if (c.order == 4) {
-    adj_w_kernel<4, 0><<<wgrd, blk, 0, st>>>(P, A);
-    if (ade) adj_ade_kernel<<<agrd, ablk, 0, st>>>(P, A);
-    if (gyro) { adj_gyro_mu_kernel<<<agrd, ablk, 0, st>>>(P, A); adj_gyro_j_kernel<<<agrd, ablk, 0, st>>>(P, A); }
-    adj_curl_kernel<4, 0><<<grd, blk, 0, st>>>(P, A);
-    adj_w_kernel<4, 1><<<wgrd, blk, 0, st>>>(P, A);
-    adj_curl_kernel<4, 1><<<grd, blk, 0, st>>>(P, A);
+    launch(ctx, false, adj_w_kernel<4, 0>, wgrd, blk, 0, st, P, A);
+    if (ade) launch(ctx, false, adj_ade_kernel, agrd, ablk, 0, st, P, A);
+    if (gyro) { launch(ctx, false, adj_gyro_mu_kernel, agrd, ablk, 0, st, P, A); launch(ctx, false, adj_gyro_j_kernel, agrd, ablk, 0, st, P, A); }
+    launch(ctx, false, adj_curl_kernel<4, 0>, grd, blk, 0, st, P, A);
+    launch(ctx, false, adj_w_kernel<4, 1>, wgrd, blk, 0, st, P, A);
+    launch(ctx, false, adj_curl_kernel<4, 1>, grd, blk, 0, st, P, A);
     ctx->launches += 6 + (ade ? 1 : 0) + (gyro ? 2 : 0);
   } else {
-    adj_w_kernel<2, 0><<<wgrd, blk, 0, st>>>(P, A);
-    if (ade) adj_ade_kernel<<<agrd, ablk, 0, st>>>(P, A);
-    if (gyro) { adj_gyro_mu_kernel<<<agrd, ablk, 0, st>>>(P, A); adj_gyro_j_kernel<<<agrd, ablk, 0, st>>>(P, A); }
-    adj_curl_kernel<2, 0><<<grd, blk, 0, st>>>(P, A);
-    adj_w_kernel<2, 1><<<wgrd, blk, 0, st>>>(P, A);
-    adj_curl_kernel<2, 1><<<grd, blk, 0, st>>>(P, A);
+    launch(ctx, false, adj_w_kernel<2, 0>, wgrd, blk, 0, st, P, A);
+    if (ade) launch(ctx, false, adj_ade_kernel, agrd, ablk, 0, st, P, A);
+    if (gyro) { launch(ctx, false, adj_gyro_mu_kernel, agrd, ablk, 0, st, P, A); launch(ctx, false, adj_gyro_j_kernel, agrd, ablk, 0, st, P, A); }
+    launch(ctx, false, adj_curl_kernel<2, 0>, grd, blk, 0, st, P, A);
+    launch(ctx, false, adj_w_kernel<2, 1>, wgrd, blk, 0, st, P, A);
+    launch(ctx, false, adj_curl_kernel<2, 1>, grd, blk, 0, st, P, A);
     ctx->launches += 6 + (ade ? 1 : 0) + (gyro ? 2 : 0);
   }
-  return DTMX_OK;
+  return launched(ctx);
 }
 
 // final state back in place, gradient to the caller (waits for the stream)
@@ -2477,7 +2506,7 @@ extern "C" int dtmx_forward_adjoint(dtmx_ctx* ctx, int nsteps, int checkpoint_ev
   for (int st = 0; st < R.N && !rc; st++) rc = fa_forward(ctx, R, st);
   if (!rc) rc = fa_forward_done(ctx, R);
   for (int seg = R.nseg - 1; seg >= 0 && !rc; seg--) {
-    fa_segment_begin(ctx, R, seg);
+    rc = fa_segment_begin(ctx, R, seg);
     for (int q = 1; q <= R.len && !rc; q++) rc = fa_recompute(ctx, R, q);
     for (int q = R.len; q >= 1 && !rc; q--) rc = fa_adjoint(ctx, R, q);
   }
@@ -2537,7 +2566,7 @@ extern "C" int dtmx_batch_forward_adjoint(dtmx_ctx* const* ctxs, int n, int nste
   for (int b = 0; b < n && !rc; b++) rc = fa_forward_done(ctxs[b], R[b]);
   const int nseg = R[0].nseg;
   for (int seg = nseg - 1; seg >= 0 && !rc; seg--) {
-    for (int b = 0; b < n; b++) fa_segment_begin(ctxs[b], R[b], seg);
+    for (int b = 0; b < n && !rc; b++) rc = fa_segment_begin(ctxs[b], R[b], seg);
     const int len = R[0].len;
     for (int q = 1; q <= len && !rc; q++)
       for (int b = 0; b < n && !rc; b++) rc = fa_recompute(ctxs[b], R[b], q);
@@ -2782,9 +2811,9 @@ extern "C" int dtmx_get_field(dtmx_ctx* ctx, int comp, float* host_out) {
   int rc = DTMX_OK;
   for (size_t r = 0; r < rows && !rc; r += per) {
     const size_t n = std::min(per, rows - r);
-    dense_rows_kernel<<<148 * 8, dim3(32, 8), 0, ctx->stream>>>(ctx->P.f[comp] + r * ctx->nzp, ctx->nzp, dense, c.nz, (long long)n, c.nz);
+    launch(ctx, false, dense_rows_kernel, 148 * 8, dim3(32, 8), 0, ctx->stream, ctx->P.f[comp] + r * ctx->nzp, ctx->nzp, dense, c.nz, (long long)n, c.nz);
     ctx->launches++;
-    rc = copy_out(ctx, host_out + r * c.nz, dense, n * c.nz * 4);
+    if (!(rc = launched(ctx))) rc = copy_out(ctx, host_out + r * c.nz, dense, n * c.nz * 4);
   }
   cudaFreeAsync(dense, ctx->stream);
   return rc;
@@ -2803,7 +2832,7 @@ extern "C" int dtmx_set_field(dtmx_ctx* ctx, int comp, const float* host_in) {
     for (size_t r = 0; r < rows && e == cudaSuccess; r += per) {
       const size_t n = std::min(per, rows - r);
       e = cudaMemcpyAsync(dense, host_in + r * c.nz, n * c.nz * 4, cudaMemcpyHostToDevice, ctx->stream);
-      dense_rows_kernel<<<148 * 8, dim3(32, 8), 0, ctx->stream>>>(dense, c.nz, ctx->P.f[comp] + r * ctx->nzp, ctx->nzp, (long long)n, c.nz);
+      launch(ctx, false, dense_rows_kernel, 148 * 8, dim3(32, 8), 0, ctx->stream, dense, c.nz, ctx->P.f[comp] + r * ctx->nzp, ctx->nzp, (long long)n, c.nz);
       ctx->launches++;
     }
     cudaFreeAsync(dense, ctx->stream);
@@ -2813,10 +2842,10 @@ extern "C" int dtmx_set_field(dtmx_ctx* ctx, int comp, const float* host_in) {
                          ctx->stream));
   }
   // non-live nodes are held at zero
-  mask_nonlive_kernel<<<148 * 4, 256, 0, ctx->stream>>>(ctx->P, comp, (long long)ctx->ncell);
+  launch(ctx, false, mask_nonlive_kernel, 148 * 4, 256, 0, ctx->stream, ctx->P, comp, (long long)ctx->ncell);
   ctx->launches++;
   CK(cudaStreamSynchronize(ctx->stream));
-  return DTMX_OK;
+  return launched(ctx);
 }
 
 extern "C" int dtmx_field_device_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]) {
@@ -2834,9 +2863,10 @@ extern "C" int dtmx_check_finite(dtmx_ctx* ctx) {
   if (!ctx) return DTMX_ERR_INVALID;
   CK(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
   for (int comp = 0; comp < 6; comp++) {
-    nonfinite_kernel<<<148 * 4, 256, 0, ctx->stream>>>(ctx->P, comp, (long long)ctx->ncell, ctx->d_flag);
+    launch(ctx, false, nonfinite_kernel, 148 * 4, 256, 0, ctx->stream, ctx->P, comp, (long long)ctx->ncell, ctx->d_flag);
     ctx->launches++;
   }
+  if (int rc = launched(ctx)) return rc;
   int flag = 0;
   CK(cudaMemcpyAsync(&flag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -3156,7 +3186,7 @@ extern "C" int dtmx_set_wait_limit(dtmx_ctx* ctx, int64_t polls) {
 }
 
 extern "C" int dtmx_fail_next(dtmx_ctx* ctx, int what, int skip) {
-  if (!ctx || what != DTMX_FAIL_ALLOC) return fail(ctx, DTMX_ERR_INVALID, "bad failure request");
+  if (!ctx || (what != DTMX_FAIL_ALLOC && what != DTMX_FAIL_LAUNCH)) return fail(ctx, DTMX_ERR_INVALID, "bad failure request");
   ctx->fail_in[what] = skip < 0 ? -1 : skip;
   return DTMX_OK;
 }

@@ -346,7 +346,7 @@ class Simulation:
 
     def fail_next(self, what, skip=0):
         """Testing aid: the (skip + 1)-th request of a kind (abi.FAIL_ALLOC: a device
-        allocation) from now on is refused on the host; skip < 0: none."""
+        allocation, abi.FAIL_LAUNCH: a kernel launch) from now on is refused on the host; skip < 0: none."""
         self._ck(self._L.dtmx_fail_next(self._h, int(what), int(skip)))
 
     @property

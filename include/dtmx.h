@@ -291,10 +291,12 @@ int  dtmx_kernel_launches(const dtmx_ctx* ctx, int64_t* n);
 int  dtmx_set_wait_limit(dtmx_ctx* ctx, int64_t polls);
 
 /* Testing aid for the paths of a refused request: the (skip + 1)-th device
- * allocation of this context from now on (DTMX_FAIL_ALLOC) fails on the host, as if the
- * memory were not there, without being asked for; skip < 0: none.  No reference
+ * allocation (DTMX_FAIL_ALLOC) or kernel launch (DTMX_FAIL_LAUNCH) of this
+ * context from now on fails on the host, as if the memory or the resources were
+ * not there, without being asked for; skip < 0: none.  No reference
  * counterpart. */
 #define DTMX_FAIL_ALLOC 0
+#define DTMX_FAIL_LAUNCH 1
 int  dtmx_fail_next(dtmx_ctx* ctx, int what, int skip);
 
 /* The context's CUDA stream (cudaStream_t), for event timing by the caller. */
