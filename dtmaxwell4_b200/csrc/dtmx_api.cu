@@ -108,7 +108,9 @@ struct dtmx_ctx {
   std::vector<uint8_t> h_mat[3];
   // sources
   std::vector<PointSrcDev> psrc;
-  PointSrcDev* d_psrc = nullptr;
+  PointSrcDev* d_psrc = nullptr;   // the sources sorted by node (prepare)
+  int2* d_psrc_run = nullptr;      // {first, count} of each node's
+  int nrun = 0;
   int has_tfsf = 0;
   dtmx_tfsf tfsf{};
   TfsfDev T{};
@@ -1497,7 +1499,7 @@ static long long launch_tail(dtmx_ctx* ctx, const Params& P, cudaStream_t st) {
   a.ticket = ctx->d_ticket;
   const int ns = (int)ctx->psrc.size();
   if (ns > TAIL_SRC) {
-    launch(ctx, ctx->early, point_source_kernel, (ns + 63) / 64, 64, 0, st, P, ctx->d_psrc, ns, ctx->d_step, c.dt);
+    launch(ctx, ctx->early, point_source_kernel, (ctx->nrun + 63) / 64, 64, 0, st, P, ctx->d_psrc, ctx->d_psrc_run, ctx->nrun, ctx->d_step, c.dt);
     nl++;
   } else {
     a.src = ctx->d_psrc; a.ns = ns;
@@ -1620,9 +1622,20 @@ static int launch_step(dtmx_ctx* ctx) {
 static int prepare(dtmx_ctx* ctx) {
   if (ctx->prepared) return DTMX_OK;
   int rc;
-  if (!ctx->psrc.empty()) {
-    if ((rc = dalloc(ctx, &ctx->d_psrc, ctx->psrc.size(), true))) return rc;
-    CK(cudaMemcpyAsync(ctx->d_psrc, ctx->psrc.data(), ctx->psrc.size() * sizeof(PointSrcDev), cudaMemcpyHostToDevice, ctx->stream));
+  std::vector<PointSrcDev> sorted = ctx->psrc;
+  std::vector<int2> runs;
+  if (!sorted.empty()) {
+    // by node, sources on one node in the order they were given
+    std::stable_sort(sorted.begin(), sorted.end(),
+                     [](const PointSrcDev& a, const PointSrcDev& b) { return std::tie(a.comp, a.id) < std::tie(b.comp, b.id); });
+    for (int q = 0; q < (int)sorted.size(); q++) {
+      if (q > 0 && sorted[q].comp == sorted[q - 1].comp && sorted[q].id == sorted[q - 1].id) runs.back().y++;
+      else runs.push_back(make_int2(q, 1));
+    }
+    if ((rc = dalloc(ctx, &ctx->d_psrc, sorted.size(), true)) || (rc = dalloc(ctx, &ctx->d_psrc_run, runs.size(), true))) return rc;
+    CK(cudaMemcpyAsync(ctx->d_psrc, sorted.data(), sorted.size() * sizeof(PointSrcDev), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_psrc_run, runs.data(), runs.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->nrun = (int)runs.size();
   }
   if (!ctx->probes.empty()) {
     if ((rc = dalloc(ctx, &ctx->d_probes, ctx->probes.size(), true))) return rc;

@@ -273,19 +273,23 @@ __device__ __forceinline__ float source_value(const PointSrcDev& s, long long n,
   return (float)(s.amp * sin(2.0 * M_PI * s.f0 * u) * exp(-(u / s.tau) * (u / s.tau)));
 }
 
-// More soft sources than the tail kernel's list holds.  Sources on one node are
-// added in their order by the first of them.
-__global__ void point_source_kernel(const __grid_constant__ Params p, const PointSrcDev* s, int ns, const long long* d_step, double dt) {
+// More soft sources than the tail kernel's list holds.  The list is sorted by node
+// when it is made, sources on one node in the order they were given; a
+// thread adds those of one node: run[q] = {first, count}.  (Without the sorted
+// list every thread searched all sources for its node's: 16384 sources took
+// 4 ms a step: 64x272x272 cells 4064 us, now 56, without sources 53.)
+__global__ void point_source_kernel(const __grid_constant__ Params p, const PointSrcDev* s, const int2* run, int nrun, const long long* d_step,
+                                    double dt) {
   pdl_wait();
   pdl_trigger();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= ns) return;
-  for (int e = 0; e < q; e++)
-    if (s[e].comp == s[q].comp && s[e].id == s[q].id) return;
-  float v = p.f[s[q].comp][s[q].id];
-  for (int e = q; e < ns; e++)
-    if (s[e].comp == s[q].comp && s[e].id == s[q].id) v += source_value(s[e], *d_step, dt);
-  p.f[s[q].comp][s[q].id] = v;
+  if (q >= nrun) return;
+  const int2 r = run[q];
+  float* f = p.f[s[r.x].comp] + s[r.x].id;
+  const long long n = *d_step;
+  float v = *f;
+  for (int e = r.x; e < r.x + r.y; e++) v += source_value(s[e], n, dt);
+  *f = v;
 }
 
 struct ProbeDev { int comp, i, j, k, mode; };
@@ -401,13 +405,11 @@ __global__ void __launch_bounds__(256) tail_kernel(const __grid_constant__ Param
   __syncthreads();
   if (!last) return;
   if (tid < a.ns) {
-    // sources on one node are added in their order by the first of them
-    bool first = true;
-    for (int q = 0; q < tid; q++) first = first && !(s.comp[q] == s.comp[tid] && s.id[q] == s.id[tid]);
-    if (first) {
+    // the list is sorted by node: the first source of a node adds those that follow it there
+    auto same = [&](int q) { return s.comp[q] == s.comp[tid] && s.id[q] == s.id[tid]; };
+    if (tid == 0 || !same(tid - 1)) {
       float v = p.f[s.comp[tid]][s.id[tid]];
-      for (int q = tid; q < a.ns; q++)
-        if (s.comp[q] == s.comp[tid] && s.id[q] == s.id[tid]) v += s.v[q];
+      for (int q = tid; q < a.ns && same(q); q++) v += s.v[q];
       p.f[s.comp[tid]][s.id[tid]] = v;
     }
   }

@@ -79,3 +79,58 @@ def test_windows_and_reads_mid_cycle(window):
     for out in got[1:]:
         for x, y in zip(out, got[0]):
             assert np.array_equal(x, y)
+
+
+def test_thousands_of_sources():
+    """Far more sources than the launch's list holds, in no order, several on one
+    node: after one step from zero fields E holds their sums, added in the
+    order given.  Tolerance: 2e-6 of the largest (FP32 sums of at most ten
+    values)."""
+    from dtmaxwell4_b200 import Simulation, abi
+    n = (20, 40, 50)
+    s = Simulation(abi.make_config(*n, courant=0.5, pml=4))
+    rng = np.random.default_rng(4)
+    want = [np.zeros(n, np.float32) for _ in range(3)]
+    dt = s.cfg.dt
+    for q in range(5000):
+        c, i, j, k = int(rng.integers(3)), 10, int(rng.integers(8, 32)), int(rng.integers(8, 42))
+        src = abi.PointSource(comp=c, i=i, j=j, k=k, waveform=abi.WAVE_GAUSS_SINE, amp=float(rng.uniform(-2, 2)), f0=0.05, tau=15.0,
+                              t0=float(rng.uniform(2, 12)))
+        s.add_point_source(src)
+        u = 0.5 * dt - src.t0
+        want[c][i, j, k] += np.float32(src.amp * np.sin(2 * np.pi * src.f0 * u) * np.exp(-(u / src.tau) ** 2))
+    s.step(1)
+    top = max(np.abs(w).max() for w in want)
+    for c in range(3):
+        assert np.abs(s.get_field(c) - want[c]).max() <= 2e-6 * top, c
+    s.close()
+
+
+def _step_us(make, n=48):
+    import time
+    s = make()
+    best = 1e9
+    s.step(n)
+    s.sync()
+    for _ in range(4):
+        t = time.perf_counter()
+        s.step(n)
+        s.sync()
+        best = min(best, (time.perf_counter() - t) / n)
+    s.close()
+    return 1e6 * best
+
+
+def test_cost_of_a_sheet_of_sources():
+    """A sheet of 128 x 128 sources is one short launch more: well below 0.3 ms a
+    step (searching the whole list for each source took 4 ms)."""
+    from dtmaxwell4_b200 import Simulation, abi
+
+    def make(m):
+        s = Simulation(abi.make_config(24, 150, 150, courant=0.5, pml=4))
+        for q in range(m * m):
+            s.add_point_source(abi.PointSource(comp=abi.EZ, i=12, j=10 + q // m, k=10 + q % m, waveform=abi.WAVE_GAUSS_SINE, amp=1e-3,
+                                               f0=0.05, tau=20.0, t0=30.0))
+        return s
+    one, sheet = _step_us(lambda: make(1)), _step_us(lambda: make(128))
+    assert sheet - one <= 300.0, (one, sheet)
