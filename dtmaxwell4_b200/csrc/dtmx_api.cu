@@ -1523,7 +1523,7 @@ static long long launch_tail(dtmx_ctx* ctx, const Params& P, cudaStream_t st) {
       b.nd = P.des_on ? P.des_n[0] * P.des_n[1] * P.des_n[2] : 0;
       b.advance = 1;
     }
-    const int blocks = std::max(1, b.nmap + (b.hist ? (3 * b.nd + 255) / 256 : 0));
+    const int blocks = std::max({1, b.nmap + (b.hist ? (3 * b.nd + 255) / 256 : 0), (b.np + 255) / 256});
     launch(ctx, ctx->early, tail_kernel, blocks, 256, 0, st, P, b, ctx->d_step);
     nl++;
     if (m && ++m->nstaged == DFT_STAGE) dft_flush(ctx, *m);

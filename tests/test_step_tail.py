@@ -134,3 +134,46 @@ def test_cost_of_a_sheet_of_sources():
         return s
     one, sheet = _step_us(lambda: make(1)), _step_us(lambda: make(128))
     assert sheet - one <= 300.0, (one, sheet)
+
+
+@pytest.mark.parametrize("every", [1, 3])
+@pytest.mark.parametrize("npr", [255, 256, 257, 1500])
+def test_many_probes(npr, every):
+    """Probes around and beyond a block of 256, next to fewer and to no DFT blocks,
+    with a source on probed nodes: the traces are the fields' values."""
+    from dtmaxwell4_b200 import Simulation, abi
+    n = (20, 22, 31)
+    rng = np.random.default_rng(npr)
+    at = [(int(rng.integers(6)),) + tuple(int(rng.integers(0, m)) for m in n) for _ in range(npr)]
+    at[npr - 1] = at[0] = (abi.EZ, 9, 10, 11)
+    for plane in (False, True):
+        s = Simulation(abi.make_config(*n, courant=0.5, pml=4, probe_every=every, probe_capacity=2))
+        s.add_point_source(abi.PointSource(comp=abi.EZ, i=9, j=10, k=11, waveform=abi.WAVE_GAUSS_SINE, amp=1.0, f0=0.05, tau=15.0, t0=4.0))
+        for c in range(6):
+            s.set_field(c, rng.standard_normal(n).astype(np.float32))
+        for p in at:
+            s.add_probe(*p)
+        if plane:
+            s.add_dft_plane(0, 9, 1 << abi.EZ, [0.3])
+        for sample in range(3):                   # (the third one has no room)
+            s.step(every)
+            f = [s.get_field(c) for c in range(6)]
+            if sample < 2:
+                want = np.array([f[c][i, j, k] for c, i, j, k in at])
+                got = s.read_probes()
+                assert got.shape == (npr, sample + 1) and np.array_equal(got[:, sample], want)
+        assert s.read_probes().shape == (npr, 2)
+        s.close()
+
+
+def test_cost_of_many_probes():
+    """20000 probes stay well below 40 us a step (one block took 100)."""
+    from dtmaxwell4_b200 import Simulation, abi
+
+    def make(npr):
+        s = Simulation(abi.make_config(24, 150, 150, courant=0.5, pml=4, probe_capacity=4096))
+        for q in range(npr):
+            s.add_probe(q % 6, 4 + q % 16, 5 + q // 150, 3 + (q * 7) % 140)
+        return s
+    few, many = _step_us(lambda: make(8)), _step_us(lambda: make(20000))
+    assert many - few <= 40.0, (few, many)
