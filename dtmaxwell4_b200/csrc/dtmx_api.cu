@@ -2861,14 +2861,19 @@ extern "C" int dtmx_set_field(dtmx_ctx* ctx, int comp, const float* host_in) {
   return launched(ctx);
 }
 
-extern "C" int dtmx_field_device_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]) {
+extern "C" int dtmx_field_current_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]) {
   if (ctx && ctx->parked) return fail(ctx, DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
   if (!ctx || comp < 0 || comp > 5 || !dptr) return fail(ctx, DTMX_ERR_INVALID, "bad field request");
-  // the caller may keep the address: the automatic engine choice leaves the arrays where they are from here on
-  pin_fields(ctx);
   *dptr = ctx->P.f[comp];
   if (strides) { strides[0] = ctx->P.g.sx; strides[1] = ctx->P.g.sy; strides[2] = 1; }
   return DTMX_OK;
+}
+
+extern "C" int dtmx_field_device_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]) {
+  const int rc = dtmx_field_current_ptr(ctx, comp, dptr, strides);
+  // the caller may keep the address: the automatic engine choice leaves the arrays where they are from here on
+  if (!rc) pin_fields(ctx);
+  return rc;
 }
 
 extern "C" int dtmx_check_finite(dtmx_ctx* ctx) {

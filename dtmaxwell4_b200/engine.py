@@ -19,7 +19,7 @@ EXPORTS = (
     "dtmx_version", "dtmx_error_string", "dtmx_create", "dtmx_destroy", "dtmx_last_error",
     "dtmx_set_materials", "dtmx_add_point_source", "dtmx_set_tfsf", "dtmx_add_probe",
     "dtmx_read_probes", "dtmx_add_dft_plane", "dtmx_read_dft", "dtmx_step", "dtmx_sync",
-    "dtmx_get_step", "dtmx_get_field", "dtmx_set_field", "dtmx_field_device_ptr",
+    "dtmx_get_step", "dtmx_get_field", "dtmx_set_field", "dtmx_field_device_ptr", "dtmx_field_current_ptr",
     "dtmx_check_finite", "dtmx_kernel_launches", "dtmx_set_engine", "dtmx_set_xchunk", "dtmx_park", "dtmx_unpark", "dtmx_set_park_pool", "dtmx_plane_state_floats", "dtmx_read_planes", "dtmx_write_planes", "dtmx_copy_planes", "dtmx_set_tile_rows", "dtmx_get_engine", "dtmx_get_stream",
     "dtmx_set_profiling", "dtmx_read_profile", "dtmx_abi_sizes", "dtmx_count_nonfinite_noalloc",
     "dtmx_tfsfsrc_set", "dtmx_ref_main", "dtmx_ref_materials", "dtmx_ref_material_table",
@@ -72,6 +72,7 @@ def load():
     L.dtmx_get_field.argtypes = [vp, ip, vp]
     L.dtmx_set_field.argtypes = [vp, ip, vp]
     L.dtmx_field_device_ptr.argtypes = [vp, ip, C.POINTER(vp), C.POINTER(C.c_int64)]
+    L.dtmx_field_current_ptr.argtypes = [vp, ip, C.POINTER(vp), C.POINTER(C.c_int64)]
     L.dtmx_check_finite.argtypes = [vp]
     L.dtmx_kernel_launches.argtypes = [vp, C.POINTER(C.c_int64)]
     L.dtmx_set_engine.argtypes = [vp, ip, ip]
@@ -400,11 +401,14 @@ class Simulation:
         self._ck(self._L.dtmx_get_stream(self._h, C.byref(v)))
         return v.value
 
-    def device_ptr(self, comp):
-        """(device address, element strides (x, y, z)) of a field component."""
+    def device_ptr(self, comp, keep=True):
+        """(device address, element strides (x, y, z)) of a field component.
+        keep=False: for a caller who asks again after each step()
+        (dtmx_field_current_ptr)."""
         p = C.c_void_p()
         st = (C.c_int64 * 3)()
-        self._ck(self._L.dtmx_field_device_ptr(self._h, comp, C.byref(p), st))
+        ask = self._L.dtmx_field_device_ptr if keep else self._L.dtmx_field_current_ptr
+        self._ck(ask(self._h, comp, C.byref(p), st))
         return p.value, (st[0], st[1], st[2])
 
     def set_profiling(self, on=True):

@@ -21,7 +21,9 @@ each rank sends its first owned E plane to the left neighbour and its last
 owned E plane to the right neighbour (3 contiguous planes per direction),
 with torch.distributed point-to-point operations (NCCL between GPUs: the
 library's device memory is sent and received in place on the context's
-stream; gloo on the host).  No collective is issued inside a step.
+stream; gloo on the host).  No collective is issued inside a step.  Each rank
+chooses its engine as a one-domain run does, so the results are that run's, bit
+for bit (the engines round a TF/SF source's correction of H differently).
 
 The CPML slabs of the x faces belong to the first and last ranks (each must
 own more planes than its slab, so that no ghost plane lies in one); the y
@@ -98,7 +100,9 @@ class _DeviceArray:
 
 class DevicePlanes:
     """x planes of a GPU Simulation as torch tensors that alias its device
-    memory: sent and received in place, ordered on the context's stream."""
+    memory: sent and received in place, ordered on the context's stream.  The
+    addresses are asked for at each use, so the context keeps its engine choice
+    (the single sweep alternates between two sets of arrays)."""
 
     def __init__(self, sim):
         import torch
@@ -107,7 +111,7 @@ class DevicePlanes:
         self.stream = torch.cuda.ExternalStream(sim.stream_handle())
 
     def _plane(self, comp, i):
-        ptr, st = self.sim.device_ptr(comp)
+        ptr, st = self.sim.device_ptr(comp, keep=False)
         return self.torch.as_tensor(_DeviceArray(ptr + 4 * i * st[0], st[0]), device="cuda")
 
     def send(self, comp, i):

@@ -274,6 +274,9 @@ int  dtmx_set_field(dtmx_ctx* ctx, int comp, const float* host_in);
  * stays at that address with engines 0, 1 and 2; engine 3 alternates between
  * two sets of arrays, so ask again after each dtmx_step. */
 int  dtmx_field_device_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]);
+/* The same for a caller who asks again after each dtmx_step: the address holds
+ * the state until then, and the engine choice stays as it is. */
+int  dtmx_field_current_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]);
 
 /* Host-side NaN/Inf check of the probe traces and a device reduction over E;
  * returns DTMX_ERR_NONFINITE if any is found. */

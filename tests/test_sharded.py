@@ -239,3 +239,58 @@ def test_sharded_single_rank_is_the_plain_run():
     assert np.array_equal(a.read_dft(da[1]), b.read_dft(db[1]))
     a.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["plane", "dipole", "none"])
+def test_two_slabs_of_one_gpu_equal_the_plain_run(kind):
+    """Two ranks' slabs stepped in turn on one GPU, their E planes handed over
+    through the device plane accessor after each step (no collective): with the
+    engine each takes by default, the fields are the default one-domain run's,
+    bit for bit, TF/SF sources included."""
+    import torch
+    from dtmaxwell4_b200 import Simulation, abi, scenarios
+    from dtmaxwell4_b200.sharded import DevicePlanes, ShardedSimulation, SlabPlan
+    if kind == "none":
+        cfg, mats, idx, src, probes, fields = _scenario()
+        sc, steps = None, 30
+    else:
+        from test_window import _tfsf_scenario
+        sc, steps = _tfsf_scenario(kind)
+        cfg = sc["cfg"]
+
+    def fill(s):
+        if sc is None:
+            _apply(s, mats, idx, src, probes, fields)
+        else:
+            scenarios.apply(s, sc)
+    slabs = []
+    for rank in range(2):
+        s = ShardedSimulation(cfg)
+        s.local.close()
+        s.plan = SlabPlan(cfg, 2, rank)           # the rank's slab without a process group
+        s.local = Simulation(s.plan.cfg)
+        s.planes = DevicePlanes(s.local)
+        fill(s)
+        slabs.append(s)
+    a, b = slabs
+    for _ in range(steps):
+        for s in slabs:
+            s.local.step(1)
+            s.sync()
+        lo, hi = a.plan.owned_local()
+        first = b.plan.owned_local()[0]
+        for c in (abi.EX, abi.EY, abi.EZ):
+            b.planes.recv(c, 0).copy_(a.planes.send(c, hi - 1))
+            a.planes.recv(c, a.plan.nxl - 1).copy_(b.planes.send(c, first))
+        torch.cuda.synchronize()
+    one = Simulation(cfg)
+    fill(one)
+    one.step(steps)
+    assert np.abs(one.get_field(abi.EZ)).max() > 1e-4
+    for c in range(6):
+        got = np.concatenate([np.asarray(s.local.get_field(c))[slice(*s.plan.owned_local())] for s in slabs])
+        assert np.array_equal(got, one.get_field(c)), c
+    one.close()
+    for s in slabs:
+        s.close()
