@@ -158,6 +158,12 @@ struct dtmx_ctx {
   FusedMaps fmaps8[2]{};              // the same for 8-row tiles
   int frows = 16;                     // tile rows of the single sweep (16 or 8; dtmx_set_tile_rows, dtmx_autotune)
   bool fused_ready = false;
+  // The automatic choice's second set may be given back to whoever needs the
+  // memory, another thread too, while no call on this context is using it.
+  std::mutex run;
+  std::atomic<std::thread::id> runner{};   // the thread that holds run
+  bool lendable = false;              // registered in lenders()
+  bool spare_others = false;          // an allocation that is not worth another context's set
   bool pinned = false;                // the caller holds the fields' addresses: see step_engine
   bool graphs_stale = false;          // the step graphs were made before that
   bool auto_per_step = false;         // the automatic choice found no room for the second set
@@ -453,15 +459,78 @@ static CUresult vmm_back(int dev, VmmBlock& b) {
   return r;
 }
 
+// the caller captures the context's stream: no allocation, no wait
+static bool capturing(const dtmx_ctx* ctx) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+// Calls that use a context's second set hold it while they run (again within
+// the same thread: a batch holds all of its contexts).
+struct Running {
+  dtmx_ctx* c;
+  explicit Running(dtmx_ctx* ctx) : c(ctx && ctx->runner.load() != std::this_thread::get_id() ? ctx : nullptr) {
+    if (!c) return;
+    c->run.lock();
+    c->runner = std::this_thread::get_id();
+  }
+  ~Running() {
+    if (!c) return;
+    c->runner = std::thread::id();
+    c->run.unlock();
+  }
+  Running(Running&& o) : c(o.c) { o.c = nullptr; }
+};
+// the contexts whose automatic choice has made a second set
+struct Lenders {
+  std::mutex mu;
+  std::vector<dtmx_ctx*> list;
+};
+static Lenders& lenders() {
+  static Lenders l;
+  return l;
+}
+static bool fused_give_back(dtmx_ctx* ctx);
+// Memory for a request of ctx that failed: the second set of this context (own: the
+// request is not made in the middle of a step that uses it), else that of
+// another one on the device that no other thread is using.  False: there is none.
+static bool free_a_set(dtmx_ctx* ctx, bool own) {
+  cudaGetLastError();
+  if (ctx->spare_others) return false;
+  if (own) {
+    const Running running(ctx);
+    if (fused_give_back(ctx)) return true;
+  }
+  Lenders& L = lenders();
+  std::lock_guard<std::mutex> lk(L.mu);
+  for (dtmx_ctx* h : L.list) {
+    if (h == ctx || h->dev != ctx->dev) continue;
+    const bool mine = h->runner.load() == std::this_thread::get_id();
+    if (!mine && !h->run.try_lock()) continue;
+    const bool got = fused_give_back(h);
+    if (!mine) h->run.unlock();
+    if (got) return true;
+  }
+  return false;
+}
+
 // device memory beside the context's own arrays (which dalloc makes); *p is nullptr without it
 template <class T>
-static cudaError_t dev_malloc(dtmx_ctx* ctx, T** p, size_t bytes) {
+static cudaError_t dev_malloc(dtmx_ctx* ctx, T** p, size_t bytes, bool own = true) {
   *p = nullptr;
-  const cudaError_t e = refuse(ctx, DTMX_FAIL_ALLOC) ? cudaErrorMemoryAllocation : cudaMalloc((void**)p, bytes);
+  cudaError_t e = refuse(ctx, DTMX_FAIL_ALLOC) ? cudaErrorMemoryAllocation : cudaMalloc((void**)p, bytes);
+  while (e == cudaErrorMemoryAllocation && free_a_set(ctx, own)) e = cudaMalloc((void**)p, bytes);
   if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); *p = nullptr; }
   return e;
 }
 
+static bool vmm_back_or_free(dtmx_ctx* ctx, VmmBlock& b) {
+  CUresult r = vmm_back(ctx->dev, b);
+  while (r == CUDA_ERROR_OUT_OF_MEMORY && free_a_set(ctx, false)) r = vmm_back(ctx->dev, b);
+  return r == CUDA_SUCCESS;
+}
+
+// an array of the context (made before the first step or in a step: its own second set stays)
 template <class T>
 static int dalloc(dtmx_ctx* ctx, T** p, size_t count, bool fixed = false) {
   if (ctx->cfg.parkable) {
@@ -476,7 +545,7 @@ static int dalloc(dtmx_ctx* ctx, T** p, size_t count, bool fixed = false) {
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
     b.size = (bytes + g - 1) / g * g;
     if (A.reserve(&b.va, b.size, 0, 0, 0) != CUDA_SUCCESS) return fail(ctx, DTMX_ERR_OOM, "address reservation");
-    if (vmm_back(ctx->dev, b) != CUDA_SUCCESS) { A.vfree(b.va, b.size); return fail(ctx, DTMX_ERR_OOM, "device memory"); }
+    if (!vmm_back_or_free(ctx, b)) { A.vfree(b.va, b.size); return fail(ctx, DTMX_ERR_OOM, "device memory"); }
     b.fixed = fixed;
     ctx->vmm.push_back(b);
     CK(cudaMemsetAsync((void*)b.va, 0, b.size, ctx->stream));
@@ -484,7 +553,7 @@ static int dalloc(dtmx_ctx* ctx, T** p, size_t count, bool fixed = false) {
     return DTMX_OK;
   }
   void* q = nullptr;
-  cudaError_t e = dev_malloc(ctx, &q, std::max<size_t>(count, 1) * sizeof(T));
+  cudaError_t e = dev_malloc(ctx, &q, std::max<size_t>(count, 1) * sizeof(T), false);
   if (e != cudaSuccess) {
     ctx->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? DTMX_ERR_OOM : DTMX_ERR_CUDA;
@@ -801,6 +870,11 @@ static void mon_free(MonTable& m) {
 
 extern "C" void dtmx_destroy(dtmx_ctx* ctx) {
   if (!ctx) return;
+  if (ctx->lendable) {
+    std::lock_guard<std::mutex> lk(lenders().mu);
+    auto& l = lenders().list;
+    l.erase(std::find(l.begin(), l.end(), ctx));
+  }
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   for (auto& g : ctx->graph16)
     if (g) cudaGraphExecDestroy(g);
@@ -1405,11 +1479,6 @@ static void work_cut(const dtmx_ctx* ctx, int rows, int budget, std::vector<int4
       }
   if (count) *count = n;
 }
-// the caller captures the context's stream: no allocation, no wait
-static bool capturing(const dtmx_ctx* ctx) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
-}
 enum { WK_STREAM, WK_SWEEP, WK_ADJ };
 constexpr int kOneWave = 40;            // most units of a piece in a single wave
 // The plan of a launch; its table is made on first use, never while a stream is captured.
@@ -1867,8 +1936,10 @@ static void fused_release(dtmx_ctx* ctx) {
 
 // The automatic choice's second set given back for another use of the memory:
 // the context goes on with the per-step engine (the state is always in P.f).
+// Not while the caller captures the stream: nothing may be freed then.
 static bool fused_give_back(dtmx_ctx* ctx) {
-  if (ctx->engine != 0 || !ctx->fused_ready || ctx->cfg.parkable) return false;
+  if (ctx->engine != 0 || !ctx->fused_ready || ctx->cfg.parkable || capturing(ctx)) return false;
+  cudaStreamSynchronize(ctx->stream);
   drop_graphs(ctx);
   ctx->fused_ready = false;
   ctx->auto_per_step = true;
@@ -1956,18 +2027,29 @@ static int launch_fused_step(dtmx_ctx* ctx) {
 //     between two sets of arrays, the per-step engine updates the one the caller
 //     holds),
 //   * while profiling (which times the H and the E kernel),
-//   * for parkable contexts and where the second set would take more than half
-//     of the free device memory (or cannot be had): it doubles the fields.
+//   * for parkable contexts, where the second set would take more than an eighth
+//     of the free device memory (or cannot be had), and once it has been given
+//     back: it doubles the fields, and the memory left is the caller's.  A
+//     request for device memory that fails, on this or another context, takes the
+//     set (free_a_set); other allocators cannot, hence the eighth.
 // Needs fused_prepare's allocations, so call it outside a capture.
 static int step_engine(dtmx_ctx* ctx) {
   if (ctx->engine != 0) return ctx->engine == 3 ? 3 : 1;
   if (ctx->pinned || ctx->profiling || ctx->cfg.parkable || ctx->auto_per_step || !fused_usable(ctx, nullptr)) return 1;
   if (!ctx->fused_ready) {
-    if (fused_set_bytes(ctx) > 0.5 * free_device_bytes() || fused_prepare(ctx) != DTMX_OK) {
+    ctx->spare_others = true;
+    const bool made = fused_set_bytes(ctx) <= 0.125 * free_device_bytes() && fused_prepare(ctx) == DTMX_OK;
+    ctx->spare_others = false;
+    if (!made) {
       fused_release(ctx);
       ctx->auto_per_step = true;
       return 1;
     }
+  }
+  if (!ctx->lendable) {
+    std::lock_guard<std::mutex> lk(lenders().mu);
+    lenders().list.push_back(ctx);
+    ctx->lendable = true;
   }
   return 3;
 }
@@ -2037,12 +2119,14 @@ static int graph_steps16(dtmx_ctx* ctx) {
 extern "C" int dtmx_step(dtmx_ctx* ctx, int nsteps) {
   if (ctx && ctx->parked) return fail(ctx, DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
   if (!ctx || nsteps < 0) return fail(ctx, DTMX_ERR_INVALID, "bad step count");
+  const Running running(ctx);
   int rc0 = prepare(ctx);
   if (rc0) return rc0;
   int left = nsteps;
   // steps that the caller captures: with engine 0 in place, one by one
   const bool captured = ctx->engine == 0 && nsteps > 0 && capturing(ctx);
   if (captured) pin_fields(ctx);
+  if (ctx->pinned) fused_give_back(ctx);
   if (ctx->engine == 2) {
     std::string why;
     if (!torre_features_ok(ctx, &why)) return fail(ctx, DTMX_ERR_UNSUPPORTED, "wavefront engine: " + why);
@@ -2191,11 +2275,9 @@ struct FaRun {
     (void)pool_kept;
     st = ctx->stream;
     void* q = nullptr;
-    if (refuse(ctx, DTMX_FAIL_ALLOC) || cudaMallocAsync(&q, bytes, ctx->stream) != cudaSuccess) {
-      // an automatic second set of fields makes room for the adjoint
-      cudaGetLastError();
-      if (!fused_give_back(ctx) || cudaMallocAsync(&q, bytes, ctx->stream) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    }
+    cudaError_t e = refuse(ctx, DTMX_FAIL_ALLOC) ? cudaErrorMemoryAllocation : cudaMallocAsync(&q, bytes, ctx->stream);
+    while (e != cudaSuccess && free_a_set(ctx, true)) e = cudaMallocAsync(&q, bytes, ctx->stream);
+    if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
     bufs.push_back(q);
     return q;
   }
@@ -2212,10 +2294,12 @@ static double fa_history_bytes(const dtmx_ctx* ctx, int nsteps) {
   const Params& P = ctx->P;
   return (double)(nsteps + 1) * 3.0 * P.des_n[0] * P.des_n[1] * P.des_n[2] * 4.0;
 }
+// the bytes of an automatic second set: as good as free
+static double lent_bytes(const dtmx_ctx* ctx) { return ctx->engine == 0 && ctx->fused_ready && !ctx->cfg.parkable ? fused_set_bytes(ctx) : 0.0; }
 static bool fa_history_fits(dtmx_ctx* ctx, int nsteps) {
   const double bytes = fa_history_bytes(ctx, nsteps);
   if (ctx->adj_budget >= 0) return bytes <= (double)ctx->adj_budget;
-  return bytes <= 0.25 * free_device_bytes();
+  return bytes <= 0.25 * (free_device_bytes() + lent_bytes(ctx));
 }
 
 // The adjoint as one sweep a step (dtmx_adjsweep.cuh): the Yee stencil without
@@ -2512,6 +2596,7 @@ extern "C" int dtmx_forward_adjoint(dtmx_ctx* ctx, int nsteps, int checkpoint_ev
                                     double* objective, float* grad_eps) {
   if (ctx && ctx->parked) return fail(ctx, DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
   if (!ctx || !objective || !grad_eps) return fail(ctx, DTMX_ERR_INVALID, "bad arguments");
+  const Running running(ctx);
   FaRun R;
   if (nsteps < 1 || checkpoint_every < 1) return fail(ctx, DTMX_ERR_INVALID, "bad arguments");
   int rc = fa_begin(ctx, R, nsteps, checkpoint_every, plane_x, omega, fa_history_fits(ctx, nsteps));
@@ -2543,6 +2628,9 @@ extern "C" int dtmx_batch_forward_adjoint(dtmx_ctx* const* ctxs, int n, int nste
   if (!ctxs || n < 1 || !plane_x || !omega || !objectives || !grads) return DTMX_ERR_INVALID;
   for (int b = 0; b < n; b++)
     if (ctxs[b] && ctxs[b]->parked) return fail(ctxs[b], DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
+  std::vector<Running> running;
+  running.reserve(n);
+  for (int b = 0; b < n; b++) running.emplace_back(ctxs[b]);
   std::vector<FaRun> R(n);
   // one context's early launches would hold room that another's kernels need
   struct Plain {
@@ -2563,15 +2651,16 @@ extern "C" int dtmx_batch_forward_adjoint(dtmx_ctx* const* ctxs, int n, int nste
   };
   // one mode for the whole batch (the segments advance in lock step)
   bool full = nsteps >= 1;
-  double total = 0.0;
+  double total = 0.0, lent = 0.0;
   bool automatic = true;
   for (int b = 0; b < n; b++) {
     full = full && ctxs[b] && fa_history_fits(ctxs[b], nsteps);
     if (!full) break;
     total += fa_history_bytes(ctxs[b], nsteps);
+    lent += lent_bytes(ctxs[b]);
     automatic = automatic && ctxs[b]->adj_budget < 0;
   }
-  if (full && automatic) full = total <= 0.25 * free_device_bytes();
+  if (full && automatic) full = total <= 0.25 * (free_device_bytes() + lent);
   for (int b = 0; b < n; b++)
     if ((rc = fa_begin(ctxs[b], R[b], nsteps, checkpoint_every, plane_x[b], omega[b], full))) { abort_all(b); return rc; }
   for (int st = 0; st < nsteps && !rc; st++)
@@ -2616,6 +2705,7 @@ extern "C" int dtmx_autotune(dtmx_ctx* ctx, int trial_steps, int* engine_out, in
                              double* ms_per_step_out) {
   if (ctx && ctx->parked) return fail(ctx, DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
   if (!ctx || trial_steps < 1) return fail(ctx, DTMX_ERR_INVALID, "bad arguments");
+  const Running running(ctx);
   int rc = prepare(ctx);
   if (rc) return rc;
   const dtmx_config& c = ctx->cfg;
@@ -2731,6 +2821,7 @@ extern "C" int dtmx_save_state(dtmx_ctx* ctx, const char* path) {
   if (!ctx || !path) return fail(ctx, DTMX_ERR_INVALID, "bad arguments");
   int rc = prepare(ctx);
   if (rc) return rc;
+  const Running running(ctx);
   const size_t sb = state_bytes(ctx);
   char* dev = nullptr;
   if (dev_malloc(ctx, &dev, sb) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "state buffer");
@@ -2775,6 +2866,7 @@ extern "C" int dtmx_load_state(dtmx_ctx* ctx, const char* path) {
   const bool ok = fread(host.data(), 1, sb, f) == sb;
   fclose(f);
   if (!ok) return fail(ctx, DTMX_ERR_INVALID, "truncated state file");
+  const Running running(ctx);
   char* dev = nullptr;
   if (dev_malloc(ctx, &dev, sb) != cudaSuccess) return fail(ctx, DTMX_ERR_OOM, "state buffer");
   cudaError_t e = cudaMemcpyAsync(dev, host.data(), sb, cudaMemcpyHostToDevice, ctx->stream);
@@ -2872,7 +2964,11 @@ extern "C" int dtmx_field_current_ptr(dtmx_ctx* ctx, int comp, void** dptr, int6
 extern "C" int dtmx_field_device_ptr(dtmx_ctx* ctx, int comp, void** dptr, int64_t strides[3]) {
   const int rc = dtmx_field_current_ptr(ctx, comp, dptr, strides);
   // the caller may keep the address: the automatic engine choice leaves the arrays where they are from here on
-  if (!rc) pin_fields(ctx);
+  if (!rc) {
+    const Running running(ctx);
+    pin_fields(ctx);
+    fused_give_back(ctx);
+  }
   return rc;
 }
 
@@ -2899,6 +2995,7 @@ extern "C" int dtmx_kernel_launches(const dtmx_ctx* ctx, int64_t* n) {
 
 extern "C" int dtmx_set_engine(dtmx_ctx* ctx, int engine, int time_block) {
   if (!ctx || engine < 0 || engine > 3 || time_block < 0) return fail(ctx, DTMX_ERR_INVALID, "bad engine");
+  const Running running(ctx);
   if (engine == 3) {
     std::string why;
     if (!fused_usable(ctx, &why)) return fail(ctx, DTMX_ERR_UNSUPPORTED, "single-sweep engine: " + why);
@@ -2911,7 +3008,10 @@ extern "C" int dtmx_set_engine(dtmx_ctx* ctx, int engine, int time_block) {
   } else {
     ctx->tblock = time_block;
   }
+  // the per-step and wavefront engines have no use for an automatic choice's second set
+  if (engine == 1 || engine == 2) fused_give_back(ctx);
   ctx->engine = engine;
+  ctx->auto_per_step = false;
   drop_graphs(ctx);
   return DTMX_OK;
 }
@@ -2968,7 +3068,7 @@ extern "C" int dtmx_unpark(dtmx_ctx* ctx) {
   CK(cudaSetDevice(ctx->dev));
   for (size_t q = 0; q < ctx->vmm.size(); q++) {
     VmmBlock& b = ctx->vmm[q];
-    if (vmm_back(ctx->dev, b) != CUDA_SUCCESS) {
+    if (!vmm_back_or_free(ctx, b)) {
       // keep the context consistent: release what was mapped again and stay parked
       const VmmApi& A = vmm_api();
       for (size_t r = 0; r < q; r++) { A.unmap(ctx->vmm[r].va, ctx->vmm[r].size); A.release(ctx->vmm[r].h); }
@@ -3176,6 +3276,7 @@ extern "C" int dtmx_write_planes(dtmx_ctx* ctx, int x0, int nplanes, const float
 
 extern "C" int dtmx_set_tile_rows(dtmx_ctx* ctx, int rows) {
   if (!ctx || (rows != 0 && rows != 8 && rows != 16)) return fail(ctx, DTMX_ERR_INVALID, "tile rows must be 8 or 16");
+  const Running running(ctx);
   ctx->frows = rows ? rows : 16;
   drop_graphs(ctx);
   return DTMX_OK;
@@ -3192,6 +3293,7 @@ extern "C" int dtmx_get_engine(dtmx_ctx* ctx, int* engine, int* time_block, int*
 
 extern "C" int dtmx_set_xchunk(dtmx_ctx* ctx, int planes) {
   if (!ctx || planes < 0) return fail(ctx, DTMX_ERR_INVALID, "bad x chunk");
+  const Running running(ctx);
   ctx->xchunk = planes;
   drop_graphs(ctx);
   return DTMX_OK;

@@ -448,7 +448,9 @@ int  dtmx_load_state(dtmx_ctx* ctx, const char* path);
 int  dtmx_count_nonfinite_noalloc(const float* const* d_fields, int nfields, int64_t nelem, int64_t* count_out);
 
 /* Engine choice for dtmx_step: 0 = auto (the single sweep where it applies and
- * its second set of arrays takes at most half of the free device memory; one
+ * its second set of arrays takes at most an eighth of the free device memory,
+ * and until a later request of this or another context for device memory
+ * needs that set; dtmx_set_engine(ctx, 1, 0) gives it back at once; one
  * launch per half step otherwise, for parkable contexts, while profiling, and
  * once the caller holds the fields' addresses, from dtmx_field_device_ptr or in
  * a graph that steps were captured into: those arrays then keep holding the

@@ -1,0 +1,202 @@
+"""The automatic engine's second set of fields is memory that others may have.
+
+A request for device memory that fails takes it, from the context that asks
+or from another one that no thread is using, and the context it was taken from
+goes on with the per-step engine: the same fields, bit for bit.  Choosing
+the per-step engine, or holding the fields' addresses, gives it back at once.
+Device memory is filled from outside (by PyTorch) up to a margin that holds
+what the call needs only if the set is given up.
+"""
+import contextlib
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+N = (160, 150, 170)                    # 18.4 MB a component as stored
+MB = 1 << 20
+
+
+def _sim(seed=1, **kw):
+    from dtmaxwell4_b200 import Simulation, abi
+    kw.setdefault("absorber", abi.ABS_NONE)
+    kw.setdefault("pml", 0)
+    s = Simulation(abi.make_config(*N, courant=0.5, **kw))
+    rng = np.random.default_rng(seed)
+    for c in (1, 3):
+        s.set_field(c, rng.standard_normal(N).astype(np.float32))
+    return s
+
+
+def _run(s, *steps):
+    for n in steps:
+        s.step(n)
+    return [s.get_field(c) for c in range(6)]
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+@contextlib.contextmanager
+def _left(nbytes):
+    """Device memory filled up to nbytes."""
+    import torch
+    t = torch.empty(max(0, _free() - nbytes), dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del t
+        torch.cuda.empty_cache()
+
+
+@pytest.fixture(scope="module")
+def want():
+    a = _sim()
+    a.set_engine(1)
+    out = {5: _run(a, 5), 12: _run(a, 7)}
+    a.close()
+    return out
+
+
+def _equal(got, ref):
+    for c in range(6):
+        assert np.array_equal(got[c], ref[c]), c
+
+
+def test_another_context_takes_it(want):
+    import torch
+    torch.zeros(1, device="cuda")
+    a = _sim()
+    a.step(5)
+    a.sync()
+    # a second context needs about 130 MB, the set is 110
+    with _left(60 * MB):
+        b = _sim(2)
+        _equal(_run(a, 7), want[12])
+        assert np.abs(b.get_field(1)).max() > 0
+        b.close()
+    a.close()
+
+
+def test_a_parked_context_takes_it_to_come_back(want):
+    b = _sim(2, parkable=True)
+    first = _run(b, 3)
+    b.park()
+    a = _sim()
+    a.step(5)
+    a.sync()
+    with _left(60 * MB):
+        b.unpark()
+        _equal([b.get_field(c) for c in range(6)], first)
+        _equal(_run(a, 7), want[12])
+    b.close()
+    a.close()
+
+
+def test_the_context_itself_takes_it(want, tmp_path):
+    """The copy of the state that a file is written from (the fields again)."""
+    a = _sim()
+    a.step(5)
+    a.sync()
+    with _left(60 * MB):
+        a.save_state(str(tmp_path / "s"))
+        _equal(_run(a, 7), want[12])
+    a.load_state(str(tmp_path / "s"))
+    _equal([a.get_field(c) for c in range(6)], want[5])
+    a.close()
+
+
+@pytest.mark.parametrize("how", ["set_engine", "device_ptr", "captured"])
+def test_given_back_when_it_has_no_use(want, how):
+    import torch
+    a = _sim()
+    a.step(2)
+    a.sync()
+    with_set = _free()
+    if how == "set_engine":
+        a.set_engine(1)
+    elif how == "device_ptr":
+        a.device_ptr(0)
+    else:
+        st = torch.cuda.ExternalStream(a.stream_handle())
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            a.step(1)
+        with torch.cuda.stream(st):
+            g.replay()
+    _equal(_run(a, 3 if how != "captured" else 2), want[5])
+    assert _free() >= with_set + 100 * MB
+    if how == "captured":
+        with torch.cuda.stream(st):
+            g.replay()
+        _equal(_run(a, 6), want[12])
+        del g
+    a.close()
+
+
+def test_a_context_in_use_by_another_thread_keeps_its_state(want):
+    """Contexts made while another thread steps: each is made or refused, and the
+    fields of the stepped one are what they should be."""
+    from dtmaxwell4_b200 import abi
+    from dtmaxwell4_b200.engine import DtmxError
+    a = _sim()
+    a.step(1)
+    a.sync()
+    out, go = [], threading.Event()
+
+    def steps():
+        go.set()
+        for _ in range(11):
+            a.step(1)
+            a.sync()
+        out.append([a.get_field(c) for c in range(6)])
+    with _left(60 * MB):
+        t = threading.Thread(target=steps)
+        t.start()
+        go.wait()
+        for _ in range(6):
+            try:
+                _sim(2).close()
+            except DtmxError as e:
+                assert e.code == abi.ERR_OOM
+        t.join()
+    _equal(out[0], want[12])
+    a.close()
+
+
+@pytest.mark.parametrize("budget", [-1, 0])
+def test_a_batch_with_refused_allocations(budget):
+    """Each allocation of one context of a batch refused in turn: the sets of the
+    batch's contexts make room, or the call reports it."""
+    from dtmaxwell4_b200 import Simulation, abi
+    from dtmaxwell4_b200.engine import DtmxError, batch_forward_adjoint
+    n = (20, 18, 21)
+
+    def make(q):
+        s = Simulation(abi.make_config(*n, courant=0.5, pml=4))
+        s.set_design((7, 6, 8), np.full((3, 4, 5, 4), 2.0 + q, np.float32))
+        s.set_field(2, np.random.default_rng(q).standard_normal(n).astype(np.float32))
+        s.set_adjoint_memory(budget)
+        return s
+    ref = None
+    done = 0
+    for k in range(-1, 60):
+        sims = [make(q) for q in range(3)]
+        sims[1].fail_next(abi.FAIL_ALLOC, k)
+        try:
+            got = batch_forward_adjoint(sims, 6, [15] * 3, [0.4] * 3, checkpoint_every=3)
+        except DtmxError as e:
+            assert e.code == abi.ERR_OOM and k >= 0
+        else:
+            done += 1
+            ref = ref or got
+            assert got[0] == ref[0] and all(np.array_equal(x, y) for x, y in zip(got[1], ref[1])), k
+        for s in sims:
+            s.close()
+    assert done >= 30
