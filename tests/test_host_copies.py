@@ -68,3 +68,52 @@ def test_spectra_are_complex_arrays():
     for k, w in enumerate(om):
         assert np.allclose(out[0, k], e * np.exp(-1j * w * dt) * dt, rtol=0, atol=1e-12 * np.abs(e).max())
     s.close()
+
+
+@pytest.mark.parametrize("n", [(9, 8, 11), (64, 161, 103), (128, 128, 64), (128, 128, 65)])
+def test_without_memory_for_the_dense_copy(n):
+    """No device memory for the dense copy of padded rows (kept by the context up to
+    4 MB, from the stream's pool above): the strided copy gives the same."""
+    from dtmaxwell4_b200 import Simulation, abi
+    s = Simulation(abi.make_config(*n, absorber=abi.ABS_NONE, pml=0))
+    a = np.random.default_rng(7).standard_normal(n).astype(np.float32)
+    for k in range(2):                            # (then with it)
+        s.fail_next(abi.FAIL_ALLOC, 0 if k == 0 else -1)
+        s.set_field(4, a)
+        s.fail_next(abi.FAIL_ALLOC, 0 if k == 0 else -1)
+        assert np.array_equal(s.get_field(4), a)
+        a = a + 1
+    s.close()
+
+
+def test_a_parked_context_keeps_no_dense_copy():
+    import torch
+    from dtmaxwell4_b200 import Simulation, abi
+    n = (100, 100, 100)
+    s = Simulation(abi.make_config(*n, absorber=abi.ABS_NONE, pml=0, parkable=True))
+    a = np.random.default_rng(8).standard_normal(n).astype(np.float32)
+    s.park()
+    without = torch.cuda.mem_get_info()[0]
+    s.unpark()
+    s.set_field(4, a)
+    s.park()
+    assert torch.cuda.mem_get_info()[0] == without
+    s.unpark()
+    assert np.array_equal(s.get_field(4), a)
+    s.close()
+
+
+def test_cost_of_setting_a_small_field():
+    """48^3 cells with padded rows: well below 250 us (a block from the pool on every
+    call took 450, the strided copy takes 160)."""
+    import time
+    from dtmaxwell4_b200 import Simulation, abi
+    s = Simulation(abi.make_config(48, 48, 48, pml=8))
+    a = np.ones((48, 48, 48), np.float32)
+    best = 1e9
+    for _ in range(12):
+        t = time.perf_counter()
+        s.set_field(2, a)
+        best = min(best, time.perf_counter() - t)
+    assert best <= 250e-6, best
+    s.close()
