@@ -1602,6 +1602,12 @@ static long long launch_tail(dtmx_ctx* ctx, const Params& P, cudaStream_t st) {
   return nl;
 }
 
+// Nodes of a half step's dipole corrections up to which a node gets eight threads
+// instead of one (tfsf_kernel).  Measured, us a step added by the corrections:
+// order 2, 19 thousand nodes 12.6 with eight and 15.9 with one, 43 thousand 22 and 16,
+// 307 thousand 126 and 30; order 4, whose nodes have up to two crossing taps of
+// a term, 32 thousand 17 and 22, 58 thousand 28 and 23, 920 thousand 378 and 122.
+constexpr long long kTapNodes2 = 28000, kTapNodes4 = 44000;
 // TF/SF corrections of one half step, and the plane wave's line
 static long long launch_tfsf(dtmx_ctx* ctx, const Params& P, cudaStream_t st, bool isH) {
   if (!ctx->has_tfsf) return 0;
@@ -1623,11 +1629,12 @@ static long long launch_tfsf(dtmx_ctx* ctx, const Params& P, cudaStream_t st, bo
     else launch(ctx, ctx->early, tfsf_plane_kernel<2>, grd, 256, 0, st, P, T, l, ctx->d_step, isH);
     return 1;
   }
-  long long mx = 1;
-  for (int r = 0; r < T.njob[hs]; r++) mx = std::max(mx, T.job[hs][r].cells);
-  const dim3 grd((unsigned)((mx * 8 + 255) / 256), std::max(1, T.njob[hs]));
-  if (o4) launch(ctx, ctx->early, tfsf_kernel<4>, grd, 256, 0, st, P, T, ctx->d_step, isH);
-  else launch(ctx, ctx->early, tfsf_kernel<2>, grd, 256, 0, st, P, T, ctx->d_step, isH);
+  long long mx = 1, all = 0;
+  for (int r = 0; r < T.njob[hs]; r++) { mx = std::max(mx, T.job[hs][r].cells); all += T.job[hs][r].cells; }
+  const bool taps = all <= (o4 ? kTapNodes4 : kTapNodes2);
+  const dim3 grd((unsigned)((mx * (taps ? 8 : 1) + 255) / 256), std::max(1, T.njob[hs]));
+  auto k = o4 ? (taps ? tfsf_kernel<4, 8> : tfsf_kernel<4, 1>) : (taps ? tfsf_kernel<2, 8> : tfsf_kernel<2, 1>);
+  launch(ctx, ctx->early, k, grd, 256, 0, st, P, T, ctx->d_step, isH);
   return 1;
 }
 // grid of the passes over the ADE box (ade_cell)

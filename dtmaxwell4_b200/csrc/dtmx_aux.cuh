@@ -113,15 +113,22 @@ __device__ __forceinline__ bool in_job(const TfsfJob& jb, int i, int j, int k) {
   return i >= jb.lo[0] && i <= jb.hi[0] && j >= jb.lo[1] && j <= jb.hi[1] && k >= jb.lo[2] && k <= jb.hi[2];
 }
 
-// Eight threads per node of a job (blockIdx.y), one for each tap of both curl
-// terms: the incident field of a tap is a chain of FP64 sines, and one thread
-// that walked a node's taps took 10 us a half step for any box (the jobs are far
-// too small to fill the chip).  A node that also lies in an earlier job of the
-// same component is left to that job, so every node is corrected exactly once
-// with the sum of all its crossing taps.
-template <int ORDER>
+// TPN threads per node of a job (blockIdx.y), by the number of nodes (kTapNodes2,
+// kTapNodes4).  Eight, one for each tap of both curl terms: the incident field of
+// a tap is a chain of FP64 sines, and on boxes too small to fill the chip its
+// latency is all there is (one thread that walks a node's taps takes 5 to 10 us a
+// half step for any small box, eight 3 to 5).  One: a node has one or two crossing
+// taps, so of eight threads most wait for the others, and where there are
+// enough nodes the work of the warps counts: order 4 on 200^3 with a box of 160
+// took 366 us a step for the corrections with eight throughout, 122 now.  The sum
+// over the taps is the same tree in both, bit for bit.
+// A node that also lies in an earlier job of the same component is left to that
+// job, so every node is corrected exactly once with the sum of all its
+// crossing taps.
+template <int ORDER, int TPN>
 __global__ void __launch_bounds__(256) tfsf_kernel(const __grid_constant__ Params p, const __grid_constant__ TfsfDev t, const long long* d_step,
                                                    int isH) {
+  static_assert(TPN == 1 || TPN == 8, "a node a thread or a tap a thread");
   pdl_wait();
   pdl_trigger();
   const long long n = *d_step;
@@ -131,18 +138,45 @@ __global__ void __launch_bounds__(256) tfsf_kernel(const __grid_constant__ Param
   if (r >= t.njob[hs]) return;
   const TfsfJob& jb = t.job[hs][r];
   // a job is a thin shell (cells < 2^31, checked when the jobs are built): 32-bit indexing
-  const long long cell8 = (long long)blockIdx.x * 256 + threadIdx.x;
-  const int cell = (int)min(cell8 >> 3, jb.cells - 1);          // (threads past the end help the last node and store nothing)
+  const long long th = (long long)blockIdx.x * 256 + threadIdx.x;
+  // (the grid is as wide as the largest job: warps past the end of this one have no node, and in its
+  // last warp the threads past it help the last node and store nothing)
+  if ((th & ~31LL) / TPN >= jb.cells) return;
+  const int cell = (int)min(th / TPN, jb.cells - 1);
   const int ey = jb.hi[1] - jb.lo[1] + 1, ez = jb.hi[2] - jb.lo[2] + 1;
   const int i = jb.lo[0] + cell / (ey * ez);
   const int rest = cell - (i - jb.lo[0]) * (ey * ez);
   const int j = jb.lo[1] + rest / ez;
   const int k = jb.lo[2] + (rest - (j - jb.lo[1]) * ez);
   const int c = jb.c;
-  double total = tfsf_tap<ORDER>(p, t, c, i, j, k, isH, isH ? (double)n : (double)n + 0.5, (threadIdx.x >> 2) & 1, threadIdx.x & 3);
+  const double tt = isH ? (double)n : (double)n + 0.5;
+  double total;
+  if (TPN == 8) {
+    total = tfsf_tap<ORDER>(p, t, c, i, j, k, isH, tt, (threadIdx.x >> 2) & 1, threadIdx.x & 3);
 #pragma unroll
-  for (int s = 1; s < 8; s <<= 1) total += __shfl_xor_sync(0xffffffffu, total, s);
-  if ((threadIdx.x & 7) != 0 || (cell8 >> 3) >= jb.cells || total == 0.0 || !is_live(p.g, c, i, j, k)) return;
+    for (int s = 1; s < 8; s <<= 1) total += __shfl_xor_sync(0xffffffffu, total, s);
+  } else {
+    total = 0.0;
+#pragma unroll 1
+    for (int term = 0; term < 2; term++) {
+      int ax[2], gs[2];
+      curl_terms(c, ax[0], gs[0], ax[1], gs[1]);
+      const int a = term ? ax[1] : ax[0], g = term ? gs[1] : gs[0], b1 = (a + 1) % 3, b2 = (a + 2) % 3;
+      auto at = [&](int b) { return b == 0 ? i : b == 1 ? j : k; };
+      // a tap crosses only where the node lies inside the box' range on the other two axes and near a face along a
+      const int B1 = 2 * at(b1) + comp_off(g, b1), B2 = 2 * at(b2) + comp_off(g, b2), S = 2 * at(a) + comp_off(c, a);
+      if (B1 < t.lo[b1] || B1 > t.hi[b1] || B2 < t.lo[b2] || B2 > t.hi[b2]) continue;
+      if ((S < t.lo[a] - 4 || S > t.lo[a] + 3) && (S < t.hi[a] - 3 || S > t.hi[a] + 4)) continue;
+      double low = 0.0, high = 0.0;                              // taps 0 + 1 and 2 + 3
+#pragma unroll 1
+      for (int q = ORDER == 2 ? 1 : 0; q < (ORDER == 2 ? 3 : 4); q++) {
+        const double v = tfsf_tap<ORDER>(p, t, c, i, j, k, isH, tt, term, q);
+        if (q < 2) low += v; else high += v;
+      }
+      total += low + high;
+    }
+  }
+  if (th % TPN != 0 || th / TPN >= jb.cells || total == 0.0 || !is_live(p.g, c, i, j, k)) return;
   for (int q = 0; q < r; q++)
     if (t.job[hs][q].c == c && in_job(t.job[hs][q], i, j, k)) return;
   const long long id = (long long)i * p.g.sx + (long long)j * p.g.sy + k;
