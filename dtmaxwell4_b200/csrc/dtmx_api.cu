@@ -1541,6 +1541,19 @@ static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, 
   return DTMX_OK;
 }
 static int plan_stream(dtmx_ctx* ctx, const WorkPlan** w) { return plan_work(ctx, WK_STREAM, TYT, ctx->cfg.order == 4 ? 3 : 4, ctx->xchunk, w); }
+// Stages of the order-4 kernels' rings (h_kernel): 4 for launches of more than four waves
+// of their CTAs and for walks of 8 planes and more, 3 otherwise.  In us a step, 3 and 4
+// stages: 1024 CTAs of 4 planes (128^3) 39.4 and 41.5, 700 (100^3) 28.8 and 30.1; 2800 (192x160x224) 121.8
+// and 115.8; 16 planes at 128^3 37.5 and 37.2, on 192x160x224 115.8 and 95.8.  Not with a
+// design region nor where most cells lie in an absorber's slabs: their loads go
+// through the L1 cache that the fourth stage takes (200^3 with a design region
+// 220 and 227, 600x600x12 with slabs of 4 278 and 286).
+static int stream_stages(const dtmx_ctx* ctx, const WorkPlan& w) {
+  double inside = 1.0;
+  for (int a = 0; a < 3; a++) inside *= 1.0 - (double)(ctx->P.ab.L[a][0] + ctx->P.ab.L[a][1]) / ctx->P.g.n[a];
+  if (ctx->P.des_on || (ctx->P.ab.kind != 0 && inside < 0.5)) return 3;
+  return (long long)w.grid.x * w.grid.y * w.grid.z > 4 * 148 * 3 || w.xchunk >= 8 ? 4 : 3;
+}
 static int plan_sweep(dtmx_ctx* ctx, const WorkPlan** w) {
   return plan_work(ctx, WK_SWEEP, ctx->frows, ctx->frows == 16 ? 3 : 5, std::min(ctx->xchunk, FX_MAX), w);
 }
@@ -1549,12 +1562,14 @@ static int set_kernel_attributes() {
   static bool done = false;
   if (done) return 0;
   auto allow = [](const void* k, size_t smem) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); };
-  allow((const void*)h_kernel<2, false>, Pipe<2, true>::SMEM_BYTES);
-  allow((const void*)h_kernel<2, true>, Pipe<2, true>::SMEM_BYTES);
-  allow((const void*)h_kernel<4, false>, Pipe<4, true>::SMEM_BYTES);
-  allow((const void*)e_kernel<2, false>, Pipe<2, false>::SMEM_BYTES);
-  allow((const void*)e_kernel<2, true>, Pipe<2, false>::SMEM_BYTES);
-  allow((const void*)e_kernel<4, false>, Pipe<4, false>::SMEM_BYTES);
+  allow((const void*)h_kernel<2, false, 3>, Pipe<2, true>::SMEM_BYTES);
+  allow((const void*)h_kernel<2, true, 3>, Pipe<2, true>::SMEM_BYTES);
+  allow((const void*)h_kernel<4, false, 3>, Pipe<4, true>::SMEM_BYTES);
+  allow((const void*)h_kernel<4, false, 4>, Pipe<4, true, 4>::SMEM_BYTES);
+  allow((const void*)e_kernel<2, false, 3>, Pipe<2, false>::SMEM_BYTES);
+  allow((const void*)e_kernel<2, true, 3>, Pipe<2, false>::SMEM_BYTES);
+  allow((const void*)e_kernel<4, false, 3>, Pipe<4, false>::SMEM_BYTES);
+  allow((const void*)e_kernel<4, false, 4>, Pipe<4, false, 4>::SMEM_BYTES);
   done = true;
   return 0;
 }
@@ -1652,13 +1667,14 @@ static int launch_step(dtmx_ctx* ctx) {
   P.xchunk = plan.xchunk;
   const int blk = STREAM_NT;
   const dim3 grd = plan.grid;
-  const bool o4 = c.order == 4;
+  const bool o4 = c.order == 4, deep = o4 && stream_stages(ctx, plan) == 4;
   cudaStream_t st = ctx->stream;
   long long nl = 0;
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], st);
-  if (o4) launch(ctx, ctx->early, h_kernel<4, false>, grd, blk, Pipe<4, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
-  else if (plan.table) launch(ctx, ctx->early, h_kernel<2, true>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, plan.work);
-  else launch(ctx, ctx->early, h_kernel<2, false>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  if (o4 && deep) launch(ctx, ctx->early, h_kernel<4, false, 4>, grd, blk, Pipe<4, true, 4>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  else if (o4) launch(ctx, ctx->early, h_kernel<4, false, 3>, grd, blk, Pipe<4, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  else if (plan.table) launch(ctx, ctx->early, h_kernel<2, true, 3>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, plan.work);
+  else launch(ctx, ctx->early, h_kernel<2, false, 3>, grd, blk, Pipe<2, true>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
   if (ctx->profiling) cudaEventRecord(ctx->ev[1], st);
   nl++;
   nl += launch_tfsf(ctx, P, st, true);
@@ -1669,9 +1685,10 @@ static int launch_step(dtmx_ctx* ctx) {
     nl++;
   }
   if (ctx->profiling) cudaEventRecord(ctx->ev[2], st);
-  if (o4) launch(ctx, ctx->early, e_kernel<4, false>, grd, blk, Pipe<4, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
-  else if (plan.table) launch(ctx, ctx->early, e_kernel<2, true>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, plan.work);
-  else launch(ctx, ctx->early, e_kernel<2, false>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  if (o4 && deep) launch(ctx, ctx->early, e_kernel<4, false, 4>, grd, blk, Pipe<4, false, 4>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  else if (o4) launch(ctx, ctx->early, e_kernel<4, false, 3>, grd, blk, Pipe<4, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
+  else if (plan.table) launch(ctx, ctx->early, e_kernel<2, true, 3>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, plan.work);
+  else launch(ctx, ctx->early, e_kernel<2, false, 3>, grd, blk, Pipe<2, false>::SMEM_BYTES, st, P, ctx->maps, Work<false>{});
   if (P.ade.Em[0] || ctx->has_gyro) {
     // dispersive and gyrotropic nodes of the E half step (e_kernel skipped them)
     const bool box = c.geometry == DTMX_GEOM_BOX;

@@ -5,7 +5,7 @@
 // source-field tiles (with y/z halo), the own values of the three updated
 // components and, for the E step on mixed planes, their material indices.  One
 // elected thread fetches all of them with cp.async.bulk.tensor (TMA, no
-// multicast) into a ring of NST shared-memory stages, LEAD planes ahead of
+// multicast) into a ring of NST shared-memory stages, ahead of
 // the ones the update reads; completion is tracked per stage by an mbarrier
 // with a transaction count.  Out-of-array boxes are zero-filled by the TMA
 // unit, which is exactly the zero-outside boundary.  Tiles at a mirror boundary
@@ -69,7 +69,7 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
-template <int ORDER, bool ISH>
+template <int ORDER, bool ISH, int NST_ = 3>
 struct Pipe {
   static constexpr int R = ORDER / 2;
   static constexpr int YL = ISH ? R : R - 1, YH = ISH ? R - 1 : R;      // halo rows of the y taps
@@ -93,7 +93,7 @@ struct Pipe {
   static constexpr int DIR = ISH ? 1 : -1;             // direction of the walk along x
   static constexpr int AHEAD = ORDER == 4 ? 1 : 0;
   static constexpr int BEHIND = ORDER == 4 ? 2 : 1;
-  static constexpr int NST = 3;
+  static constexpr int NST = NST_;
   static constexpr int BASE = ISH ? 2 : 1;             // queue slot of x offset 0 (dstencil taps v0..v3)
   static constexpr size_t SMEM_BYTES = (size_t)NST * STAGE * 4 + MAXMAT * 3 * 4 + NST * 8 + 128;
 };
@@ -215,9 +215,9 @@ __device__ __forceinline__ void absorb4(int kind, const Q4& d, const float (&c0)
   put4(mem, vec && lm == 15u, m & lm, nv);
 }
 
-template <int ORDER, bool ISH, bool TAB>
+template <int ORDER, bool ISH, bool TAB, int NST_>
 __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, const Work<TAB>& work, float* dsm) {
-  using P = Pipe<ORDER, ISH>;
+  using P = Pipe<ORDER, ISH, NST_>;
   constexpr int NST = P::NST, AHEAD = P::AHEAD, BEHIND = P::BEHIND, BASE = P::BASE, DIR = P::DIR;
   constexpr int c0 = ISH ? 0 : 3, cf = ISH ? 3 : 0;          // source and updated components
   constexpr int O = ISH ? 0 : 1;                             // half-coordinate offset of the updated nodes along their derivative axes
@@ -495,19 +495,25 @@ __device__ __forceinline__ void stream_body(const Params& p, const TmaMaps& m, c
   }
 }
 
-// 4 CTAs per SM: what shared memory allows for the 3-stage rings
-template <int ORDER, bool TAB>
+// CTAs per SM: 4 at order 2, what shared memory allows for 3 stages; 3 at order 4, whose
+// registers (146) allow no more, with 3 or 4 stages.  Order 4 holds two of its
+// stages resident, so a ring of 3 has one plane in flight: large launches are
+// then bound by the copies' latency (640x640x384 without absorber 2318 us a step,
+// with 4 stages 1886; 256^3 265 and 223; with a 10-cell CPML 384^3 966 and 859).
+// The fourth stage costs a little where a short walk starts from cached fields
+// (128^3 39.4 and 41.5 us; stream_stages).
+template <int ORDER, bool TAB, int NST>
 __global__ void __launch_bounds__(STREAM_NT, ORDER == 2 ? 4 : 3)
     h_kernel(const __grid_constant__ Params p, const __grid_constant__ TmaMaps m, const __grid_constant__ Work<TAB> work) {
   extern __shared__ __align__(128) float dsm[];
-  stream_body<ORDER, true, TAB>(p, m, work, dsm);
+  stream_body<ORDER, true, TAB, NST>(p, m, work, dsm);
 }
 
-template <int ORDER, bool TAB>
+template <int ORDER, bool TAB, int NST>
 __global__ void __launch_bounds__(STREAM_NT, ORDER == 2 ? 4 : 3)
     e_kernel(const __grid_constant__ Params p, const __grid_constant__ TmaMaps m, const __grid_constant__ Work<TAB> work) {
   extern __shared__ __align__(128) float dsm[];
-  stream_body<ORDER, false, TAB>(p, m, work, dsm);
+  stream_body<ORDER, false, TAB, NST>(p, m, work, dsm);
 }
 
 }  // namespace dtmx
