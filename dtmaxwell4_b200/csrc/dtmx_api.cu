@@ -109,7 +109,7 @@ struct dtmx_ctx {
   // sources
   std::vector<PointSrcDev> psrc;
   PointSrcDev* d_psrc = nullptr;   // the sources sorted by node (prepare)
-  int2* d_psrc_run = nullptr;      // {first, count} of each node's
+  int2* d_psrc_run = nullptr;      // {first, count} of each node's (more sources than the tail's list holds)
   int nrun = 0;
   int has_tfsf = 0;
   dtmx_tfsf tfsf{};
@@ -1727,10 +1727,13 @@ static int prepare(dtmx_ctx* ctx) {
       if (q > 0 && sorted[q].comp == sorted[q - 1].comp && sorted[q].id == sorted[q - 1].id) runs.back().y++;
       else runs.push_back(make_int2(q, 1));
     }
-    if ((rc = dalloc(ctx, &ctx->d_psrc, sorted.size(), true)) || (rc = dalloc(ctx, &ctx->d_psrc_run, runs.size(), true))) return rc;
+    if ((rc = dalloc(ctx, &ctx->d_psrc, sorted.size(), true))) return rc;
     CK(cudaMemcpyAsync(ctx->d_psrc, sorted.data(), sorted.size() * sizeof(PointSrcDev), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_psrc_run, runs.data(), runs.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
-    ctx->nrun = (int)runs.size();
+    if (sorted.size() > TAIL_SRC) {
+      if ((rc = dalloc(ctx, &ctx->d_psrc_run, runs.size(), true))) return rc;
+      CK(cudaMemcpyAsync(ctx->d_psrc_run, runs.data(), runs.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
+      ctx->nrun = (int)runs.size();
+    }
   }
   if (!ctx->probes.empty()) {
     if ((rc = dalloc(ctx, &ctx->d_probes, ctx->probes.size(), true))) return rc;
@@ -1903,14 +1906,22 @@ static int fused_prepare(dtmx_ctx* ctx) {
     cudaFuncSetAttribute(fused_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FL<8>::SMEM);
     attr = true;
   }
-  const dtmx_config& c = ctx->cfg;
-  int rc = DTMX_OK;
-  for (int comp = 0; comp < 6 && !rc; comp++) rc = dalloc(ctx, &ctx->f_alt[comp], ctx->nstore + 64);
-  for (int a = 0; a < 3 && !rc; a++) {
-    const size_t th = (size_t)(ctx->P.ab.L[a][0] + ctx->P.ab.L[a][1]);
-    if (!ctx->P.ab.aux[a][2] || !th) continue;
-    const size_t cnt = th * (ctx->ncell / (size_t)(a == 0 ? c.nx : a == 1 ? c.ny : c.nz));
-    for (int q = 0; q < 2 && !rc; q++) rc = dalloc(ctx, &ctx->hax_alt[a][q], cnt);
+  // one allocation, cut up (twelve of them cost the first step of a 128^3 grid 3.6 ms), but for parkable contexts,
+  // whose arrays are parked one by one; the first array's address is the block's (fused_release)
+  float** arr[12];
+  size_t len[12], total = 0;
+  int na = 0, rc = DTMX_OK;
+  auto want = [&](float** q, size_t n) { arr[na] = q; len[na++] = n; total += (n + 63) / 64 * 64; };
+  for (int comp = 0; comp < 6; comp++) want(&ctx->f_alt[comp], ctx->nstore + 64);
+  for (int a = 0; a < 3; a++)
+    for (int q = 0; q < 2; q++)
+      if (ctx->P.ab.aux[a][2]) want(&ctx->hax_alt[a][q], (size_t)(ctx->P.ab.L[a][0] + ctx->P.ab.L[a][1]) * (ctx->ncell / (size_t)ctx->P.g.n[a]));
+  if (ctx->cfg.parkable) {
+    for (int q = 0; q < na && !rc; q++) rc = dalloc(ctx, arr[q], len[q]);
+  } else {
+    float* block = nullptr;
+    rc = dalloc(ctx, &block, total);
+    for (int q = 0; q < na && !rc; q++) { *arr[q] = block; block += (len[q] + 63) / 64 * 64; }
   }
   // maps of the per-step kernels over the second set, so either engine runs from either buffer
   if (!rc) {
@@ -1945,7 +1956,8 @@ static double fused_set_bytes(const dtmx_ctx* ctx) {
   return 4.0 * n;
 }
 
-// Give a half-made second set back (plain allocations: the automatic choice leaves parkable contexts alone).
+// Give the second set back, half-made or whole (plain allocations: the automatic choice leaves parkable
+// contexts alone): the block, or after an odd number of swaps the arrays allocated first; pointers into a block free nothing.
 static void fused_release(dtmx_ctx* ctx) {
   if (ctx->fused_ready) return;
   cudaStreamSynchronize(ctx->stream);
