@@ -202,13 +202,18 @@ constexpr long long kWaitPolls = 1LL << 26;
 // 1 MB, lets the next piece come in while it moves the last one to the caller's
 // buffer, and takes piece after piece until none is left.  The slots (8 MB)
 // belong to the process, are used by one read at a time (another one meanwhile
-// takes the driver's path) and are freed with the last context.
+// takes the driver's path) and are freed with the last context.  Pinning them
+// takes 3 to 10 ms, as much as they save on 32 MB of fresh pages (8.4 MB 2.2 ms by
+// the driver's copy, 1.05 through the slots) and more than they save where the
+// caller's pages have been touched (0.45 and 0.4 to 0.6), so they are made by a read of 32
+// MB, or by the one that brings the bytes read without them to 64 MB.
 struct ReadSlots {
   std::mutex use, life;
   char* buf = nullptr;
+  size_t plain = 0;             // bytes of large reads that took the driver's path for want of slots
   int contexts = 0;
 };
-constexpr size_t kReadPiece = 1 << 20, kReadMin = 4 << 20;
+constexpr size_t kReadPiece = 1 << 20, kReadMin = 4 << 20, kReadWorth = 32 << 20;
 constexpr int kReadThreads = 4;
 static ReadSlots& read_slots() {
   static ReadSlots s;
@@ -226,6 +231,7 @@ static void read_slots_drop() {
   std::lock_guard<std::mutex> us(S.use);
   if (S.buf) cudaFreeHost(S.buf);
   S.buf = nullptr;
+  S.plain = 0;
 }
 
 // the calling thread's device while it uses another one
@@ -251,11 +257,13 @@ static cudaError_t copy_to_host(int dev, cudaStream_t st, void* host, const void
   }
   std::unique_lock<std::mutex> lk(S.use, std::defer_lock);
   if (!direct && !lk.try_lock()) direct = true;
+  if (!direct && !S.buf && bytes < kReadWorth && (S.plain += bytes) < 2 * kReadWorth) direct = true;
   if (!direct && !S.buf && cudaHostAlloc((void**)&S.buf, kReadPiece * 2 * kReadThreads, cudaHostAllocPortable) != cudaSuccess) {
     cudaGetLastError();
     S.buf = nullptr;
     direct = true;
   }
+  if (direct && lk.owns_lock()) lk.unlock();
   cudaError_t e = cudaSuccess;
   if (!direct) {
     const size_t pieces = (bytes + kReadPiece - 1) / kReadPiece;

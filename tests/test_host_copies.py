@@ -9,6 +9,19 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(scope="module", autouse=True)
+def slots():
+    """The threaded read's pinned slots: made by a read of 32 MB, kept while a context
+    lives."""
+    from dtmaxwell4_b200 import Simulation, abi
+    s = Simulation(abi.make_config(512, 128, 128, absorber=abi.ABS_NONE, pml=0))
+    a = np.random.default_rng(1).standard_normal(s.shape).astype(np.float32)
+    s.set_field(0, a)
+    assert np.array_equal(s.get_field(0), a)      # 33.6 MB
+    yield
+    s.close()
+
+
 @pytest.mark.parametrize("n", [(9, 8, 11), (64, 161, 103), (40, 64, 512), (1100, 33, 31)])
 def test_field_roundtrip(n):
     import torch
@@ -117,3 +130,4 @@ def test_cost_of_setting_a_small_field():
         best = min(best, time.perf_counter() - t)
     assert best <= 250e-6, best
     s.close()
+

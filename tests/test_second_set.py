@@ -204,7 +204,7 @@ def test_a_batch_with_refused_allocations(budget):
 
 def test_cost_of_the_first_steps():
     """The first 16 steps of a 128^3 grid with the set-up of the automatic engine in them:
-    well below 3 ms (5 with an allocation for each of the set's twelve arrays; the 16
+    well below 4 ms (5 with an allocation for each of the set's twelve arrays; the 16
     steps take 0.6)."""
     import time
     from dtmaxwell4_b200 import Simulation, abi
@@ -217,4 +217,4 @@ def test_cost_of_the_first_steps():
         s.sync()
         best = min(best, time.perf_counter() - t)
         s.close()
-    assert best <= 3e-3, best
+    assert best <= 4e-3, best
