@@ -78,7 +78,7 @@ struct VmmBlock {
 // the pieces of a streaming launch (plan_work)
 struct WorkPlan {
   bool table = false, alone = false;   // alone: to be launched when the kernel ahead has finished
-  int xchunk = 0;
+  int xchunk = 0, longest = 0;         // planes of equal pieces; of the longest piece
   dim3 grid;
   Work<true> work{};
 };
@@ -1501,6 +1501,7 @@ static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, 
   auto it = ctx->work.find(key);
   if (it == ctx->work.end()) {
     WorkPlan w;
+    std::vector<int4> v;
     bool keep = true;
     w.xchunk = planes;
     if (planes == 0) {
@@ -1514,7 +1515,6 @@ static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, 
           if (n <= fit) break;
         }
       }
-      std::vector<int4> v;
       int4* d = nullptr;
       if (budget <= kOneWave) {
         // no table while the caller captures the stream, nor without memory for one: equal pieces serve
@@ -1538,6 +1538,9 @@ static int plan_work(dtmx_ctx* ctx, int kind, int rows, int per_sm, int planes, 
       }
     }
     if (!w.table) w.grid = dim3(ntz, nty, (c.nx + w.xchunk - 1) / w.xchunk);
+    w.longest = std::min(w.xchunk, c.nx);
+    for (const int4& e : v)
+      if (w.table) w.longest = std::max(w.longest, e.w - e.z);
     if (!keep) {
       ctx->work_once = w;
       if (plan) *plan = &ctx->work_once;
@@ -3372,6 +3375,19 @@ extern "C" int dtmx_set_xchunk(dtmx_ctx* ctx, int planes) {
   const Running running(ctx);
   ctx->xchunk = planes;
   drop_graphs(ctx);
+  return DTMX_OK;
+}
+
+extern "C" int dtmx_work_pieces(dtmx_ctx* ctx, int kernel, int* equal_cost, int* pieces, int* longest) {
+  if (ctx && ctx->parked) return fail(ctx, DTMX_ERR_STATE, "the context is parked (dtmx_unpark first)");
+  if (!ctx || kernel < 0 || kernel > 2) return fail(ctx, DTMX_ERR_INVALID, "bad kernel");
+  const Running running(ctx);
+  const WorkPlan* w;
+  const int rc = kernel == 0 ? plan_stream(ctx, &w) : kernel == 1 ? plan_sweep(ctx, &w) : plan_work(ctx, WK_ADJ, 16, 3, 0, &w);
+  if (rc) return rc;
+  if (equal_cost) *equal_cost = w->table ? 1 : 0;
+  if (pieces) *pieces = (int)(w->grid.x * w->grid.y * w->grid.z);
+  if (longest) *longest = w->longest;
   return DTMX_OK;
 }
 

@@ -26,7 +26,7 @@ EXPORTS = (
     "dtmx_set_design", "dtmx_forward_adjoint", "dtmx_batch_forward_adjoint", "dtmx_autotune",
     "dtmx_write_arr", "dtmx_save_state", "dtmx_load_state",
     "dtmx_add_dft_patch", "dtmx_add_flux_box", "dtmx_read_flux", "dtmx_flux_faces",
-    "dtmx_set_adjoint_memory", "dtmx_ntff", "dtmx_set_wait_limit", "dtmx_fail_next",
+    "dtmx_set_adjoint_memory", "dtmx_ntff", "dtmx_set_wait_limit", "dtmx_fail_next", "dtmx_work_pieces",
 )
 
 
@@ -100,6 +100,7 @@ def load():
                                              C.POINTER(C.c_double), C.POINTER(vp)]
     L.dtmx_count_nonfinite_noalloc.argtypes = [C.POINTER(C.c_void_p), C.c_int, C.c_int64, C.POINTER(C.c_int64)]
     L.dtmx_set_wait_limit.argtypes = [vp, C.c_int64]
+    L.dtmx_work_pieces.argtypes = [vp, ip, C.POINTER(ip), C.POINTER(ip), C.POINTER(ip)]
     L.dtmx_fail_next.argtypes = [vp, ip, ip]
     _lib = L
     return L
@@ -294,6 +295,13 @@ class Simulation:
         v = [C.c_int() for _ in range(4)]
         self._ck(self._L.dtmx_get_engine(self._h, *[C.byref(x) for x in v]))
         return tuple(x.value for x in v)
+
+    def work_pieces(self, kernel):
+        """(equal cost, pieces, planes of the longest) of a launch of the per-step
+        kernels (0), the single sweep (1) or the single-sweep adjoint (2)."""
+        v = [C.c_int() for _ in range(3)]
+        self._ck(self._L.dtmx_work_pieces(self._h, int(kernel), *[C.byref(x) for x in v]))
+        return bool(v[0].value), v[1].value, v[2].value
 
     # ---- differentiation
     def set_design(self, lo, eps):

@@ -520,6 +520,12 @@ int  dtmx_set_tile_rows(dtmx_ctx* ctx, int rows);
  * dtmx_autotune); any pointer may be NULL.  No reference counterpart. */
 int  dtmx_get_engine(dtmx_ctx* ctx, int* engine, int* time_block, int* xchunk, int* tile_rows);
 
+/* How a launch is cut along x: kernel 0 the per-step kernels, 1 the single
+ * sweep, 2 the single-sweep adjoint; whether the pieces are of equal cost (a table)
+ * or of equal length, their number and the planes of the longest.  Any pointer
+ * may be NULL.  No reference counterpart. */
+int  dtmx_work_pieces(dtmx_ctx* ctx, int kernel, int* equal_cost, int* pieces, int* longest);
+
 /* Time every applicable engine configuration for trial_steps steps from the
  * current state (probes and DFT planes paused; the state is restored after
  * each trial) and keep the fastest: the per-step engine with x chunks of 4 to 64

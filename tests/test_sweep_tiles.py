@@ -50,22 +50,25 @@ def test_tile_edges_equal_the_per_step_engine(n, pml, rows):
         assert np.array_equal(got[c], want[c]), (c, np.abs(got[c] - want[c]).max())
 
 
-@pytest.mark.parametrize("n,pml", [
-    ((70, 40, 40), ((6, 6), (6, 6), (6, 6))),        # one wave, pieces of one plane
-    ((61, 170, 150), ((6, 6), (6, 6), (6, 6))),      # one wave, pieces of equal cost
-    ((44, 300, 290), ((6, 5), (0, 7), (8, 8))),      # one wave of long pieces
-    ((20, 520, 530), ((6, 5), (0, 7), (8, 8))),      # several waves
-    ((150, 17, 20), None),                           # pieces as long as a CTA's tables allow (64 planes)
+# cuts: by kernel (0 per-step, 1 single sweep), equal cost or not and the planes of the longest piece
+@pytest.mark.parametrize("n,pml,cuts", [
+    ((70, 40, 40), ((6, 6), (6, 6), (6, 6)), ((False, 1), (False, 1))),       # one wave, pieces of one plane
+    ((61, 170, 150), ((6, 6), (6, 6), (6, 6)), ((True, 12), (True, 15))),     # one wave, pieces of equal cost
+    ((30, 300, 290), ((6, 5), (0, 7), (8, 8)), ((True, 15), (True, 27))),     # one wave of long pieces
+    ((44, 300, 290), ((6, 5), (0, 7), (8, 8)), ((True, 22), (False, 6))),     # one wave / several
+    ((20, 520, 530), ((6, 5), (0, 7), (8, 8)), ((False, 4), (False, 6))),     # several waves
+    ((150, 17, 20), None, ((False, 1), (False, 1))),
 ])
-def test_pieces_of_equal_cost(n, pml):
+def test_pieces_of_equal_cost(n, pml, cuts):
     """The tile columns cut into pieces of equal cost (automatic) against equal
-    pieces of 7 planes, on both streaming engines."""
+    pieces of 7 planes and of as many as a CTA's tables hold (64 planes, in the
+    single sweep), on both streaming engines."""
     from dtmaxwell4_b200 import Simulation, abi
     cfg = abi.make_config(*n, courant=0.5, absorber=abi.ABS_CPML if pml else abi.ABS_NONE, pml=pml or 0)
     rng = np.random.default_rng(3)
     fields = [rng.standard_normal(n).astype(np.float32) for _ in range(6)]
     got = []
-    for engine, planes in ((1, 7), (1, 0), (3, 7), (3, 0)):
+    for engine, planes in ((1, 7), (1, 0), (3, 7), (3, 0), (1, 200), (3, 200)):
         s = Simulation(cfg)
         for c in range(6):
             s.set_field(c, fields[c])
@@ -73,6 +76,12 @@ def test_pieces_of_equal_cost(n, pml):
         s.set_xchunk(planes)
         s.step(5)
         got.append([s.get_field(c) for c in range(6)])
+        kernel = 0 if engine == 1 else 1
+        equal, _, longest = s.work_pieces(kernel)
+        if planes == 0:
+            assert (equal, longest) == cuts[kernel]
+        else:
+            assert (equal, longest) == (False, min(planes, n[0], 64 if engine == 3 else 200))
         s.close()
     for out in got[1:]:
         for c in range(6):
