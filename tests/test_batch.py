@@ -35,3 +35,27 @@ def test_batch_equals_separate_runs(budget):
             assert np.array_equal(s.get_field(c), sims[b].get_field(c))
         s.close()
         sims[b].close()
+
+
+def test_cost_of_a_first_batch():
+    """The first batch on new contexts takes at most three of a later one (four to five
+    where the pool passed blocks between streams in flight)."""
+    import time
+    from dtmaxwell4_b200 import Simulation, abi, engine
+    n, best = (64, 64, 64), 1e9
+    for _ in range(4):
+        sims = []
+        for q in range(8):
+            s = Simulation(abi.make_config(*n, courant=0.4, pml=6))
+            s.set_design((32, 32, 32), np.full((3, 6, 6, 6), 2.0, np.float32))
+            s.set_field(2, np.random.default_rng(q).standard_normal(n).astype(np.float32))
+            sims.append(s)
+        t = []
+        for _ in range(3):
+            a = time.perf_counter()
+            engine.batch_forward_adjoint(sims, 30, [54] * 8, [0.4] * 8)
+            t.append(time.perf_counter() - a)
+        best = min(best, t[0] / min(t[1:]))
+        for s in sims:
+            s.close()
+    assert best <= 3.0, best
