@@ -61,13 +61,6 @@ __device__ __forceinline__ Str4 str_same(const float* c) {
   for (int e = 0; e < 4; e++) { r.b[e] = c[0]; r.a[e] = c[1]; r.g[e] = c[2]; }
   return r;
 }
-__device__ __forceinline__ Str4 str_row(const float* c) {
-  Str4 r;
-  const Q4 b = ld4(c), a = ld4(c + 36), g = ld4(c + 72);
-#pragma unroll
-  for (int e = 0; e < 4; e++) { r.b[e] = b.v[e]; r.a[e] = a.v[e]; r.g[e] = g.v[e]; }
-  return r;
-}
 
 // Coefficient tables: x planes x0-1 .. x0+FX_MAX, rows j0-1 .. j0+TY, columns
 // k0-1 .. k0+32 (the columns start at entry 3, so that k0 is 16-byte aligned).

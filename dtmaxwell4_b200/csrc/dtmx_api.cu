@@ -625,10 +625,6 @@ static void setup_grid(dtmx_ctx* ctx) {
       g.all_lo[a] = std::max(g.all_lo[a], g.live_lo[comp][a]);
       g.all_hi[a] = std::min(g.all_hi[a], g.live_hi[comp][a]);
     }
-    // a zero side never needs the boundary mapping: in-array non-live cells
-    // hold zero and out-of-array boxes are zero-filled by the TMA unit
-    g.safe_lo[a] = g.btype[a][0] == 0 ? -(1 << 28) : g.all_lo[a];
-    g.safe_hi[a] = g.btype[a][1] == 0 ? (1 << 28) : g.all_hi[a];
   }
 }
 

@@ -21,17 +21,19 @@
 
 namespace dtmx {
 
-constexpr int TZ = 32;          // tile extent along z (one warp)
+constexpr int TZ = 32;          // tile extent along z: eight threads of four nodes
 constexpr int TYT = 16;          // tile extent along y
 constexpr int MAXMAT = 64;
 constexpr int MAXPOLE = 2;
 
 // Programmatic dependent launch.  A step is a chain of launches on one stream, on
-// small grids of a few microseconds each.  Every kernel of the chain lets the
-// next one start its set-up (pdl_trigger) and itself waits for the one before
-// (pdl_wait) ahead of anything that one may have written; what comes before
-// the wait reads only tables that no step changes.  Each kernel waits in all
-// its threads, so a finished kernel means that all before it have finished.
+// small grids of a few microseconds each.  Every kernel of the chain waits for the
+// one before (pdl_wait) ahead of anything that one may have written; what comes
+// before the wait reads only tables that no step changes.  All but the per-step
+// field kernels and the DFT fold let the next one start its set-up (pdl_trigger);
+// after those it starts when they end.  Each kernel waits in all its threads (the
+// fold is launched without the attribute), so a finished kernel means that all
+// before it have finished.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -43,7 +45,6 @@ struct Grid {
   long long sx, sy;          // element strides of x and y (z stride 1)
   int live_lo[6][3], live_hi[6][3];
   int all_lo[3], all_hi[3];  // index range live for every component
-  int safe_lo[3], safe_hi[3];// index range whose taps need no mirror mapping (zero sides unbounded)
   int btype[3][2], bplane[3][2];
   int bsE[3][2], bsH[3][2];
   int box;                   // box geometry: every node of the array is live, zero outside
@@ -74,7 +75,6 @@ struct Ade {
   float* Jp[3][MAXPOLE];
   float* Jm[3][MAXPOLE];
   float* Jg[2][3];           // gyrotropic current, double-buffered
-  int gnew;                  // buffer holding J^{n+1/2} during the E half step
 };
 
 struct Params {

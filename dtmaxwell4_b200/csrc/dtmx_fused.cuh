@@ -43,7 +43,7 @@
 // a step (algorithmic bytes at 5.4 TB/s), without absorber 508 -> 454 us (6.0
 // TB/s), 128^3 with a 10-cell CPML 57 -> 40 us.
 //
-// The node updates are the expressions of plane_update (dtmx_device.cuh), in
+// The node updates are the expressions of stream_body (dtmx_stream.cuh), in
 // the same order with the same explicitly rounded operations (sums with an
 // exact zero and products with an exact one left out), so without a TF/SF
 // source this engine's fields equal the per-step engine's.  With one, the H
@@ -147,7 +147,7 @@ __device__ __forceinline__ void cpml4(const Q4& d, const float (&b)[4], const fl
   if (store) put4(mem, vec, m, nv);
 }
 
-// CPML corrections of four nodes (the arithmetic of absorb_apply3) from their
+// CPML corrections of four nodes (the arithmetic of absorb4) from their
 // scaled derivative terms dxy etc. (component, axis); inc += sum over the axes.
 template <int TY, bool ISH>
 __device__ __forceinline__ void fused_cpml(const Params& p, const FusedArgs& fa, const FNode& f, int i, int xs, const float* fco, int xrow,

@@ -29,7 +29,7 @@
 // shared-memory stages by TMA; eight (TY/4) consumer warps compute, each
 // thread four consecutive z nodes of one y row (float4 shared-memory reads,
 // float4 global stores).  x taps come from per-level register queues that
-// advance one plane per wave step.  Arithmetic is that of plane_update (same
+// advance one plane per wave step.  Arithmetic is that of stream_body (same
 // expressions in the same order), so the engine is bit-identical to the
 // one-launch-per-half-step engine.
 #pragma once
@@ -105,9 +105,6 @@ __device__ __forceinline__ void st_release(int* q, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;\n" ::"l"(q), "r"(v) : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;\n" ::: "memory"); }
-__device__ __forceinline__ void named_bar(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(nthreads) : "memory");
-}
 __device__ __forceinline__ float4 lds4(const float* q) { return *reinterpret_cast<const float4*>(q); }
 __device__ __forceinline__ float f4(const float4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
 
