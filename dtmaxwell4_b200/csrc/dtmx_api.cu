@@ -347,11 +347,12 @@ static bool refuse(dtmx_ctx* ctx, int what) { return ctx->fail_in[what] >= 0 && 
 // A launch; early: it may start its set-up before the kernel ahead of it on the
 // stream has finished (pdl_wait in the kernel).  Captured into graphs like any
 // other.  A context takes early launches up to 2^23 cells (kEarlyCells) and
-// outside a batch: a 48^3 step 11.9 -> 11.1 us, 77x201x55 17.3 -> 15.9, a gradient
-// on 192x160x128 20.1 -> 19.3 ms, order 4 on 6.9 M cells 177 -> 173; on 25 M cells with
-// a gyrotropic layer 402 -> 409 us and on 57 M with TF/SF and dispersive passes
-// 672 -> 700, and the waiting CTAs take room from the other contexts of a batch
-// (23.2 -> 23.7 ms).
+// outside a batch, where the waiting CTAs take room from the other contexts
+// (23.2 -> 23.7 ms).  Measured without and with them, us a step, a Drude sphere with
+// TF/SF at order 2 / a gyrotropic layer / order 4 with TF/SF: 1 M cells 50.9 and 48.6 / 37.2 and
+// 37.4 / 58.7 and 55.9; 8.0 M 163.5 and 162.7 / 174.8 and 177.3 / 223.6 and 222.0; 10.1 M 179.2 and
+// 182.4 / 199.0 and 202.1 / 245.3 and 242.0; 16.8 M 237.7 and 253.9 / 267.7 and 271.5 / 326 and 324; a
+// plain grid gains 1 to 2 % up to 1 M cells and nothing above.
 // A launch that failed is kept in the context until launched() reports it.
 template <class... P, class... A>
 static cudaError_t launch(dtmx_ctx* ctx, bool early, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
@@ -1444,7 +1445,7 @@ extern "C" int dtmx_ntff(dtmx_ctx* ctx, int id, int ndir, const double* theta, c
 //     kernel ahead.  The single sweep's pieces below six planes stay equal: the lookup
 //     ahead of the first copy costs them more than it evens out (96^3: 18.7 -> 20.7 us).
 //     The order-4 per-step kernels stay at equal pieces (64.5 + 54.0 -> 75.1 + 55.3 us in
-//     the reference geometry).
+//     the reference geometry, 180x180x128; not measured on other grids).
 //   * Otherwise several waves of equal pieces: of 6 to 32 planes for the single sweep
 //     (192x160x128: 68 us with 6, 77 with 12; 384^3: 634 us with 32, 641 with 10, 669
 //     with 64), 4 to 10 for the per-step kernels (384^3 712 us with 10, 830 with about 40).
