@@ -164,6 +164,7 @@ struct dtmx_ctx {
   std::mutex run;
   std::atomic<std::thread::id> runner{};   // the thread that holds run
   bool lendable = false;              // registered in lenders()
+  bool set_in_graph = false;          // a graph of the caller's uses the second set: it stays
   double fa_reserved = 0.0;           // bytes that fa_reserve has asked for
   bool spare_others = false;          // an allocation that is not worth another context's set
   bool pinned = false;                // the caller holds the fields' addresses: see step_engine
@@ -1985,7 +1986,7 @@ static void fused_release(dtmx_ctx* ctx) {
 // the context goes on with the per-step engine (the state is always in P.f).
 // Not while the caller captures the stream: nothing may be freed then.
 static bool fused_give_back(dtmx_ctx* ctx) {
-  if (ctx->engine != 0 || !ctx->fused_ready || ctx->cfg.parkable || capturing(ctx)) return false;
+  if (ctx->engine != 0 || !ctx->fused_ready || ctx->cfg.parkable || ctx->set_in_graph || capturing(ctx)) return false;
   cudaStreamSynchronize(ctx->stream);
   drop_graphs(ctx);
   ctx->fused_ready = false;
@@ -2170,9 +2171,12 @@ extern "C" int dtmx_step(dtmx_ctx* ctx, int nsteps) {
   int rc0 = prepare(ctx);
   if (rc0) return rc0;
   int left = nsteps;
-  // steps that the caller captures: with engine 0 in place, one by one
-  const bool captured = ctx->engine == 0 && nsteps > 0 && capturing(ctx);
+  if (int rc = launched(ctx)) return rc;         // (of an earlier call that ended with another error)
+  // steps that the caller captures: with engine 0 in place, one by one; with engine 3 on both sets,
+  // which then stay
+  const bool any = (ctx->engine == 0 || ctx->engine == 3) && nsteps > 0 && capturing(ctx), captured = any && ctx->engine == 0;
   if (captured) pin_fields(ctx);
+  if (any && ctx->engine == 3) ctx->set_in_graph = true;
   if (ctx->pinned) fused_give_back(ctx);
   if (ctx->engine == 2) {
     std::string why;

@@ -140,6 +140,32 @@ def test_given_back_when_it_has_no_use(want, how):
     a.close()
 
 
+def test_a_set_in_the_callers_graph_stays(want):
+    """Two steps of the single sweep, chosen by the caller, in a graph of the caller's: no
+    other engine choice frees the set that replays use."""
+    import torch
+    a = _sim()
+    a.set_engine(3)
+    a.step(2)
+    a.sync()
+    st = torch.cuda.ExternalStream(a.stream_handle())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        a.step(2)
+    with_set = _free()
+    a.set_engine(0)
+    a.set_engine(1)
+    a.step(1)                                    # in place: the state stays where the replays expect it
+    with _left(60 * MB):
+        pass
+    assert _free() <= with_set + 16 * MB
+    with torch.cuda.stream(st):
+        g.replay()
+    _equal([a.get_field(c) for c in range(6)], want[5])
+    del g
+    a.close()
+
+
 def test_a_context_in_use_by_another_thread_keeps_its_state(want):
     """Contexts made while another thread steps: each is made or refused, and the
     fields of the stepped one are what they should be."""
